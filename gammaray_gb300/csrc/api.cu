@@ -339,6 +339,8 @@ gr_status gr_film_create(uint32_t w, uint32_t h, gr_film** out) {
     size_t bytes = static_cast<size_t>(w) * h * sizeof(float4);
     GR_CUDA_TRY(f->pixels.ensure(bytes));
     GR_CUDA_TRY(cudaMemset(f->pixels.ptr, 0, bytes));
+    GR_CUDA_TRY(cudaEventCreateWithFlags(&f->cleared, cudaEventDisableTiming));
+    GR_CUDA_TRY(cudaEventRecord(f->cleared, 0));
     cudaGetDevice(&f->device);
     *out = f.release();
     return GR_OK;
@@ -353,6 +355,7 @@ gr_status gr_film_clear(gr_film* f) {
     if (!f) return fail(GR_ERR_INVALID_ARGUMENT, "null film");
     GR_CUDA_TRY(cudaMemset(f->pixels.ptr, 0, static_cast<size_t>(f->width) * f->height * sizeof(float4)));
     if (f->splat.ptr) GR_CUDA_TRY(cudaMemset(f->splat.ptr, 0, static_cast<size_t>(f->width) * f->height * sizeof(float4)));
+    GR_CUDA_TRY(cudaEventRecord(f->cleared, 0));
     f->passes = 0;
     return GR_OK;
 }
@@ -530,12 +533,13 @@ gr_status gr_render(gr_scene* s, const gr_camera* c, const gr_render_params* p, 
     if (!s || !c || !f) return fail(GR_ERR_INVALID_ARGUMENT, "null argument");
     GR_TRY(check_render_params(p));
     std::lock_guard<std::mutex> g(s->mu);
+    GR_CUDA_TRY(cudaStreamWaitEvent(s->stream, f->cleared, 0));
     float4* splat = nullptr;
     if (p->integrator == GR_INTEGRATOR_BDPT && p->light_tracing) {
         if (!f->splat.ptr) {
             size_t bytes = static_cast<size_t>(f->width) * f->height * sizeof(float4);
             GR_CUDA_TRY(f->splat.ensure(bytes));
-            GR_CUDA_TRY(cudaMemset(f->splat.ptr, 0, bytes));
+            GR_CUDA_TRY(cudaMemsetAsync(f->splat.ptr, 0, bytes, s->stream));
         }
         splat = f->splat.as<float4>();
     }

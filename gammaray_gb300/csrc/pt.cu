@@ -13,7 +13,9 @@
 //            atomic per warp (ballot + popc)
 //   film     after the last bounce, the deterministic tile gather in film.cu
 // Extend and shade run as grid-stride loops over the device-side queue count, so the
-// host never waits for a bounce; it polls the count two bounces behind to stop.
+// host never waits for a bounce; it polls the count two bounces behind to stop.  Once
+// few paths are left (or a render has few from the start), one launch carries them to
+// their end (the path loop).
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
@@ -59,6 +61,31 @@ template <int NT>
 constexpr uint32_t shade_per() {
     return NT == 128 ? SHADE_PER_THREAD : (NT == 384 ? 96u : SHADE_BIG_PER);
 }
+
+// Queues of at most PATH_LOOP_MAX paths are carried to their end by one launch
+// (k_pt_finish) instead of an extension and a shading launch per bounce; a group that
+// starts that small needs no queue at all.  Below it a bounce is bounded by latency: its
+// two launches take about 30 us however few paths are left, and on meshes the slowest ray
+// of each bounce alone takes 90-140 us.  Above it the wavefront's sorted shading and
+// refilled extension win.  Measured, wavefront against path loop (us per render):
+//   Cornell box, depth 8     5 k paths 377 / 181, 66 k 400 / 258, 393 k 545 / 611
+//   50 k triangles, depth 12 8 k paths - / 295, 240 k 1361 / 598, 393 k 955 / 760
+//   102 k triangles, 66 k paths 1256 / 463
+// and as the end of a larger render: 641 x 359 x 9 spp, unbounded depth 2439 -> 1695,
+// 512 x 512 x 4 spp 2080 -> 1480, 1024 x 1024 x 64 spp 28.61 -> 28.40 ms.
+constexpr uint32_t PATH_LOOP_MAX = 1u << 18;
+// Depths the path loop takes: one launch carries a path to its end, so its length has to
+// be bounded, by max_depth or by the roulette (at most 3/4 survive a bounce beyond
+// rr_aggressive_depth).  Other settings keep a launch per bounce.
+constexpr uint32_t PATH_LOOP_DEPTH = 256;
+constexpr uint32_t PATH_LOOP_RR_DEPTH = 64;
+// At 4 blocks per SM it has 128 registers; it uses 112.
+constexpr int PATH_LOOP_BLOCKS = 4;
+// Lanes of a warp that carry paths when there are too few to fill every warp: lanes of a
+// warp wait for each other, but fewer lanes per warp repeat the shading code.  4 / 8 / 16
+// / 32 measured 193 / 181 / 170 / 181 us on 5 k paths of the Cornell box, 280 / 295 / 316
+// / 324 us on 8 k of a mesh.
+constexpr uint32_t PATH_LOOP_MIN_LANES = 8;
 
 struct PTParams {
     DevCamera cam;
@@ -133,6 +160,35 @@ GR_D void push_path(bool alive, uint32_t* count_out, uint32_t slot, V3 o, V3 d, 
     }
 }
 
+// One vertex of PathTracerIntegrator::integrate (render/integrators.rs:42-100) at the hit
+// h = (t, leaf-order primitive or -1, u, v) of the ray (o, d): emission into L, the next
+// throughput in tp and the next ray.  Returns whether the path goes on.
+GR_D bool shade_hit(const DeviceScene& s, const PTParams& p, uint32_t depth, uint64_t key, V3 o, V3 d, float4 h,
+                    V3& tp, V3& L, V3& new_o, V3& new_d) {
+    const int32_t k = __float_as_int(h.y);
+    if (k < 0) {
+        if (s.has_env) L = L + mul(tp, V3{s.env[0], s.env[1], s.env[2]});
+        return false;
+    }
+    const uint32_t base = DIM_CAMERA_WALK + 4 * depth;
+    uint32_t prim;
+    Frame f = hit_frame(s, k, o, d, h.x, h.z, h.w, prim);
+    const DevMaterial& m = s.materials[__ldg(s.prim_material + prim)];
+    MaterialSample ms = sample_world(m, -d, f, true, uniform01(key, base), uniform01(key, base + 1),
+                                     uniform01(key, base + 2));
+    L = L + mul(tp, ms.emission);
+    tp = mul(tp, ms.radiance * (fabsf(dot(f.normal, ms.outgoing)) / ms.pdf));
+    new_o = nudge(o + (d * h.x), ms.outgoing);
+    new_d = ms.outgoing;
+    if (depth > p.rr_depth || nearly_zero(tp)) {
+        float rv = uniform01(key, base + 3);
+        float lum = luminance(tp);
+        float prob = depth > p.rr_aggr ? clamped_lerp(0.10f, 0.75f, lum) : clamped_lerp(0.25f, 1.00f, lum);
+        tp = rv < prob ? tp / prob : v3zero();
+    }
+    return !is_zero(tp) && (p.max_depth == 0 || depth + 1 < p.max_depth);
+}
+
 // Material-sorted shading (shade_sort.cuh): each block sorts its chunk of the queue by
 // code path (chosen lobe type, the material's lobe types), then shades it in that order.
 
@@ -185,29 +241,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_shade(DeviceScene s, PTParams 
                     sb = q_state[2 * static_cast<size_t>(q) + 1];
                 }
                 V3 tp = V3{sa.x, sa.y, sa.z}, L = V3{sa.w, sb.x, sb.y};
-                int32_t k = __float_as_int(h.y);
-                if (k < 0) {
-                    if (s.has_env) L = L + mul(tp, V3{s.env[0], s.env[1], s.env[2]});
-                } else {
-                    uint32_t prim;
-                    Frame f = hit_frame(s, k, o, d, h.x, h.z, h.w, prim);
-                    const DevMaterial& m = s.materials[__ldg(s.prim_material + prim)];
-                    uint64_t key = state_key(sb);
-                    MaterialSample ms = sample_world(m, -d, f, true, uniform01(key, base), uniform01(key, base + 1),
-                                                     uniform01(key, base + 2));
-                    L = L + mul(tp, ms.emission);
-                    tp = mul(tp, ms.radiance * (fabsf(dot(f.normal, ms.outgoing)) / ms.pdf));
-                    new_o = nudge(o + (d * h.x), ms.outgoing);
-                    new_d = ms.outgoing;
-                    if (depth > p.rr_depth || nearly_zero(tp)) {
-                        float rv = uniform01(key, base + 3);
-                        float lum = luminance(tp);
-                        float prob =
-                            depth > p.rr_aggr ? clamped_lerp(0.10f, 0.75f, lum) : clamped_lerp(0.25f, 1.00f, lum);
-                        tp = rv < prob ? tp / prob : v3zero();
-                    }
-                    alive = !is_zero(tp) && (p.max_depth == 0 || depth + 1 < p.max_depth);
-                }
+                alive = shade_hit(s, p, depth, state_key(sb), o, d, h, tp, L, new_o, new_d);
                 if (alive) {
                     sa = make_float4(tp.x, tp.y, tp.z, L.x);
                     sb = make_float4(L.y, L.z, sb.z, sb.w);
@@ -257,6 +291,93 @@ gr_status launch_shade(uint32_t n_bound, bool first, cudaStream_t st, A... a) {
     if (first) return big ? launch_shade_nt<SHADE_BIG, true>(n_bound, st, a...)
                           : launch_shade_nt<128, true>(n_bound, st, a...);
     return big ? launch_shade_nt<SHADE_BIG, false>(n_bound, st, a...) : launch_shade_nt<128, false>(n_bound, st, a...);
+}
+
+// A bounce's queue, as the path loop reads it.
+struct PathQueue {
+    const uint32_t* count;
+    const uint32_t* slot;
+    const float4* o;
+    const float4* d;
+    const float4* state;
+};
+
+// Carries paths to their end (run_paths): CAMERA, the n_paths paths of a group from their
+// camera rays (no queue; their film positions are written here); else the queue of bounce
+// `depth0`.  Bound by latency: dependent node and record loads of one traversal step
+// after another, and the instruction fetch of the shading code.
+template <int W, bool CAMERA>
+__global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
+    k_pt_finish(DeviceScene s, PTParams p, uint32_t depth0, uint32_t n_paths, PathQueue queue, float2* __restrict__ st,
+                float4* __restrict__ L_buf, uint32_t lanes, uint32_t* fetch, int* err, unsigned long long* rays) {
+    extern __shared__ unsigned char smem[];
+    int2 spill[MAX_STACK - SMEM_STACK];
+    const StackView stk = thread_stack(smem, spill);
+    const uint32_t n = CAMERA ? n_paths : *queue.count;
+    V3 tp, L;
+    uint64_t key = 0;
+    uint32_t slot = 0, depth = 0;
+    auto take = [&](uint32_t q, V3& o, V3& d) {
+        depth = depth0;
+        if (CAMERA) {
+            slot = q;
+            const uint32_t pass_local = fast_div(q, p.by_npix);
+            const uint32_t pixel = q - pass_local * p.npix;
+            const uint32_t row = fast_div(pixel, p.by_width), col = pixel - row * p.width;
+            key = path_key(p.seed, p.first_pass + pass_local, pixel);
+            float fs, ft;
+            film_sample_point(p.width, p.height, row, col, key, fs, ft);
+            camera_ray(p.cam, fs, ft, o, d);
+            st[q] = make_float2(fs, ft);
+            tp = v3one();
+            L = v3zero();
+        } else {
+            slot = queue.slot[q];
+            const float4 o4 = queue.o[q], d4 = queue.d[q];
+            const float4 sa = queue.state[2 * static_cast<size_t>(q)], sb = queue.state[2 * static_cast<size_t>(q) + 1];
+            o = V3{o4.x, o4.y, o4.z};
+            d = V3{d4.x, d4.y, d4.z};
+            tp = V3{sa.x, sa.y, sa.z};
+            L = V3{sa.w, sb.x, sb.y};
+            key = state_key(sb);
+        }
+        return true;
+    };
+    auto shade = [&](uint32_t, const TravState& t, V3& no, V3& nd) {
+        const float4 h = make_float4(t.closest, __int_as_float(t.hit), t.hu, t.hv);
+        const bool alive = shade_hit(s, p, depth, key, t.o, t.d, h, tp, L, no, nd);
+        ++depth;
+        if (!alive) L_buf[slot] = make_float4(L.x, L.y, L.z, 0.0f);
+        return alive;
+    };
+    count_rays(run_paths<W>(s, stk, n, lanes, fetch, err, take, shade), rays);
+}
+
+template <int W, bool CAMERA>
+gr_status launch_finish_w(const DeviceScene& s, const PTParams& p, uint32_t depth, uint32_t most, const PathQueue& q,
+                          float2* film_pos, float4* L_buf, uint32_t* fetch, int* err, unsigned long long* rays,
+                          cudaStream_t st) {
+    const size_t smem = step_stack_smem_bytes(BLOCK);
+    int per_sm = 0;
+    GR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pt_finish<W, CAMERA>, BLOCK, smem));
+    const uint32_t warps = static_cast<uint32_t>(std::max(1, per_sm) * device_sm_count()) * (BLOCK / 32);
+    const uint32_t lanes = std::min(32u, std::max(PATH_LOOP_MIN_LANES, (most + warps - 1) / warps));
+    const uint32_t need_warps = (most + lanes - 1) / lanes;
+    const uint32_t grid = (std::min(warps, need_warps) + BLOCK / 32 - 1) / (BLOCK / 32);
+    k_pt_finish<W, CAMERA><<<grid, BLOCK, smem, st>>>(s, p, depth, most, q, film_pos, L_buf, lanes, fetch, err, rays);
+    GR_CUDA_TRY(cudaGetLastError());
+    return GR_OK;
+}
+
+// The paths of a queue of at most `most` entries (CAMERA: of a group of `most` camera
+// paths) to their end.  *fetch is zero.
+template <bool CAMERA, class... A>
+gr_status launch_finish(const DeviceScene& s, A... a) {
+    switch (s.width) {
+        case 2: return launch_finish_w<2, CAMERA>(s, a...);
+        case 4: return launch_finish_w<4, CAMERA>(s, a...);
+        default: return launch_finish_w<8, CAMERA>(s, a...);
+    }
 }
 
 __global__ void k_samples_out(uint32_t n, const float2* __restrict__ st, const float4* __restrict__ L, float* out) {
@@ -350,28 +471,62 @@ gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
     p.rr_depth = rp.rr_depth;
     p.rr_aggr = rp.rr_aggressive_depth;
     uint64_t launches = 0;
+    // Whether the path loop may take this render's short queues (it counts no traversal).
+    const bool bounded = rp.max_depth ? rp.max_depth <= PATH_LOOP_DEPTH
+                                      : std::max(rp.rr_depth, rp.rr_aggressive_depth) <= PATH_LOOP_RR_DEPTH;
+    const bool loop_ok = bounded && !display && !(rp.flags & GR_RENDER_COUNT_TRAVERSAL);
 
     for (uint32_t done = 0; done < total; done += group) {
         uint32_t g = std::min(group, total - done);
         uint32_t n = g * npix;
         p.first_pass = rp.first_pass + done;
-        int r0 = -1, r1 = -1;
-        if (timed) GR_TRY_S(mark(r0));
-        k_set_count<<<1, 1, 0, st>>>(cnt + CNT_QUEUE0, n);
-        GR_CUDA_TRY(cudaGetLastError());
-        uint32_t bound = n;  // an upper bound of the current queue length
-        k_raygen<<<(n + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(p, n, ps.st.as<float2>(), ps.q_o[0].as<float4>(),
-                                                            ps.q_d[0].as<float4>());
-        GR_CUDA_TRY(cudaGetLastError());
-        ++launches;
-        GR_TRY_S(sync_check(st, "raygen", 0, n));
-        if (timed) {
-            GR_TRY_S(mark(r1));
-            raygen_pairs.emplace_back(r0, r1);
+        // Carries the queue of `depth` (depth 0: the group's camera paths, which need no
+        // queue) to its end.  Its time counts as extension (GR_RENDER_TIME_KERNELS).
+        auto finish = [&](uint32_t depth, uint32_t most) -> gr_status {
+            int e0 = -1, e1 = -1;
+            if (timed) GR_TRY_S(mark(e0));
+            GR_CUDA_TRY(cudaMemsetAsync(cnt + CNT_FETCH, 0, sizeof(uint32_t), st));
+            const int cur = depth & 1;
+            const PathQueue q{cnt + cur, ps.q_slot[cur].as<uint32_t>(), ps.q_o[cur].as<float4>(),
+                              ps.q_d[cur].as<float4>(), ps.q_state[cur].as<float4>()};
+            GR_TRY_S(depth == 0 ? launch_finish<true>(job.scene, p, 0, most, q, ps.st.as<float2>(),
+                                                      ps.light.as<float4>(), cnt + CNT_FETCH, err, rays, st)
+                                : launch_finish<false>(job.scene, p, depth, most, q, ps.st.as<float2>(),
+                                                       ps.light.as<float4>(), cnt + CNT_FETCH, err, rays, st));
+            ++launches;
+            GR_TRY_S(sync_check(st, "path loop", depth, n));
+            if (timed) {
+                GR_TRY_S(mark(e1));
+                ext_pairs.emplace_back(e0, e1);
+            }
+            return GR_OK;
+        };
+        const bool small = loop_ok && n <= PATH_LOOP_MAX;
+        if (small) {
+            GR_TRY_S(finish(0, n));
+        } else {
+            int r0 = -1, r1 = -1;
+            if (timed) GR_TRY_S(mark(r0));
+            k_set_count<<<1, 1, 0, st>>>(cnt + CNT_QUEUE0, n);
+            GR_CUDA_TRY(cudaGetLastError());
+            k_raygen<<<(n + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(p, n, ps.st.as<float2>(), ps.q_o[0].as<float4>(),
+                                                                ps.q_d[0].as<float4>());
+            GR_CUDA_TRY(cudaGetLastError());
+            ++launches;
+            GR_TRY_S(sync_check(st, "raygen", 0, n));
+            if (timed) {
+                GR_TRY_S(mark(r1));
+                raygen_pairs.emplace_back(r0, r1);
+            }
         }
-        for (uint32_t depth = 0;; ++depth) {
+        uint32_t bound = n;  // an upper bound of the current queue length
+        for (uint32_t depth = 0; !small; ++depth) {
             if (p.max_depth && depth >= p.max_depth) break;
             int cur = depth & 1, nxt = cur ^ 1;
+            if (depth > 0 && loop_ok && bound <= PATH_LOOP_MAX) {
+                GR_TRY_S(finish(depth, bound));
+                break;
+            }
             int e0 = -1, e1 = -1;
             if (timed) GR_TRY_S(mark(e0));
             gr_status s1 = extend_any(job.scene, (rp.flags & GR_RENDER_COUNT_TRAVERSAL) != 0, n, cnt + cur,

@@ -159,6 +159,12 @@ struct gr_film {
     mutable gr::DevBuf readback;  // accum and weight planes for gr_film_read (a cache); allocated on first use
     uint32_t passes = 0;
     int device = 0;
+    // Recorded on the default stream after the film was cleared there; a render's own
+    // stream waits for it.
+    cudaEvent_t cleared = nullptr;
+    ~gr_film() {
+        if (cleared) cudaEventDestroy(cleared);
+    }
 };
 
 namespace gr {

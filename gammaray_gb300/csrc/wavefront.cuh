@@ -154,6 +154,92 @@ __global__ void GR_EXTEND_BOUNDS k_extend_refill(DeviceScene s, const uint32_t* 
     }
 }
 
+// Path loop: a warp carries paths from their first ray to their end without going back
+// to a queue.  Its lanes trace, one traversal step each per iteration, until every path
+// of the warp has its closest hit, then all of them shade, and the survivors trace their
+// next rays; lanes whose paths ended take other paths.  One launch replaces an extension
+// and a shading launch per bounce, and a slow ray delays its own warp's paths instead of
+// every path of its bounce.
+//   n       paths; path index q goes to take() once
+//   lanes   lanes of each warp that carry paths (1..32): few paths are spread over the
+//           whole grid, since lanes of one warp wait for each other
+//   fetch   a zeroed counter; the first warps * lanes paths are handed out by position
+//           (neighbouring ones to different blocks, so a costly part of an image does not
+//           fall on one SM), the rest from it
+//   take(q, o, d)         loads path q and its next ray; false: it has none
+//   shade(q, t, no, nd)   shades the hit in t (t.hit, t.closest, t.hu, t.hv); true and the
+//                         next ray in (no, nd) when the path goes on
+// Every warp intrinsic runs where control flow is warp-uniform (each condition around one
+// comes from ballots or from the shuffled base), and every loop ends: a traversal
+// iteration steps a lane whose ray has the scene's step budget, each path is handed out
+// once and ends by its depth limit or roulette.  Returns the rays this lane traced.
+template <int W, class Take, class Shade>
+GR_D uint32_t run_paths(const DeviceScene& s, const StackView& stk, uint32_t n, uint32_t lanes, uint32_t* fetch,
+                        int* err, const Take& take, const Shade& shade) {
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned below = (1u << lane) - 1u;
+    const bool use = lane < lanes;
+    const uint32_t warps = blockDim.x >> 5;
+    const uint32_t first = gridDim.x * warps * lanes;  // paths handed out by position
+    const uint32_t refill_at = lanes < 4u ? 1u : lanes / 4u;
+    TravState t;
+    t.hit = -1;
+    uint32_t q = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * lanes + lane, steps = 0, traced = 0;
+    bool busy = false, exhausted = first >= n;
+    auto start = [&](V3 o, V3 d) {
+        trav_init(t, o, d, FLT_MAX);
+        steps = 0;
+        ++traced;
+        busy = true;
+    };
+    if (use && q < n) {
+        V3 o, d;
+        if (take(q, o, d)) start(o, d);
+    }
+    for (;;) {
+        const unsigned idle = __ballot_sync(0xffffffffu, use && !busy);
+        if (!exhausted && static_cast<uint32_t>(__popc(idle)) >= refill_at) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(fetch, static_cast<uint32_t>(__popc(idle)));
+            base = __shfl_sync(0xffffffffu, base, 0) + first;
+            exhausted = static_cast<uint64_t>(base) + __popc(idle) >= n;
+            if (use && !busy) {
+                q = base + __popc(idle & below);
+                V3 o, d;
+                if (q < n && take(q, o, d)) start(o, d);
+            }
+        }
+        // No lane busy and paths left: every lane is idle, so the next iteration takes
+        // paths or learns that none are left.
+        if (__ballot_sync(0xffffffffu, busy) == 0u && exhausted) break;
+        bool trav = busy;
+        while (__any_sync(0xffffffffu, trav)) {
+            if (trav) {
+                bool done = trav_step<W, false, false>(s, t, stk, err, nullptr);
+                if (!done && ++steps > s.step_budget) {
+                    atomicExch(err, 2);
+                    atomicExch(err + 1, static_cast<int>(q));
+                    t.hit = -1;
+                    done = true;
+                }
+                trav = !done;
+            }
+        }
+        if (busy) {
+            V3 no, nd;
+            if (shade(q, t, no, nd)) start(no, nd);
+            else busy = false;
+        }
+    }
+    return traced;
+}
+
+// Adds the warp's traced rays to *rays (one atomic per warp; every lane calls it).
+GR_D void count_rays(uint32_t traced, unsigned long long* rays) {
+    const uint32_t sum = __reduce_add_sync(0xffffffffu, traced);
+    if ((threadIdx.x & 31u) == 0 && sum) atomicAdd(rays, static_cast<unsigned long long>(sum));
+}
+
 // Appends this lane's ray to the next queue with one atomic per warp (ballot + popc).
 // Every lane of the warp must call it (warp-uniform trip counts).
 GR_D void push_warp(bool alive, uint32_t* count_out, uint32_t slot, V3 o, V3 d, uint32_t* __restrict__ nslot,

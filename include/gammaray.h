@@ -260,7 +260,8 @@ typedef struct gr_render_params {
 #define GR_RENDER_COUNT_TRAVERSAL 1u
 /* Time every extension (closest-hit) and shade launch with CUDA events on the render
  * stream (gr_render_stats.extend_ms / shade_ms), and for the path tracer its camera
- * rays and film accumulation (raygen_ms / film_ms). */
+ * rays and film accumulation (raygen_ms / film_ms).  The path tracer's launch that
+ * carries few paths to their end, extension and shading in one, counts as extension. */
 #define GR_RENDER_TIME_KERNELS 2u
 
 void gr_render_params_default(int32_t integrator, gr_render_params* out);
