@@ -23,6 +23,7 @@
 #include <utility>
 #include <vector>
 
+#include "path_order.cuh"
 #include "runtime.hpp"
 #include "shade_sort.cuh"
 #include "wavefront.cuh"
@@ -89,8 +90,7 @@ constexpr uint32_t PATH_LOOP_MIN_LANES = 8;
 
 struct PTParams {
     DevCamera cam;
-    uint32_t width, height, npix;
-    FastDiv by_npix, by_width;  // divisions by npix and width
+    PathOrder order;  // which sample a camera-ray entry is
     uint32_t first_pass;
     uint64_t seed;
     uint32_t max_depth, rr_depth, rr_aggr;
@@ -105,36 +105,41 @@ struct PTParams {
 // arrays at random.  A finished path writes its radiance to its slot (the index of its
 // film position), which the film gather reads.
 //
-// The first queue (camera rays) holds only rays: its entry q is path q (slot q), whose
-// state is unit throughput, no radiance and the key of its pass and pixel, so shading
-// makes that state instead of reading it; and their one origin (the pinhole's) is stored
-// once, in q_o[0].  Raygen writes 24 bytes per path.
+// The first queue (camera rays) holds only rays, each with its slot in the direction's w:
+// their state is unit throughput, no radiance and the key of the slot's pass and pixel, so
+// shading makes that state instead of reading it; and their one origin (the pinhole's) is
+// stored once, in q_o[0].  Raygen writes 24 bytes per path.
 GR_D uint64_t state_key(float4 b) {
     return (static_cast<uint64_t>(__float_as_uint(b.w)) << 32) | __float_as_uint(b.z);
 }
 
-// The random key of path q of the group (pass first_pass + q / npix, pixel q % npix).
-GR_D uint64_t first_key(const PTParams& p, uint32_t q) {
-    const uint32_t pass_local = fast_div(q, p.by_npix);
-    return path_key(p.seed, p.first_pass + pass_local, q - pass_local * p.npix);
+// The random key of sample `slot` of the group (pass first_pass + slot / npix, pixel
+// slot % npix).
+GR_D uint64_t first_key(const PTParams& p, uint32_t slot) {
+    const uint32_t pass = fast_div(slot, p.order.by_npix);
+    return path_key(p.seed, p.first_pass + pass, slot - pass * p.order.npix);
+}
+
+// The camera ray of queue entry q; its film position goes to st[slot].
+GR_D uint32_t camera_path(const PTParams& p, uint32_t q, float2* __restrict__ st, uint64_t& key, V3& o, V3& d) {
+    const PathSample ps = path_sample(p.order, q);
+    key = path_key(p.seed, p.first_pass + ps.pass, ps.row * p.order.width + ps.col);
+    float s, t;
+    film_sample_point(p.order.width, p.order.height, ps.row, ps.col, key, s, t);
+    camera_ray(p.cam, s, t, o, d);
+    st[ps.slot] = make_float2(s, t);
+    return ps.slot;
 }
 
 __global__ void __launch_bounds__(BLOCK) k_raygen(PTParams p, uint32_t n, float2* __restrict__ st,
                                                   float4* __restrict__ q_o, float4* __restrict__ q_d) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    uint32_t pass_local = fast_div(i, p.by_npix);
-    uint32_t pixel = i - pass_local * p.npix;
-    uint32_t row = fast_div(pixel, p.by_width);
-    uint32_t col = pixel - row * p.width;
-    uint64_t k = path_key(p.seed, p.first_pass + pass_local, pixel);
-    float s, t;
-    film_sample_point(p.width, p.height, row, col, k, s, t);
+    uint64_t key;
     V3 o, d;
-    camera_ray(p.cam, s, t, o, d);
-    st[i] = make_float2(s, t);
+    const uint32_t slot = camera_path(p, i, st, key, o, d);
     if (i == 0) q_o[0] = make_float4(o.x, o.y, o.z, 0.0f);  // the pinhole origin, the same for every ray
-    q_d[i] = make_float4(d.x, d.y, d.z, 0.0f);
+    q_d[i] = make_float4(d.x, d.y, d.z, __uint_as_float(slot));
 }
 
 // Appends this lane's surviving path (slot, ray, state) to the next queue with one atomic
@@ -214,7 +219,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_shade(DeviceScene s, PTParams 
         const uint32_t cn = min(chunk, n - c0);
         sort_chunk<NT, PER>(sm, cn, per, [&](uint32_t i) {
             uint32_t q = c0 + i;
-            const uint64_t key = FIRST ? first_key(p, q) : state_key(q_state[2 * q + 1]);
+            const uint64_t key = FIRST ? first_key(p, __float_as_uint(q_d[q].w)) : state_key(q_state[2 * q + 1]);
             return shade_bucket(s, __float_as_int(q_hit[q].y), uniform01(key, base), 0);
         });
         // Every lane runs every step so that all of them reach the ballot in push_path.
@@ -230,8 +235,8 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_shade(DeviceScene s, PTParams 
                 float4 o4 = q_o[FIRST ? 0u : q], d4 = q_d[q];  // camera rays share q_o[0]
                 V3 o = V3{o4.x, o4.y, o4.z}, d = V3{d4.x, d4.y, d4.z};
                 if (FIRST) {
-                    slot = q;
-                    const uint64_t k0 = first_key(p, q);
+                    slot = __float_as_uint(d4.w);
+                    const uint64_t k0 = first_key(p, slot);
                     sa = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
                     sb = make_float4(0.0f, 0.0f, __uint_as_float(static_cast<uint32_t>(k0)),
                                      __uint_as_float(static_cast<uint32_t>(k0 >> 32)));
@@ -255,8 +260,9 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_shade(DeviceScene s, PTParams 
     }
 }
 
-// DisplayColorIntegrator: one bounce, so the queue is the camera rays (entry q is path q).
+// DisplayColorIntegrator: one bounce, so the queue is the camera rays (slots in q_d).
 __global__ void __launch_bounds__(BLOCK) k_shade_display(DeviceScene s, const uint32_t* __restrict__ count_in,
+                                                         const float4* __restrict__ q_d,
                                                          const float4* __restrict__ q_hit, float4* __restrict__ L_buf) {
     const uint32_t n = *count_in;
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
@@ -268,7 +274,7 @@ __global__ void __launch_bounds__(BLOCK) k_shade_display(DeviceScene s, const ui
             const DevMaterial& m = s.materials[__ldg(s.prim_material + prim)];
             c = make_float4(m.display[0], m.display[1], m.display[2], 0.0f);
         }
-        L_buf[q] = c;
+        L_buf[__float_as_uint(q_d[q].w)] = c;
     }
 }
 
@@ -320,15 +326,7 @@ __global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
     auto take = [&](uint32_t q, V3& o, V3& d) {
         depth = depth0;
         if (CAMERA) {
-            slot = q;
-            const uint32_t pass_local = fast_div(q, p.by_npix);
-            const uint32_t pixel = q - pass_local * p.npix;
-            const uint32_t row = fast_div(pixel, p.by_width), col = pixel - row * p.width;
-            key = path_key(p.seed, p.first_pass + pass_local, pixel);
-            float fs, ft;
-            film_sample_point(p.width, p.height, row, col, key, fs, ft);
-            camera_ray(p.cam, fs, ft, o, d);
-            st[q] = make_float2(fs, ft);
+            slot = camera_path(p, q, st, key, o, d);
             tp = v3one();
             L = v3zero();
         } else {
@@ -460,11 +458,6 @@ gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
 
     PTParams p;
     p.cam = job.camera;
-    p.width = job.width;
-    p.by_width = make_fastdiv(job.width);
-    p.height = job.height;
-    p.npix = npix;
-    p.by_npix = make_fastdiv(npix);
     p.qcap = static_cast<uint32_t>(static_cast<size_t>(group) * npix);
     p.seed = rp.seed;
     p.max_depth = display ? 1 : rp.max_depth;
@@ -480,6 +473,7 @@ gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
         uint32_t g = std::min(group, total - done);
         uint32_t n = g * npix;
         p.first_pass = rp.first_pass + done;
+        p.order = make_path_order(job.width, job.height, g);
         // Carries the queue of `depth` (depth 0: the group's camera paths, which need no
         // queue) to its end.  Its time counts as extension (GR_RENDER_TIME_KERNELS).
         auto finish = [&](uint32_t depth, uint32_t most) -> gr_status {
@@ -542,8 +536,8 @@ gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
             }
             if (display) {
                 int grid = resident_grid(k_shade_display, 0, n);
-                k_shade_display<<<grid, BLOCK, 0, st>>>(job.scene, cnt + cur, ps.q_hit.as<float4>(),
-                                                        ps.light.as<float4>());
+                k_shade_display<<<grid, BLOCK, 0, st>>>(job.scene, cnt + cur, ps.q_d[cur].as<float4>(),
+                                                        ps.q_hit.as<float4>(), ps.light.as<float4>());
                 GR_CUDA_TRY(cudaGetLastError());
                 ++launches;
                 break;
@@ -757,11 +751,7 @@ extern "C" gr_status gr_render_static(gr_scene* sc, const gr_camera* camera, con
     const bool display = rp->integrator == GR_INTEGRATOR_DISPLAY_COLOR;
     PTParams p;
     p.cam = make_camera(*camera);
-    p.width = width;
-    p.by_width = make_fastdiv(width);
-    p.height = height;
-    p.npix = npix;
-    p.by_npix = make_fastdiv(npix);
+    p.order = make_path_order(width, height, 1);
     p.qcap = npix;
     p.seed = rp->seed;
     p.max_depth = display ? 1 : rp->max_depth;
@@ -783,7 +773,7 @@ extern "C" gr_status gr_render_static(gr_scene* sc, const gr_camera* camera, con
             GR_CUDA_TRY(cudaGetLastError());
             if (display) {
                 int grid = resident_grid(k_shade_display, 0, n);
-                k_shade_display<<<grid, BLOCK, 0, st>>>(sc->dev, cnt + cur, q_hit, light);
+                k_shade_display<<<grid, BLOCK, 0, st>>>(sc->dev, cnt + cur, q_d[cur], q_hit, light);
                 GR_CUDA_TRY(cudaGetLastError());
                 break;
             }
