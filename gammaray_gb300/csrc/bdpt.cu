@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(BLOCK) k_bdpt_shadow(DeviceScene s, const uint
                                                        float3 cam, int* err, unsigned long long* shadow_rays) {
     extern __shared__ unsigned char smem[];
     int2 spill[MAX_STACK - SMEM_STACK];
-    const StackView stk = thread_stack(smem, spill);
+    const auto stk = thread_stack<BLOCK>(smem, spill);
     const uint32_t n = *count;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(shadow_rays, static_cast<unsigned long long>(n));
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {

@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
                 float4* __restrict__ L_buf, uint32_t lanes, uint32_t* fetch, int* err, unsigned long long* rays) {
     extern __shared__ unsigned char smem[];
     int2 spill[MAX_STACK - SMEM_STACK];
-    const StackView stk = thread_stack(smem, spill);
+    const auto stk = thread_stack<BLOCK>(smem, spill);
     const uint32_t n = CAMERA ? n_paths : *queue.count;
     V3 tp, L;
     uint64_t key = 0;

@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(QUERY_BLOCK) k_trace(DeviceScene s, const floa
                                                        int* err) {
     extern __shared__ unsigned char smem[];
     int2 spill[MAX_STACK - SMEM_STACK];
-    const StackView stk = thread_stack(smem, spill);
+    const auto stk = thread_stack<QUERY_BLOCK>(smem, spill);
     uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float* r = rays + 6 * i;
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(QUERY_BLOCK) k_visibility(DeviceScene s, const
                                                             uint64_t n, uint8_t* __restrict__ vis, int* err) {
     extern __shared__ unsigned char smem[];
     int2 spill[MAX_STACK - SMEM_STACK];
-    const StackView stk = thread_stack(smem, spill);
+    const auto stk = thread_stack<QUERY_BLOCK>(smem, spill);
     uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float* p = pairs + 6 * i;

@@ -34,14 +34,6 @@ constexpr uint32_t SHADE_PER_THREAD = GR_SHADE_PER_THREAD;
 constexpr uint32_t SHADE_BIG_PER = GR_SHADE_BIG_PER;
 static_assert(SHADE_BIG_PER >= 1 && SHADE_BIG_PER <= 85, "768 x per chunk positions fit 16 bits");
 
-// Rays per thread per chunk when the extension kernels trace their queue grouped by
-// direction (octant and dominant axis; 0: no sort).  Measured on the path-tracer
-// workload: 8 -> +2.2%; 2, 32 and 64 slower (the barrier per chunk waits for the chunk's
-// slowest ray, which outweighs the coherence gained).
-#ifndef GR_EXTEND_SORT
-#define GR_EXTEND_SORT 8
-#endif
-
 // The sort's shared memory (dynamic, sort_smem_bytes(NT, PER) bytes at the start of the
 // block's dynamic shared memory): bucket sizes, then per-entry bucket and sorted order.
 struct SortView {

@@ -67,11 +67,6 @@ GR_D float intersect_prim(const float4 p0, const float4 p1, const float4 p2, V3 
 // child[slot] without dynamic register indexing (keeps the node in registers).
 template <int W>
 GR_D int32_t select_child(const float (&f)[8 * W], uint32_t slot) {
-    if (W == 4) {  // by the slot's two bits: three selects
-        const float lo = (slot & 1u) ? f[6 * W + 1] : f[6 * W];
-        const float hi = (slot & 1u) ? f[6 * W + 3] : f[6 * W + 2];
-        return __float_as_int((slot & 2u) ? hi : lo);
-    }
     int32_t r = 0;
 #pragma unroll
     for (int j = 0; j < W; ++j)
@@ -81,16 +76,6 @@ GR_D int32_t select_child(const float (&f)[8 * W], uint32_t slot) {
 
 template <int N>
 GR_D void sort_keys(uint32_t (&k)[N]) {
-    if (N == 4) {  // the 5-comparator network for 4 keys
-        const int pairs[5][2] = {{0, 1}, {2, 3}, {0, 2}, {1, 3}, {1, 2}};
-#pragma unroll
-        for (int c = 0; c < 5; ++c) {
-            uint32_t a = k[pairs[c][0]], b = k[pairs[c][1]];
-            k[pairs[c][0]] = min(a, b);
-            k[pairs[c][1]] = max(a, b);
-        }
-        return;
-    }
     // Odd-even transposition network, fully unrolled (N <= 8).
 #pragma unroll
     for (int pass = 0; pass < N; ++pass) {
@@ -124,22 +109,45 @@ namespace gr {
 constexpr int SMEM_STACK = GR_SMEM_STACK;
 static_assert(SMEM_STACK >= 1 && SMEM_STACK <= MAX_STACK, "shared stack part within the stack bound");
 
-// Extension kernels that refill their warps (k_extend_refill, k_eng_extend_refill): a
-// warp takes new rays for its idle lanes once at least this many are idle; 0 selects the
-// kernels with one ray per thread and no refill.  On the path-tracer workload (102,422
-// triangles, 1024 x 1024, 64 spp) 0 / 4 / 8 / 16 measured 1298 / 1511 / 1565 / 1586
-// Msamples/s.
-#ifndef GR_EXTEND_REFILL
-#define GR_EXTEND_REFILL 16
-#endif
+// A warp tracing rays from a queue (trace_queue) takes new rays for its idle lanes once
+// EXTEND_REFILL of them are idle, and tests leaves once EXTEND_LEAVES of its lanes stand at
+// one (or none stands at a node), not whenever one does: a step runs either the node test
+// or the leaf test for the whole warp.  On the path-tracer workload (102,422 triangles,
+// 1024 x 1024, 64 spp) testing leaves at once took 15.3 ms of extension per render, and
+// waiting for 4 / 6 / 8 / 12 lanes 15.2 / 14.4 / 14.3 / 15.1 (refilling at 16); refilling
+// at 8 / 12 / 16 / 20 / 24 (waiting for 8) 15.7 / 14.7 / 14.3 / 14.1 / 14.4.
+constexpr int EXTEND_REFILL = 20;
+constexpr int EXTEND_LEAVES = 8;
 
-// The two arrays a traversal step reads.  A kernel whose lanes trace rays of different
-// scenes keeps one per lane in registers instead of reloading them through a scene
-// record at every step.
+// What a traversal step reads.  A kernel whose lanes trace rays of different scenes keeps
+// one per lane in registers instead of reloading it through a scene record at every step.
 struct TraceScene {
     const float4* nodes;
     const float4* prims;
+    uint32_t step_budget;
 };
+
+// Two floats in one 64-bit register, added or multiplied by one instruction; each half is
+// rounded as the scalar operation rounds it.
+struct F2 {
+    unsigned long long v;
+};
+GR_D F2 pack2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+GR_D void unpack2(F2 p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v)); }
+GR_D F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+GR_D F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
 
 struct TravState {
     V3 o, d, inv;
@@ -166,30 +174,47 @@ GR_D void trav_init(TravState& t, V3 o, V3 d, float t_max) {
 }
 
 // Stack entries are (child reference, entry distance bits) pairs, one 64-bit access each.
+// STRIDE: threads of the block, so that an entry's address is the column's plus a
+// constant shift.
+template <int STRIDE>
 struct StackView {
-    int2* s;      // this thread's shared column (stride = blockDim.x entries)
-    int stride;
+    int2* s;      // this thread's shared column
     int2* spill;  // local overflow, MAX_STACK - SMEM_STACK entries
-    GR_D void push(int sp, int32_t ref, float te) const {
-        const int2 e = make_int2(ref, __float_as_int(te));
-        if (sp < SMEM_STACK) s[sp * stride] = e;
+    static constexpr int stride = STRIDE;
+    GR_D int2* at(int sp) const { return s + sp * STRIDE; }
+    GR_D void push(int sp, int32_t ref, uint32_t te_bits) const {
+        const int2 e = make_int2(ref, static_cast<int>(te_bits));
+        if (sp < SMEM_STACK) s[sp * STRIDE] = e;
         else spill[sp - SMEM_STACK] = e;
     }
     GR_D void pop(int sp, int32_t& ref, float& te) const {
         int2 e;
-        if (sp < SMEM_STACK) e = s[sp * stride];  // shared and local loads kept apart
+        if (sp < SMEM_STACK) e = s[sp * STRIDE];  // shared and local loads kept apart
         else e = spill[sp - SMEM_STACK];
         ref = e.x;
         te = __int_as_float(e.y);
     }
 };
 
+constexpr uint32_t KEY_MISS = 0xFFFFFFFFu;  // sorts after every hit child
+
+// One comparator of the sorting network at width 4, each key with its child reference.
+GR_D void order_pair(uint32_t& ka, uint32_t& kb, int32_t& ra, int32_t& rb) {
+    const bool swap = kb < ka;
+    const uint32_t k = swap ? kb : ka;
+    kb = swap ? ka : kb;
+    ka = k;
+    const int32_t r = swap ? rb : ra;
+    rb = swap ? ra : rb;
+    ra = r;
+}
+
 // Tests one wide node against the ray: pushes the far hit children (sorted by entry
 // distance, nearest last) and makes the nearest hit child the current reference.
 // Returns false when no child is hit.  A push beyond MAX_STACK sets *err = 1 and
 // `overflow`.
-template <int W, bool COUNT, class S>
-GR_D bool visit_node(const S& s, TravState& t, const StackView& stk, int* err, uint32_t* counts,
+template <int W, bool COUNT, class S, class K>
+GR_D bool visit_node(const S& s, TravState& t, const K& stk, int* err, uint32_t* counts,
                      bool& overflow) {
     const float inflate = 1.0f + 2.0f * gamma_n(3.0f);
     if (COUNT) counts[0] += 1;
@@ -225,35 +250,82 @@ GR_D bool visit_node(const S& s, TravState& t, const StackView& stk, int* err, u
     }
     uint32_t key[W];
     int h = 0;
+    // The slab test (tmin <= tmax, tmax > 0, tmin < closest) on te = max(tmin, 0): the same
+    // result (closest > 0), except that a box whose far distance is exactly 0 counts as
+    // hit, which can only add a node to visit.
+    auto child_key = [&](int j, float tmin, float tmax) {
+        const float te = fmaxf(tmin, 0.0f);
+        const bool hit = te <= tmax && te < t.closest;
+        key[j] = hit ? ((__float_as_uint(te) & ~7u) | static_cast<uint32_t>(j)) : KEY_MISS;
+        h += hit ? 1 : 0;
+    };
+    if (W % 4 == 0) {  // rows 0-2 near, 3-5 far; two children per packed operation
+        const F2 nox = pack2(-t.o.x, -t.o.x), noy = pack2(-t.o.y, -t.o.y), noz = pack2(-t.o.z, -t.o.z);
+        const F2 ix = pack2(t.inv.x, t.inv.x), iy = pack2(t.inv.y, t.inv.y), iz = pack2(t.inv.z, t.inv.z);
+        auto plane = [&](int row, int j, F2 no, F2 inv, float& a, float& b) {
+            unpack2(mul2(add2(pack2(f[row * W + j], f[row * W + j + 1]), no), inv), a, b);
+        };
 #pragma unroll
-    for (int j = 0; j < W; ++j) {
-        float t0x, t1x, t0y, t1y, t0z, t1z;
-        if (W % 4 == 0) {  // rows 0-2 near, 3-5 far
-            t0x = (f[0 * W + j] - t.o.x) * t.inv.x;
-            t0y = (f[1 * W + j] - t.o.y) * t.inv.y;
-            t0z = (f[2 * W + j] - t.o.z) * t.inv.z;
-            t1x = (f[3 * W + j] - t.o.x) * t.inv.x;
-            t1y = (f[4 * W + j] - t.o.y) * t.inv.y;
-            t1z = (f[5 * W + j] - t.o.z) * t.inv.z;
-        } else {
+        for (int j = 0; j < W; j += 2) {
+            float ax, bx, ay, by, az, bz;
+            plane(0, j, nox, ix, ax, bx);
+            plane(1, j, noy, iy, ay, by);
+            plane(2, j, noz, iz, az, bz);
+            const float na = fmaxf(fmaxf(ax, ay), az), nb2 = fmaxf(fmaxf(bx, by), bz);
+            plane(3, j, nox, ix, ax, bx);
+            plane(4, j, noy, iy, ay, by);
+            plane(5, j, noz, iz, az, bz);
+            float fa, fb;
+            unpack2(mul2(pack2(fminf(fminf(ax, ay), az), fminf(fminf(bx, by), bz)), pack2(inflate, inflate)), fa, fb);
+            child_key(j, na, fa);
+            child_key(j + 1, nb2, fb);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
             float lx = f[0 * W + j], ly = f[1 * W + j], lz = f[2 * W + j];
             float hx = f[3 * W + j], hy = f[4 * W + j], hz = f[5 * W + j];
-            t0x = ((t.nx ? hx : lx) - t.o.x) * t.inv.x;
-            t1x = ((t.nx ? lx : hx) - t.o.x) * t.inv.x;
-            t0y = ((t.ny ? hy : ly) - t.o.y) * t.inv.y;
-            t1y = ((t.ny ? ly : hy) - t.o.y) * t.inv.y;
-            t0z = ((t.nz ? hz : lz) - t.o.z) * t.inv.z;
-            t1z = ((t.nz ? lz : hz) - t.o.z) * t.inv.z;
+            float t0x = ((t.nx ? hx : lx) - t.o.x) * t.inv.x;
+            float t1x = ((t.nx ? lx : hx) - t.o.x) * t.inv.x;
+            float t0y = ((t.ny ? hy : ly) - t.o.y) * t.inv.y;
+            float t1y = ((t.ny ? ly : hy) - t.o.y) * t.inv.y;
+            float t0z = ((t.nz ? hz : lz) - t.o.z) * t.inv.z;
+            float t1z = ((t.nz ? lz : hz) - t.o.z) * t.inv.z;
+            child_key(j, fmaxf(fmaxf(t0x, t0y), t0z), fminf(fminf(t1x, t1y), t1z) * inflate);
         }
-        float tmin = fmaxf(fmaxf(t0x, t0y), t0z);
-        float tmax = fminf(fminf(t1x, t1y), t1z) * inflate;
-        // The slab test (tmin <= tmax, tmax > 0, tmin < closest) on te = max(tmin, 0):
-        // the same result (closest > 0), except that a box whose far distance is exactly
-        // 0 counts as hit, which can only add a node to visit.
-        float te = fmaxf(tmin, 0.0f);
-        bool hit = te <= tmax && te < t.closest;
-        key[j] = hit ? ((__float_as_uint(te) & ~7u) | static_cast<uint32_t>(j)) : 0xFFFFFFFFu;
-        h += hit ? 1 : 0;
+    }
+    // Width 4: the 5-comparator network with the child references carried along (instead
+    // of picked by the sorted slots: the path loop's meshes 0.996 -> 0.944 ms), and one
+    // bounds test for all pushes.
+    if (W == 4) {
+        int32_t c[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = __float_as_int(f[6 * W + j % W]);
+        order_pair(key[0], key[1], c[0], c[1]);
+        order_pair(key[2], key[3 % W], c[2], c[3]);
+        order_pair(key[0], key[2], c[0], c[2]);
+        order_pair(key[1], key[3 % W], c[1], c[3]);
+        order_pair(key[1], key[2], c[1], c[2]);
+        if (key[0] == KEY_MISS) return false;
+        const int n = (key[1] != KEY_MISS ? 1 : 0) + (key[2] != KEY_MISS ? 1 : 0) + (key[3 % W] != KEY_MISS ? 1 : 0);
+        const int top = t.sp + n;
+        if (top <= SMEM_STACK) {
+            int2* e = stk.at(top);
+            if (key[1] != KEY_MISS) e[-K::stride] = make_int2(c[1], static_cast<int>(key[1] & ~7u));
+            if (key[2] != KEY_MISS) e[-2 * K::stride] = make_int2(c[2], static_cast<int>(key[2] & ~7u));
+            if (key[3 % W] != KEY_MISS) e[-3 * K::stride] = make_int2(c[3], static_cast<int>(key[3 % W] & ~7u));
+        } else if (top <= MAX_STACK) {
+#pragma unroll
+            for (int j = 3; j >= 1; --j)
+                if (key[j % W] != KEY_MISS) stk.push(top - j, c[j], key[j % W] & ~7u);
+        } else {
+            *err = 1;
+            overflow = true;
+            return false;
+        }
+        t.sp = top;
+        t.ref = c[0];
+        return true;
     }
     if (h == 0) return false;
     sort_keys<W>(key);
@@ -265,7 +337,7 @@ GR_D bool visit_node(const S& s, TravState& t, const StackView& stk, int* err, u
 #pragma unroll
     for (int j = W - 1; j >= 1; --j) {
         if (j < h) {
-            stk.push(t.sp, select_child<W>(f, key[j] & 7u), __uint_as_float(key[j] & ~7u));
+            stk.push(t.sp, select_child<W>(f, key[j] & 7u), key[j] & ~7u);
             ++t.sp;
         }
     }
@@ -299,7 +371,8 @@ GR_D bool visit_leaf(const S& s, TravState& t, int32_t ref, uint32_t* counts) {
 
 // Pops the next stacked child that can still hold a closer hit into t.ref.  Returns
 // false when the stack is exhausted.
-GR_D bool pop_next(TravState& t, const StackView& stk) {
+template <class K>
+GR_D bool pop_next(TravState& t, const K& stk) {
     while (t.sp > 0) {
         --t.sp;
         int32_t r;
@@ -316,8 +389,8 @@ GR_D bool pop_next(TravState& t, const StackView& stk) {
 // One traversal step.  Returns true when the ray is finished (t.hit / t.closest hold
 // the closest hit).  With ANY_HIT it finishes at the first hit closer than t_max.
 // S is DeviceScene or TraceScene: the step functions read only `nodes` and `prims`.
-template <int W, bool ANY_HIT, bool COUNT, class S>
-GR_D bool trav_step(const S& s, TravState& t, const StackView& stk, int* err, uint32_t* counts) {
+template <int W, bool ANY_HIT, bool COUNT, class S, class K>
+GR_D bool trav_step(const S& s, TravState& t, const K& stk, int* err, uint32_t* counts) {
     if (t.ref >= 0) {
         bool overflow = false;
         bool descended = visit_node<W, COUNT>(s, t, stk, err, counts, overflow);
@@ -337,10 +410,11 @@ inline size_t step_stack_smem_bytes(int threads) {
 }
 
 // A thread's traversal stack: its column of the block's shared stack (dynamic shared
-// memory starting at `smem`, step_stack_smem_bytes(blockDim.x) bytes) and its local
+// memory starting at `smem`, step_stack_smem_bytes(STRIDE) bytes, STRIDE = blockDim.x) and its local
 // spill array.
-GR_D StackView thread_stack(unsigned char* smem, int2* spill) {
-    return StackView{reinterpret_cast<int2*>(smem) + threadIdx.x, static_cast<int>(blockDim.x), spill};
+template <int STRIDE>
+GR_D StackView<STRIDE> thread_stack(unsigned char* smem, int2* spill) {
+    return StackView<STRIDE>{reinterpret_cast<int2*>(smem) + threadIdx.x, spill};
 }
 
 // Traces one ray to the end.  ANY_HIT: stops at the first hit closer than t_max (shadow
@@ -349,8 +423,8 @@ GR_D StackView thread_stack(unsigned char* smem, int2* spill) {
 // ray's index there.  A stack overflow (impossible for trees the builds accept) sets
 // *err = 1.  With COUNT, counts[0] / counts[1] accumulate nodes visited / primitives
 // tested.
-template <int W, bool ANY_HIT, bool COUNT = false>
-GR_D TraceResult trace_ray(const DeviceScene& s, V3 o, V3 d, float t_max, const StackView& stk, int* err,
+template <int W, bool ANY_HIT, bool COUNT = false, class K>
+GR_D TraceResult trace_ray(const DeviceScene& s, V3 o, V3 d, float t_max, const K& stk, int* err,
                            int* err_ray = nullptr, uint32_t ray = 0, uint32_t* counts = nullptr) {
     TravState t;
     trav_init(t, o, d, t_max);
@@ -364,5 +438,98 @@ GR_D TraceResult trace_ray(const DeviceScene& s, V3 o, V3 d, float t_max, const 
     }
     return TraceResult{t.closest, t.hit, t.hu, t.hv};
 }
+
+// ---------------------------------------------------------------------------
+// Queue traversal: a warp keeps its lanes busy across rays q = 0 .. n - 1.
+//   grab(k, lane)    the first of the next k rays (a counter shared by the whole grid or
+//                    by the warp alone; rays >= n are not there)
+//   load(q, t)       starts ray q (trav_init), or returns false when nothing is to trace
+//   scene()          this lane's scene: nodes, prims and step budget
+//   store(q, t)      the finished ray: t.hit / t.closest / t.hu / t.hv
+// Each iteration every busy lane that is at a node, or else every one that is at a leaf,
+// takes one traversal step (see EXTEND_LEAVES); once enough lanes are idle, the warp
+// grabs that many rays and hands them to its idle lanes.  So a lane whose ray ended early
+// starts another one, instead of idling until the warp's longest ray ends.  A ray that
+// takes more than its scene's step budget is abandoned as a miss: *err = 2 and, if err_ray
+// is given, its index there.  With ANY_HIT a ray ends at its first hit.
+//
+// Every warp intrinsic runs where control flow is warp-uniform: the loop's iterations are
+// the same for all lanes, the refill condition depends on ballot results and on the
+// grabbed base only, and the loop ends on a ballot.  It terminates: an iteration steps at
+// least one busy lane (each ray has the step budget, and each ray is handed out once), or
+// finds every lane idle, refills and gets rays or learns that none are left.
+//
+// Bound by instruction issue (71-77% active) and the L1 data pipe (54-67%: 112 bytes per
+// lane and node) on camera rays and first bounces, by node-load latency further on.
+template <int W, bool ANY_HIT, bool COUNT, class K, class Grab, class SceneOf, class Load, class Store>
+GR_D void trace_queue(uint32_t n, const K& stk, int* err, int* err_ray, uint32_t* counts, const Grab& grab,
+                      const SceneOf& scene, const Load& load, const Store& store) {
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned below = (1u << lane) - 1u;
+    TravState t;
+    uint32_t q = 0, steps = 0;
+    bool busy = false, exhausted = false;
+    for (;;) {
+        const unsigned idle = __ballot_sync(0xffffffffu, !busy);
+        if (!exhausted && __popc(idle) >= EXTEND_REFILL) {
+            const uint32_t base = grab(static_cast<uint32_t>(__popc(idle)), lane);
+            exhausted = static_cast<uint64_t>(base) + __popc(idle) >= n;
+            if (!busy) {
+                q = base + __popc(idle & below);
+                if (q < n) {
+                    busy = load(q, t);
+                    steps = 0;
+                }
+            }
+        }
+        const bool leaf = busy && t.ref < 0, node = busy && t.ref >= 0;
+        const unsigned leaves = __ballot_sync(0xffffffffu, leaf), nodes = __ballot_sync(0xffffffffu, node);
+        if ((leaves | nodes) == 0u) {  // every lane idle: grab again, or none is left
+            if (exhausted) break;
+            continue;
+        }
+        bool pop = false, done = false;
+        if (nodes == 0u || __popc(leaves) >= EXTEND_LEAVES) {
+            if (leaf) {
+                done = visit_leaf<ANY_HIT, COUNT>(scene(), t, t.ref, counts);
+                pop = !done;
+                ++steps;
+            }
+        } else if (node) {
+            bool overflow = false;
+            pop = !visit_node<W, COUNT>(scene(), t, stk, err, counts, overflow);
+            ++steps;
+            if (overflow) {
+                t.hit = -1;
+                done = true;
+                pop = false;
+            }
+        }
+        if (pop) done = !pop_next(t, stk);
+        if (busy) {
+            if (!done && steps > scene().step_budget) {
+                atomicExch(err, 2);
+                if (err_ray) atomicExch(err_ray, static_cast<int>(q));
+                t.hit = -1;
+                done = true;
+            }
+            if (done) {
+                store(q, t);
+                busy = false;
+            }
+        }
+    }
+}
+
+// Rays handed out from a counter in global memory, zero before the launch: one atomic per
+// refill.
+struct SharedCounter {
+    uint32_t* next;
+    GR_D uint32_t operator()(uint32_t k, unsigned lane) const {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(next, k);
+        return __shfl_sync(0xffffffffu, base, 0);
+    }
+};
 
 }  // namespace gr
