@@ -8,18 +8,18 @@
 //   extend    closest hit (shared with the path tracer)
 //   shade     random_walk (integrators.rs:138-229) for both walks: Material::sample_world,
 //             throughput, shading-normal correction on light paths, roulette from
-//             length rr_len; each vertex is stored SoA, the escape vertex too
-//   order     paths counting-sorted by (camera, light) walk length, so the connection
-//             kernels' warps run loops of equal trip counts
-//   connect   per path, every strategy (c >= 1, l >= 0, c + l <= max) in the reference's
-//             loop order: connect() (integrators.rs:269-343) without the visibility test,
+//             length rr_len; each surface vertex is stored (an escape connects to nothing)
+//   mis       per walk vertex, the part of the MIS weights that no connection changes
+//   order     paths counting-sorted by (camera, light) walk length; the strategies of all
+//             paths laid out as items, all paths of one strategy (c, l) next to each other
+//   connect   per item, connect() (integrators.rs:269-343) without the visibility test,
 //             times its weight; terms that need one queue a shadow ray
 //   light_trace  with light tracing, every light-walk vertex inside the image gets a
-//             camera term (its own kernel)
+//             camera term (its own items and kernel)
 //   shadow    Bvh::visibility (bvh.rs:460-477) as an any-hit query
-//   gather    per path, sums the weighted strategy terms in loop order (deterministic,
-//             same order as the reference); visible light-tracing terms are added to
-//             the film's splat buffer with atomics
+//   gather    per path, sums the weighted strategy terms in the reference's loop order
+//             (deterministic)
+//   splat     visible light-tracing terms are added to the film's splat buffer, with atomics
 //   film      the deterministic splat of film.cu
 #include <algorithm>
 #include <cstdlib>
@@ -39,8 +39,8 @@ constexpr float E_NO_TEST = 0.0f;  // entry flags (float in .w)
 constexpr float E_PENDING = 1.0f;
 constexpr float E_VISIBLE = 2.0f;
 constexpr float E_OCCLUDED = 3.0f;
-constexpr int CNT_ENTRIES = 12;
 constexpr int CNT_SHADOWQ = 13;
+constexpr int CNT_SHADOWF = 14;  // shadow rays handed out
 
 // The pinhole camera seen from the scene (light-tracing and MIS extensions): position,
 // world directions of its x, y, z axes (the camera matrix is a rotation and a
@@ -85,16 +85,20 @@ GR_D float to_area(float pdf, V3 from, V3 to, V3 ng) {
     return pdf * (fabsf(dot(ng, v)) / sqrtf(d2)) / d2;
 }
 
-// Stored vertex (BdptVertex, integrators.rs:107-130) as 8 float4, field-major:
+// Stored vertex (BdptVertex, integrators.rs:107-130) as 8 float4, one 128-byte line: the
+// shading and connection kernels reach vertices in sorted orders, so a vertex is written
+// and read by one thread at a time.
 //   0: point, prim     1: incoming, connectible   2: normal, tp.x   3: tangent, tp.y
 //   4: binormal, tp.z  5: geom_normal, material   6: emission
-//   7: MIS extension: area pdf of the vertex from its predecessor on its walk (afwd) and
-//      from its successor (arev), specular-sample flag
+//   7: MIS extension: while the walks run, area pdf of the vertex from its predecessor on
+//      its walk (afwd) and from its successor (arev), specular-sample flag; after
+//      k_bdpt_mis, the vertex's MisPart
 struct Verts {
     float4* v;
     uint32_t nslots;
+    GR_D uint32_t record(uint32_t k, uint32_t slot) const { return k * nslots + slot; }
     GR_D float4& at(uint32_t k, int f, uint32_t slot) const {
-        return v[(static_cast<size_t>(k) * VREC + f) * nslots + slot];
+        return v[static_cast<size_t>(record(k, slot)) * VREC + f];
     }
 };
 
@@ -278,12 +282,10 @@ __global__ void __launch_bounds__(BSBLOCK, 768 / BSBLOCK) k_bdpt_shade(DeviceSce
                 uint32_t k = vcount[slot];
                 int32_t pk = __float_as_int(h.y);
                 if (pk < 0) {
-                    // As if a black infinite light was hit (integrators.rs:210-225).  The
-                    // throughput at the escape is kept for the environment extension.
-                    Frame z{v3zero(), v3zero(), v3zero(), v3zero()};
-                    store_vertex(vs, k, slot, v3zero(), NO_INDEX, -d, false, z, tp, 0, v3zero());
-                    vs.at(k, 7, slot) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    vcount[slot] = k + 1;
+                    // As if a black infinite light was hit (integrators.rs:210-225).  Such a
+                    // vertex connects to nothing and every term with it is zero, so it is
+                    // not stored or counted.  The throughput at the escape is kept for
+                    // the environment extension.
                     if (walk == 0) {
                         escape[path] = make_float4(tp.x, tp.y, tp.z, 0.0f);
                         flags[path] |= F_ESCAPE;
@@ -345,12 +347,6 @@ __global__ void __launch_bounds__(BSBLOCK, 768 / BSBLOCK) k_bdpt_shade(DeviceSce
 GR_D size_t entry_cap(const BdptParams& p) { return static_cast<size_t>(p.n) * (p.max_len * (p.max_len + 1) / 2); }
 GR_D size_t shadow_cap(const BdptParams& p) { return entry_cap(p) + (p.lt ? static_cast<size_t>(p.n) * p.max_len : 0); }
 
-GR_D uint32_t num_entries(uint32_t cs, uint32_t ls, uint32_t max_len) {
-    uint32_t e = 0;
-    for (uint32_t c = 1; c <= cs; ++c) e += min(ls, max_len - c) + 1;
-    return e;
-}
-
 // ---------------------------------------------------- MIS extension (power heuristic)
 // Veach 1997 eq. 10.9 with beta = 2, in the ratio form of PBRT 3e section 16.3.4: per
 // vertex the area pdfs of generating it along its own walk (afwd) and from the other
@@ -389,38 +385,68 @@ GR_D float remap0(float x) { return x != 0.0f ? x : 1.0f; }
 // loop (each ratio squared and summed unless the vertex or the one before it is a delta
 // vertex) regrouped, so a weight costs O(1) and P advances by one step per vertex.
 // skip0: the camera walk's k = 0 term (the light-tracing strategy) is left out.
-struct WalkMis {
-    VPdf v1{0.0f, 0.0f, false}, v2{0.0f, 0.0f, false}, v3{0.0f, 0.0f, false};  // vertices n-1, n-2, n-3
-    float P = 0.0f;  // P(n - 3)
-    uint32_t n = 0;
-    bool skip0 = false;
-
-    GR_D bool cond_interior(uint32_t k, const VPdf& v, const VPdf& before) const {
-        return !v.delta && !(k >= 1 && before.delta) && !(k == 0 && skip0);
+// What a weight needs of a walk for a connection at vertex n - 1, which depends on the walk
+// alone: one float4 per vertex, made once by k_bdpt_mis.
+struct MisPart {
+    float fwd1, fwd2;  // remap0(afwd) of vertices n - 1 and n - 2
+    float rest;        // [cond(n - 2)] + P(n - 3)
+    float cond1;       // [cond(n - 1)]
+};
+GR_D MisPart load_mis(const Verts& vs, uint32_t k, uint32_t slot) {
+    const float4 f7 = vs.at(k, 7, slot);
+    return MisPart{f7.x, f7.y, f7.z, f7.w};
+}
+// The walk's part for its first n vertices (n >= 1), the connection's reverse pdfs given.
+GR_D float mis_part(const MisPart& m, uint32_t n, float rev1, float rev2) {
+    const float a = remap0(rev1) / m.fwd1;
+    float sum = m.cond1 != 0.0f ? a * a : 0.0f;
+    if (n >= 2) {
+        const float ab = a * (remap0(rev2) / m.fwd2);
+        sum += ab * ab * m.rest;
     }
-    // Moves the connection one vertex out: v is the record of vertex n.
-    GR_D void push(const VPdf& v) {
-        if (n >= 2) {  // vertex n - 2 becomes interior
-            float q = remap0(v2.arev) / remap0(v2.afwd);
-            P = q * q * ((cond_interior(n - 2, v2, v3) ? 1.0f : 0.0f) + P);
+    return sum;
+}
+
+// Turns each vertex's pdf record into its MisPart, one thread per walk.
+__global__ void __launch_bounds__(BLOCK) k_bdpt_mis(BdptParams p, Verts vs, const uint32_t* __restrict__ vcount) {
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot >= p.nslots) return;
+    const uint32_t count = vcount[slot];
+    bool skip0 = false;
+    if ((slot & 1u) == 0u) {
+        bool lt_possible = false;
+        if (p.lt && count > 0) {
+            const float4 f0 = vs.at(0, 0, slot);
+            float ss, tt, dd, cv;
+            lt_possible = p.view.project(V3{f0.x, f0.y, f0.z}, ss, tt, dd, cv);
+        }
+        skip0 = !lt_possible;
+    }
+    auto cond_interior = [&](uint32_t k, const VPdf& v, const VPdf& before) {
+        return !v.delta && !(k >= 1 && before.delta) && !(k == 0 && skip0);
+    };
+    VPdf v1{0.0f, 0.0f, false}, v2 = v1, v3 = v1;  // vertices n - 1, n - 2, n - 3
+    float P = 0.0f;                                // P(n - 3)
+    for (uint32_t n = 1; n <= count; ++n) {
+        const VPdf v = load_pdf(vs, n - 1, slot);
+        if (n >= 3) {  // vertex n - 3 becomes interior
+            const float q = remap0(v2.arev) / remap0(v2.afwd);
+            P = q * q * ((cond_interior(n - 3, v2, v3) ? 1.0f : 0.0f) + P);
         }
         v3 = v2;
         v2 = v1;
         v1 = v;
-        ++n;
-    }
-    GR_D float part(float rev1, float rev2) const {
-        if (n == 0) return 0.0f;
-        float a = remap0(rev1) / remap0(v1.afwd);
-        bool c1 = n == 1 ? !skip0 : !v2.delta;
-        float sum = c1 ? a * a : 0.0f;
-        if (n >= 2) {
-            float ab = a * (remap0(rev2) / remap0(v2.afwd));
-            sum += ab * ab * ((cond_interior(n - 2, v2, v3) ? 1.0f : 0.0f) + P);
+        MisPart m{remap0(v1.afwd), 1.0f, 0.0f, 0.0f};
+        if (n == 1) {
+            m.cond1 = skip0 ? 0.0f : 1.0f;
+        } else {
+            m.cond1 = v2.delta ? 0.0f : 1.0f;
+            m.fwd2 = remap0(v2.afwd);
+            m.rest = (cond_interior(n - 2, v2, v3) ? 1.0f : 0.0f) + P;
         }
-        return sum;
+        vs.at(n - 1, 7, slot) = make_float4(m.fwd1, m.fwd2, m.rest, m.cond1);
     }
-};
+}
 
 struct VPos {
     V3 point, ng;
@@ -467,12 +493,11 @@ static __device__ __noinline__ VEval eval_vertex(const DevMaterial& m, V3 wi, V3
     return e;
 }
 
-// MIS weight of camera strategy (c >= 1, l >= 0) with a non-zero connection; cw and lw
-// stand at c and l vertices.  For l >= 1, ez and ey are the connection's evaluations at
+// MIS weight of camera strategy (c >= 1, l >= 0) with a non-zero connection.  For l >= 1, ez and ey are the connection's evaluations at
 // z (camera side, toward y) and y (light side, toward z; for l = 1 the light's
 // direction pdf in pdf_fwd).
-GR_D float strategy_weight(const DeviceScene& s, const Verts& vs, uint32_t i, const WalkMis& cw, const WalkMis& lw,
-                           uint32_t c, uint32_t l, const Vtx& z, const Vtx* y, const VEval& ez, const VEval& ey) {
+GR_D float strategy_weight(const DeviceScene& s, const Verts& vs, uint32_t i, uint32_t c, uint32_t l, const Vtx& z,
+                           const Vtx* y, const VEval& ez, const VEval& ey) {
     float z_rev = 0.0f, zm_rev = 0.0f, y_rev = 0.0f, ym_rev = 0.0f;
     if (l == 0) {  // the camera walk hit a light
         z_rev = light_point_pdf(s, z.prim);
@@ -492,23 +517,44 @@ GR_D float strategy_weight(const DeviceScene& s, const Verts& vs, uint32_t i, co
             ym_rev = to_area(ey.pdf_rev, y->point, yp.point, yp.ng);
         }
     }
-    return 1.0f / (1.0f + cw.part(z_rev, zm_rev) + lw.part(y_rev, ym_rev));
+    const float camera_part = mis_part(load_mis(vs, c - 1, 2 * i), c, z_rev, zm_rev);
+    const float light_part = l ? mis_part(load_mis(vs, l - 1, 2 * i + 1), l, y_rev, ym_rev) : 0.0f;
+    return 1.0f / (1.0f + camera_part + light_part);
 }
 
-// ------------------------------------------ connection order: paths by walk lengths
-// The connection kernel runs a thread per path through loops over both walks' vertices;
-// paths of equal (camera, light) vertex counts make warps of equal trip counts.  A
-// counting sort of the path indices by that pair (17 x 17 buckets, walks <= 16) gives
-// the order; which thread handles which path changes no result.
-constexpr uint32_t LEN_BUCKETS = 17 * 17;
+// ------------------------------------------------ connection items: paths by strategy
+// Paths are counting-sorted by their (camera, light) vertex counts (17 x 17 buckets, walks
+// <= 16), so the paths with cs camera vertices and at least l light vertices are
+// consecutive: from start[17 cs + l] to start[17 (cs + 1)].  The strategies of all paths
+// are items: item t belongs to a segment (l, c, cs), the paths of exactly cs camera and at
+// least l light vertices doing strategy (c, l), and is the (t - base)-th of that range.
+// Segments of one l and c follow each other, so a warp evaluates one strategy of 32 paths:
+// one connection each, instead of one path each with its own loops over both walks.
+// Light-tracing items are segments (l, cs) in the same way.  Which thread handles which
+// path changes no result.
+constexpr uint32_t LENS = 17;
+constexpr uint32_t LEN_BUCKETS = LENS * LENS;
+constexpr uint32_t MAX_SEGMENTS = 1496;    // sum over c of (17 - c)^2, walks <= 16
+constexpr uint32_t MAX_LT_SEGMENTS = 272;  // 16 x 17
+
+struct Items {
+    uint32_t hist[LEN_BUCKETS];       // paths per bucket, then next free position
+    uint32_t start[LEN_BUCKETS + 1];  // first position of each bucket
+    uint32_t segments, lt_segments;
+    uint32_t base[MAX_SEGMENTS + 1];  // first item per segment, then the number of items
+    uint32_t what[MAX_SEGMENTS];      // (l << 16) | (c << 8) | cs
+    uint32_t at[LENS * LENS * LENS];  // base of segment (l, c, cs)
+    uint32_t lt_base[MAX_LT_SEGMENTS + 1];
+    uint32_t lt_what[MAX_LT_SEGMENTS];  // (l << 8) | cs
+};
 
 GR_D uint32_t len_bucket(const uint32_t* vcount, const uint32_t* flags, uint32_t i) {
     if (flags[i] & F_SKIP) return 0;
-    return min(vcount[2 * i], 16u) * 17u + min(vcount[2 * i + 1], 16u);
+    return min(vcount[2 * i], 16u) * LENS + min(vcount[2 * i + 1], 16u);
 }
 
 __global__ void __launch_bounds__(BLOCK) k_bdpt_len_count(uint32_t n, const uint32_t* __restrict__ vcount,
-                                                          const uint32_t* __restrict__ flags, uint32_t* hist) {
+                                                          const uint32_t* __restrict__ flags, Items* items) {
     __shared__ uint32_t h[LEN_BUCKETS];
     for (uint32_t b = threadIdx.x; b < LEN_BUCKETS; b += blockDim.x) h[b] = 0;
     __syncthreads();
@@ -516,21 +562,94 @@ __global__ void __launch_bounds__(BLOCK) k_bdpt_len_count(uint32_t n, const uint
         atomicAdd(&h[len_bucket(vcount, flags, i)], 1u);
     __syncthreads();
     for (uint32_t b = threadIdx.x; b < LEN_BUCKETS; b += blockDim.x)
-        if (h[b]) atomicAdd(&hist[b], h[b]);
+        if (h[b]) atomicAdd(&items->hist[b], h[b]);
 }
 
-// One thread: bucket counts -> first positions (exclusive prefix sum), in place.
-__global__ void k_bdpt_len_scan(uint32_t* hist) {
-    uint32_t run = 0;
-    for (uint32_t b = 0; b < LEN_BUCKETS; ++b) {
-        uint32_t c = hist[b];
-        hist[b] = run;
-        run += c;
+// Exclusive prefix sum of one value per thread of a PLAN_THREADS-thread block; `total`
+// gets the sum.
+constexpr uint32_t PLAN_THREADS = 512;
+GR_D uint32_t block_scan(uint32_t* sm, uint32_t v, uint32_t& total) {
+    const uint32_t t = threadIdx.x;
+    __syncthreads();  // sm is free
+    sm[t] = v;
+    __syncthreads();
+    for (uint32_t o = 1; o < PLAN_THREADS; o <<= 1) {
+        const uint32_t x = t >= o ? sm[t - o] : 0u;
+        __syncthreads();
+        sm[t] += x;
+        __syncthreads();
+    }
+    total = sm[PLAN_THREADS - 1];
+    return sm[t] - v;
+}
+
+// One block: bucket counts -> first positions, and the segments of the items.
+__global__ void __launch_bounds__(PLAN_THREADS) k_bdpt_items(Items* items, uint32_t max_len, uint32_t lt) {
+    __shared__ uint32_t sm[PLAN_THREADS], start[LEN_BUCKETS + 1];
+    const uint32_t t = threadIdx.x;
+    static_assert(LEN_BUCKETS < PLAN_THREADS, "one bucket per thread");
+    uint32_t total;
+    const uint32_t first = block_scan(sm, t < LEN_BUCKETS ? items->hist[t] : 0u, total);
+    if (t < LEN_BUCKETS) {
+        start[t] = first;
+        items->hist[t] = first;
+        items->start[t] = first;
+    }
+    if (t == 0) {
+        start[LEN_BUCKETS] = total;
+        items->start[LEN_BUCKETS] = total;
+    }
+    __syncthreads();
+    auto paths = [&](uint32_t cs, uint32_t l) { return start[(cs + 1) * LENS] - start[cs * LENS + l]; };
+    // Segments in the order l, c, cs, each thread a run of PER of them.
+    constexpr uint32_t PER = (MAX_SEGMENTS + PLAN_THREADS - 1) / PLAN_THREADS;
+    uint32_t what[PER], size[PER], mine = 0, count = 0;
+    for (uint32_t k = 0; k < PER; ++k) what[k] = size[k] = 0;
+    for (uint32_t l = 0; l < max_len; ++l)
+        for (uint32_t c = 1; c + l <= max_len; ++c) {
+            const uint32_t n = max_len - c + 1;  // cs = c .. max_len
+            for (uint32_t k = 0; k < PER; ++k) {
+                const uint32_t g = t * PER + k;
+                if (g >= count && g < count + n) {
+                    const uint32_t cs = c + (g - count);
+                    what[k] = (l << 16) | (c << 8) | cs;
+                    size[k] = paths(cs, l);
+                    mine += size[k];
+                }
+            }
+            count += n;
+        }
+    uint32_t base = block_scan(sm, mine, total);
+    for (uint32_t k = 0; k < PER; ++k) {
+        const uint32_t g = t * PER + k;
+        if (g >= count) break;
+        items->what[g] = what[k];
+        items->base[g] = base;
+        items->at[((what[k] >> 16) * LENS + ((what[k] >> 8) & 255u)) * LENS + (what[k] & 255u)] = base;
+        base += size[k];
+    }
+    if (t == 0) {
+        items->segments = count;
+        items->base[count] = total;
+    }
+    // Light-tracing segments: l = 1 .. max_len, cs = 0 .. max_len (a camera walk that
+    // escapes at once has no vertex).
+    const uint32_t lt_count = lt ? max_len * (max_len + 1) : 0u;
+    const uint32_t l = t / (max_len + 1) + 1, cs = t % (max_len + 1);
+    const uint32_t n = t < lt_count ? paths(cs, l) : 0u;
+    base = block_scan(sm, n, total);
+    if (t < lt_count) {
+        items->lt_what[t] = (l << 8) | cs;
+        items->lt_base[t] = base;
+    }
+    if (t == 0) {
+        items->lt_segments = lt_count;
+        items->lt_base[lt_count] = total;
     }
 }
 
 __global__ void __launch_bounds__(BLOCK) k_bdpt_len_scatter(uint32_t n, const uint32_t* __restrict__ vcount,
-                                                            const uint32_t* __restrict__ flags, uint32_t* pos,
+                                                            const uint32_t* __restrict__ flags, Items* items,
                                                             uint32_t* __restrict__ order) {
     const unsigned lane = threadIdx.x & 31u;
     for (uint32_t b = blockIdx.x * blockDim.x; b < n; b += gridDim.x * blockDim.x) {
@@ -541,249 +660,244 @@ __global__ void __launch_bounds__(BLOCK) k_bdpt_len_scatter(uint32_t n, const ui
         const unsigned same = __match_any_sync(0xffffffffu, key);
         const int leader = __ffs(same) - 1;
         uint32_t base = 0;
-        if (in && static_cast<int>(lane) == leader) base = atomicAdd(&pos[key], static_cast<uint32_t>(__popc(same)));
+        if (in && static_cast<int>(lane) == leader)
+            base = atomicAdd(&items->hist[key], static_cast<uint32_t>(__popc(same)));
         base = __shfl_sync(0xffffffffu, base, leader);
         if (in) order[base + __popc(same & ((1u << lane) - 1u))] = i;
     }
 }
 
-// connect() for every strategy of one path, in the reference's loop order, each term
-// times its weight (uniform or MIS).
-// Threads per block of the connection kernel (paths are taken in walk-length order, so a
-// larger block keeps more of an SM's warps on paths of equal loop trip counts).  At 160
-// registers, 384 threads is one block per SM; on the 512 x 512 16-spp MIS + light-tracing
-// render 128 / 384 measured 185 / 192 Msamples/s (uniform weights: 315 / 314).
+// The segment of item t: the last one whose base is <= t (empty segments share their base
+// with the next, which is then taken).
+GR_D uint32_t find_segment(const uint32_t* base, uint32_t segments, uint32_t t) {
+    uint32_t lo = 0, hi = segments;
+    while (hi - lo > 1) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if (base[mid] <= t) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// One strategy of one path per thread: connect() without its visibility test, times the
+// strategy's weight (uniform or MIS), into entries[t]; terms that need the test queue a
+// shadow ray.
+// Bound by divergence (the two materials of a connection differ within a warp) and by the
+// instruction fetch of the mixture.  512 x 512 x 16 spp with MIS: one thread per path,
+// looping over its strategies, 4.94 ms; items 3.54 (with field-major vertices replaced by
+// whole lines), without the escapes' vertices 1.62.  Cornell box, 200 x 150 x 4 spp, length
+// 16: 841 -> 164 us.  Sorting chunks of items by the two materials' lobes cost as much as
+// it saved; 3 / 4 / 5 blocks per SM measured the same (9.58 / 9.60 / 9.55 ms per render; 4 has no spills).
 #ifndef GR_CONNECT_BLOCK
-#define GR_CONNECT_BLOCK 384
+#define GR_CONNECT_BLOCK 128
 #endif
 #ifndef GR_CONNECT_MIN_BLOCKS
-#define GR_CONNECT_MIN_BLOCKS 1
+#define GR_CONNECT_MIN_BLOCKS 4
 #endif
-__global__ void __launch_bounds__(GR_CONNECT_BLOCK, GR_CONNECT_MIN_BLOCKS) k_bdpt_connect(DeviceScene s, BdptParams p, Verts vs,
-                                                        const uint32_t* __restrict__ vcount,
-                                                        const uint32_t* __restrict__ flags, uint32_t* counters,
-                                                        uint32_t* __restrict__ entry_base, float4* __restrict__ entries,
-                                                        uint4* __restrict__ shadow_q,
-                                                        const uint32_t* __restrict__ order) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= p.n) return;
-    const uint32_t i = order[t];
-    uint32_t fl = flags[i];
-    if (fl & F_SKIP) return;
-    uint32_t cs = vcount[2 * i], ls = vcount[2 * i + 1];
-    uint32_t ne = num_entries(cs, ls, p.max_len);
-    uint32_t base = ne ? atomicAdd(counters + CNT_ENTRIES, ne) : 0;
-    entry_base[i] = base;
-    bool lt_possible = false;
-    if (p.lt && cs > 0) {
-        VPos z1 = load_pos(vs, 0, 2 * i);
-        float4 f0 = vs.at(0, 0, 2 * i);
-        float ss, tt, dd, cv;
-        lt_possible = __float_as_uint(f0.w) != NO_INDEX && p.view.project(z1.point, ss, tt, dd, cv);
-    }
+__global__ void __launch_bounds__(GR_CONNECT_BLOCK, GR_CONNECT_MIN_BLOCKS)
+    k_bdpt_connect(DeviceScene s, BdptParams p, Verts vs, const Items* __restrict__ items,
+                   const uint32_t* __restrict__ order, uint32_t* counters, float4* __restrict__ entries,
+                   uint4* __restrict__ shadow_q) {
+    __shared__ uint32_t base[MAX_SEGMENTS + 1];
+    const uint32_t segments = items->segments;
+    for (uint32_t k = threadIdx.x; k <= segments; k += blockDim.x) base[k] = items->base[k];
+    __syncthreads();
+    const uint32_t total = base[segments];
     const uint32_t extra = p.lt ? 1u : 0u;
-    uint32_t j = base;
-    WalkMis cw;
-    cw.skip0 = !lt_possible;
-    for (uint32_t c = 1; c <= cs; ++c) {
-        Vtx cv = load_vertex(vs, c - 1, 2 * i);
-        if (p.mis) cw.push(load_pdf(vs, c - 1, 2 * i));
-        WalkMis lw;
-        for (uint32_t l = 0; l <= ls && c + l <= p.max_len; ++l) {
-            V3 term = v3zero();
-            float flag = E_NO_TEST;
-            Vtx lv;
-            VEval ez{v3zero(), 0.0f, 0.0f}, ey{v3zero(), 0.0f, 0.0f};
-            if (l == 0) {
-                if (cv.prim != NO_INDEX) term = mul(cv.tp, cv.emission);
-            } else {
-                lv = load_vertex(vs, l - 1, 2 * i + 1);
-                if (p.mis) lw.push(load_pdf(vs, l - 1, 2 * i + 1));
-                if (cv.prim != NO_INDEX && lv.prim != NO_INDEX && cv.connectible && lv.connectible) {
-                    V3 c2l = normalized(lv.point - cv.point);
-                    V3 l2c = -c2l;  // equals normalized(cv.point - lv.point) bit for bit
-                    const DevMaterial& cm = s.materials[cv.material];
-                    const DevMaterial& lm = s.materials[lv.material];
-                    ez = eval_vertex(cm, cv.incoming, c2l, cv.frame, true, p.mis);
-                    V3 cr = ez.f;
-                    V3 ce;
-                    if (l == 1) {
-                        ce = light_world(lm, l2c, lv.frame);
-                        ey.pdf_fwd = light_dir_pdf(lv.frame, l2c);
-                    } else {
-                        ey = eval_vertex(lm, lv.incoming, l2c, lv.frame, false, p.mis);
-                        ce = ey.f;
-                    }
-                    float g = fabsf(dot(cv.frame.normal, c2l));
-                    float cdn = convert_density(cv.point, lv.point, lv.frame);
-                    term = mul(mul(mul(cv.tp, cr), ce), lv.tp) * (g * cdn);
-                    if (!nearly_zero(term)) {
-                        flag = E_PENDING;
-                        uint32_t sq = agg_inc(counters + CNT_SHADOWQ);
-                        // float4 index of field 0 (point) of each vertex
-                        if (GR_IN_RANGE(sq, shadow_cap(p)))
-                            shadow_q[sq] = make_uint4(j, (c - 1) * VREC * p.nslots + 2 * i,
-                                                      (l - 1) * VREC * p.nslots + 2 * i + 1, 0);
-                    }
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+        const uint32_t g = find_segment(base, segments, t);
+        const uint32_t what = __ldg(&items->what[g]);
+        const uint32_t l = what >> 16, c = (what >> 8) & 255u, cs = what & 255u;
+        const uint32_t i = order[__ldg(&items->start[cs * LENS + l]) + (t - base[g])];
+        V3 term = v3zero();
+        float flag = E_NO_TEST;
+        const Vtx cv = load_vertex(vs, c - 1, 2 * i);
+        Vtx lv;
+        VEval ez{v3zero(), 0.0f, 0.0f}, ey{v3zero(), 0.0f, 0.0f};
+        if (l == 0) {
+            term = mul(cv.tp, cv.emission);
+        } else if (cv.connectible) {
+            lv = load_vertex(vs, l - 1, 2 * i + 1);
+            if (lv.connectible) {
+                V3 c2l = normalized(lv.point - cv.point);
+                V3 l2c = -c2l;  // equals normalized(cv.point - lv.point) bit for bit
+                const DevMaterial& cm = s.materials[cv.material];
+                const DevMaterial& lm = s.materials[lv.material];
+                ez = eval_vertex(cm, cv.incoming, c2l, cv.frame, true, p.mis);
+                V3 cr = ez.f;
+                V3 ce;
+                if (l == 1) {
+                    ce = light_world(lm, l2c, lv.frame);
+                    ey.pdf_fwd = light_dir_pdf(lv.frame, l2c);
+                } else {
+                    ey = eval_vertex(lm, lv.incoming, l2c, lv.frame, false, p.mis);
+                    ce = ey.f;
+                }
+                float gcos = fabsf(dot(cv.frame.normal, c2l));
+                float cdn = convert_density(cv.point, lv.point, lv.frame);
+                term = mul(mul(mul(cv.tp, cr), ce), lv.tp) * (gcos * cdn);
+                if (!nearly_zero(term)) {
+                    flag = E_PENDING;
+                    uint32_t sq = agg_inc(counters + CNT_SHADOWQ);
+                    if (GR_IN_RANGE(sq, shadow_cap(p)))  // the two vertices' records
+                        shadow_q[sq] = make_uint4(t, vs.record(c - 1, 2 * i), vs.record(l - 1, 2 * i + 1), 0);
                 }
             }
-            float w;
-            if (!p.mis) w = 1.0f / static_cast<float>(c + l + extra);  // integrators.rs:345-354
-            else w = is_zero(term) ? 0.0f : strategy_weight(s, vs, i, cw, lw, c, l, cv, l ? &lv : nullptr, ez, ey);
-            term = term * w;
-            if (GR_IN_RANGE(j, entry_cap(p))) entries[j] = make_float4(term.x, term.y, term.z, flag);
-            ++j;
         }
+        float w;
+        if (!p.mis) w = 1.0f / static_cast<float>(c + l + extra);  // integrators.rs:345-354
+        else w = is_zero(term) ? 0.0f : strategy_weight(s, vs, i, c, l, cv, l ? &lv : nullptr, ez, ey);
+        term = term * w;
+        if (GR_IN_RANGE(t, entry_cap(p))) entries[t] = make_float4(term.x, term.y, term.z, flag);
     }
-
 }
 
-// The light-tracing strategy (t = 1, an MIS extension): each light-walk vertex inside
-// the image gets a camera term in lt[i * max_len + l - 1] (value, flag) and its film
-// pixel in lt_pixel.  A kernel of its own, after the connections, so that neither
-// kernel carries the other's code and registers.
+// The light-tracing strategy (t = 1, an MIS extension), one light-walk vertex per thread:
+// inside the image it gets a camera term in lt[t] (value, flag) and its film pixel in
+// lt_pixel[t].
 __global__ void __launch_bounds__(BLOCK) k_bdpt_light_trace(DeviceScene s, BdptParams p, Verts vs,
-                                                            const uint32_t* __restrict__ vcount,
-                                                            const uint32_t* __restrict__ flags, uint32_t* counters,
+                                                            const Items* __restrict__ items,
+                                                            const uint32_t* __restrict__ order, uint32_t* counters,
                                                             uint4* __restrict__ shadow_q, float4* __restrict__ lt,
-                                                            uint32_t* __restrict__ lt_pixel,
-                                                            const uint32_t* __restrict__ order) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= p.n) return;
-    const uint32_t i = order[t];
-    if (flags[i] & F_SKIP) return;
-    const uint32_t ls = vcount[2 * i + 1];
-    // Light tracing: light-walk vertex y -> camera.  We / pdf of a pinhole camera is
-    // 1 / (area cos^3 dist^2) (PBRT 3e section 16.1.1).
-    const uint32_t lmax = min(ls, p.max_len);
-    WalkMis lw;
-    for (uint32_t l = 1; l <= p.max_len; ++l) {
-        size_t e = static_cast<size_t>(i) * p.max_len + (l - 1);
+                                                            uint32_t* __restrict__ lt_pixel) {
+    __shared__ uint32_t base[MAX_LT_SEGMENTS + 1];
+    const uint32_t segments = items->lt_segments;
+    for (uint32_t k = threadIdx.x; k <= segments; k += blockDim.x) base[k] = items->lt_base[k];
+    __syncthreads();
+    const uint32_t total = base[segments];
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+        const uint32_t g = find_segment(base, segments, t);
+        const uint32_t what = __ldg(&items->lt_what[g]);
+        const uint32_t l = what >> 8, cs = what & 255u;
+        const uint32_t i = order[__ldg(&items->start[cs * LENS + l]) + (t - base[g])];
+        // Light-walk vertex y -> camera.  We / pdf of a pinhole camera is
+        // 1 / (area cos^3 dist^2) (PBRT 3e section 16.1.1).
         float4 out = make_float4(0.0f, 0.0f, 0.0f, E_NO_TEST);
         uint32_t pix = 0;
-        if (l <= lmax) {
-            Vtx y = load_vertex(vs, l - 1, 2 * i + 1);
-            if (p.mis) lw.push(load_pdf(vs, l - 1, 2 * i + 1));
-            float ss, tt, dist, cvw;
-            if (y.prim != NO_INDEX && y.connectible && p.view.project(y.point, ss, tt, dist, cvw)) {
-                V3 w_yc = (p.view.pos - y.point) / dist;
-                const DevMaterial& ym = s.materials[y.material];
-                VEval ev{v3zero(), 0.0f, 0.0f};
-                if (l >= 2) ev = eval_vertex(ym, y.incoming, w_yc, y.frame, false, p.mis);
-                V3 F = l == 1 ? light_world(ym, w_yc, y.frame) : ev.f;
-                float g = fabsf(dot(y.frame.normal, w_yc)) / (p.view.area * cvw * cvw * cvw * dist * dist);
-                V3 L = mul(y.tp, F) * g;
-                if (!nearly_zero(L)) {
-                    float w;
-                    if (!p.mis) {
-                        w = 1.0f / static_cast<float>(l + 1);
-                    } else {
-                        float y_rev = to_area(p.view.dir_pdf(cvw), p.view.pos, y.point, y.frame.geom_normal);
-                        float ym_rev = 0.0f;
-                        if (l >= 2) {
-                            VPos yp = load_pos(vs, l - 2, 2 * i + 1);
-                            ym_rev = to_area(ev.pdf_rev, y.point, yp.point, yp.ng);
-                        }
-                        w = 1.0f / (1.0f + lw.part(y_rev, ym_rev));
+        const Vtx y = load_vertex(vs, l - 1, 2 * i + 1);
+        float ss, tt, dist, cvw;
+        if (y.connectible && p.view.project(y.point, ss, tt, dist, cvw)) {
+            V3 w_yc = (p.view.pos - y.point) / dist;
+            const DevMaterial& ym = s.materials[y.material];
+            VEval ev{v3zero(), 0.0f, 0.0f};
+            if (l >= 2) ev = eval_vertex(ym, y.incoming, w_yc, y.frame, false, p.mis);
+            V3 F = l == 1 ? light_world(ym, w_yc, y.frame) : ev.f;
+            float gcos = fabsf(dot(y.frame.normal, w_yc)) / (p.view.area * cvw * cvw * cvw * dist * dist);
+            V3 L = mul(y.tp, F) * gcos;
+            if (!nearly_zero(L)) {
+                float w;
+                if (!p.mis) {
+                    w = 1.0f / static_cast<float>(l + 1);
+                } else {
+                    float y_rev = to_area(p.view.dir_pdf(cvw), p.view.pos, y.point, y.frame.geom_normal);
+                    float ym_rev = 0.0f;
+                    if (l >= 2) {
+                        VPos yp = load_pos(vs, l - 2, 2 * i + 1);
+                        ym_rev = to_area(ev.pdf_rev, y.point, yp.point, yp.ng);
                     }
-                    L = L * w;
-                    uint32_t col = min(p.width - 1, static_cast<uint32_t>(floorf(0.5f * (ss + 1.0f) * p.width)));
-                    uint32_t row = min(p.height - 1, static_cast<uint32_t>(floorf(0.5f * (tt + 1.0f) * p.height)));
-                    pix = row * p.width + col;
-                    out = make_float4(L.x, L.y, L.z, E_PENDING);
-                    uint32_t sq = agg_inc(counters + CNT_SHADOWQ);
-                    if (GR_IN_RANGE(sq, shadow_cap(p)))
-                        shadow_q[sq] = make_uint4(static_cast<uint32_t>(e), (l - 1) * VREC * p.nslots + 2 * i + 1, 0, 1);
+                    w = 1.0f / (1.0f + mis_part(load_mis(vs, l - 1, 2 * i + 1), l, y_rev, ym_rev));
                 }
+                L = L * w;
+                uint32_t col = min(p.width - 1, static_cast<uint32_t>(floorf(0.5f * (ss + 1.0f) * p.width)));
+                uint32_t row = min(p.height - 1, static_cast<uint32_t>(floorf(0.5f * (tt + 1.0f) * p.height)));
+                pix = row * p.width + col;
+                out = make_float4(L.x, L.y, L.z, E_PENDING);
+                uint32_t sq = agg_inc(counters + CNT_SHADOWQ);
+                if (GR_IN_RANGE(sq, shadow_cap(p))) shadow_q[sq] = make_uint4(t, vs.record(l - 1, 2 * i + 1), 0, 1);
             }
         }
-        lt[e] = out;
-        lt_pixel[e] = pix;
+        if (GR_IN_RANGE(t, static_cast<size_t>(p.n) * p.max_len)) {
+            lt[t] = out;
+            lt_pixel[t] = pix;
+        }
     }
 }
 
-// Shadow query entries: (entry, float4 index of vertex a's point, of vertex b's point,
-// kind).  Kind 0 connects two walk vertices (their strategy entry); kind 1 connects the
-// camera to vertex a (a light-tracing entry in lt).
+// Shadow query entries: (entry, record of vertex a, of vertex b, kind).  Kind 0 connects
+// two walk vertices (their strategy entry); kind 1 connects the camera to vertex a (a
+// light-tracing entry in lt).
 template <int W>
-__global__ void __launch_bounds__(BLOCK) k_bdpt_shadow(DeviceScene s, const uint32_t* __restrict__ count,
+__global__ void __launch_bounds__(BLOCK) k_bdpt_shadow(DeviceScene s, uint32_t* counters,
                                                        const uint4* __restrict__ shadow_q, const float4* __restrict__ v0,
                                                        float4* __restrict__ entries, float4* __restrict__ lt,
                                                        float3 cam, int* err, unsigned long long* shadow_rays) {
     extern __shared__ unsigned char smem[];
     int2 spill[MAX_STACK - SMEM_STACK];
     const auto stk = thread_stack<BLOCK>(smem, spill);
-    const uint32_t n = *count;
+    const uint32_t n = counters[CNT_SHADOWQ];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(shadow_rays, static_cast<unsigned long long>(n));
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-        uint4 e = shadow_q[q];
-        V3 a, b;
-        if (e.w == 1) {  // Bvh::visibility(camera, y), as the oracle's light-tracing test
-            float4 y4 = v0[e.y];
-            a = V3{cam.x, cam.y, cam.z};
-            b = V3{y4.x, y4.y, y4.z};
-        } else {
-            float4 a4 = v0[e.y], b4 = v0[e.z];
-            a = V3{a4.x, a4.y, a4.z};
-            b = V3{b4.x, b4.y, b4.z};
-        }
-        bool visible;
-        if (fabsf(a.x - b.x) < 1e-3f && fabsf(a.y - b.y) < 1e-3f && fabsf(a.z - b.z) < 1e-3f) {
-            visible = false;
-        } else {
-            V3 d = normalized(b - a);
-            V3 o = nudge(a, d);
-            float target = magnitude(b - o);
-            TraceResult r = trace_ray<W, true>(s, o, d, target - 1e-3f, stk, err);
-            visible = r.k < 0;
-        }
-        (e.w == 1 ? lt : entries)[e.x].w = visible ? E_VISIBLE : E_OCCLUDED;
-    }
+    uint4 e = make_uint4(0, 0, 0, 0);
+    auto answer = [&](bool visible) { (e.w == 1 ? lt : entries)[e.x].w = visible ? E_VISIBLE : E_OCCLUDED; };
+    trace_queue<W, true, false>(
+        n, stk, err, nullptr, nullptr, SharedCounter{counters + CNT_SHADOWF}, [&]() -> const DeviceScene& { return s; },
+        [&](uint32_t q, TravState& t) {
+            e = shadow_q[q];
+            V3 a, b;
+            if (e.w == 1) {  // Bvh::visibility(camera, y), as the oracle's light-tracing test
+                float4 y4 = v0[static_cast<size_t>(e.y) * VREC];
+                a = V3{cam.x, cam.y, cam.z};
+                b = V3{y4.x, y4.y, y4.z};
+            } else {
+                float4 a4 = v0[static_cast<size_t>(e.y) * VREC], b4 = v0[static_cast<size_t>(e.z) * VREC];
+                a = V3{a4.x, a4.y, a4.z};
+                b = V3{b4.x, b4.y, b4.z};
+            }
+            if (fabsf(a.x - b.x) < 1e-3f && fabsf(a.y - b.y) < 1e-3f && fabsf(a.z - b.z) < 1e-3f) {
+                answer(false);
+                return false;
+            }
+            const V3 d = normalized(b - a);
+            const V3 o = nudge(a, d);
+            trav_init(t, o, d, magnitude(b - o) - 1e-3f);
+            return true;
+        },
+        [&](uint32_t, const TravState& t) { answer(t.hit < 0); });
 }
 
-// Sums each path's weighted strategy terms in loop order; adds visible light-tracing
-// terms to `splat` (atomics; null: dropped, as for per-path sample output).
+// Sums each path's weighted strategy terms in loop order.  Threads take the paths in the
+// items' order, so the entries of one strategy are read consecutively.
 __global__ void __launch_bounds__(BLOCK) k_bdpt_gather(DeviceScene s, BdptParams p,
                                                        const uint32_t* __restrict__ vcount,
                                                        const uint32_t* __restrict__ flags,
                                                        const float4* __restrict__ escape,
-                                                       const uint32_t* __restrict__ entry_base,
-                                                       const float4* __restrict__ entries, float4* __restrict__ L_out,
-                                                       const float4* __restrict__ lt,
-                                                       const uint32_t* __restrict__ lt_pixel, float4* splat) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n) return;
-    uint32_t fl = flags[i];
+                                                       const Items* __restrict__ items,
+                                                       const uint32_t* __restrict__ order,
+                                                       const float4* __restrict__ entries, float4* __restrict__ L_out) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= p.n) return;
+    const uint32_t i = order[t];
+    const uint32_t fl = flags[i];
     V3 light = v3zero();
     if (s.has_env && (fl & F_ESCAPE)) {
         float4 e = escape[i];
         light = light + mul(V3{e.x, e.y, e.z}, V3{s.env[0], s.env[1], s.env[2]});
     }
     if (!(fl & F_SKIP)) {
-        uint32_t cs = vcount[2 * i], ls = vcount[2 * i + 1];
-        uint32_t j = entry_base[i];
+        const uint32_t cs = vcount[2 * i], ls = vcount[2 * i + 1];
         for (uint32_t c = 1; c <= cs; ++c) {
-            for (uint32_t l = 0; l <= ls; ++l) {
-                if (c + l > p.max_len) continue;
-                float4 e = entries[j++];
+            for (uint32_t l = 0; l <= ls && c + l <= p.max_len; ++l) {
+                const uint32_t at = __ldg(&items->at[(l * LENS + c) * LENS + cs]);
+                const float4 e = entries[at + (t - __ldg(&items->start[cs * LENS + l]))];
                 V3 term = (e.w == E_NO_TEST || e.w == E_VISIBLE) ? V3{e.x, e.y, e.z} : v3zero();
                 light = light + term;  // weighted in k_bdpt_connect
             }
         }
-        if (p.lt && splat) {
-            const uint32_t lmax = min(ls, p.max_len);
-            for (uint32_t l = 1; l <= lmax; ++l) {
-                size_t e = static_cast<size_t>(i) * p.max_len + (l - 1);
-                float4 v = lt[e];
-                if (v.w != E_VISIBLE) continue;
-                float* d = reinterpret_cast<float*>(splat + lt_pixel[e]);
-                atomicAdd(d, v.x);
-                atomicAdd(d + 1, v.y);
-                atomicAdd(d + 2, v.z);
-            }
-        }
     }
     L_out[i] = make_float4(light.x, light.y, light.z, 0.0f);
+}
+
+// Adds the visible light-tracing terms to the film's splat buffer.
+__global__ void __launch_bounds__(BLOCK) k_bdpt_splat(const Items* __restrict__ items, const float4* __restrict__ lt,
+                                                      const uint32_t* __restrict__ lt_pixel, float4* splat) {
+    const uint32_t total = items->lt_base[items->lt_segments];
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+        const float4 v = lt[t];
+        if (v.w != E_VISIBLE) continue;
+        float* d = reinterpret_cast<float*>(splat + lt_pixel[t]);
+        atomicAdd(d, v.x);
+        atomicAdd(d + 1, v.y);
+        atomicAdd(d + 2, v.z);
+    }
 }
 
 __global__ void k_bdpt_samples_out(uint32_t n, const float2* __restrict__ st, const float4* __restrict__ L,
@@ -800,14 +914,12 @@ __global__ void k_bdpt_samples_out(uint32_t n, const float2* __restrict__ st, co
 uint32_t max_pairs(uint32_t max_len) { return max_len * (max_len + 1) / 2; }
 
 template <int W>
-gr_status shadow_launch(const DeviceScene& s, uint32_t cap, const uint32_t* count, const uint4* q, const float4* v0,
+gr_status shadow_launch(const DeviceScene& s, uint32_t cap, uint32_t* counters, const uint4* q, const float4* v0,
                         float4* entries, float4* lt, float3 cam, int* err, unsigned long long* shadow_rays,
                         cudaStream_t st) {
     size_t smem = step_stack_smem_bytes(BLOCK);
-    GR_CUDA_TRY(
-        cudaFuncSetAttribute(k_bdpt_shadow<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     int grid = resident_grid(k_bdpt_shadow<W>, smem, cap);
-    k_bdpt_shadow<W><<<grid, BLOCK, smem, st>>>(s, count, q, v0, entries, lt, cam, err, shadow_rays);
+    k_bdpt_shadow<W><<<grid, BLOCK, smem, st>>>(s, counters, q, v0, entries, lt, cam, err, shadow_rays);
     GR_CUDA_TRY(cudaGetLastError());
     return GR_OK;
 }
@@ -817,7 +929,7 @@ gr_status shadow_launch(const DeviceScene& s, uint32_t cap, const uint32_t* coun
 size_t BdptState::bytes_per_path(uint32_t max_len) {
     const size_t pairs = max_pairs(max_len);
     return 2 * (2 * (4 + 16 + 16) + 16 + 16) + 8 + 8 + 16  // queues, hits, throughput; key, st, light
-           + 2 * max_len * VREC * 16 + 2 * 4 + 4 + 16 + 4     // vertices, counts, flags, escape, entry base
+           + 2 * max_len * VREC * 16 + 2 * 4 + 4 + 16         // vertices, counts, flags, escape
            + pairs * 16 + (pairs + max_len) * 16 + max_len * (16 + 4) + 4;  // entries, shadow queue, lt, order
 }
 
@@ -839,14 +951,13 @@ cudaError_t BdptState::ensure(size_t paths, uint32_t max_len) {
     if ((e = vcount.ensure(slots * sizeof(uint32_t))) != cudaSuccess) return e;
     if ((e = flags.ensure(paths * sizeof(uint32_t))) != cudaSuccess) return e;
     if ((e = escape.ensure(paths * sizeof(float4))) != cudaSuccess) return e;
-    if ((e = entry_base.ensure(paths * sizeof(uint32_t))) != cudaSuccess) return e;
     if ((e = entries.ensure(pairs * sizeof(float4))) != cudaSuccess) return e;
     const size_t lt_n = paths * max_len;  // light-tracing terms
     if ((e = shadow.ensure((pairs + lt_n) * sizeof(uint4))) != cudaSuccess) return e;
     if ((e = lt.ensure(lt_n * sizeof(float4))) != cudaSuccess) return e;
     if ((e = lt_pixel.ensure(lt_n * sizeof(uint32_t))) != cudaSuccess) return e;
     if ((e = order.ensure(paths * sizeof(uint32_t))) != cudaSuccess) return e;
-    if ((e = len_hist.ensure(2 * LEN_BUCKETS * sizeof(uint32_t))) != cudaSuccess) return e;
+    if ((e = items.ensure(sizeof(Items))) != cudaSuccess) return e;
     return cudaSuccess;
 }
 
@@ -907,7 +1018,7 @@ gr_status render_bdpt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
         p.first_pass = rp.first_pass + done;
         Verts vs{bs.verts.as<float4>(), p.nslots};
         GR_CUDA_TRY(cudaMemsetAsync(cnt + CNT_QUEUE0, 0, sizeof(uint32_t), st));
-        GR_CUDA_TRY(cudaMemsetAsync(cnt + CNT_ENTRIES, 0, 2 * sizeof(uint32_t), st));
+        GR_CUDA_TRY(cudaMemsetAsync(cnt + CNT_SHADOWQ, 0, 2 * sizeof(uint32_t), st));
         k_bdpt_raygen<<<(p.n + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(
             job.scene, p, vs, bs.vcount.as<uint32_t>(), ps.tp.as<float4>(), bs.flags.as<uint32_t>(),
             ps.key.as<unsigned long long>(), ps.st.as<float2>(), bs.escape.as<float4>(), cnt + CNT_QUEUE0,
@@ -934,44 +1045,55 @@ gr_status render_bdpt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
             GR_CUDA_TRY(cudaGetLastError());
             launches += 2;
         }
+        Items* items = bs.items.as<Items>();
         {
             const int sgrid = static_cast<int>(std::min<uint32_t>((p.n + BLOCK - 1) / BLOCK, 1024u));
-            uint32_t* hist = bs.len_hist.as<uint32_t>();
-            GR_CUDA_TRY(cudaMemsetAsync(hist, 0, LEN_BUCKETS * sizeof(uint32_t), st));
-            k_bdpt_len_count<<<sgrid, BLOCK, 0, st>>>(p.n, bs.vcount.as<uint32_t>(), bs.flags.as<uint32_t>(), hist);
-            k_bdpt_len_scan<<<1, 1, 0, st>>>(hist);
-            k_bdpt_len_scatter<<<sgrid, BLOCK, 0, st>>>(p.n, bs.vcount.as<uint32_t>(), bs.flags.as<uint32_t>(), hist,
+            GR_CUDA_TRY(cudaMemsetAsync(items->hist, 0, sizeof(items->hist), st));
+            k_bdpt_len_count<<<sgrid, BLOCK, 0, st>>>(p.n, bs.vcount.as<uint32_t>(), bs.flags.as<uint32_t>(), items);
+            k_bdpt_items<<<1, PLAN_THREADS, 0, st>>>(items, max_len, p.lt);
+            k_bdpt_len_scatter<<<sgrid, BLOCK, 0, st>>>(p.n, bs.vcount.as<uint32_t>(), bs.flags.as<uint32_t>(), items,
                                                        bs.order.as<uint32_t>());
             GR_CUDA_TRY(cudaGetLastError());
             launches += 3;
         }
-        k_bdpt_connect<<<(p.n + GR_CONNECT_BLOCK - 1) / GR_CONNECT_BLOCK, GR_CONNECT_BLOCK, 0, st>>>(
-            job.scene, p, vs, bs.vcount.as<uint32_t>(), bs.flags.as<uint32_t>(), cnt, bs.entry_base.as<uint32_t>(),
-            bs.entries.as<float4>(), bs.shadow.as<uint4>(), bs.order.as<uint32_t>());
+        if (p.mis) {
+            k_bdpt_mis<<<(p.nslots + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(p, vs, bs.vcount.as<uint32_t>());
+            GR_CUDA_TRY(cudaGetLastError());
+            ++launches;
+        }
+        // The number of items is known on the device only: every resident block, looping.
+        const uint32_t all = p.n * max_pairs(max_len);
+        k_bdpt_connect<<<resident_grid(k_bdpt_connect, 0, all, GR_CONNECT_BLOCK), GR_CONNECT_BLOCK, 0, st>>>(
+            job.scene, p, vs, items, bs.order.as<uint32_t>(), cnt, bs.entries.as<float4>(), bs.shadow.as<uint4>());
         GR_CUDA_TRY(cudaGetLastError());
         if (p.lt) {
-            k_bdpt_light_trace<<<(p.n + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(
-                job.scene, p, vs, bs.vcount.as<uint32_t>(), bs.flags.as<uint32_t>(), cnt, bs.shadow.as<uint4>(),
-                bs.lt.as<float4>(), bs.lt_pixel.as<uint32_t>(), bs.order.as<uint32_t>());
+            k_bdpt_light_trace<<<resident_grid(k_bdpt_light_trace, 0, p.n * max_len), BLOCK, 0, st>>>(
+                job.scene, p, vs, items, bs.order.as<uint32_t>(), cnt, bs.shadow.as<uint4>(), bs.lt.as<float4>(),
+                bs.lt_pixel.as<uint32_t>());
             GR_CUDA_TRY(cudaGetLastError());
             ++launches;
         }
         uint32_t cap = p.n * (max_pairs(max_len) + (p.lt ? max_len : 0u));
         gr_status s2;
         switch (job.scene.width) {
-            case 2: s2 = shadow_launch<2>(job.scene, cap, cnt + CNT_SHADOWQ, bs.shadow.as<uint4>(),
-                                          bs.verts.as<float4>(), bs.entries.as<float4>(), bs.lt.as<float4>(), cam_pos, err, shadow, st); break;
-            case 4: s2 = shadow_launch<4>(job.scene, cap, cnt + CNT_SHADOWQ, bs.shadow.as<uint4>(),
-                                          bs.verts.as<float4>(), bs.entries.as<float4>(), bs.lt.as<float4>(), cam_pos, err, shadow, st); break;
-            default: s2 = shadow_launch<8>(job.scene, cap, cnt + CNT_SHADOWQ, bs.shadow.as<uint4>(),
-                                           bs.verts.as<float4>(), bs.entries.as<float4>(), bs.lt.as<float4>(), cam_pos, err, shadow, st); break;
+            case 2: s2 = shadow_launch<2>(job.scene, cap, cnt, bs.shadow.as<uint4>(), bs.verts.as<float4>(),
+                                          bs.entries.as<float4>(), bs.lt.as<float4>(), cam_pos, err, shadow, st); break;
+            case 4: s2 = shadow_launch<4>(job.scene, cap, cnt, bs.shadow.as<uint4>(), bs.verts.as<float4>(),
+                                          bs.entries.as<float4>(), bs.lt.as<float4>(), cam_pos, err, shadow, st); break;
+            default: s2 = shadow_launch<8>(job.scene, cap, cnt, bs.shadow.as<uint4>(), bs.verts.as<float4>(),
+                                           bs.entries.as<float4>(), bs.lt.as<float4>(), cam_pos, err, shadow, st); break;
         }
         if (s2 != GR_OK) return s2;
         k_bdpt_gather<<<(p.n + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(
-            job.scene, p, bs.vcount.as<uint32_t>(), bs.flags.as<uint32_t>(), bs.escape.as<float4>(),
-            bs.entry_base.as<uint32_t>(), bs.entries.as<float4>(), ps.light.as<float4>(), bs.lt.as<float4>(),
-            bs.lt_pixel.as<uint32_t>(), job.splat);
+            job.scene, p, bs.vcount.as<uint32_t>(), bs.flags.as<uint32_t>(), bs.escape.as<float4>(), items,
+            bs.order.as<uint32_t>(), bs.entries.as<float4>(), ps.light.as<float4>());
         GR_CUDA_TRY(cudaGetLastError());
+        if (p.lt && job.splat) {
+            k_bdpt_splat<<<resident_grid(k_bdpt_splat, 0, p.n * max_len), BLOCK, 0, st>>>(
+                items, bs.lt.as<float4>(), bs.lt_pixel.as<uint32_t>(), job.splat);
+            GR_CUDA_TRY(cudaGetLastError());
+            ++launches;
+        }
         launches += 3;
         if (job.film) {
             DevBuf& fs = device_work().film_sched;

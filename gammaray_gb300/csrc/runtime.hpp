@@ -83,8 +83,8 @@ struct PathState {
 // demand).  Walks are addressed by slot (2 per path: camera, light).
 struct BdptState {
     DevBuf q_slot[2], q_o[2], q_d[2], q_hit, tp, key, st, light;
-    DevBuf verts, vcount, flags, escape, entry_base, entries, shadow, lt, lt_pixel;
-    DevBuf order, len_hist;  // paths ordered by walk lengths for the connection kernel
+    DevBuf verts, vcount, flags, escape, entries, shadow, lt, lt_pixel;
+    DevBuf order, items;  // paths ordered by walk lengths, and their strategies laid out as items
     cudaError_t ensure(size_t paths, uint32_t max_len);
     static size_t bytes_per_path(uint32_t max_len);  // device bytes ensure() needs per path
 };
