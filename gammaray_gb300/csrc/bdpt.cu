@@ -6,10 +6,10 @@
 //   raygen    per path: jitter + camera ray (camera walk, slot 2i) and Bvh::sample_light
 //             + the light vertex (light walk, slot 2i+1), both pushed to one queue
 //   extend    closest hit (shared with the path tracer)
+//   (once few walks are left, or from the start, one launch carries them to their end)
 //   shade     random_walk (integrators.rs:138-229) for both walks: Material::sample_world,
 //             throughput, shading-normal correction on light paths, roulette from
 //             length rr_len; each surface vertex is stored (an escape connects to nothing)
-//   mis       per walk vertex, the part of the MIS weights that no connection changes
 //   order     paths counting-sorted by (camera, light) walk length; the strategies of all
 //             paths laid out as items, all paths of one strategy (c, l) next to each other
 //   connect   per item, connect() (integrators.rs:269-343) without the visibility test,
@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "path_order.cuh"
 #include "runtime.hpp"
 #include "shade_sort.cuh"
 #include "wavefront.cuh"
@@ -67,7 +68,8 @@ struct PinholeView {
 struct BdptParams {
     DevCamera cam;
     PinholeView view;
-    uint32_t width, height, npix, first_pass;
+    PathOrder order;  // which sample a path is
+    uint32_t width, height, first_pass;
     uint64_t seed;
     uint32_t max_len, rr_len;
     uint32_t n;       // paths in this group
@@ -90,9 +92,7 @@ GR_D float to_area(float pdf, V3 from, V3 to, V3 ng) {
 // and read by one thread at a time.
 //   0: point, prim     1: incoming, connectible   2: normal, tp.x   3: tangent, tp.y
 //   4: binormal, tp.z  5: geom_normal, material   6: emission
-//   7: MIS extension: while the walks run, area pdf of the vertex from its predecessor on
-//      its walk (afwd) and from its successor (arev), specular-sample flag; after
-//      k_bdpt_mis, the vertex's MisPart
+//   7: MIS extension: the vertex's MisPart
 struct Verts {
     float4* v;
     uint32_t nslots;
@@ -138,15 +138,6 @@ GR_D void store_vertex(const Verts& vs, uint32_t k, uint32_t slot, V3 point, uin
     vs.at(k, 6, slot) = make_float4(emission.x, emission.y, emission.z, 0.0f);
 }
 
-struct VPdf {
-    float afwd, arev;
-    bool delta;
-};
-GR_D VPdf load_pdf(const Verts& vs, uint32_t k, uint32_t slot) {
-    float4 f7 = vs.at(k, 7, slot);
-    return VPdf{f7.x, f7.y, f7.z != 0.0f};
-}
-
 // Warp-aggregated counter increment for divergent code (the lanes active here).
 GR_D uint32_t agg_inc(uint32_t* ctr) {
     unsigned m = __activemask();
@@ -173,34 +164,141 @@ GR_D float convert_density(V3 prev, V3 next, const Frame& nf) {  // integrators.
     return fabsf(dot(nf.normal, p2n)) / (dist * dist);
 }
 
-__global__ void __launch_bounds__(BLOCK) k_bdpt_raygen(DeviceScene s, BdptParams p, Verts vs,
-                                                       uint32_t* __restrict__ vcount, float4* __restrict__ tp_buf,
-                                                       uint32_t* __restrict__ flags,
-                                                       unsigned long long* __restrict__ key_buf,
-                                                       float2* __restrict__ st_buf, float4* __restrict__ escape,
-                                                       uint32_t* count_out, uint32_t* __restrict__ nslot,
-                                                       float4* __restrict__ no, float4* __restrict__ nd) {
+// What a weight needs of a walk for a connection at its vertex n - 1 (n vertices), given the
+// connection's own reverse pdfs rev1 and rev2 at vertices n - 1 and n - 2:
+//   a = remap0(rev1) / remap0(afwd[n-1]),  b = remap0(rev2) / remap0(afwd[n-2]),
+//   part = [cond(n-1)] a^2 + (a b)^2 ([cond(n-2)] + P(n-3)),
+// where P(m) = q(m)^2 ([cond(m)] + P(m-1)), q(m) = remap0(arev[m]) / remap0(afwd[m]), sums
+// the vertices whose reverse pdfs the connection leaves alone; afwd and arev are the area
+// pdfs of a vertex from its predecessor and from its successor.  This is the chained-ratio
+// loop (each ratio squared and summed unless the vertex or the one before it is a delta
+// vertex) regrouped, so a weight costs O(1).  Everything but rev1 and rev2 depends on the
+// walk alone and is known when vertex n - 1 is made: one float4 per vertex.  The camera
+// walk's k = 0 term (the light-tracing strategy) is left out where that strategy is.
+struct MisPart {
+    float fwd1, fwd2;  // remap0(afwd) of vertices n - 1 and n - 2
+    float rest;        // [cond(n - 2)] + P(n - 3)
+    float cond1;       // [cond(n - 1)]
+};
+GR_D float remap0(float x) { return x != 0.0f ? x : 1.0f; }
+GR_D MisPart load_mis(const Verts& vs, uint32_t k, uint32_t slot) {
+    const float4 f7 = vs.at(k, 7, slot);
+    return MisPart{f7.x, f7.y, f7.z, f7.w};
+}
+GR_D void store_mis(const Verts& vs, uint32_t k, uint32_t slot, const MisPart& m) {
+    vs.at(k, 7, slot) = make_float4(m.fwd1, m.fwd2, m.rest, m.cond1);
+}
+GR_D float mis_part(const MisPart& m, uint32_t n, float rev1, float rev2) {
+    const float a = remap0(rev1) / m.fwd1;
+    float sum = m.cond1 != 0.0f ? a * a : 0.0f;
+    if (n >= 2) {
+        const float ab = a * (remap0(rev2) / m.fwd2);
+        sum += ab * ab * m.rest;
+    }
+    return sum;
+}
+
+// A walk between two vertices.  It travels with its ray in the queue, two float4 per entry
+//   (tp.xyz, pdf) (key low, key high, k, flags)
+// and with the MIS extension two more
+//   (prev.xyz, fwd) (ng.xyz, rest)
+// read where the entry sits and written where the surviving walk is pushed.
+struct Walk {
+    V3 tp;
+    float pdf;      // solid-angle pdf of the walk's next direction (0 after a specular sample)
+    uint64_t key;
+    uint32_t k;     // index of its next vertex
+    uint32_t flags; // MIS extension: W_DELTA, W_SKIP0
+    V3 prev, ng;    // MIS extension: its last vertex and the geometric normal there
+    float fwd;      // remap0(afwd) of its last vertex
+    float rest;     // MisPart::rest of its next vertex
+};
+constexpr uint32_t W_DELTA = 1u;  // the last vertex sampled a specular lobe
+constexpr uint32_t W_SKIP0 = 2u;  // camera walk: no light-tracing strategy reaches its first vertex
+
+template <bool MIS>
+GR_D Walk load_walk(const float4* __restrict__ q_state, size_t q) {
+    const float4* e = q_state + q * (MIS ? 4 : 2);
+    const float4 a = e[0], b = e[1];
+    Walk w;
+    w.tp = V3{a.x, a.y, a.z};
+    w.pdf = a.w;
+    w.key = (static_cast<uint64_t>(__float_as_uint(b.y)) << 32) | __float_as_uint(b.x);
+    w.k = __float_as_uint(b.z);
+    w.flags = __float_as_uint(b.w);
+    w.prev = w.ng = v3zero();
+    w.fwd = w.rest = 0.0f;
+    if (MIS) {
+        const float4 c = e[2], d = e[3];
+        w.prev = V3{c.x, c.y, c.z};
+        w.fwd = c.w;
+        w.ng = V3{d.x, d.y, d.z};
+        w.rest = d.w;
+    }
+    return w;
+}
+
+// Appends this lane's walk and its next ray to a queue with one atomic per warp.  Every lane
+// of the warp must call it.
+template <bool MIS>
+GR_D void push_walk(bool alive, uint32_t* count_out, uint32_t slot, V3 o, V3 d, const Walk& w,
+                    uint32_t* __restrict__ nslot, float4* __restrict__ no, float4* __restrict__ nd,
+                    float4* __restrict__ nstate, uint32_t cap) {
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned m = __ballot_sync(0xffffffffu, alive);
+    if (!m) return;
+    const int leader = __ffs(m) - 1;
+    uint32_t base = 0;
+    if (lane == static_cast<unsigned>(leader)) base = atomicAdd(count_out, static_cast<uint32_t>(__popc(m)));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (alive) {
+        const uint32_t pos = base + __popc(m & ((1u << lane) - 1u));
+        if (!GR_IN_RANGE(pos, cap)) return;
+        nslot[pos] = slot;
+        no[pos] = make_float4(o.x, o.y, o.z, 0.0f);
+        nd[pos] = make_float4(d.x, d.y, d.z, 0.0f);
+        float4* e = nstate + static_cast<size_t>(pos) * (MIS ? 4 : 2);
+        e[0] = make_float4(w.tp.x, w.tp.y, w.tp.z, w.pdf);
+        e[1] = make_float4(__uint_as_float(static_cast<uint32_t>(w.key)),
+                           __uint_as_float(static_cast<uint32_t>(w.key >> 32)), __uint_as_float(w.k),
+                           __uint_as_float(w.flags));
+        if (MIS) {
+            e[2] = make_float4(w.prev.x, w.prev.y, w.prev.z, w.fwd);
+            e[3] = make_float4(w.ng.x, w.ng.y, w.ng.z, w.rest);
+        }
+    }
+}
+
+// Per path: vertex counts of both walks, flags and the throughput at the camera walk's
+// escape (with F_ESCAPE).
+struct PathOut {
+    uint32_t* vcount;
+    uint32_t* flags;
+    float4* escape;
+};
+
+template <bool MIS>
+__global__ void __launch_bounds__(BLOCK) k_bdpt_raygen(DeviceScene s, BdptParams p, Verts vs, PathOut out,
+                                                       float2* __restrict__ st_buf, uint32_t* count_out,
+                                                       uint32_t* __restrict__ nslot, float4* __restrict__ no,
+                                                       float4* __restrict__ nd, float4* __restrict__ nstate) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     bool cam_alive = false, light_alive = false;
     V3 co = v3zero(), cd = v3zero(), lo = v3zero(), ld = v3zero();
+    Walk cw{}, lw{};
     if (i < p.n) {
-        uint32_t pass_local = i / p.npix;
-        uint32_t pixel = i - pass_local * p.npix;
-        uint32_t row = pixel / p.width, col = pixel - (pixel / p.width) * p.width;
-        uint64_t key = path_key(p.seed, p.first_pass + pass_local, pixel);
+        const PathSample ps = path_sample(p.order, i);
+        uint64_t key = path_key(p.seed, p.first_pass + ps.pass, ps.row * p.width + ps.col);
         float s0, t0;
-        film_sample_point(p.width, p.height, row, col, key, s0, t0);
+        film_sample_point(p.width, p.height, ps.row, ps.col, key, s0, t0);
         camera_ray(p.cam, s0, t0, co, cd);
-        key_buf[i] = key;
-        st_buf[i] = make_float2(s0, t0);
-        escape[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        uint32_t fl = 0;
-        vcount[2 * i] = 0;
-        // .w carries the solid-angle pdf of the walk's next direction (MIS extension).
-        float cam_pdf = (p.mis || p.lt) ? p.view.dir_pdf(dot(cd, -p.view.axis[2])) : 0.0f;
-        tp_buf[2 * i] = make_float4(1.0f, 1.0f, 1.0f, cam_pdf);
+        st_buf[ps.slot] = make_float2(s0, t0);
+        uint32_t fl = 0, light_vertices = 0;
+        cw.tp = v3one();
+        cw.pdf = MIS ? p.view.dir_pdf(dot(cd, -p.view.axis[2])) : 0.0f;
+        cw.key = lw.key = key;
+        cw.prev = p.view.pos;
         cam_alive = p.max_len > 0;
-        vcount[2 * i + 1] = 0;
         if (s.num_lights > 0) {
             float u[6];
             for (int k = 0; k < 6; ++k) u[k] = uniform01(key, DIM_LIGHT_SAMPLE + k);
@@ -214,18 +312,106 @@ __global__ void __launch_bounds__(BLOCK) k_bdpt_raygen(DeviceScene s, BdptParams
                         (fabsf(dot(ls.frame.geom_normal, ls.direction)) / (ls.point_pdf * ls.dir_pdf));
                 store_vertex(vs, 0, 2 * i + 1, ls.origin, ls.prim, v3zero(), true, ls.frame, v3one() / ls.point_pdf,
                              mi, v3zero());
-                vs.at(0, 7, 2 * i + 1) = make_float4(ls.point_pdf, 0.0f, 0.0f, 0.0f);
-                vcount[2 * i + 1] = 1;
-                tp_buf[2 * i + 1] = make_float4(ie.x, ie.y, ie.z, ls.dir_pdf);
+                light_vertices = 1;
+                lw.tp = ie;
+                lw.pdf = ls.dir_pdf;
+                lw.k = 1;
+                if (MIS) {
+                    lw.fwd = remap0(ls.point_pdf);
+                    store_mis(vs, 0, 2 * i + 1, MisPart{lw.fwd, 1.0f, 0.0f, 1.0f});
+                    lw.prev = ls.origin;
+                    lw.ng = ls.frame.geom_normal;
+                    lw.rest = 1.0f;
+                }
                 light_alive = !is_zero(ie) && 1 < p.max_len;
                 lo = nudge(ls.origin, ls.direction);
                 ld = ls.direction;
             }
         }
-        flags[i] = fl;
+        out.vcount[2 * i] = 0;
+        out.vcount[2 * i + 1] = light_vertices;
+        out.flags[i] = fl;
     }
-    push_warp(cam_alive, count_out, 2 * i, co, cd, nslot, no, nd, p.nslots);
-    push_warp(light_alive, count_out, 2 * i + 1, lo, ld, nslot, no, nd, p.nslots);
+    push_walk<MIS>(cam_alive, count_out, 2 * i, co, cd, cw, nslot, no, nd, nstate, p.nslots);
+    push_walk<MIS>(light_alive, count_out, 2 * i + 1, lo, ld, lw, nslot, no, nd, nstate, p.nslots);
+}
+
+// One vertex of random_walk (integrators.rs:138-229) at the hit h = (t, leaf-order primitive
+// or -1, u, v) of walk `slot`'s ray (o, d): stores the vertex and advances w.  Returns
+// whether the walk goes on, with its next ray; a walk that ends leaves its vertex count.
+template <bool MIS>
+GR_D bool walk_vertex(const DeviceScene& s, const BdptParams& p, const Verts& vs, const PathOut& out, uint32_t slot,
+                      Walk& w, V3 o, V3 d, float4 h, V3& new_o, V3& new_d) {
+    const uint32_t walk = slot & 1u, path = slot >> 1, k = w.k;
+    const bool c2l = walk == 0;
+    const int32_t pk = __float_as_int(h.y);
+    if (pk < 0) {
+        // As if a black infinite light was hit (integrators.rs:210-225).  Such a vertex
+        // connects to nothing and every term with it is zero, so it is not stored or
+        // counted.  The throughput at the escape is kept for the environment extension.
+        if (walk == 0) {
+            out.escape[path] = make_float4(w.tp.x, w.tp.y, w.tp.z, 0.0f);
+            out.flags[path] |= F_ESCAPE;
+        }
+        out.vcount[slot] = k;
+        return false;
+    }
+    uint32_t prim;
+    Frame f = hit_frame(s, pk, o, d, h.x, h.z, h.w, prim);
+    uint32_t mi = __ldg(s.prim_material + prim);
+    const DevMaterial& m = s.materials[mi];
+    uint32_t base = (walk ? DIM_LIGHT_WALK : DIM_CAMERA_WALK) + 4 * k;
+    V3 incoming = -d;
+    V3 hit_point = o + (d * h.x);
+    MaterialSample ms = sample_world(m, incoming, f, c2l, uniform01(w.key, base), uniform01(w.key, base + 1),
+                                     uniform01(w.key, base + 2));
+    bool connectible = count_lobes(m, LOBE_DIFFUSE | LOBE_GLOSSY) != 0;
+    V3 ntp = mul(w.tp, ms.radiance * (fabsf(dot(f.normal, ms.outgoing)) / ms.pdf));
+    ntp = ntp * correct_shading_normal(incoming, ms.outgoing, f, c2l);
+    store_vertex(vs, k, slot, hit_point, prim, incoming, connectible, f, w.tp, mi, ms.emission);
+    const bool delta = (ms.kind & LOBE_SPECULAR) != 0;
+    if (MIS) {
+        // Area pdf of this vertex from its predecessor, and of the predecessor from this
+        // vertex (reverse BSDF pdf; zero after a specular sample, PBRT 3e section 16.3.2).
+        MisPart part;
+        part.fwd1 = remap0(to_area(w.pdf, w.prev, hit_point, f.geom_normal));
+        float P = 0.0f;  // P(k - 1), which the next vertex's part needs
+        if (k == 0) {  // of a camera walk
+            float ss, tt, dd, cv;
+            if (!(p.lt && p.view.project(hit_point, ss, tt, dd, cv))) w.flags |= W_SKIP0;
+            part.fwd2 = 1.0f;
+            part.rest = 0.0f;
+            part.cond1 = w.flags & W_SKIP0 ? 0.0f : 1.0f;
+        } else {
+            part.fwd2 = w.fwd;
+            part.rest = w.rest;
+            part.cond1 = w.flags & W_DELTA ? 0.0f : 1.0f;
+            const float rev = delta ? 0.0f : pdf_world(m, ms.outgoing, incoming, f);
+            const float q = remap0(to_area(rev, hit_point, w.prev, w.ng)) / w.fwd;
+            P = q * q * w.rest;
+        }
+        store_mis(vs, k, slot, part);
+        const bool before_delta = k >= 1 && (w.flags & W_DELTA);
+        const bool cond = !delta && !before_delta && !(k == 0 && (w.flags & W_SKIP0));
+        w.rest = (cond ? 1.0f : 0.0f) + P;
+        w.fwd = part.fwd1;
+        w.prev = hit_point;
+        w.ng = f.geom_normal;
+        w.flags = (w.flags & ~W_DELTA) | (delta ? W_DELTA : 0u);
+    }
+    if (k + 1 >= p.rr_len || nearly_zero(ntp)) {
+        float rv = uniform01(w.key, base + 3);
+        float prob = clamped_lerp(0.25f, 0.75f, luminance(ntp));
+        ntp = rv < prob ? ntp / prob : v3zero();
+    }
+    const bool alive = !is_zero(ntp) && k + 1 < p.max_len;
+    new_o = nudge(hit_point, ms.outgoing);
+    new_d = ms.outgoing;
+    w.tp = ntp;
+    w.pdf = delta ? 0.0f : ms.pdf;
+    w.k = k + 1;
+    if (!alive) out.vcount[slot] = k + 1;
+    return alive;
 }
 
 // BDPT walk shading in blocks of GR_BDPT_SHADE_BLOCK threads (128 or 768), each sorting its
@@ -238,16 +424,13 @@ constexpr int BSBLOCK = GR_BDPT_SHADE_BLOCK;
 static_assert(BSBLOCK == 128 || BSBLOCK == 768, "BDPT shading block of 128 or 768 threads");
 constexpr uint32_t BSHADE_PER_THREAD = BSBLOCK == 128 ? SHADE_PER_THREAD : SHADE_BIG_PER;
 
-__global__ void __launch_bounds__(BSBLOCK, 768 / BSBLOCK) k_bdpt_shade(DeviceScene s, BdptParams p, Verts vs,
-                                                      const uint32_t* __restrict__ count_in,
-                                                      const uint32_t* __restrict__ q_slot,
-                                                      const float4* __restrict__ q_o, const float4* __restrict__ q_d,
-                                                      const float4* __restrict__ q_hit, uint32_t* __restrict__ vcount,
-                                                      float4* __restrict__ tp_buf,
-                                                      const unsigned long long* __restrict__ key_buf,
-                                                      uint32_t* __restrict__ flags, float4* __restrict__ escape,
-                                                      uint32_t* count_out, uint32_t* __restrict__ nslot,
-                                                      float4* __restrict__ no, float4* __restrict__ nd) {
+template <bool MIS>
+__global__ void __launch_bounds__(BSBLOCK, 768 / BSBLOCK)
+    k_bdpt_shade(DeviceScene s, BdptParams p, Verts vs, PathOut out, const uint32_t* __restrict__ count_in,
+                 const uint32_t* __restrict__ q_slot, const float4* __restrict__ q_o, const float4* __restrict__ q_d,
+                 const float4* __restrict__ q_hit, const float4* __restrict__ q_state, uint32_t* count_out,
+                 uint32_t* __restrict__ nslot, float4* __restrict__ no, float4* __restrict__ nd,
+                 float4* __restrict__ nstate) {
     extern __shared__ unsigned char dsmem[];
     const SortView sm = sort_view<BSBLOCK, BSHADE_PER_THREAD>(dsmem);
     const uint32_t n = *count_in;
@@ -258,88 +441,58 @@ __global__ void __launch_bounds__(BSBLOCK, 768 / BSBLOCK) k_bdpt_shade(DeviceSce
     for (uint32_t c0 = blockIdx.x * chunk; c0 < n; c0 += gridDim.x * chunk) {
         const uint32_t cn = min(chunk, n - c0);
         sort_chunk<BSBLOCK, BSHADE_PER_THREAD>(sm, cn, per, [&](uint32_t i) {
-            uint32_t q = c0 + i;
-            uint32_t sl = q_slot[q];
-            uint32_t w = sl & 1u;
-            uint32_t dim = (w ? DIM_LIGHT_WALK : DIM_CAMERA_WALK) + 4 * vcount[sl];
-            return shade_bucket(s, __float_as_int(q_hit[q].y), uniform01(key_buf[sl >> 1], dim), w);
+            const uint32_t q = c0 + i;
+            const uint32_t w = q_slot[q] & 1u;
+            const float4 b = q_state[static_cast<size_t>(q) * (MIS ? 4 : 2) + 1];
+            const uint64_t key = (static_cast<uint64_t>(__float_as_uint(b.y)) << 32) | __float_as_uint(b.x);
+            const uint32_t dim = (w ? DIM_LIGHT_WALK : DIM_CAMERA_WALK) + 4 * __float_as_uint(b.z);
+            return shade_bucket(s, __float_as_int(q_hit[q].y), uniform01(key, dim), w);
         });
         for (uint32_t e = 0; e < per; ++e) {
             uint32_t i = e * BSBLOCK + threadIdx.x;
             bool alive = false;
             uint32_t slot = 0;
             V3 new_o = v3zero(), new_d = v3zero();
+            Walk w{};
             if (i < cn) {
                 uint32_t q = c0 + sm.order[i];
                 slot = q_slot[q];
-                const uint32_t walk = slot & 1u, path = slot >> 1;
-                const bool c2l = walk == 0;
-                float4 h = q_hit[q];
-                float4 o4 = q_o[q], d4 = q_d[q];
-                V3 o = V3{o4.x, o4.y, o4.z}, d = V3{d4.x, d4.y, d4.z};
-                float4 t4 = tp_buf[slot];
-                V3 tp = V3{t4.x, t4.y, t4.z};
-                uint32_t k = vcount[slot];
-                int32_t pk = __float_as_int(h.y);
-                if (pk < 0) {
-                    // As if a black infinite light was hit (integrators.rs:210-225).  Such a
-                    // vertex connects to nothing and every term with it is zero, so it is
-                    // not stored or counted.  The throughput at the escape is kept for
-                    // the environment extension.
-                    if (walk == 0) {
-                        escape[path] = make_float4(tp.x, tp.y, tp.z, 0.0f);
-                        flags[path] |= F_ESCAPE;
-                    }
-                } else {
-                    uint32_t prim;
-                    Frame f = hit_frame(s, pk, o, d, h.x, h.z, h.w, prim);
-                    uint32_t mi = __ldg(s.prim_material + prim);
-                    const DevMaterial& m = s.materials[mi];
-                    uint64_t key = key_buf[path];
-                    uint32_t base = (walk ? DIM_LIGHT_WALK : DIM_CAMERA_WALK) + 4 * k;
-                    V3 incoming = -d;
-                    V3 hit_point = o + (d * h.x);
-                    MaterialSample ms = sample_world(m, incoming, f, c2l, uniform01(key, base), uniform01(key, base + 1),
-                                                     uniform01(key, base + 2));
-                    bool connectible = count_lobes(m, LOBE_DIFFUSE | LOBE_GLOSSY) != 0;
-                    V3 ntp = mul(tp, ms.radiance * (fabsf(dot(f.normal, ms.outgoing)) / ms.pdf));
-                    ntp = ntp * correct_shading_normal(incoming, ms.outgoing, f, c2l);
-                    store_vertex(vs, k, slot, hit_point, prim, incoming, connectible, f, tp, mi, ms.emission);
-                    const bool delta = (ms.kind & LOBE_SPECULAR) != 0;
-                    if (p.mis || p.lt) {
-                        // Area pdfs (MIS extension): this vertex from its predecessor, and the
-                        // predecessor from this vertex (reverse BSDF pdf; zero after a
-                        // specular sample, PBRT 3e section 16.3.2).
-                        const bool has_prev = walk == 1 || k > 0;
-                        V3 prev = p.view.pos;
-                        if (has_prev) {
-                            float4 pp = vs.at(k - 1, 0, slot);
-                            prev = V3{pp.x, pp.y, pp.z};
-                        }
-                        float afwd = to_area(t4.w, prev, hit_point, f.geom_normal);
-                        vs.at(k, 7, slot) = make_float4(afwd, 0.0f, delta ? 1.0f : 0.0f, 0.0f);
-                        if (has_prev) {
-                            float4 pn = vs.at(k - 1, 5, slot);
-                            float rev = delta ? 0.0f : pdf_world(m, ms.outgoing, incoming, f);
-                            vs.at(k - 1, 7, slot).y = to_area(rev, hit_point, prev, V3{pn.x, pn.y, pn.z});
-                        }
-                    }
-                    vcount[slot] = k + 1;
-                    if (k + 1 >= p.rr_len || nearly_zero(ntp)) {
-                        float rv = uniform01(key, base + 3);
-                        float prob = clamped_lerp(0.25f, 0.75f, luminance(ntp));
-                        ntp = rv < prob ? ntp / prob : v3zero();
-                    }
-                    alive = !is_zero(ntp) && k + 1 < p.max_len;
-                    new_o = nudge(hit_point, ms.outgoing);
-                    new_d = ms.outgoing;
-                    if (alive) tp_buf[slot] = make_float4(ntp.x, ntp.y, ntp.z, delta ? 0.0f : ms.pdf);
-                }
+                const float4 o4 = q_o[q], d4 = q_d[q];
+                w = load_walk<MIS>(q_state, q);
+                alive = walk_vertex<MIS>(s, p, vs, out, slot, w, V3{o4.x, o4.y, o4.z}, V3{d4.x, d4.y, d4.z}, q_hit[q],
+                                         new_o, new_d);
             }
-            push_warp(alive, count_out, slot, new_o, new_d, nslot, no, nd, p.nslots);
+            push_walk<MIS>(alive, count_out, slot, new_o, new_d, w, nslot, no, nd, nstate, p.nslots);
         }
         __syncthreads();  // sm is reused by the next chunk
     }
+}
+
+// Carries a queue's walks to their end (run_paths, wavefront.cuh).
+template <int W, bool MIS>
+__global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
+    k_bdpt_walks(DeviceScene s, BdptParams p, Verts vs, PathOut out, const uint32_t* __restrict__ count,
+                 const uint32_t* __restrict__ q_slot, const float4* __restrict__ q_o, const float4* __restrict__ q_d,
+                 const float4* __restrict__ q_state, uint32_t lanes, uint32_t* fetch, int* err,
+                 unsigned long long* rays) {
+    extern __shared__ unsigned char smem[];
+    int2 spill[MAX_STACK - SMEM_STACK];
+    const auto stk = thread_stack<BLOCK>(smem, spill);
+    uint32_t slot = 0;
+    Walk w{};
+    auto take = [&](uint32_t q, V3& o, V3& d) {
+        slot = q_slot[q];
+        const float4 o4 = q_o[q], d4 = q_d[q];
+        o = V3{o4.x, o4.y, o4.z};
+        d = V3{d4.x, d4.y, d4.z};
+        w = load_walk<MIS>(q_state, q);
+        return true;
+    };
+    auto shade = [&](uint32_t, const TravState& t, V3& no, V3& nd) {
+        const float4 h = make_float4(t.closest, __int_as_float(t.hit), t.hu, t.hv);
+        return walk_vertex<MIS>(s, p, vs, out, slot, w, t.o, t.d, h, no, nd);
+    };
+    count_rays(run_paths<W>(s, stk, *count, lanes, fetch, err, take, shade), rays);
 }
 
 // Capacities of the strategy entries and of the shadow queue, as BdptState::ensure sizes
@@ -354,7 +507,7 @@ GR_D size_t shadow_cap(const BdptParams& p) { return entry_cap(p) + (p.lt ? stat
 // connection, delta (specular) vertices skipped and zero pdfs counted as 1.  The
 // strategies are (c camera-walk, l light-walk vertices), c + l <= max_len, and with
 // light tracing also c = 0.  The oracle states the same weight as a loop over the
-// strategies (orender.hpp, mis_weight); WalkMis below regroups it.
+// strategies (orender.hpp, mis_weight); MisPart regroups it.
 
 // Area pdf with which Bvh::sample_light picks a point of light prim `prim`
 // (bvh.rs:481-496, mesh.rs:310-327, sphere.rs:103-111).
@@ -372,80 +525,6 @@ GR_D float light_point_pdf(const DeviceScene& s, uint32_t prim) {
 GR_D float light_dir_pdf(const Frame& f, V3 w) {
     float c = dot(f.geom_normal, w);
     return c > 0.0f ? c * FRAC_1_PI : 0.0f;
-}
-
-GR_D float remap0(float x) { return x != 0.0f ? x : 1.0f; }
-
-// One walk's part of the MIS sum for a connection at its vertex n - 1.  With the
-// connection's reverse pdfs rev1 (vertex n - 1) and rev2 (vertex n - 2),
-//   a = remap0(rev1) / remap0(afwd[n-1]),  b = remap0(rev2) / remap0(afwd[n-2]),
-//   part = [cond(n-1)] a^2 + (a b)^2 ([cond(n-2)] + P(n-3)),
-// where P(m) = q(m)^2 ([cond(m)] + P(m-1)), q(m) = remap0(arev[m]) / remap0(afwd[m]), sums
-// the vertices whose reverse pdfs the connection leaves alone.  This is the chained-ratio
-// loop (each ratio squared and summed unless the vertex or the one before it is a delta
-// vertex) regrouped, so a weight costs O(1) and P advances by one step per vertex.
-// skip0: the camera walk's k = 0 term (the light-tracing strategy) is left out.
-// What a weight needs of a walk for a connection at vertex n - 1, which depends on the walk
-// alone: one float4 per vertex, made once by k_bdpt_mis.
-struct MisPart {
-    float fwd1, fwd2;  // remap0(afwd) of vertices n - 1 and n - 2
-    float rest;        // [cond(n - 2)] + P(n - 3)
-    float cond1;       // [cond(n - 1)]
-};
-GR_D MisPart load_mis(const Verts& vs, uint32_t k, uint32_t slot) {
-    const float4 f7 = vs.at(k, 7, slot);
-    return MisPart{f7.x, f7.y, f7.z, f7.w};
-}
-// The walk's part for its first n vertices (n >= 1), the connection's reverse pdfs given.
-GR_D float mis_part(const MisPart& m, uint32_t n, float rev1, float rev2) {
-    const float a = remap0(rev1) / m.fwd1;
-    float sum = m.cond1 != 0.0f ? a * a : 0.0f;
-    if (n >= 2) {
-        const float ab = a * (remap0(rev2) / m.fwd2);
-        sum += ab * ab * m.rest;
-    }
-    return sum;
-}
-
-// Turns each vertex's pdf record into its MisPart, one thread per walk.
-__global__ void __launch_bounds__(BLOCK) k_bdpt_mis(BdptParams p, Verts vs, const uint32_t* __restrict__ vcount) {
-    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= p.nslots) return;
-    const uint32_t count = vcount[slot];
-    bool skip0 = false;
-    if ((slot & 1u) == 0u) {
-        bool lt_possible = false;
-        if (p.lt && count > 0) {
-            const float4 f0 = vs.at(0, 0, slot);
-            float ss, tt, dd, cv;
-            lt_possible = p.view.project(V3{f0.x, f0.y, f0.z}, ss, tt, dd, cv);
-        }
-        skip0 = !lt_possible;
-    }
-    auto cond_interior = [&](uint32_t k, const VPdf& v, const VPdf& before) {
-        return !v.delta && !(k >= 1 && before.delta) && !(k == 0 && skip0);
-    };
-    VPdf v1{0.0f, 0.0f, false}, v2 = v1, v3 = v1;  // vertices n - 1, n - 2, n - 3
-    float P = 0.0f;                                // P(n - 3)
-    for (uint32_t n = 1; n <= count; ++n) {
-        const VPdf v = load_pdf(vs, n - 1, slot);
-        if (n >= 3) {  // vertex n - 3 becomes interior
-            const float q = remap0(v2.arev) / remap0(v2.afwd);
-            P = q * q * ((cond_interior(n - 3, v2, v3) ? 1.0f : 0.0f) + P);
-        }
-        v3 = v2;
-        v2 = v1;
-        v1 = v;
-        MisPart m{remap0(v1.afwd), 1.0f, 0.0f, 0.0f};
-        if (n == 1) {
-            m.cond1 = skip0 ? 0.0f : 1.0f;
-        } else {
-            m.cond1 = v2.delta ? 0.0f : 1.0f;
-            m.fwd2 = remap0(v2.afwd);
-            m.rest = (cond_interior(n - 2, v2, v3) ? 1.0f : 0.0f) + P;
-        }
-        vs.at(n - 1, 7, slot) = make_float4(m.fwd1, m.fwd2, m.rest, m.cond1);
-    }
 }
 
 struct VPos {
@@ -883,7 +962,7 @@ __global__ void __launch_bounds__(BLOCK) k_bdpt_gather(DeviceScene s, BdptParams
             }
         }
     }
-    L_out[i] = make_float4(light.x, light.y, light.z, 0.0f);
+    L_out[path_sample(p.order, i).slot] = make_float4(light.x, light.y, light.z, 0.0f);
 }
 
 // Adds the visible light-tracing terms to the film's splat buffer.
@@ -924,11 +1003,76 @@ gr_status shadow_launch(const DeviceScene& s, uint32_t cap, uint32_t* counters, 
     return GR_OK;
 }
 
+template <int W, bool MIS>
+gr_status walks_launch(const DeviceScene& s, const BdptParams& p, const Verts& vs, const PathOut& out, uint32_t most,
+                       BdptState& bs, int cur, uint32_t* cnt, int* err, unsigned long long* rays, cudaStream_t st) {
+    const size_t smem = step_stack_smem_bytes(BLOCK);
+    uint32_t lanes = 0;
+    const int grid = path_loop_grid(k_bdpt_walks<W, MIS>, smem, most, lanes);
+    k_bdpt_walks<W, MIS><<<grid, BLOCK, smem, st>>>(s, p, vs, out, cnt + cur, bs.q_slot[cur].as<uint32_t>(),
+                                                    bs.q_o[cur].as<float4>(), bs.q_d[cur].as<float4>(),
+                                                    bs.q_state[cur].as<float4>(), lanes, cnt + CNT_FETCH, err, rays);
+    GR_CUDA_TRY(cudaGetLastError());
+    return GR_OK;
+}
+
+// Both walks of a group's paths: raygen, then bounce by bounce; once at most PATH_LOOP_MAX
+// walks are left (as the host reads two bounces behind), one launch carries them to their
+// end: Cornell box, 200 x 150 x 4 spp, length 16, 636 us of extension and shading -> 404.
+template <bool MIS>
+gr_status run_walks(const DeviceScene& s, const BdptParams& p, const Verts& vs, BdptState& bs, uint32_t* cnt, int* err,
+                    unsigned long long* rays, uint64_t& launches, cudaStream_t st) {
+    const PathOut out{bs.vcount.as<uint32_t>(), bs.flags.as<uint32_t>(), bs.escape.as<float4>()};
+    BounceReadback& rb = device_work().readback;  // the caller holds device_work().mu
+    GR_CUDA_TRY(rb.ensure());
+    k_bdpt_raygen<MIS><<<(p.n + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(
+        s, p, vs, out, bs.st.as<float2>(), cnt + CNT_QUEUE0, bs.q_slot[0].as<uint32_t>(), bs.q_o[0].as<float4>(),
+        bs.q_d[0].as<float4>(), bs.q_state[0].as<float4>());
+    GR_CUDA_TRY(cudaGetLastError());
+    ++launches;
+    uint32_t bound = p.nslots;  // an upper bound of the current queue length
+    // Every walk ends within max_len bounces (one vertex per bounce).
+    for (uint32_t depth = 0; depth < p.max_len; ++depth) {
+        const int cur = depth & 1, nxt = cur ^ 1;
+        if (bound <= PATH_LOOP_MAX) {
+            GR_CUDA_TRY(cudaMemsetAsync(cnt + CNT_FETCH, 0, sizeof(uint32_t), st));
+            switch (s.width) {
+                case 2: GR_TRY_S((walks_launch<2, MIS>(s, p, vs, out, bound, bs, cur, cnt, err, rays, st))); break;
+                case 4: GR_TRY_S((walks_launch<4, MIS>(s, p, vs, out, bound, bs, cur, cnt, err, rays, st))); break;
+                default: GR_TRY_S((walks_launch<8, MIS>(s, p, vs, out, bound, bs, cur, cnt, err, rays, st)));
+            }
+            ++launches;
+            break;
+        }
+        GR_TRY_S(extend_any(s, false, bound, cnt + cur, bs.q_o[cur].as<float4>(), bs.q_d[cur].as<float4>(),
+                            bs.q_hit.as<float4>(), err, rays, cnt + CNT_FETCH, st, false));
+        GR_CUDA_TRY(cudaGetLastError());
+        GR_CUDA_TRY(cudaMemsetAsync(cnt + nxt, 0, sizeof(uint32_t), st));
+        const size_t ssmem = sort_smem_bytes(BSBLOCK, BSHADE_PER_THREAD);
+        GR_CUDA_TRY(allow_sort_smem(k_bdpt_shade<MIS>, ssmem));
+        k_bdpt_shade<MIS><<<resident_grid(k_bdpt_shade<MIS>, ssmem, bound, BSBLOCK), BSBLOCK, ssmem, st>>>(
+            s, p, vs, out, cnt + cur, bs.q_slot[cur].as<uint32_t>(), bs.q_o[cur].as<float4>(),
+            bs.q_d[cur].as<float4>(), bs.q_hit.as<float4>(), bs.q_state[cur].as<float4>(), cnt + nxt,
+            bs.q_slot[nxt].as<uint32_t>(), bs.q_o[nxt].as<float4>(), bs.q_d[nxt].as<float4>(),
+            bs.q_state[nxt].as<float4>());
+        GR_CUDA_TRY(cudaGetLastError());
+        launches += 2;
+        GR_CUDA_TRY(cudaMemcpyAsync(rb.host + (depth & 3), cnt + nxt, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        GR_CUDA_TRY(cudaEventRecord(rb.ev[depth & 3], st));
+        if (depth >= 2) {
+            GR_CUDA_TRY(cudaEventSynchronize(rb.ev[(depth - 2) & 3]));
+            bound = rb.host[(depth - 2) & 3];  // walks only leave the queue
+            if (bound == 0) break;
+        }
+    }
+    return GR_OK;
+}
+
 }  // namespace
 
 size_t BdptState::bytes_per_path(uint32_t max_len) {
     const size_t pairs = max_pairs(max_len);
-    return 2 * (2 * (4 + 16 + 16) + 16 + 16) + 8 + 8 + 16  // queues, hits, throughput; key, st, light
+    return 2 * (2 * (4 + 16 + 16 + 64) + 16) + 8 + 16      // queues (with state), hits; st, light
            + 2 * max_len * VREC * 16 + 2 * 4 + 4 + 16         // vertices, counts, flags, escape
            + pairs * 16 + (pairs + max_len) * 16 + max_len * (16 + 4) + 4;  // entries, shadow queue, lt, order
 }
@@ -941,10 +1085,9 @@ cudaError_t BdptState::ensure(size_t paths, uint32_t max_len) {
         if ((e = q_slot[k].ensure(slots * sizeof(uint32_t))) != cudaSuccess) return e;
         if ((e = q_o[k].ensure(slots * sizeof(float4))) != cudaSuccess) return e;
         if ((e = q_d[k].ensure(slots * sizeof(float4))) != cudaSuccess) return e;
+        if ((e = q_state[k].ensure(slots * 4 * sizeof(float4))) != cudaSuccess) return e;
     }
     if ((e = q_hit.ensure(slots * sizeof(float4))) != cudaSuccess) return e;
-    if ((e = tp.ensure(slots * sizeof(float4))) != cudaSuccess) return e;
-    if ((e = key.ensure(paths * sizeof(unsigned long long))) != cudaSuccess) return e;
     if ((e = st.ensure(paths * sizeof(float2))) != cudaSuccess) return e;
     if ((e = light.ensure(paths * sizeof(float4))) != cudaSuccess) return e;
     if ((e = verts.ensure(slots * max_len * VREC * sizeof(float4))) != cudaSuccess) return e;
@@ -996,7 +1139,6 @@ gr_status render_bdpt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
     p.cam = job.camera;
     p.width = job.width;
     p.height = job.height;
-    p.npix = npix;
     p.seed = rp.seed;
     p.max_len = max_len;
     p.rr_len = rp.rr_depth;
@@ -1019,32 +1161,9 @@ gr_status render_bdpt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
         Verts vs{bs.verts.as<float4>(), p.nslots};
         GR_CUDA_TRY(cudaMemsetAsync(cnt + CNT_QUEUE0, 0, sizeof(uint32_t), st));
         GR_CUDA_TRY(cudaMemsetAsync(cnt + CNT_SHADOWQ, 0, 2 * sizeof(uint32_t), st));
-        k_bdpt_raygen<<<(p.n + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(
-            job.scene, p, vs, bs.vcount.as<uint32_t>(), ps.tp.as<float4>(), bs.flags.as<uint32_t>(),
-            ps.key.as<unsigned long long>(), ps.st.as<float2>(), bs.escape.as<float4>(), cnt + CNT_QUEUE0,
-            ps.q_slot[0].as<uint32_t>(), ps.q_o[0].as<float4>(), ps.q_d[0].as<float4>());
-        GR_CUDA_TRY(cudaGetLastError());
-        ++launches;
-        // Every walk ends within max_len bounces (one vertex per bounce).
-        for (uint32_t depth = 0; depth < max_len; ++depth) {
-            int cur = depth & 1, nxt = cur ^ 1;
-            gr_status s1 = extend_any(job.scene, false, p.nslots, cnt + cur, ps.q_o[cur].as<float4>(),
-                                      ps.q_d[cur].as<float4>(), ps.q_hit.as<float4>(), err, rays, cnt + CNT_FETCH, st, false);
-            if (s1 != GR_OK) return s1;
-            GR_CUDA_TRY(cudaGetLastError());
-            GR_CUDA_TRY(cudaMemsetAsync(cnt + nxt, 0, sizeof(uint32_t), st));
-            const size_t ssmem = sort_smem_bytes(BSBLOCK, BSHADE_PER_THREAD);
-            GR_CUDA_TRY(allow_sort_smem(k_bdpt_shade, ssmem));
-            int grid = resident_grid(k_bdpt_shade, ssmem, p.nslots, BSBLOCK);
-            k_bdpt_shade<<<grid, BSBLOCK, ssmem, st>>>(job.scene, p, vs, cnt + cur, ps.q_slot[cur].as<uint32_t>(),
-                                                 ps.q_o[cur].as<float4>(), ps.q_d[cur].as<float4>(),
-                                                 ps.q_hit.as<float4>(), bs.vcount.as<uint32_t>(), ps.tp.as<float4>(),
-                                                 ps.key.as<unsigned long long>(), bs.flags.as<uint32_t>(),
-                                                 bs.escape.as<float4>(), cnt + nxt, ps.q_slot[nxt].as<uint32_t>(),
-                                                 ps.q_o[nxt].as<float4>(), ps.q_d[nxt].as<float4>());
-            GR_CUDA_TRY(cudaGetLastError());
-            launches += 2;
-        }
+        p.order = make_path_order(job.width, job.height, g);
+        GR_TRY_S(p.mis || p.lt ? run_walks<true>(job.scene, p, vs, bs, cnt, err, rays, launches, st)
+                               : run_walks<false>(job.scene, p, vs, bs, cnt, err, rays, launches, st));
         Items* items = bs.items.as<Items>();
         {
             const int sgrid = static_cast<int>(std::min<uint32_t>((p.n + BLOCK - 1) / BLOCK, 1024u));
@@ -1055,11 +1174,6 @@ gr_status render_bdpt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
                                                        bs.order.as<uint32_t>());
             GR_CUDA_TRY(cudaGetLastError());
             launches += 3;
-        }
-        if (p.mis) {
-            k_bdpt_mis<<<(p.nslots + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(p, vs, bs.vcount.as<uint32_t>());
-            GR_CUDA_TRY(cudaGetLastError());
-            ++launches;
         }
         // The number of items is known on the device only: every resident block, looping.
         const uint32_t all = p.n * max_pairs(max_len);

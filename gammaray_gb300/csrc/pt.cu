@@ -28,12 +28,6 @@
 #include "shade_sort.cuh"
 #include "wavefront.cuh"
 
-#define GR_TRY_S(expr)                \
-    do {                              \
-        gr_status s__ = (expr);       \
-        if (s__ != GR_OK) return s__; \
-    } while (0)
-
 namespace gr {
 
 namespace {
@@ -62,31 +56,6 @@ template <int NT>
 constexpr uint32_t shade_per() {
     return NT == 128 ? SHADE_PER_THREAD : (NT == 384 ? 96u : SHADE_BIG_PER);
 }
-
-// Queues of at most PATH_LOOP_MAX paths are carried to their end by one launch
-// (k_pt_finish) instead of an extension and a shading launch per bounce; a group that
-// starts that small needs no queue at all.  Below it a bounce is bounded by latency: its
-// two launches take about 30 us however few paths are left, and on meshes the slowest ray
-// of each bounce alone takes 90-140 us.  Above it the wavefront's sorted shading and
-// refilled extension win.  Measured, wavefront against path loop (us per render):
-//   Cornell box, depth 8     5 k paths 377 / 181, 66 k 400 / 258, 393 k 545 / 611
-//   50 k triangles, depth 12 8 k paths - / 295, 240 k 1361 / 598, 393 k 955 / 760
-//   102 k triangles, 66 k paths 1256 / 463
-// and as the end of a larger render: 641 x 359 x 9 spp, unbounded depth 2439 -> 1695,
-// 512 x 512 x 4 spp 2080 -> 1480, 1024 x 1024 x 64 spp 28.61 -> 28.40 ms.
-constexpr uint32_t PATH_LOOP_MAX = 1u << 18;
-// Depths the path loop takes: one launch carries a path to its end, so its length has to
-// be bounded, by max_depth or by the roulette (at most 3/4 survive a bounce beyond
-// rr_aggressive_depth).  Other settings keep a launch per bounce.
-constexpr uint32_t PATH_LOOP_DEPTH = 256;
-constexpr uint32_t PATH_LOOP_RR_DEPTH = 64;
-// At 4 blocks per SM it has 128 registers; it uses 112.
-constexpr int PATH_LOOP_BLOCKS = 4;
-// Lanes of a warp that carry paths when there are too few to fill every warp: lanes of a
-// warp wait for each other, but fewer lanes per warp repeat the shading code.  4 / 8 / 16
-// / 32 measured 193 / 181 / 170 / 181 us on 5 k paths of the Cornell box, 280 / 295 / 316
-// / 324 us on 8 k of a mesh.
-constexpr uint32_t PATH_LOOP_MIN_LANES = 8;
 
 struct PTParams {
     DevCamera cam;
@@ -356,12 +325,8 @@ gr_status launch_finish_w(const DeviceScene& s, const PTParams& p, uint32_t dept
                           float2* film_pos, float4* L_buf, uint32_t* fetch, int* err, unsigned long long* rays,
                           cudaStream_t st) {
     const size_t smem = step_stack_smem_bytes(BLOCK);
-    int per_sm = 0;
-    GR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pt_finish<W, CAMERA>, BLOCK, smem));
-    const uint32_t warps = static_cast<uint32_t>(std::max(1, per_sm) * device_sm_count()) * (BLOCK / 32);
-    const uint32_t lanes = std::min(32u, std::max(PATH_LOOP_MIN_LANES, (most + warps - 1) / warps));
-    const uint32_t need_warps = (most + lanes - 1) / lanes;
-    const uint32_t grid = (std::min(warps, need_warps) + BLOCK / 32 - 1) / (BLOCK / 32);
+    uint32_t lanes = 0;
+    const int grid = path_loop_grid(k_pt_finish<W, CAMERA>, smem, most, lanes);
     k_pt_finish<W, CAMERA><<<grid, BLOCK, smem, st>>>(s, p, depth, most, q, film_pos, L_buf, lanes, fetch, err, rays);
     GR_CUDA_TRY(cudaGetLastError());
     return GR_OK;

@@ -19,6 +19,13 @@ namespace gr {
 
 void set_error(const std::string& msg);
 
+// Passes on a gr_status other than GR_OK.
+#define GR_TRY_S(expr)                \
+    do {                              \
+        gr_status s__ = (expr);       \
+        if (s__ != GR_OK) return s__; \
+    } while (0)
+
 #define GR_CUDA_TRY(expr)                                                                          \
     do {                                                                                           \
         cudaError_t e__ = (expr);                                                                  \
@@ -82,7 +89,7 @@ struct PathState {
 // BDPT walk queues, vertex storage, strategy entries and the shadow queue (grown on
 // demand).  Walks are addressed by slot (2 per path: camera, light).
 struct BdptState {
-    DevBuf q_slot[2], q_o[2], q_d[2], q_hit, tp, key, st, light;
+    DevBuf q_slot[2], q_o[2], q_d[2], q_state[2], q_hit, st, light;
     DevBuf verts, vcount, flags, escape, entries, shadow, lt, lt_pixel;
     DevBuf order, items;  // paths ordered by walk lengths, and their strategies laid out as items
     cudaError_t ensure(size_t paths, uint32_t max_len);

@@ -56,6 +56,31 @@ __global__ void __launch_bounds__(BLOCK) k_extend_refill(DeviceScene s, const ui
     }
 }
 
+// Queues of at most PATH_LOOP_MAX paths are carried to their end by one launch
+// (k_pt_finish) instead of an extension and a shading launch per bounce; a group that
+// starts that small needs no queue at all.  Below it a bounce is bounded by latency: its
+// two launches take about 30 us however few paths are left, and on meshes the slowest ray
+// of each bounce alone takes 90-140 us.  Above it the wavefront's sorted shading and
+// refilled extension win.  Measured, wavefront against path loop (us per render):
+//   Cornell box, depth 8     5 k paths 377 / 181, 66 k 400 / 258, 393 k 545 / 611
+//   50 k triangles, depth 12 8 k paths - / 295, 240 k 1361 / 598, 393 k 955 / 760
+//   102 k triangles, 66 k paths 1256 / 463
+// and as the end of a larger render: 641 x 359 x 9 spp, unbounded depth 2439 -> 1695,
+// 512 x 512 x 4 spp 2080 -> 1480, 1024 x 1024 x 64 spp 28.61 -> 28.40 ms.
+constexpr uint32_t PATH_LOOP_MAX = 1u << 18;
+// Depths the path loop takes: one launch carries a path to its end, so its length has to
+// be bounded, by max_depth or by the roulette (at most 3/4 survive a bounce beyond
+// rr_aggressive_depth).  Other settings keep a launch per bounce.
+constexpr uint32_t PATH_LOOP_DEPTH = 256;
+constexpr uint32_t PATH_LOOP_RR_DEPTH = 64;
+// At 4 blocks per SM it has 128 registers; it uses 112.
+constexpr int PATH_LOOP_BLOCKS = 4;
+// Lanes of a warp that carry paths when there are too few to fill every warp: lanes of a
+// warp wait for each other, but fewer lanes per warp repeat the shading code.  4 / 8 / 16
+// / 32 measured 193 / 181 / 170 / 181 us on 5 k paths of the Cornell box, 280 / 295 / 316
+// / 324 us on 8 k of a mesh.
+constexpr uint32_t PATH_LOOP_MIN_LANES = 8;
+
 // Path loop: a warp carries paths from their first ray to their end without going back
 // to a queue.  Its lanes trace, one traversal step each per iteration, until every path
 // of the warp has its closest hit, then all of them shade, and the survivors trace their
@@ -142,26 +167,6 @@ GR_D void count_rays(uint32_t traced, unsigned long long* rays) {
     if ((threadIdx.x & 31u) == 0 && sum) atomicAdd(rays, static_cast<unsigned long long>(sum));
 }
 
-// Appends this lane's ray to the next queue with one atomic per warp (ballot + popc).
-// Every lane of the warp must call it (warp-uniform trip counts).
-GR_D void push_warp(bool alive, uint32_t* count_out, uint32_t slot, V3 o, V3 d, uint32_t* __restrict__ nslot,
-                    float4* __restrict__ no, float4* __restrict__ nd, uint32_t cap) {
-    const unsigned lane = threadIdx.x & 31;
-    unsigned m = __ballot_sync(0xffffffffu, alive);
-    if (!m) return;
-    int leader = __ffs(m) - 1;
-    uint32_t base = 0;
-    if (lane == static_cast<unsigned>(leader)) base = atomicAdd(count_out, static_cast<uint32_t>(__popc(m)));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (alive) {
-        uint32_t pos = base + __popc(m & ((1u << lane) - 1u));
-        if (!GR_IN_RANGE(pos, cap)) return;
-        nslot[pos] = slot;
-        no[pos] = make_float4(o.x, o.y, o.z, 0.0f);
-        nd[pos] = make_float4(d.x, d.y, d.z, 0.0f);
-    }
-}
-
 // Blocks of `block` threads for n items: every block the device can hold at once (SMs x
 // resident blocks per SM, asked of the current device at each launch), or fewer when n
 // needs fewer.
@@ -174,6 +179,19 @@ int resident_grid(K kernel, size_t smem, uint32_t n, int block = BLOCK) {
     uint32_t need = (n + block - 1) / block;
     uint32_t cap = static_cast<uint32_t>(sm * per_sm);
     return static_cast<int>(std::max(1u, std::min(need, cap)));
+}
+
+// Grid of a path-loop kernel (blocks of BLOCK threads) for at most `most` paths, and the
+// lanes of each warp that carry them.
+template <class K>
+int path_loop_grid(K kernel, size_t smem, uint32_t most, uint32_t& lanes) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, BLOCK, smem) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+    const uint32_t warps = static_cast<uint32_t>(per_sm * device_sm_count()) * (BLOCK / 32);
+    lanes = std::min(32u, std::max(PATH_LOOP_MIN_LANES, (most + warps - 1) / warps));
+    const uint32_t need = (most + lanes - 1) / lanes;
+    return static_cast<int>((std::min(warps, need) + BLOCK / 32 - 1) / (BLOCK / 32));
 }
 
 // `fetch`: the kernel's ray counter, zeroed here before each launch.
