@@ -554,15 +554,11 @@ static __device__ __noinline__ VEval eval_vertex(const DevMaterial& m, V3 wi, V3
 #pragma unroll 1
     for (int k = 0; k < m.n_lobes; ++k) {
         const DevLobe& L = m.lobe[k];
-        if ((refl && (L.kind & LOBE_REFLECTION)) || (!refl && (L.kind & LOBE_TRANSMISSION)))
-            e.f = e.f + lobe_f(L, il, ol, c2l);
-        // Both directions through one call site (one inlined copy of the lobe pdfs).
-#pragma unroll 1
-        for (int d = 0; pdfs && d < 2; ++d) {
-            float q = lobe_pdf(L, d ? ol : il, d ? il : ol);
-            if (d) pr += q;
-            else pf += q;
-        }
+        const bool value = (refl && (L.kind & LOBE_REFLECTION)) || (!refl && (L.kind & LOBE_TRANSMISSION));
+        const LobeEval v = lobe_eval(L, il, ol, c2l, (value ? WANT_F : 0u) | (pdfs ? WANT_PDF | WANT_REV : 0u));
+        if (value) e.f = e.f + v.f;
+        pf += v.pdf;
+        pr += v.rev;
     }
     if (pdfs && m.n_lobes) {
         const float n = static_cast<float>(m.n_lobes);
