@@ -339,9 +339,11 @@ __global__ void __launch_bounds__(BLOCK) k_bdpt_raygen(DeviceScene s, BdptParams
 // One vertex of random_walk (integrators.rs:138-229) at the hit h = (t, leaf-order primitive
 // or -1, u, v) of walk `slot`'s ray (o, d): stores the vertex and advances w.  Returns
 // whether the walk goes on, with its next ray; a walk that ends leaves its vertex count.
+// `lobe`: the lobe already picked (sorted_lobe), or ANY_LOBE.
+constexpr uint32_t ANY_LOBE = 0xFFFFFFFFu;
 template <bool MIS>
 GR_D bool walk_vertex(const DeviceScene& s, const BdptParams& p, const Verts& vs, const PathOut& out, uint32_t slot,
-                      Walk& w, V3 o, V3 d, float4 h, V3& new_o, V3& new_d) {
+                      Walk& w, uint32_t lobe, V3 o, V3 d, float4 h, V3& new_o, V3& new_d) {
     const uint32_t walk = slot & 1u, path = slot >> 1, k = w.k;
     const bool c2l = walk == 0;
     const int32_t pk = __float_as_int(h.y);
@@ -363,8 +365,9 @@ GR_D bool walk_vertex(const DeviceScene& s, const BdptParams& p, const Verts& vs
     uint32_t base = (walk ? DIM_LIGHT_WALK : DIM_CAMERA_WALK) + 4 * k;
     V3 incoming = -d;
     V3 hit_point = o + (d * h.x);
-    MaterialSample ms = sample_world(m, incoming, f, c2l, uniform01(w.key, base), uniform01(w.key, base + 1),
-                                     uniform01(w.key, base + 2));
+    if (lobe == ANY_LOBE) lobe = pick_lobe(m, uniform01(w.key, base));
+    MaterialSample ms = sample_lobe(m, incoming, f, c2l, static_cast<int>(lobe), uniform01(w.key, base + 1),
+                                    uniform01(w.key, base + 2));
     bool connectible = count_lobes(m, LOBE_DIFFUSE | LOBE_GLOSSY) != 0;
     V3 ntp = mul(w.tp, ms.radiance * (fabsf(dot(f.normal, ms.outgoing)) / ms.pdf));
     ntp = ntp * correct_shading_normal(incoming, ms.outgoing, f, c2l);
@@ -422,7 +425,7 @@ GR_D bool walk_vertex(const DeviceScene& s, const BdptParams& p, const Verts& vs
 #endif
 constexpr int BSBLOCK = GR_BDPT_SHADE_BLOCK;
 static_assert(BSBLOCK == 128 || BSBLOCK == 768, "BDPT shading block of 128 or 768 threads");
-constexpr uint32_t BSHADE_PER_THREAD = BSBLOCK == 128 ? SHADE_PER_THREAD : SHADE_BIG_PER;
+constexpr uint32_t BSHADE_PER_THREAD = BSBLOCK == 128 ? SHADE_PER_THREAD : SHADE_ONE_CHUNK;
 
 template <bool MIS>
 __global__ void __launch_bounds__(BSBLOCK, 768 / BSBLOCK)
@@ -436,7 +439,8 @@ __global__ void __launch_bounds__(BSBLOCK, 768 / BSBLOCK)
     const uint32_t n = *count_in;
     // Material-sorted shading (shade_sort.cuh), by (walk, material, chosen lobe).
     // Block-uniform chunk loop.
-    const uint32_t per = chunk_per_thread<BSBLOCK, BSHADE_PER_THREAD>(n, gridDim.x);
+    const uint32_t per =
+        chunk_per_thread<BSBLOCK, BSBLOCK == 128 ? BSHADE_PER_THREAD : SHADE_BIG_PER, BSHADE_PER_THREAD>(n, gridDim.x);
     const uint32_t chunk = chunk_entries<BSBLOCK>(n, gridDim.x, per);
     for (uint32_t c0 = blockIdx.x * chunk; c0 < n; c0 += gridDim.x * chunk) {
         const uint32_t cn = min(chunk, n - c0);
@@ -455,12 +459,13 @@ __global__ void __launch_bounds__(BSBLOCK, 768 / BSBLOCK)
             V3 new_o = v3zero(), new_d = v3zero();
             Walk w{};
             if (i < cn) {
-                uint32_t q = c0 + sm.order[i];
+                const uint32_t at = sm.order[i];
+                uint32_t q = c0 + at;
                 slot = q_slot[q];
                 const float4 o4 = q_o[q], d4 = q_d[q];
                 w = load_walk<MIS>(q_state, q);
-                alive = walk_vertex<MIS>(s, p, vs, out, slot, w, V3{o4.x, o4.y, o4.z}, V3{d4.x, d4.y, d4.z}, q_hit[q],
-                                         new_o, new_d);
+                alive = walk_vertex<MIS>(s, p, vs, out, slot, w, sorted_lobe(sm, at), V3{o4.x, o4.y, o4.z},
+                                         V3{d4.x, d4.y, d4.z}, q_hit[q], new_o, new_d);
             }
             push_walk<MIS>(alive, count_out, slot, new_o, new_d, w, nslot, no, nd, nstate, p.nslots);
         }
@@ -490,7 +495,7 @@ __global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
     };
     auto shade = [&](uint32_t, const TravState& t, V3& no, V3& nd) {
         const float4 h = make_float4(t.closest, __int_as_float(t.hit), t.hu, t.hv);
-        return walk_vertex<MIS>(s, p, vs, out, slot, w, t.o, t.d, h, no, nd);
+        return walk_vertex<MIS>(s, p, vs, out, slot, w, ANY_LOBE, t.o, t.d, h, no, nd);
     };
     count_rays(run_paths<W>(s, stk, *count, lanes, fetch, err, take, shade), rays);
 }

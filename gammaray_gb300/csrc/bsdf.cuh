@@ -421,7 +421,7 @@ struct MaterialSample {
     uint32_t kind;
 };
 
-// material.rs:140-235.  u0 picks the lobe, u1 and u2 feed the lobe's sampler.
+// material.rs:140-235 once the lobe r is picked; u1 and u2 feed its sampler.
 //
 // The reference sums the chosen lobe's value and pdf first, then every other lobe's in
 // index order.  One loop does all of it: step -1 is the chosen lobe, steps 0..n-1 the
@@ -429,13 +429,11 @@ struct MaterialSample {
 // the mixture uses it, it made the shading kernels too large for the instruction
 // cache.  The first term is assigned rather than added to zero, so the sums (and the
 // signs of zeros) are the reference's.
-GR_D MaterialSample sample_world(const DevMaterial& m, V3 wi, const Frame& f, bool c2l, float u0, float u1,
-                                 float u2) {
+GR_D MaterialSample sample_lobe(const DevMaterial& m, V3 wi, const Frame& f, bool c2l, int r, float u1, float u2) {
     V3 il = world_to_local(wi, f.tangent, f.binormal, f.normal);
     V3 emission = light_world(m, wi, f);
     int n = m.n_lobes;
     if (n == 0) return MaterialSample{emission, v3zero(), v3zero(), 1.0f, LOBE_NONE};
-    int r = static_cast<int>(range_index(u0, static_cast<uint32_t>(n)));
     uint32_t kind = m.lobe[r].kind;
     V3 o;
     float given_pdf;
@@ -464,6 +462,15 @@ GR_D MaterialSample sample_world(const DevMaterial& m, V3 wi, const Frame& f, bo
     pdf /= static_cast<float>(n);
     if (pdf == 0.0f) return MaterialSample{emission, v3zero(), ow, 1.0f, LOBE_NONE};
     return MaterialSample{emission, radiance, ow, pdf, kind};
+}
+
+// The lobe that u0 picks (material.rs:151-153); 0 for a material without lobes.
+GR_D uint32_t pick_lobe(const DevMaterial& m, float u0) {
+    return m.n_lobes ? range_index(u0, static_cast<uint32_t>(m.n_lobes)) : 0u;
+}
+GR_D MaterialSample sample_world(const DevMaterial& m, V3 wi, const Frame& f, bool c2l, float u0, float u1,
+                                 float u2) {
+    return sample_lobe(m, wi, f, c2l, static_cast<int>(pick_lobe(m, u0)), u1, u2);
 }
 
 }  // namespace gr

@@ -21,7 +21,11 @@ constexpr int EBLOCK = 128;
 #endif
 constexpr int ESBLOCK = GR_ENG_SHADE_BLOCK;
 static_assert(ESBLOCK == 128 || ESBLOCK == 768, "engine shading block of 128 or 768 threads");
-constexpr uint32_t ESHADE_PER_THREAD = ESBLOCK == 128 ? SHADE_PER_THREAD : SHADE_BIG_PER;
+// Entries per thread per chunk: fewer than the path tracer's, since the sort also reads an
+// entry's job and depth (two more lines that have to stay in L1).  12 images in a batch /
+// 6 served requests: 32 / 12 / 8 / 6 / 4 measured 10.81 / 9.91 / 9.97 / 9.78 / 9.73 and 19.40
+// / 18.48 / 18.34 / 18.19 / 18.06 ms.
+constexpr uint32_t ESHADE_PER_THREAD = ESBLOCK == 128 ? SHADE_PER_THREAD : 4;
 
 // Path state.  The queue entry of a live path carries its ray, its job (o.w), its depth
 // (d.w) and its state, two float4:
@@ -289,7 +293,8 @@ __global__ void __launch_bounds__(ESBLOCK, 768 / ESBLOCK)
             V3 new_o = v3zero(), new_d = v3zero();
             float4 sa = make_float4(0.0f, 0.0f, 0.0f, 0.0f), sb = sa;
             if (i < cn) {
-                uint32_t q = c0 + sm.order[i];
+                const uint32_t at = sm.order[i];
+                uint32_t q = c0 + at;
                 slot = q_slot[q];
                 float4 h = q_hit[q];
                 float4 o4 = q_o[q], d4 = q_d[q];
@@ -317,8 +322,8 @@ __global__ void __launch_bounds__(ESBLOCK, 768 / ESBLOCK)
                     const DevMaterial& m = s.materials[__ldg(s.prim_material + prim)];
                     uint64_t key = state_key(hb);
                     uint32_t base = DIM_CAMERA_WALK + 4 * depth;
-                    MaterialSample ms = sample_world(m, -d, f, true, uniform01(key, base), uniform01(key, base + 1),
-                                                     uniform01(key, base + 2));
+                    MaterialSample ms = sample_lobe(m, -d, f, true, static_cast<int>(sorted_lobe(sm, at)),
+                                                    uniform01(key, base + 1), uniform01(key, base + 2));
                     L = L + mul(tp, ms.emission);
                     tp = mul(tp, ms.radiance * (fabsf(dot(f.normal, ms.outgoing)) / ms.pdf));
                     new_o = nudge(o + (d * h.x), ms.outgoing);

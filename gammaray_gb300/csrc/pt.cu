@@ -51,10 +51,10 @@ __global__ void k_set_count(uint32_t* c, uint32_t n) { *c = n; }
 #endif
 constexpr int SHADE_BIG = GR_SHADE_BLOCK;
 static_assert(SHADE_BIG == 128 || SHADE_BIG == 384 || SHADE_BIG == 768, "shading block of 128, 384 or 768 threads");
-// Entries per thread per chunk: 64 at 128 threads, SHADE_BIG_PER at 768 (shade_sort.cuh).
+// Most entries per thread of one chunk (shade_sort.cuh).
 template <int NT>
 constexpr uint32_t shade_per() {
-    return NT == 128 ? SHADE_PER_THREAD : (NT == 384 ? 96u : SHADE_BIG_PER);
+    return NT == 128 ? SHADE_PER_THREAD : SHADE_ONE_CHUNK;
 }
 
 struct PTParams {
@@ -137,8 +137,10 @@ GR_D void push_path(bool alive, uint32_t* count_out, uint32_t slot, V3 o, V3 d, 
 // One vertex of PathTracerIntegrator::integrate (render/integrators.rs:42-100) at the hit
 // h = (t, leaf-order primitive or -1, u, v) of the ray (o, d): emission into L, the next
 // throughput in tp and the next ray.  Returns whether the path goes on.
-GR_D bool shade_hit(const DeviceScene& s, const PTParams& p, uint32_t depth, uint64_t key, V3 o, V3 d, float4 h,
-                    V3& tp, V3& L, V3& new_o, V3& new_d) {
+// `lobe`: the lobe already picked (sorted_lobe), or ANY_LOBE.
+constexpr uint32_t ANY_LOBE = 0xFFFFFFFFu;
+GR_D bool shade_hit(const DeviceScene& s, const PTParams& p, uint32_t depth, uint64_t key, uint32_t lobe, V3 o, V3 d,
+                    float4 h, V3& tp, V3& L, V3& new_o, V3& new_d) {
     const int32_t k = __float_as_int(h.y);
     if (k < 0) {
         if (s.has_env) L = L + mul(tp, V3{s.env[0], s.env[1], s.env[2]});
@@ -148,8 +150,9 @@ GR_D bool shade_hit(const DeviceScene& s, const PTParams& p, uint32_t depth, uin
     uint32_t prim;
     Frame f = hit_frame(s, k, o, d, h.x, h.z, h.w, prim);
     const DevMaterial& m = s.materials[__ldg(s.prim_material + prim)];
-    MaterialSample ms = sample_world(m, -d, f, true, uniform01(key, base), uniform01(key, base + 1),
-                                     uniform01(key, base + 2));
+    if (lobe == ANY_LOBE) lobe = pick_lobe(m, uniform01(key, base));
+    MaterialSample ms =
+        sample_lobe(m, -d, f, true, static_cast<int>(lobe), uniform01(key, base + 1), uniform01(key, base + 2));
     L = L + mul(tp, ms.emission);
     tp = mul(tp, ms.radiance * (fabsf(dot(f.normal, ms.outgoing)) / ms.pdf));
     new_o = nudge(o + (d * h.x), ms.outgoing);
@@ -179,16 +182,19 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_shade(DeviceScene s, PTParams 
     extern __shared__ unsigned char dsmem[];
     constexpr uint32_t PER = shade_per<NT>();
     const SortView sm = sort_view<NT, PER>(dsmem);
+    // Bounce 0: the keys of a chunk, made once for its sort and its shading.
+    uint64_t* keys = reinterpret_cast<uint64_t*>(dsmem + sort_smem_bytes(NT, PER));
     const uint32_t n = *count_in;
     const uint32_t base = DIM_CAMERA_WALK + 4 * depth;
     // Block-uniform chunk loop (sort_chunk's barriers need every thread).
-    const uint32_t per = chunk_per_thread<NT, PER>(n, gridDim.x);
+    const uint32_t per = chunk_per_thread<NT, NT == 128 ? PER : SHADE_BIG_PER, PER>(n, gridDim.x);
     const uint32_t chunk = chunk_entries<NT>(n, gridDim.x, per);
     for (uint32_t c0 = blockIdx.x * chunk; c0 < n; c0 += gridDim.x * chunk) {
         const uint32_t cn = min(chunk, n - c0);
         sort_chunk<NT, PER>(sm, cn, per, [&](uint32_t i) {
             uint32_t q = c0 + i;
             const uint64_t key = FIRST ? first_key(p, __float_as_uint(q_d[q].w)) : state_key(q_state[2 * q + 1]);
+            if (FIRST) keys[i] = key;
             return shade_bucket(s, __float_as_int(q_hit[q].y), uniform01(key, base), 0);
         });
         // Every lane runs every step so that all of them reach the ballot in push_path.
@@ -199,13 +205,14 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_shade(DeviceScene s, PTParams 
             V3 new_o = v3zero(), new_d = v3zero();
             float4 sa = make_float4(0.0f, 0.0f, 0.0f, 0.0f), sb = sa;
             if (i < cn) {
-                uint32_t q = c0 + sm.order[i];
+                const uint32_t at = sm.order[i];
+                uint32_t q = c0 + at;
                 float4 h = q_hit[q];
                 float4 o4 = q_o[FIRST ? 0u : q], d4 = q_d[q];  // camera rays share q_o[0]
                 V3 o = V3{o4.x, o4.y, o4.z}, d = V3{d4.x, d4.y, d4.z};
                 if (FIRST) {
                     slot = __float_as_uint(d4.w);
-                    const uint64_t k0 = first_key(p, slot);
+                    const uint64_t k0 = keys[at];
                     sa = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
                     sb = make_float4(0.0f, 0.0f, __uint_as_float(static_cast<uint32_t>(k0)),
                                      __uint_as_float(static_cast<uint32_t>(k0 >> 32)));
@@ -215,7 +222,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_shade(DeviceScene s, PTParams 
                     sb = q_state[2 * static_cast<size_t>(q) + 1];
                 }
                 V3 tp = V3{sa.x, sa.y, sa.z}, L = V3{sa.w, sb.x, sb.y};
-                alive = shade_hit(s, p, depth, state_key(sb), o, d, h, tp, L, new_o, new_d);
+                alive = shade_hit(s, p, depth, state_key(sb), sorted_lobe(sm, at), o, d, h, tp, L, new_o, new_d);
                 if (alive) {
                     sa = make_float4(tp.x, tp.y, tp.z, L.x);
                     sb = make_float4(L.y, L.z, sb.z, sb.w);
@@ -249,7 +256,7 @@ __global__ void __launch_bounds__(BLOCK) k_shade_display(DeviceScene s, const ui
 
 template <int NT, bool FIRST, class... A>
 gr_status launch_shade_nt(uint32_t n_bound, cudaStream_t st, A... a) {
-    const size_t smem = sort_smem_bytes(NT, shade_per<NT>());
+    const size_t smem = sort_smem_bytes(NT, shade_per<NT>()) + (FIRST ? NT * shade_per<NT>() * sizeof(uint64_t) : 0);
     GR_CUDA_TRY(allow_sort_smem(k_shade<NT, FIRST>, smem));
     // Every resident block; each picks its entries per thread from the queue length.
     int grid = resident_grid(k_shade<NT, FIRST>, smem, n_bound, NT);
@@ -312,7 +319,7 @@ __global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
     };
     auto shade = [&](uint32_t, const TravState& t, V3& no, V3& nd) {
         const float4 h = make_float4(t.closest, __int_as_float(t.hit), t.hu, t.hv);
-        const bool alive = shade_hit(s, p, depth, key, t.o, t.d, h, tp, L, no, nd);
+        const bool alive = shade_hit(s, p, depth, key, ANY_LOBE, t.o, t.d, h, tp, L, no, nd);
         ++depth;
         if (!alive) L_buf[slot] = make_float4(L.x, L.y, L.z, 0.0f);
         return alive;

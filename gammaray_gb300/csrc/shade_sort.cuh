@@ -13,26 +13,19 @@ namespace gr {
 
 constexpr uint32_t SORT_BUCKETS = 32;
 
-// Most queue entries each thread of a shading block sorts and shades per chunk.  Larger
-// chunks give fuller warps per bucket and amortise the sort's barriers; on the
-// path-tracer workload 4 -> 8 -> 16 entries per thread measured 937 -> 1011 -> 1070
-// Msamples/s.  The entries per thread of a launch are chosen from the queue length
-// (chunk_per_thread) so that small queues still spread over every block.
-#ifndef GR_SHADE_PER_THREAD
-#define GR_SHADE_PER_THREAD 64
-#endif
-constexpr uint32_t SHADE_PER_THREAD = GR_SHADE_PER_THREAD;
-// Entries per thread per chunk of the 768-thread shading blocks (one per SM): 85 at most
-// (768 x 85 chunk positions fit 16 bits).  A block sorts its whole chunk (reading every
-// entry's hit and key) before it shades it; at 85 per thread the chunks of all SMs (about
-// 476 MB of those lines) overflow L2 between the two reads.  On the path-tracer workload
-// (102,422 triangles, 1024 x 1024, 64 spp) 16 / 24 / 32 / 40 / 64 / 85 measured shading
-// 9.39 (with an L2 prefetch) / 9.08 / 9.10 / 9.43 / 9.69 / 10.32 ms per render.
-#ifndef GR_SHADE_BIG_PER
-#define GR_SHADE_BIG_PER 32
-#endif
-constexpr uint32_t SHADE_BIG_PER = GR_SHADE_BIG_PER;
-static_assert(SHADE_BIG_PER >= 1 && SHADE_BIG_PER <= 85, "768 x per chunk positions fit 16 bits");
+// Queue entries per thread per chunk.  A block sorts its whole chunk (reading every entry's
+// hit and key) before it shades it, and the chunk has to stay in L1 between the two: at 8
+// entries of 768 threads (one block per SM) its hits and rays are 196 KB.  Larger chunks
+// give fuller warps per bucket and amortise the sort's barriers, but read those lines from
+// L2 again.  On the path-tracer workload (102,422 triangles, 1024 x 1024, 64 spp) 4 / 6 / 8
+// / 12 / 16 / 32 / 48 measured shading 6.95 / 6.78 / 6.69 / 6.82 / 6.91 / 7.38 / 7.79 ms per
+// render (with rows of the image instead of patches in the queue, 32 was best, 9.10).  A
+// queue of up to SHADE_ONE_CHUNK entries per thread is one chunk all the same: Cornell box,
+// 9 per thread, two chunks 0.564, one 0.533 ms.
+constexpr uint32_t SHADE_BIG_PER = 8;
+constexpr uint32_t SHADE_ONE_CHUNK = 12;
+// Of 128-thread blocks, six per SM (queues too short to fill every SM with larger blocks).
+constexpr uint32_t SHADE_PER_THREAD = 32;
 
 // The sort's shared memory (dynamic, sort_smem_bytes(NT, PER) bytes at the start of the
 // block's dynamic shared memory): bucket sizes, then per-entry bucket and sorted order.
@@ -42,7 +35,7 @@ struct SortView {
     uint16_t* order;
 };
 
-inline size_t sort_smem_bytes(uint32_t nt, uint32_t per) {
+GR_HD size_t sort_smem_bytes(uint32_t nt, uint32_t per) {
     return SORT_BUCKETS * sizeof(uint32_t) + static_cast<size_t>(nt) * per * (sizeof(uint8_t) + sizeof(uint16_t));
 }
 
@@ -61,12 +54,15 @@ GR_D SortView sort_view(unsigned char* smem) {
     return SortView{count, bucket, order};
 }
 
-// Entries per thread for a queue of n entries over `blocks` blocks of NT threads: about
-// one chunk per block, at most PER.
-template <uint32_t NT, uint32_t PER>
+// Entries per thread for a queue of n entries over `blocks` blocks of NT threads: one chunk
+// per block if that is at most MOST per thread, else as few equal ones as keep it at most
+// PER.
+template <uint32_t NT, uint32_t PER, uint32_t MOST = PER>
 GR_D uint32_t chunk_per_thread(uint32_t n, uint32_t blocks) {
-    uint32_t per = (n + blocks * NT - 1) / (blocks * NT);
-    return per < 1 ? 1 : (per > PER ? PER : per);
+    const uint32_t per = (n + blocks * NT - 1) / (blocks * NT);  // of a block, in all
+    if (per <= MOST) return per < 1 ? 1 : per;
+    const uint32_t chunks = (per + PER - 1) / PER;
+    return (per + chunks - 1) / chunks;
 }
 
 // Entries per chunk for a queue of n entries over `blocks` blocks of NT threads taking
@@ -81,8 +77,8 @@ GR_D uint32_t chunk_entries(uint32_t n, uint32_t blocks, uint32_t per) {
     return c == 0 ? 32u : (c < NT ? c : NT);
 }
 
-// Sorts positions 0..cn-1 (cn <= NT * per, per <= PER) by bucket_of(i) < SORT_BUCKETS
-// into sm.order.  Every thread of an NT-thread block must call it with the same cn and
+// Sorts positions 0..cn-1 (cn <= NT * per, per <= PER) by bucket_of(i) % SORT_BUCKETS
+// into sm.order; sm.bucket[i] keeps bucket_of(i) (8 bits).  Every thread of an NT-thread block must call it with the same cn and
 // per.  It ends with a barrier; the caller needs one more before the next call reuses
 // `sm`.  Within a bucket the order is unspecified.
 template <uint32_t NT, uint32_t PER, class F>
@@ -97,7 +93,7 @@ GR_D void sort_chunk(const SortView& sm, uint32_t cn, uint32_t per, F bucket_of)
         if (i < cn) {
             uint32_t b = bucket_of(i);
             sm.bucket[i] = static_cast<uint8_t>(b);
-            atomicAdd(&sm.count[b], 1u);
+            atomicAdd(&sm.count[b % SORT_BUCKETS], 1u);
         }
     }
     __syncthreads();
@@ -113,7 +109,7 @@ GR_D void sort_chunk(const SortView& sm, uint32_t cn, uint32_t per, F bucket_of)
     __syncthreads();
     for (uint32_t e = 0; e < per; ++e) {
         uint32_t i = e * NT + tid;
-        if (i < cn) sm.order[atomicAdd(&sm.count[sm.bucket[i]], 1u)] = static_cast<uint16_t>(i);
+        if (i < cn) sm.order[atomicAdd(&sm.count[sm.bucket[i] % SORT_BUCKETS], 1u)] = static_cast<uint16_t>(i);
     }
     __syncthreads();
 }
@@ -123,7 +119,8 @@ GR_D void sort_chunk(const SortView& sm, uint32_t cn, uint32_t per, F bucket_of)
 // (material.rs:151-153) and the material's lobe types, which the mixture's f / pdf loop
 // runs through.  Six lobe types use buckets 1-30 (5 each), the lobe set and `salt` (a
 // walk kind) choosing among the 5.  Materials of any scene or job with the same lobe
-// types share a bucket.
+// types share a bucket.  The lobe's index sits above the bucket, so that shading does not
+// draw u0 again (sorted_lobe).
 GR_D uint32_t shade_bucket(const DeviceScene& s, int32_t k, float u0, uint32_t salt) {
     if (k < 0) return 0;
     uint32_t prim = __float_as_uint(__ldg(s.prims + 3 * static_cast<size_t>(k)).w);
@@ -132,7 +129,10 @@ GR_D uint32_t shade_bucket(const DeviceScene& s, int32_t k, float u0, uint32_t s
     if (nl == 0) return 1;
     const uint32_t r = range_index(u0, nl);
     const uint32_t chosen = static_cast<uint32_t>(m.lobe[r].type);
-    return 1 + 5 * (chosen % 6) + ((m.lobe_set + salt) * 0x9E3779B1u >> 16) % 5;
+    return (1 + 5 * (chosen % 6) + ((m.lobe_set + salt) * 0x9E3779B1u >> 16) % 5) | (r * SORT_BUCKETS);
 }
+static_assert(MAX_LOBES * SORT_BUCKETS <= 256, "bucket and lobe index in 8 bits");
+// The lobe that shade_bucket picked for position i of the sorted chunk.
+GR_D uint32_t sorted_lobe(const SortView& sm, uint32_t i) { return sm.bucket[i] / SORT_BUCKETS; }
 
 }  // namespace gr
