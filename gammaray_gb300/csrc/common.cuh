@@ -138,6 +138,30 @@ struct Frame {
     V3 normal, tangent, binormal, geom_normal;
 };
 
+#ifdef __CUDACC__
+// Two floats in one 64-bit register, added or multiplied by one instruction; each half is
+// rounded as the scalar operation rounds it.
+struct F2 {
+    unsigned long long v;
+};
+GR_D F2 pack2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+GR_D void unpack2(F2 p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v)); }
+GR_D F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+GR_D F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+#endif
+
 // ---------------------------------------------------------------- random numbers
 // Counter-based: a SplitMix64 finaliser (Steele, Lea & Flood 2014) keyed on
 // (seed, pass, path) and indexed by dimension; identical on host and device.

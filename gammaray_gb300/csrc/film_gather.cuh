@@ -29,14 +29,19 @@ constexpr int FILM_THREADS = FILM_TILE_W * FILM_TILE_H;  // 384, one per tile pi
 constexpr int FILM_WARPS = FILM_THREADS / 32;
 constexpr int FILM_ROWS_PER_WARP = FILM_SPAN_H / FILM_WARPS;  // 2
 constexpr int FILM_WIN = 2 * FILM_HALO + 1;                   // 9 candidate rows and columns per pixel
+constexpr uint32_t WIN_TOP = ~(0xFFFFFFFFu >> FILM_WIN);      // the top FILM_WIN bits
+constexpr int FILM_ROWS = 3;                                  // rows of candidates a pixel takes at a time
+static_assert(FILM_WIN % FILM_ROWS == 0 && FILM_ROWS * FILM_WIN <= 32, "whole groups of rows in a word");
 constexpr int FILM_FOOT = 5;                                  // columns (rows) one sample covers, at most
 static_assert(FILM_SPAN_W == 32 && FILM_THREADS % 32 == 0 && FILM_SPAN_H % FILM_WARPS == 0,
               "one warp per neighbourhood row, the rows shared evenly");
-// Gather blocks resident per SM, the register cap of the gather kernels (40 registers at
-// 4, 56 at 3); 46.8 KB of shared memory per block allows 4.  On the path-tracer workload
-// (1024 x 1024, 64 passes) 2 / 3 / 4 measured 4.21 / 3.42 / 3.22 ms of film accumulation.
+// Gather blocks resident per SM, the register cap of the gather kernels (56 registers at 3,
+// 40 with spills at 4).  Bound by instruction issue: of 3.08 ms for 64 passes of 1024 x 1024,
+// staging takes 1.1 and accumulation 1.65.  3 / 4 blocks measured 3.08 / 3.18 ms there, 104 /
+// 113 us on 16 passes of 256 x 256; with one row of candidates at a time, factors one by one
+// and scalar sums, 3.22 ms and 121 us.  Tiles 32 high (80 KB, 2 blocks): 3.12 and 119.
 #ifndef GR_FILM_BLOCKS_PER_SM
-#define GR_FILM_BLOCKS_PER_SM 4
+#define GR_FILM_BLOCKS_PER_SM 3
 #endif
 
 // Film tiles of a width x height image.
@@ -48,9 +53,9 @@ GR_HD uint32_t film_tiles_y(uint32_t height) { return (height + FILM_TILE_H - 1)
 //   mx[t % 5][k]         mitchell1((ox + t - col_discr) / 2) for each tile column t it
 //                        covers; its at most 5 consecutive columns have distinct t % 5
 //   my[t % 5][k]         likewise for the tile rows t it covers
-//   colmask[row][t]      bit c set when sample (row, c) covers tile column t
-//   rowmask[row][t]      bit c set when sample (row, c) covers tile row t
-// so sample (row, c) covers pixel (tx, ty) when bit c is set in
+//   colmask[row][t]      bit 31 - c set when sample (row, c) covers tile column t
+//   rowmask[row][t]      bit 31 - c set when sample (row, c) covers tile row t
+// so sample (row, c) covers pixel (tx, ty) when bit 31 - c is set in
 // colmask[row][tx] & rowmask[row][ty], and its weight there is mx[tx % 5] * my[ty % 5]:
 // the reference's product of the same two factors.
 struct StagedSample {
@@ -72,6 +77,32 @@ GR_D uint32_t transpose32(uint32_t x, unsigned lane) {
         x = (lane & s) ? ((x & ~m[i]) | ((y >> s) & m[i])) : ((x & m[i]) | ((y & m[i]) << s));
     }
     return x;
+}
+
+// Mitchell factors of the tile columns (rows) a footprint covers: discrete positions
+// first .. last of the image, tile positions lo .. hi of them (lo <= hi) at `origin`, of a
+// sample at `at`, into m[t % FILM_FOOT][k].
+GR_D void stage_factors(float (&m)[FILM_FOOT][FILM_SPAN_N], int k, int first, int last, int lo, int hi, int origin,
+                        float at) {
+    const float f0 = static_cast<float>(first);
+    const float d0 = fabsf(f0 - at), d1 = fabsf((f0 + 1.0f) - at), d2 = fabsf((f0 + 2.0f) - at),
+                d3 = fabsf((f0 + 3.0f) - at);
+    if (last - first == 3 && fminf(d0, d3) > 1.0f && fmaxf(d1, d2) <= 1.0f) {
+        // A whole footprint between two pixel centres (almost every sample): two factors
+        // on each side of the filter's knot.  |2x| of mitchell1's argument is the distance.
+        float v[4];
+        mitchell_pair<true>(d0, d3, v[0], v[3]);
+        mitchell_pair<false>(d1, d2, v[1], v[2]);
+        const int t0 = first - origin;
+        int s = (t0 + 2 * FILM_FOOT) % FILM_FOOT;  // t0 >= -3
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+            if (t0 + f >= lo && t0 + f <= hi) m[s][k] = v[f];
+            s = s == FILM_FOOT - 1 ? 0 : s + 1;
+        }
+        return;
+    }
+    for (int t = lo; t <= hi; ++t) m[t % FILM_FOOT][k] = mitchell1((static_cast<float>(origin + t) - at) / 2.0f);
 }
 
 // Adds the samples of `npass` passes, in pass order, to the tile (ox, oy) of `film`.
@@ -102,6 +133,7 @@ GR_D void gather_passes(StagedSample& sm, uint32_t width, uint32_t height, int o
     const bool col_in = scol >= 0 && scol < static_cast<int>(width);
     const float* mxs = sm.mx[tx % FILM_FOOT];
     const float* mys = sm.my[ty % FILM_FOOT];
+    F2 sum0 = pack2(acc.x, acc.y), sum1 = pack2(acc.z, acc.w);
     float2 rs[FILM_ROWS_PER_WARP];
     V3 rc[FILM_ROWS_PER_WARP];
     auto load = [&](uint32_t pass) {
@@ -140,44 +172,43 @@ GR_D void gather_passes(StagedSample& sm, uint32_t width, uint32_t height, int o
                 int r0 = max(0, mnr - oy), r1 = min(FILM_TILE_H - 1, mxr - oy);
                 if (c0 <= c1 && r0 <= r1) {
                     sm.color[k] = make_float4(rc[j].x, rc[j].y, rc[j].z, 0.0f);
-#pragma unroll
-                    for (int f = 0; f < FILM_FOOT; ++f) {
-                        int t = c0 + f;
-                        if (t <= c1) sm.mx[t % FILM_FOOT][k] = mitchell1((static_cast<float>(ox + t) - cd) / 2.0f);
-                    }
-#pragma unroll
-                    for (int f = 0; f < FILM_FOOT; ++f) {
-                        int t = r0 + f;
-                        if (t <= r1) sm.my[t % FILM_FOOT][k] = mitchell1((static_cast<float>(oy + t) - rd) / 2.0f);
-                    }
+                    stage_factors(sm.mx, k, mnc, mxc, c0, c1, ox, cd);
+                    stage_factors(sm.my, k, mnr, mxr, r0, r1, oy, rd);
                     cm = (2u << c1) - (1u << c0);
                     rm = (2u << r1) - (1u << r0);
                 }
             }
-            const uint32_t xc = transpose32(cm, lane), yc = transpose32(rm, lane);
+            const uint32_t xc = __brev(transpose32(cm, lane)), yc = __brev(transpose32(rm, lane));
             if (lane < static_cast<unsigned>(FILM_TILE_W)) sm.colmask[row][lane] = xc;
             if (lane < static_cast<unsigned>(FILM_TILE_H)) sm.rowmask[row][lane] = yc;
         }
         __syncthreads();
         if (pass + 1 < npass) load(pass + 1);  // in flight while this pass accumulates
         if (!inside) continue;
+        // Candidates (footprints reach 4 px), FILM_ROWS rows at a time, since the lanes of a
+        // warp loop to the largest count among them: from the top bit down, columns
+        // tx .. tx + 8 of the first row, then of the next.
 #pragma unroll
-        for (int dy = 0; dy < FILM_WIN; ++dy) {
-            const int row = ty + dy;
-            // candidates: columns tx .. tx + 8 of the row (footprints reach 4 px)
-            uint32_t m = ((sm.colmask[row][tx] & sm.rowmask[row][ty]) >> tx) & ((1u << FILM_WIN) - 1u);
+        for (int dy = 0; dy < FILM_WIN; dy += FILM_ROWS) {
+            uint32_t m = 0u;
+#pragma unroll
+            for (int r = 0; r < FILM_ROWS; ++r)
+                m |= (((sm.colmask[ty + dy + r][tx] & sm.rowmask[ty + dy + r][ty]) << tx) & WIN_TOP) >> (r * FILM_WIN);
+            const int k0 = (ty + dy) * FILM_SPAN_W + tx;
             while (m) {
-                const int k = row * FILM_SPAN_W + tx + __ffs(m) - 1;
-                m &= m - 1;
+                const int b = __clz(m);
+                m ^= 0x80000000u >> b;
+                const int k = k0 + b + (b >= FILM_WIN ? FILM_SPAN_W - FILM_WIN : 0) +
+                              (b >= 2 * FILM_WIN ? FILM_SPAN_W - FILM_WIN : 0);
                 const float4 c = sm.color[k];
                 const float wgt = mxs[k] * mys[k];
-                acc.x = acc.x + c.x * wgt;
-                acc.y = acc.y + c.y * wgt;
-                acc.z = acc.z + c.z * wgt;
-                acc.w += wgt;
+                sum0 = add2(sum0, pack2(c.x * wgt, c.y * wgt));
+                sum1 = add2(sum1, pack2(c.z * wgt, wgt));
             }
         }
     }
+    unpack2(sum0, acc.x, acc.y);
+    unpack2(sum1, acc.z, acc.w);
 }
 
 // Samples of one pass stored linearly: sample (row, col) at base + row * width + col of

@@ -127,28 +127,6 @@ struct TraceScene {
     uint32_t step_budget;
 };
 
-// Two floats in one 64-bit register, added or multiplied by one instruction; each half is
-// rounded as the scalar operation rounds it.
-struct F2 {
-    unsigned long long v;
-};
-GR_D F2 pack2(float a, float b) {
-    F2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-    return r;
-}
-GR_D void unpack2(F2 p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v)); }
-GR_D F2 add2(F2 a, F2 b) {
-    F2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
-GR_D F2 mul2(F2 a, F2 b) {
-    F2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
-
 struct TravState {
     V3 o, d, inv;
     float closest;
