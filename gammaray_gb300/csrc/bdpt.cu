@@ -478,11 +478,12 @@ template <int W, bool MIS>
 __global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
     k_bdpt_walks(DeviceScene s, BdptParams p, Verts vs, PathOut out, const uint32_t* __restrict__ count,
                  const uint32_t* __restrict__ q_slot, const float4* __restrict__ q_o, const float4* __restrict__ q_d,
-                 const float4* __restrict__ q_state, uint32_t lanes, uint32_t* fetch, int* err,
-                 unsigned long long* rays) {
+                 const float4* __restrict__ q_state, uint32_t* fetch, int* err, unsigned long long* rays) {
     extern __shared__ unsigned char smem[];
     int2 spill[MAX_STACK - SMEM_STACK];
     const auto stk = thread_stack<BLOCK>(smem, spill);
+    const uint32_t n = *count;
+    if (n == 0) return;
     uint32_t slot = 0;
     Walk w{};
     auto take = [&](uint32_t q, V3& o, V3& d) {
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
         const float4 h = make_float4(t.closest, __int_as_float(t.hit), t.hu, t.hv);
         return walk_vertex<MIS>(s, p, vs, out, slot, w, ANY_LOBE, t.o, t.d, h, no, nd);
     };
-    count_rays(run_paths<W>(s, stk, *count, lanes, fetch, err, take, shade), rays);
+    count_rays(run_paths<W>(s, stk, n, fetch, err, take, shade), rays);
 }
 
 // Capacities of the strategy entries and of the shadow queue, as BdptState::ensure sizes
@@ -1008,17 +1009,16 @@ template <int W, bool MIS>
 gr_status walks_launch(const DeviceScene& s, const BdptParams& p, const Verts& vs, const PathOut& out, uint32_t most,
                        BdptState& bs, int cur, uint32_t* cnt, int* err, unsigned long long* rays, cudaStream_t st) {
     const size_t smem = step_stack_smem_bytes(BLOCK);
-    uint32_t lanes = 0;
-    const int grid = path_loop_grid(k_bdpt_walks<W, MIS>, smem, most, lanes);
-    k_bdpt_walks<W, MIS><<<grid, BLOCK, smem, st>>>(s, p, vs, out, cnt + cur, bs.q_slot[cur].as<uint32_t>(),
+    const int grid = path_loop_grid(k_bdpt_walks<W, MIS>, smem, most);
+    k_bdpt_walks<W, MIS><<<grid, BLOCK, smem, st>>>(s, p, vs, out, cnt + CNT_LOOP, bs.q_slot[cur].as<uint32_t>(),
                                                     bs.q_o[cur].as<float4>(), bs.q_d[cur].as<float4>(),
-                                                    bs.q_state[cur].as<float4>(), lanes, cnt + CNT_FETCH, err, rays);
+                                                    bs.q_state[cur].as<float4>(), cnt + CNT_LOOP_FETCH, err, rays);
     GR_CUDA_TRY(cudaGetLastError());
     return GR_OK;
 }
 
 // Both walks of a group's paths: raygen, then bounce by bounce; once at most PATH_LOOP_MAX
-// walks are left (as the host reads two bounces behind), one launch carries them to their
+// walks are left, one launch carries them to their
 // end: Cornell box, 200 x 150 x 4 spp, length 16, 636 us of extension and shading -> 404.
 template <bool MIS>
 gr_status run_walks(const DeviceScene& s, const BdptParams& p, const Verts& vs, BdptState& bs, uint32_t* cnt, int* err,
@@ -1031,40 +1031,37 @@ gr_status run_walks(const DeviceScene& s, const BdptParams& p, const Verts& vs, 
         bs.q_d[0].as<float4>(), bs.q_state[0].as<float4>());
     GR_CUDA_TRY(cudaGetLastError());
     ++launches;
-    uint32_t bound = p.nslots;  // an upper bound of the current queue length
+    QueueOutlook look(p.nslots);
     // Every walk ends within max_len bounces (one vertex per bounce).
     for (uint32_t depth = 0; depth < p.max_len; ++depth) {
         const int cur = depth & 1, nxt = cur ^ 1;
-        if (bound <= PATH_LOOP_MAX) {
-            GR_CUDA_TRY(cudaMemsetAsync(cnt + CNT_FETCH, 0, sizeof(uint32_t), st));
+        const bool loop = look.offer();
+        GR_TRY_S(bounce_begin(rb, cnt, depth, loop ? PATH_LOOP_MAX : 0u, st));
+        if (loop) {
+            const uint32_t most = std::min(look.bound, PATH_LOOP_MAX);
             switch (s.width) {
-                case 2: GR_TRY_S((walks_launch<2, MIS>(s, p, vs, out, bound, bs, cur, cnt, err, rays, st))); break;
-                case 4: GR_TRY_S((walks_launch<4, MIS>(s, p, vs, out, bound, bs, cur, cnt, err, rays, st))); break;
-                default: GR_TRY_S((walks_launch<8, MIS>(s, p, vs, out, bound, bs, cur, cnt, err, rays, st)));
+                case 2: GR_TRY_S((walks_launch<2, MIS>(s, p, vs, out, most, bs, cur, cnt, err, rays, st))); break;
+                case 4: GR_TRY_S((walks_launch<4, MIS>(s, p, vs, out, most, bs, cur, cnt, err, rays, st))); break;
+                default: GR_TRY_S((walks_launch<8, MIS>(s, p, vs, out, most, bs, cur, cnt, err, rays, st)));
             }
             ++launches;
-            break;
+            if (look.bound <= PATH_LOOP_MAX) break;  // the path loop takes it whatever its length
         }
-        GR_TRY_S(extend_any(s, false, bound, cnt + cur, bs.q_o[cur].as<float4>(), bs.q_d[cur].as<float4>(),
+        GR_TRY_S(extend_any(s, false, look.bound, cnt + cur, bs.q_o[cur].as<float4>(), bs.q_d[cur].as<float4>(),
                             bs.q_hit.as<float4>(), err, rays, cnt + CNT_FETCH, st, false));
         GR_CUDA_TRY(cudaGetLastError());
-        GR_CUDA_TRY(cudaMemsetAsync(cnt + nxt, 0, sizeof(uint32_t), st));
         const size_t ssmem = sort_smem_bytes(BSBLOCK, BSHADE_PER_THREAD);
         GR_CUDA_TRY(allow_sort_smem(k_bdpt_shade<MIS>, ssmem));
-        k_bdpt_shade<MIS><<<resident_grid(k_bdpt_shade<MIS>, ssmem, bound, BSBLOCK), BSBLOCK, ssmem, st>>>(
+        k_bdpt_shade<MIS><<<resident_grid(k_bdpt_shade<MIS>, ssmem, look.bound, BSBLOCK), BSBLOCK, ssmem, st>>>(
             s, p, vs, out, cnt + cur, bs.q_slot[cur].as<uint32_t>(), bs.q_o[cur].as<float4>(),
             bs.q_d[cur].as<float4>(), bs.q_hit.as<float4>(), bs.q_state[cur].as<float4>(), cnt + nxt,
             bs.q_slot[nxt].as<uint32_t>(), bs.q_o[nxt].as<float4>(), bs.q_d[nxt].as<float4>(),
             bs.q_state[nxt].as<float4>());
         GR_CUDA_TRY(cudaGetLastError());
         launches += 2;
-        GR_CUDA_TRY(cudaMemcpyAsync(rb.host + (depth & 3), cnt + nxt, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        GR_CUDA_TRY(cudaEventRecord(rb.ev[depth & 3], st));
-        if (depth >= 2) {
-            GR_CUDA_TRY(cudaEventSynchronize(rb.ev[(depth - 2) & 3]));
-            bound = rb.host[(depth - 2) & 3];  // walks only leave the queue
-            if (bound == 0) break;
-        }
+        bool more = true;
+        GR_TRY_S(bounce_wait(rb, depth, look, more));
+        if (!more) break;
     }
     return GR_OK;
 }

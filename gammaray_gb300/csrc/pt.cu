@@ -13,8 +13,8 @@
 //            atomic per warp (ballot + popc)
 //   film     after the last bounce, the deterministic tile gather in film.cu
 // Extend and shade run as grid-stride loops over the device-side queue count, so the
-// host never waits for a bounce; it polls the count two bounces behind to stop.  Once
-// few paths are left (or a render has few from the start), one launch carries them to
+// device never waits for the host; the host hears of each bounce's start while the bounce
+// runs, to stop.  Once few paths are left (or a render has few from the start), one launch carries them to
 // their end (the path loop).
 #include <algorithm>
 #include <cstdlib>
@@ -291,11 +291,12 @@ struct PathQueue {
 template <int W, bool CAMERA>
 __global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
     k_pt_finish(DeviceScene s, PTParams p, uint32_t depth0, uint32_t n_paths, PathQueue queue, float2* __restrict__ st,
-                float4* __restrict__ L_buf, uint32_t lanes, uint32_t* fetch, int* err, unsigned long long* rays) {
+                float4* __restrict__ L_buf, uint32_t* fetch, int* err, unsigned long long* rays) {
     extern __shared__ unsigned char smem[];
     int2 spill[MAX_STACK - SMEM_STACK];
     const auto stk = thread_stack<BLOCK>(smem, spill);
     const uint32_t n = CAMERA ? n_paths : *queue.count;
+    if (n == 0) return;
     V3 tp, L;
     uint64_t key = 0;
     uint32_t slot = 0, depth = 0;
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
         if (!alive) L_buf[slot] = make_float4(L.x, L.y, L.z, 0.0f);
         return alive;
     };
-    count_rays(run_paths<W>(s, stk, n, lanes, fetch, err, take, shade), rays);
+    count_rays(run_paths<W>(s, stk, n, fetch, err, take, shade), rays);
 }
 
 template <int W, bool CAMERA>
@@ -332,9 +333,8 @@ gr_status launch_finish_w(const DeviceScene& s, const PTParams& p, uint32_t dept
                           float2* film_pos, float4* L_buf, uint32_t* fetch, int* err, unsigned long long* rays,
                           cudaStream_t st) {
     const size_t smem = step_stack_smem_bytes(BLOCK);
-    uint32_t lanes = 0;
-    const int grid = path_loop_grid(k_pt_finish<W, CAMERA>, smem, most, lanes);
-    k_pt_finish<W, CAMERA><<<grid, BLOCK, smem, st>>>(s, p, depth, most, q, film_pos, L_buf, lanes, fetch, err, rays);
+    const int grid = path_loop_grid(k_pt_finish<W, CAMERA>, smem, most);
+    k_pt_finish<W, CAMERA><<<grid, BLOCK, smem, st>>>(s, p, depth, most, q, film_pos, L_buf, fetch, err, rays);
     GR_CUDA_TRY(cudaGetLastError());
     return GR_OK;
 }
@@ -406,8 +406,6 @@ gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
     unsigned long long* rays = reinterpret_cast<unsigned long long*>(cnt + CNT_RAYS);
     BounceReadback& rb = device_work().readback;  // the caller holds device_work().mu
     GR_CUDA_TRY(rb.ensure());
-    uint32_t* host_cnt = rb.host;
-    cudaEvent_t* evs = rb.ev;
 
     // Optional per-kernel timing: one event pair per extend / shade launch.
     const bool timed = (rp.flags & GR_RENDER_TIME_KERNELS) != 0;
@@ -446,19 +444,19 @@ gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
         uint32_t n = g * npix;
         p.first_pass = rp.first_pass + done;
         p.order = make_path_order(job.width, job.height, g);
-        // Carries the queue of `depth` (depth 0: the group's camera paths, which need no
-        // queue) to its end.  Its time counts as extension (GR_RENDER_TIME_KERNELS).
+        // Carries what k_bounce_begin gave the path loop at `depth` (depth 0: the group's
+        // camera paths, which need no queue) to its end.  Its time counts as extension
+        // (GR_RENDER_TIME_KERNELS).
         auto finish = [&](uint32_t depth, uint32_t most) -> gr_status {
             int e0 = -1, e1 = -1;
             if (timed) GR_TRY_S(mark(e0));
-            GR_CUDA_TRY(cudaMemsetAsync(cnt + CNT_FETCH, 0, sizeof(uint32_t), st));
             const int cur = depth & 1;
-            const PathQueue q{cnt + cur, ps.q_slot[cur].as<uint32_t>(), ps.q_o[cur].as<float4>(),
+            const PathQueue q{cnt + CNT_LOOP, ps.q_slot[cur].as<uint32_t>(), ps.q_o[cur].as<float4>(),
                               ps.q_d[cur].as<float4>(), ps.q_state[cur].as<float4>()};
             GR_TRY_S(depth == 0 ? launch_finish<true>(job.scene, p, 0, most, q, ps.st.as<float2>(),
-                                                      ps.light.as<float4>(), cnt + CNT_FETCH, err, rays, st)
+                                                      ps.light.as<float4>(), cnt + CNT_LOOP_FETCH, err, rays, st)
                                 : launch_finish<false>(job.scene, p, depth, most, q, ps.st.as<float2>(),
-                                                       ps.light.as<float4>(), cnt + CNT_FETCH, err, rays, st));
+                                                       ps.light.as<float4>(), cnt + CNT_LOOP_FETCH, err, rays, st));
             ++launches;
             GR_TRY_S(sync_check(st, "path loop", depth, n));
             if (timed) {
@@ -469,6 +467,7 @@ gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
         };
         const bool small = loop_ok && n <= PATH_LOOP_MAX;
         if (small) {
+            if (done) GR_CUDA_TRY(cudaMemsetAsync(cnt + CNT_LOOP_FETCH, 0, sizeof(uint32_t), st));
             GR_TRY_S(finish(0, n));
         } else {
             int r0 = -1, r1 = -1;
@@ -485,17 +484,19 @@ gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
                 raygen_pairs.emplace_back(r0, r1);
             }
         }
-        uint32_t bound = n;  // an upper bound of the current queue length
+        QueueOutlook look(n);
         for (uint32_t depth = 0; !small; ++depth) {
             if (p.max_depth && depth >= p.max_depth) break;
             int cur = depth & 1, nxt = cur ^ 1;
-            if (depth > 0 && loop_ok && bound <= PATH_LOOP_MAX) {
-                GR_TRY_S(finish(depth, bound));
-                break;
+            const bool loop = depth > 0 && loop_ok && look.offer();
+            GR_TRY_S(bounce_begin(rb, cnt, depth, loop ? PATH_LOOP_MAX : 0u, st));
+            if (loop) {
+                GR_TRY_S(finish(depth, std::min(look.bound, PATH_LOOP_MAX)));
+                if (look.bound <= PATH_LOOP_MAX) break;  // the path loop takes it whatever its length
             }
             int e0 = -1, e1 = -1;
             if (timed) GR_TRY_S(mark(e0));
-            gr_status s1 = extend_any(job.scene, (rp.flags & GR_RENDER_COUNT_TRAVERSAL) != 0, n, cnt + cur,
+            gr_status s1 = extend_any(job.scene, (rp.flags & GR_RENDER_COUNT_TRAVERSAL) != 0, look.bound, cnt + cur,
                                       ps.q_o[cur].as<float4>(), ps.q_d[cur].as<float4>(), ps.q_hit.as<float4>(), err,
                                       rays, cnt + CNT_FETCH, st, depth == 0);
             if (s1 != GR_OK) return s1;
@@ -514,9 +515,8 @@ gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
                 ++launches;
                 break;
             }
-            GR_CUDA_TRY(cudaMemsetAsync(cnt + nxt, 0, sizeof(uint32_t), st));
             if (timed) GR_TRY_S(mark(e0));
-            GR_TRY_S(launch_shade(bound, depth == 0, st, job.scene, p, depth, cnt + cur, ps.q_slot[cur].as<uint32_t>(),
+            GR_TRY_S(launch_shade(look.bound, depth == 0, st, job.scene, p, depth, cnt + cur, ps.q_slot[cur].as<uint32_t>(),
                                   ps.q_o[cur].as<float4>(), ps.q_d[cur].as<float4>(), ps.q_hit.as<float4>(),
                                   ps.q_state[cur].as<float4>(), ps.light.as<float4>(), cnt + nxt,
                                   ps.q_slot[nxt].as<uint32_t>(), ps.q_o[nxt].as<float4>(), ps.q_d[nxt].as<float4>(),
@@ -528,16 +528,9 @@ gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
                 GR_TRY_S(mark(e1));
                 shade_pairs.emplace_back(e0, e1);
             }
-            GR_CUDA_TRY(cudaMemcpyAsync(host_cnt + (depth & 3), cnt + nxt, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                        st));
-            GR_CUDA_TRY(cudaEventRecord(evs[depth & 3], st));
-            if (depth >= 2) {
-                GR_CUDA_TRY(cudaEventSynchronize(evs[(depth - 2) & 3]));
-                if (host_cnt[(depth - 2) & 3] == 0) break;
-                // Paths only leave the queue within a group, so the length known for
-                // bounce depth - 1 bounds every later bounce's.
-                bound = host_cnt[(depth - 2) & 3];
-            }
+            bool more = true;
+            GR_TRY_S(bounce_wait(rb, depth, look, more));
+            if (!more) break;
         }
         if (job.film) {
             int f0 = -1, f1 = -1;
@@ -740,6 +733,7 @@ extern "C" gr_status gr_render_static(gr_scene* sc, const gr_camera* camera, con
         for (uint32_t depth = 0;; ++depth) {
             if (p.max_depth && depth >= p.max_depth) break;
             int cur = depth & 1, nxt = cur ^ 1;
+            GR_CUDA_TRY(cudaMemsetAsync(cnt + CNT_FETCH, 0, sizeof(uint32_t), st));
             GR_TRY_S(extend_any(sc->dev, false, n, cnt + cur, q_o[cur], q_d[cur], q_hit, err, rays, cnt + CNT_FETCH,
                                 st, depth == 0));
             GR_CUDA_TRY(cudaGetLastError());

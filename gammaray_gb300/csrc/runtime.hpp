@@ -98,8 +98,8 @@ struct BdptState {
 
 // The large wavefront buffers are shared by every scene on a device (renders on one
 // GPU run one after another anyway); a scene keeps only its small counter block.
-// The path tracer's view of its queue lengths: a pinned copy of the last four bounces'
-// counts and an event after each copy.  Made once per device and kept (freeing pinned
+// The host's view of the queue lengths: what the last four bounces' starts saw, written to
+// pinned memory by k_bounce_begin, and an event after each.  Made once per device and kept (freeing pinned
 // memory synchronises the device), so a render starts without host allocations.
 struct BounceReadback {
     uint32_t* host = nullptr;
@@ -111,7 +111,7 @@ struct BounceReadback {
             cudaError_t r = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
             if (r != cudaSuccess) return r;
         }
-        return cudaHostAlloc(reinterpret_cast<void**>(&host), 4 * sizeof(uint32_t), cudaHostAllocDefault);
+        return cudaHostAlloc(reinterpret_cast<void**>(&host), 4 * 2 * sizeof(uint32_t), cudaHostAllocDefault);
     }
 };
 
@@ -132,7 +132,9 @@ constexpr int CNT_SHADOW = 6;  // 64-bit counter at index 6..7
 constexpr int CNT_NODES = 8;   // 64-bit: BVH nodes visited (GR_RENDER_COUNT_TRAVERSAL)
 constexpr int CNT_PRIMS = 10;  // 64-bit: primitives tested
 constexpr int CNT_FETCH = 12;  // rays handed out by the refilling extension kernel (per launch)
-constexpr int NUM_COUNTERS = 16;
+constexpr int CNT_LOOP = 16;  // paths the path loop carries to their end at this bounce (k_bounce_begin)
+constexpr int CNT_LOOP_FETCH = 18;  // paths the path loop has handed out
+constexpr int NUM_COUNTERS = 20;
 
 struct SceneBuffers {
     DevBuf nodes, prims, tri_nidx, tri_uvidx, normals, uvs, prim_material, materials, lights, light_tris,

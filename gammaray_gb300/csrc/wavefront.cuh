@@ -66,7 +66,9 @@ __global__ void __launch_bounds__(BLOCK) k_extend_refill(DeviceScene s, const ui
 //   50 k triangles, depth 12 8 k paths - / 295, 240 k 1361 / 598, 393 k 955 / 760
 //   102 k triangles, 66 k paths 1256 / 463
 // and as the end of a larger render: 641 x 359 x 9 spp, unbounded depth 2439 -> 1695,
-// 512 x 512 x 4 spp 2080 -> 1480, 1024 x 1024 x 64 spp 28.61 -> 28.40 ms.
+// 512 x 512 x 4 spp 2080 -> 1480, 1024 x 1024 x 64 spp 28.61 -> 28.40 ms.  Taking over at
+// 2^18 / 2^19 / 2^20 paths: 1242 / 1330 / 1308 us on the second of these, 1.10 / 1.22 / 1.42
+// ms on 1 M paths of the Cornell box.
 constexpr uint32_t PATH_LOOP_MAX = 1u << 18;
 // Depths the path loop takes: one launch carries a path to its end, so its length has to
 // be bounded, by max_depth or by the roulette (at most 3/4 survive a bounce beyond
@@ -88,9 +90,7 @@ constexpr uint32_t PATH_LOOP_MIN_LANES = 8;
 // and a shading launch per bounce, and a slow ray delays its own warp's paths instead of
 // every path of its bounce.
 //   n       paths; path index q goes to take() once
-//   lanes   lanes of each warp that carry paths (1..32): few paths are spread over the
-//           whole grid, since lanes of one warp wait for each other
-//   fetch   a zeroed counter; the first warps * lanes paths are handed out by position
+//   fetch   a zeroed counter; the first paths, one per lane, are handed out by position
 //           (neighbouring ones to different blocks, so a costly part of an image does not
 //           fall on one SM), the rest from it
 //   take(q, o, d)         loads path q and its next ray; false: it has none
@@ -101,13 +101,16 @@ constexpr uint32_t PATH_LOOP_MIN_LANES = 8;
 // iteration steps a lane whose ray has the scene's step budget, each path is handed out
 // once and ends by its depth limit or roulette.  Returns the rays this lane traced.
 template <int W, class K, class Take, class Shade>
-GR_D uint32_t run_paths(const DeviceScene& s, const K& stk, uint32_t n, uint32_t lanes, uint32_t* fetch,
-                        int* err, const Take& take, const Shade& shade) {
+GR_D uint32_t run_paths(const DeviceScene& s, const K& stk, uint32_t n, uint32_t* fetch, int* err, const Take& take,
+                        const Shade& shade) {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    // Lanes of a warp that carry paths: as many as spread them over the whole grid, since
+    // lanes of one warp wait for each other.
+    const uint32_t lanes = min(32u, max(PATH_LOOP_MIN_LANES, (n + warps - 1) / warps));
     const bool use = lane < lanes;
-    const uint32_t warps = blockDim.x >> 5;
-    const uint32_t first = gridDim.x * warps * lanes;  // paths handed out by position
+    const uint32_t first = warps * lanes;  // paths handed out by position
     const uint32_t refill_at = lanes < 4u ? 1u : lanes / 4u;
     TravState t;
     t.hit = -1;
@@ -181,26 +184,68 @@ int resident_grid(K kernel, size_t smem, uint32_t n, int block = BLOCK) {
     return static_cast<int>(std::max(1u, std::min(need, cap)));
 }
 
-// Grid of a path-loop kernel (blocks of BLOCK threads) for at most `most` paths, and the
-// lanes of each warp that carry them.
+// Grid of a path-loop kernel (blocks of BLOCK threads) for at most `most` paths.
 template <class K>
-int path_loop_grid(K kernel, size_t smem, uint32_t most, uint32_t& lanes) {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, BLOCK, smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    const uint32_t warps = static_cast<uint32_t>(per_sm * device_sm_count()) * (BLOCK / 32);
-    lanes = std::min(32u, std::max(PATH_LOOP_MIN_LANES, (most + warps - 1) / warps));
-    const uint32_t need = (most + lanes - 1) / lanes;
-    return static_cast<int>((std::min(warps, need) + BLOCK / 32 - 1) / (BLOCK / 32));
+int path_loop_grid(K kernel, size_t smem, uint32_t most) {
+    return resident_grid(kernel, smem, (most + PATH_LOOP_MIN_LANES - 1) / PATH_LOOP_MIN_LANES * 32u);
 }
 
-// `fetch`: the kernel's ray counter, zeroed here before each launch.
+// The start of a bounce whose queue is `cur`: a queue of at most `take` paths goes to the
+// path loop (its length to CNT_LOOP, and the bounce's own launches find it empty).  The
+// device decides, so the queue goes there at the first bounce that is short enough; the
+// host reads (paths the loop takes, queue length) from `seen`, pinned host memory, while the
+// bounce runs.  Clears the counters of the bounce's launches.
+__global__ void k_bounce_begin(uint32_t* cnt, int cur, uint32_t take, uint32_t* seen) {
+    const uint32_t q = cnt[cur];
+    const bool taken = q <= take;
+    cnt[CNT_LOOP] = taken ? q : 0u;
+    if (taken) cnt[cur] = 0u;
+    cnt[cur ^ 1] = 0u;
+    cnt[CNT_FETCH] = 0u;
+    cnt[CNT_LOOP_FETCH] = 0u;
+    seen[0] = taken ? q : 0u;
+    seen[1] = q;
+    __threadfence_system();
+}
+
+gr_status bounce_begin(const BounceReadback& rb, uint32_t* cnt, uint32_t depth, uint32_t take, cudaStream_t st) {
+    const uint32_t k = depth & 3;
+    k_bounce_begin<<<1, 1, 0, st>>>(cnt, static_cast<int>(depth & 1), take, rb.host + 2 * k);
+    GR_CUDA_TRY(cudaGetLastError());
+    GR_CUDA_TRY(cudaEventRecord(rb.ev[k], st));
+    return GR_OK;
+}
+
+// What the host knows of a group's queue: `bound`, an upper bound of its current length (a
+// queue only gets shorter), and the length expected at the next bounce, which falls about
+// as it fell last.
+struct QueueOutlook {
+    uint32_t bound;
+    uint64_t expected;
+    explicit QueueOutlook(uint32_t n) : bound(n), expected(n) {}
+    // Whether to offer the next bounce's queue to the path loop: a launch that finds it too
+    // long costs about 5 us, one left out on a short queue 30 us and more.
+    bool offer() const { return expected <= PATH_LOOP_MAX + PATH_LOOP_MAX / 2 || bound <= PATH_LOOP_MAX; }
+};
+
+// Waits for what bounce `depth` began with (the bounce itself still runs); `more`: false when
+// it was the last one.
+gr_status bounce_wait(const BounceReadback& rb, uint32_t depth, QueueOutlook& out, bool& more) {
+    const uint32_t k = depth & 3;
+    GR_CUDA_TRY(cudaEventSynchronize(rb.ev[k]));
+    const uint32_t before = out.bound, seen = rb.host[2 * k + 1];
+    out.bound = seen;
+    out.expected = before ? static_cast<uint64_t>(seen) * seen / before : 0u;
+    more = rb.host[2 * k] == 0 && seen != 0;
+    return GR_OK;
+}
+
+// `fetch`: the kernel's ray counter, zero before the launch.
 template <int W, bool COUNT>
 gr_status extend_launch(const DeviceScene& s, uint32_t cap_n, const uint32_t* count, const float4* qo,
                         const float4* qd, float4* qh, int* err, unsigned long long* rays, uint32_t* fetch,
                         cudaStream_t st, bool one_origin) {
     const size_t smem = step_stack_smem_bytes(BLOCK);
-    GR_CUDA_TRY(cudaMemsetAsync(fetch, 0, sizeof(uint32_t), st));
     const int grid = resident_grid(k_extend_refill<W, COUNT>, smem, cap_n);
     k_extend_refill<W, COUNT><<<grid, BLOCK, smem, st>>>(s, count, qo, qd, qh, err, rays, fetch, one_origin);
     return GR_OK;
