@@ -498,13 +498,13 @@ __global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
         const float4 h = make_float4(t.closest, __int_as_float(t.hit), t.hu, t.hv);
         return walk_vertex<MIS>(s, p, vs, out, slot, w, ANY_LOBE, t.o, t.d, h, no, nd);
     };
-    count_rays(run_paths<W>(s, stk, n, fetch, err, take, shade), rays);
+    count_rays(run_paths<W>(stk, n, fetch, err, err + 1, [&]() -> const DeviceScene& { return s; }, take, shade), rays);
 }
 
 // Capacities of the strategy entries and of the shadow queue, as BdptState::ensure sizes
 // them (checked builds test every write against them).
-GR_D size_t entry_cap(const BdptParams& p) { return static_cast<size_t>(p.n) * (p.max_len * (p.max_len + 1) / 2); }
-GR_D size_t shadow_cap(const BdptParams& p) { return entry_cap(p) + (p.lt ? static_cast<size_t>(p.n) * p.max_len : 0); }
+[[maybe_unused]] GR_D size_t entry_cap(const BdptParams& p) { return static_cast<size_t>(p.n) * (p.max_len * (p.max_len + 1) / 2); }
+[[maybe_unused]] GR_D size_t shadow_cap(const BdptParams& p) { return entry_cap(p) + (p.lt ? static_cast<size_t>(p.n) * p.max_len : 0); }
 
 // ---------------------------------------------------- MIS extension (power heuristic)
 // Veach 1997 eq. 10.9 with beta = 2, in the ratio form of PBRT 3e section 16.3.4: per

@@ -4,6 +4,7 @@
 
 #include "engine.hpp"
 #include "film_gather.cuh"
+#include "path_loop.cuh"
 #include "shade_sort.cuh"
 #include "traverse.cuh"
 
@@ -74,30 +75,54 @@ GR_D uint32_t find_unit(const DevUnit* __restrict__ units, uint32_t lo, uint32_t
     return lo;
 }
 
-// Single thread: what to gather and how many paths to issue this iteration.
-__global__ void k_eng_plan(EngineCtl* c, const DevJob* __restrict__ jobs, const DevUnit* __restrict__ units,
-                           const uint32_t* __restrict__ unit_done, uint32_t cap, uint32_t ring, int cur) {
+// One block of GATHER_MAX threads: what to gather and how many paths to issue this
+// iteration.  The threads look at one unit each; thread 0 then decides from shared memory
+// (one thread reading the units one after another took 108 us on 192 finished units).
+__global__ void __launch_bounds__(GATHER_MAX) k_eng_plan(EngineCtl* c, const DevJob* __restrict__ jobs,
+                                                         const DevUnit* __restrict__ units,
+                                                         const uint32_t* __restrict__ unit_done, uint32_t cap,
+                                                         uint32_t ring, int cur) {
+    __shared__ uint32_t is_first[GATHER_MAX], gcount[GATHER_MAX], gtiles[GATHER_MAX], unit_group[GATHER_MAX],
+        fill[GATHER_MAX];
+    __shared__ uint32_t s_n, s_groups;
+    const uint32_t t = threadIdx.x;
     // Finished units, consecutive from the oldest, grouped by job (pass order kept).
-    uint32_t u = c->g_lo, n = 0, groups = 0;
-    uint32_t gjob[GATHER_MAX];
-    uint32_t tmp[GATHER_MAX];
-    uint32_t tmp_group[GATHER_MAX];
-    while (u < c->units_count && n < GATHER_MAX) {
-        DevUnit U = units[u];
-        if (unit_done[u] < U.npix) break;
-        uint32_t g = 0;
-        while (g < groups && gjob[g] != U.job) ++g;
-        if (g == groups) {
-            gjob[groups] = U.job;
-            c->gather_group_count[groups] = 0;
-            ++groups;
-        }
-        c->gather_group_count[g] += 1;
-        tmp[n] = u;
-        tmp_group[n] = g;
-        ++n;
-        ++u;
+    const uint32_t lo = c->g_lo, most = min(static_cast<uint32_t>(GATHER_MAX), c->units_count - lo);
+    if (t == 0) s_n = most;
+    __syncthreads();
+    uint32_t job = 0;
+    if (t < most) {
+        const DevUnit U = units[lo + t];
+        job = U.job;
+        if (unit_done[lo + t] < U.npix) atomicMin(&s_n, t);
     }
+    fill[t] = job;
+    __syncthreads();
+    const uint32_t found = s_n;
+    // A job's group is numbered by its first unit.
+    uint32_t first_of_job = 0;
+    if (t < found)
+        while (fill[first_of_job] != job) ++first_of_job;
+    const bool leader = t < found && first_of_job == t;
+    gcount[t] = 0;
+    is_first[t] = leader ? 1u : 0u;
+    if (t == 0) s_groups = 0;
+    __syncthreads();
+    uint32_t rank = 0;  // leaders before this unit's
+    if (t < found)
+        for (uint32_t k = 0; k < first_of_job; ++k) rank += is_first[k];
+    if (leader) {
+        atomicAdd(&s_groups, 1u);
+        const DevJob& J = jobs[job];
+        gtiles[rank] = film_tiles_x(J.width) * film_tiles_y(J.height);
+    }
+    if (t < found) {
+        atomicAdd(&gcount[rank], 1u);
+        unit_group[t] = rank;
+    }
+    __syncthreads();
+    if (t != 0) return;
+    uint32_t u = lo + found, n = found, groups = s_groups;
     // Gather in larger batches: a call adds several passes per film tile, so the
     // film's read-modify-write and the staging prologue are paid once for them.  Wait
     // until half a capacity of finished paths is waiting, unless the unit list is full,
@@ -112,15 +137,13 @@ __global__ void k_eng_plan(EngineCtl* c, const DevJob* __restrict__ jobs, const 
     }
     uint32_t first = 0, tiles = 0;
     for (uint32_t g = 0; g < groups; ++g) {
-        c->gather_group_first[g] = first;
+        c->gather_group_first[g] = fill[g] = first;
+        c->gather_group_count[g] = gcount[g];
         c->gather_group_tiles[g] = tiles;
-        const DevJob& J = jobs[gjob[g]];
-        tiles += film_tiles_x(J.width) * film_tiles_y(J.height);
-        first += c->gather_group_count[g];
+        tiles += gtiles[g];
+        first += gcount[g];
     }
-    uint32_t fill[GATHER_MAX];
-    for (uint32_t g = 0; g < groups; ++g) fill[g] = c->gather_group_first[g];
-    for (uint32_t k = 0; k < n; ++k) c->gather_units[fill[tmp_group[k]]++] = tmp[k];
+    for (uint32_t k = 0; k < n; ++k) c->gather_units[fill[unit_group[k]]++] = lo + k;
     c->gather_n = n;
     c->gather_groups = groups;
     c->gather_tiles = tiles;
@@ -132,6 +155,13 @@ __global__ void k_eng_plan(EngineCtl* c, const DevJob* __restrict__ jobs, const 
     unsigned long long rem = c->paths_total - c->gcur;
     unsigned long long lim = c->gather_lo_prefix + ring - c->gcur;  // ring slots free of ungathered samples
     unsigned long long nf = min(room, min(rem, lim));
+    if (nf && c->paths_total > c->gather_lo_prefix + ring) {
+        // A unit's paths start in patches, over all of its slots (fill): a unit starts only
+        // when every slot of it is free.
+        const uint32_t last = find_unit(units, c->g_lo, c->units_count, c->gcur + nf - 1);
+        const unsigned long long begin = units[last].prefix;
+        if (begin >= c->gcur && begin + units[last].npix > c->gather_lo_prefix + ring) nf = begin - c->gcur;
+    }
     c->fill_n = static_cast<uint32_t>(nf);
     c->fill_base = c->gcur;
     // The fill's camera rays go after the last shade's survivors, at fixed positions.
@@ -142,6 +172,11 @@ __global__ void k_eng_plan(EngineCtl* c, const DevJob* __restrict__ jobs, const 
         c->fill_uhi = find_unit(units, c->fill_ulo, c->units_count, c->gcur + nf - 1);
     }
     c->gcur += nf;
+    const uint32_t queue = c->q[cur];
+    const bool loop = c->gcur == c->paths_total && queue <= PATH_LOOP_MAX && !c->loop_off;
+    c->loop_n = loop ? queue : 0u;
+    c->loop_fetch = 0;
+    if (loop) c->q[cur] = 0;
     c->done = c->g_lo == c->units_count ? 1u : 0u;
     c->iter += 1;
     c->fetch = 0;  // the extension kernel of this iteration starts handing out rays at 0
@@ -196,9 +231,8 @@ __global__ void __launch_bounds__(FILM_THREADS, GR_FILM_BLOCKS_PER_SM)
     }
 }
 
-// Starts the next fill_n paths in their ring slots (coalesced: consecutive paths,
-// consecutive slots) and queues their camera rays at the positions the plan reserved
-// (no atomics).
+// Starts the next fill_n paths in their ring slots and queues their camera rays at the
+// positions the plan reserved (no atomics).
 __global__ void __launch_bounds__(EBLOCK) k_eng_fill(EngineCtl* c, const DevJob* __restrict__ jobs,
                                                      const DevUnit* __restrict__ units, uint32_t mask,
                                                      uint4* __restrict__ s_cold, uint32_t* __restrict__ q_slot,
@@ -209,15 +243,16 @@ __global__ void __launch_bounds__(EBLOCK) k_eng_fill(EngineCtl* c, const DevJob*
     const uint32_t ulo = c->fill_ulo, uhi = c->fill_uhi + 1;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const unsigned long long p = base + i;
-        const uint32_t slot = static_cast<uint32_t>(p & mask);
         const uint32_t u = find_unit(units, ulo, uhi, p);
         const DevUnit U = units[u];
-        const uint32_t pixel = static_cast<uint32_t>(p - U.prefix);
         const DevJob& J = jobs[U.job];
-        const uint32_t row = pixel / J.width, col = pixel - row * J.width;
-        const uint64_t key = path_key(J.seed, U.pass, pixel);
+        // The unit's paths start in patches of pixels (path_order.cuh); a path's slot is its
+        // pixel's, as the gather reads it.
+        const PathSample ps = path_sample(J.order, static_cast<uint32_t>(p - U.prefix));
+        const uint32_t slot = static_cast<uint32_t>((U.prefix + ps.slot) & mask);
+        const uint64_t key = path_key(J.seed, U.pass, ps.slot);
         float s, t;
-        film_sample_point(J.width, J.height, row, col, key, s, t);
+        film_sample_point(J.width, J.height, ps.row, ps.col, key, s, t);
         V3 o, d;
         camera_ray(J.cam, s, t, o, d);
         s_cold[slot] = make_uint4(u, 0, __float_as_uint(s), __float_as_uint(t));
@@ -233,7 +268,8 @@ __global__ void __launch_bounds__(EBLOCK) k_eng_fill(EngineCtl* c, const DevJob*
 }
 
 // Closest hit for the queued rays of all jobs (trace_queue, rays handed out from c->fetch,
-// which the plan zeroes); each lane keeps its ray's scene.
+// which the plan zeroes); each lane keeps its ray's scene.  Capped at 56 registers for 9
+// blocks of 128 per SM (a few spilled) a 12-image batch took 9.69 instead of 9.51 ms.
 template <int W, int BS>
 __global__ void __launch_bounds__(BS) k_eng_extend_refill(EngineCtl* c, int cur, const DevJob* __restrict__ jobs,
                                                    const float4* __restrict__ q_o, const float4* __restrict__ q_d,
@@ -256,6 +292,92 @@ __global__ void __launch_bounds__(BS) k_eng_extend_refill(EngineCtl* c, int cur,
         [&](uint32_t q, const TravState& t) {
             q_hit[q] = make_float4(t.closest, __int_as_float(t.hit), t.hu, t.hv);
         });
+}
+
+// One vertex of a job's path at the hit h = (t, leaf-order primitive or -1, u, v) of the ray
+// (o, d): radiance into L, the next throughput in tp and the next ray.  Returns whether the
+// path goes on.  `lobe`: the lobe already picked (sorted_lobe), or ANY_LOBE.
+constexpr uint32_t ANY_LOBE = 0xFFFFFFFFu;
+GR_D bool shade_job(const DevJob& J, uint32_t depth, uint64_t key, uint32_t lobe, V3 o, V3 d, float4 h, V3& tp, V3& L,
+                    V3& new_o, V3& new_d) {
+    const DeviceScene& s = J.scene;
+    const int32_t k = __float_as_int(h.y);
+    if (!J.live) return false;  // cancelled: drop the path
+    if (k < 0) {
+        // DisplayColorIntegrator returns black on a miss (render/integrators.rs:29-31).
+        if (s.has_env && !J.display) L = L + mul(tp, V3{s.env[0], s.env[1], s.env[2]});
+        return false;
+    }
+    if (J.display) {
+        uint32_t prim = __float_as_uint(__ldg(s.prims + 3 * static_cast<size_t>(k)).w);
+        const DevMaterial& m = s.materials[__ldg(s.prim_material + prim)];
+        L = V3{m.display[0], m.display[1], m.display[2]};
+        return false;
+    }
+    // PathTracerIntegrator::integrate (render/integrators.rs:42-100), one segment.
+    uint32_t prim;
+    Frame f = hit_frame(s, k, o, d, h.x, h.z, h.w, prim);
+    const DevMaterial& m = s.materials[__ldg(s.prim_material + prim)];
+    const uint32_t base = DIM_CAMERA_WALK + 4 * depth;
+    if (lobe == ANY_LOBE) lobe = pick_lobe(m, uniform01(key, base));
+    MaterialSample ms =
+        sample_lobe(m, -d, f, true, static_cast<int>(lobe), uniform01(key, base + 1), uniform01(key, base + 2));
+    L = L + mul(tp, ms.emission);
+    tp = mul(tp, ms.radiance * (fabsf(dot(f.normal, ms.outgoing)) / ms.pdf));
+    new_o = nudge(o + (d * h.x), ms.outgoing);
+    new_d = ms.outgoing;
+    if (depth > J.rr_depth || nearly_zero(tp)) {
+        float rv = uniform01(key, base + 3);
+        float lum = luminance(tp);
+        float prob = depth > J.rr_aggr ? clamped_lerp(0.10f, 0.75f, lum) : clamped_lerp(0.25f, 1.00f, lum);
+        tp = rv < prob ? tp / prob : v3zero();
+    }
+    return !is_zero(tp) && (J.max_depth == 0 || depth + 1 < J.max_depth);
+}
+
+// Carries the queue's last paths to their end (run_paths), as the plan decides.
+template <int W>
+__global__ void __launch_bounds__(EBLOCK, PATH_LOOP_BLOCKS)
+    k_eng_loop(EngineCtl* c, const DevJob* __restrict__ jobs, uint32_t* unit_done, const uint32_t* __restrict__ q_slot,
+               const float4* __restrict__ q_o, const float4* __restrict__ q_d, const float4* __restrict__ q_state,
+               float4* __restrict__ s_hot, const uint4* __restrict__ s_cold) {
+    extern __shared__ unsigned char smem[];
+    int2 spill[MAX_STACK - SMEM_STACK];
+    const auto stk = thread_stack<EBLOCK>(smem, spill);
+    const uint32_t n = c->loop_n;
+    if (n == 0) return;
+    TraceScene s{nullptr, nullptr, 0u};
+    V3 tp, L;
+    uint64_t key = 0;
+    uint32_t slot = 0, job = 0, depth = 0;
+    auto take = [&](uint32_t q, V3& o, V3& d) {
+        const float4 o4 = q_o[q], d4 = q_d[q];
+        const float4 ha = q_state[2 * static_cast<size_t>(q)], hb = q_state[2 * static_cast<size_t>(q) + 1];
+        slot = q_slot[q];
+        job = __float_as_uint(o4.w);
+        depth = __float_as_uint(d4.w);
+        const DeviceScene& js = jobs[job].scene;
+        s = TraceScene{js.nodes, js.prims, js.step_budget};
+        o = V3{o4.x, o4.y, o4.z};
+        d = V3{d4.x, d4.y, d4.z};
+        tp = V3{ha.x, ha.y, ha.z};
+        L = V3{ha.w, hb.x, hb.y};
+        key = state_key(hb);
+        return true;
+    };
+    auto shade = [&](uint32_t, const TravState& t, V3& no, V3& nd) {
+        const float4 h = make_float4(t.closest, __int_as_float(t.hit), t.hu, t.hv);
+        const bool alive = shade_job(jobs[job], depth, key, ANY_LOBE, t.o, t.d, h, tp, L, no, nd);
+        ++depth;
+        if (!alive) {
+            s_hot[slot] = make_float4(L.x, L.y, L.z, 0.0f);
+            atomicAdd(unit_done + s_cold[slot].x, 1u);
+        }
+        return alive;
+    };
+    count_rays(run_paths<W>(stk, n, &c->loop_fetch, &c->err, nullptr, [&]() -> const TraceScene& { return s; }, take,
+                            shade),
+               &c->rays);
 }
 
 __global__ void __launch_bounds__(ESBLOCK, 768 / ESBLOCK)
@@ -300,43 +422,10 @@ __global__ void __launch_bounds__(ESBLOCK, 768 / ESBLOCK)
                 float4 o4 = q_o[q], d4 = q_d[q];
                 job = __float_as_uint(o4.w);
                 depth = __float_as_uint(d4.w);
-                const DevJob& J = jobs[job];
-                const DeviceScene& s = J.scene;
-                V3 o = V3{o4.x, o4.y, o4.z}, d = V3{d4.x, d4.y, d4.z};
-                float4 ha = q_state[2 * static_cast<size_t>(q)], hb = q_state[2 * static_cast<size_t>(q) + 1];
+                const float4 ha = q_state[2 * static_cast<size_t>(q)], hb = q_state[2 * static_cast<size_t>(q) + 1];
                 V3 tp = V3{ha.x, ha.y, ha.z}, L = V3{ha.w, hb.x, hb.y};
-                int32_t k = __float_as_int(h.y);
-                if (!J.live) {
-                    // cancelled: drop the path
-                } else if (k < 0) {
-                    // DisplayColorIntegrator returns black on a miss (render/integrators.rs:29-31).
-                    if (s.has_env && !J.display) L = L + mul(tp, V3{s.env[0], s.env[1], s.env[2]});
-                } else if (J.display) {
-                    uint32_t prim = __float_as_uint(__ldg(s.prims + 3 * static_cast<size_t>(k)).w);
-                    const DevMaterial& m = s.materials[__ldg(s.prim_material + prim)];
-                    L = V3{m.display[0], m.display[1], m.display[2]};
-                } else {
-                    // PathTracerIntegrator::integrate (render/integrators.rs:42-100), one segment.
-                    uint32_t prim;
-                    Frame f = hit_frame(s, k, o, d, h.x, h.z, h.w, prim);
-                    const DevMaterial& m = s.materials[__ldg(s.prim_material + prim)];
-                    uint64_t key = state_key(hb);
-                    uint32_t base = DIM_CAMERA_WALK + 4 * depth;
-                    MaterialSample ms = sample_lobe(m, -d, f, true, static_cast<int>(sorted_lobe(sm, at)),
-                                                    uniform01(key, base + 1), uniform01(key, base + 2));
-                    L = L + mul(tp, ms.emission);
-                    tp = mul(tp, ms.radiance * (fabsf(dot(f.normal, ms.outgoing)) / ms.pdf));
-                    new_o = nudge(o + (d * h.x), ms.outgoing);
-                    new_d = ms.outgoing;
-                    if (depth > J.rr_depth || nearly_zero(tp)) {
-                        float rv = uniform01(key, base + 3);
-                        float lum = luminance(tp);
-                        float prob =
-                            depth > J.rr_aggr ? clamped_lerp(0.10f, 0.75f, lum) : clamped_lerp(0.25f, 1.00f, lum);
-                        tp = rv < prob ? tp / prob : v3zero();
-                    }
-                    alive = !is_zero(tp) && (J.max_depth == 0 || depth + 1 < J.max_depth);
-                }
+                alive = shade_job(jobs[job], depth, state_key(hb), sorted_lobe(sm, at), V3{o4.x, o4.y, o4.z},
+                                  V3{d4.x, d4.y, d4.z}, h, tp, L, new_o, new_d);
                 // A live path carries (throughput, radiance, key) to its next queue entry; a
                 // finished one leaves its radiance in its slot, which with the cold record's
                 // film position is all the gather reads.
@@ -451,11 +540,23 @@ gr_status Engine::init(const EngineConfig& cfg, cudaStream_t) {
     return record_pair();
 }
 
+template <int W>
+gr_status Engine::launch_loop(EngineCtl* c, int cur) {
+    const size_t smem = step_stack_smem_bytes(EBLOCK);
+    const int grid = grid_for(reinterpret_cast<const void*>(k_eng_loop<W>), EBLOCK, smem, cfg_.capacity);
+    k_eng_loop<W><<<grid, EBLOCK, smem, st_>>>(c, jobs_.as<DevJob>(), unit_done_.as<uint32_t>(),
+                                               q_slot_[cur].as<uint32_t>(), q_o_[cur].as<float4>(),
+                                               q_d_[cur].as<float4>(), q_state_[cur].as<float4>(),
+                                               s_hot_.as<float4>(), s_cold_.as<uint4>());
+    GR_CUDA_TRY(cudaGetLastError());
+    return GR_OK;
+}
+
 gr_status Engine::enqueue_iteration(int cur) {
     EngineCtl* c = ctl_.as<EngineCtl>();
     const uint32_t C = cfg_.capacity;
     const int nxt = cur ^ 1;
-    k_eng_plan<<<1, 1, 0, st_>>>(c, jobs_.as<DevJob>(), units_.as<DevUnit>(), unit_done_.as<uint32_t>(), C, ring_, cur);
+    k_eng_plan<<<1, GATHER_MAX, 0, st_>>>(c, jobs_.as<DevJob>(), units_.as<DevUnit>(), unit_done_.as<uint32_t>(), C, ring_, cur);
     GR_CUDA_TRY(cudaGetLastError());
     const int ggrid = grid_for(reinterpret_cast<const void*>(k_eng_gather), FILM_THREADS, 0, 1u << 30);
     k_eng_gather<<<ggrid, FILM_THREADS, 0, st_>>>(c, jobs_.as<DevJob>(), units_.as<DevUnit>(),
@@ -466,6 +567,11 @@ gr_status Engine::enqueue_iteration(int cur) {
                                           s_cold_.as<uint4>(), q_slot_[cur].as<uint32_t>(), q_o_[cur].as<float4>(),
                                           q_d_[cur].as<float4>(), q_state_[cur].as<float4>(), C);
     GR_CUDA_TRY(cudaGetLastError());
+    switch (cfg_.width) {
+        case 2: GR_ETRY(launch_loop<2>(c, cur)); break;
+        case 8: GR_ETRY(launch_loop<8>(c, cur)); break;
+        default: GR_ETRY(launch_loop<4>(c, cur));
+    }
     switch (cfg_.width) {
         case 2:
             GR_ETRY(launch_extend_w<2>(cfg_.block, c, cur, jobs_.as<DevJob>(), q_o_[cur].as<float4>(),
@@ -526,6 +632,11 @@ gr_status Engine::add_job(const DevJob& job, uint32_t first_pass, uint32_t passe
     h_jobs_.push_back(job);
     GR_CUDA_TRY(cudaMemcpyAsync(jobs_.as<DevJob>() + index, &h_jobs_.back(), sizeof(DevJob), cudaMemcpyHostToDevice,
                                 st_));
+    if (!path_loop_bounded(job.max_depth, job.rr_depth, job.rr_aggr)) {
+        static const uint32_t off = 1;
+        GR_CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<char*>(ctl_.ptr) + offsetof(EngineCtl, loop_off), &off,
+                                    sizeof(off), cudaMemcpyHostToDevice, st_));
+    }
     std::vector<std::pair<uint32_t, uint32_t>> u;
     for (uint32_t k = 0; k < passes; ++k) u.emplace_back(index, first_pass + k);
     if (!u.empty()) return append_units(u);
@@ -701,6 +812,7 @@ DevJob make_job(gr_scene* scene, const gr_camera& cam, const gr_render_params& p
     j.rr_depth = p.rr_depth;
     j.rr_aggr = p.rr_aggressive_depth;
     j.live = 1;
+    j.order = make_path_order(width, height, 1);
     return j;
 }
 

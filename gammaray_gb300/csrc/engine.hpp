@@ -5,12 +5,14 @@
 // (round-robin over jobs, pass by pass).  A live path's state travels with its ray in
 // the queue; global path p has slot p mod ring of a ring holding its film position and,
 // once it finishes, its radiance.  Every iteration:
-//   plan    (1 thread) picks the finished units to gather (consecutive from the oldest)
+//   plan    (1 block) picks the finished units to gather (consecutive from the oldest)
 //           and how many new paths to issue (queue room, ring slots already gathered)
 //   gather  splats the picked units into their films from their ring slots (the
 //           deterministic tile gather); each film tile adds its job's units in pass
 //           order, every resident block taking (tile, units) items from a counter
 //   fill    starts the next paths in their slots (jitter, camera ray) and queues them
+//   loop    once nothing is left to issue and few paths are live, one launch carries them
+//           to their end (path_loop.cuh); extend and shade then have nothing to do
 //   extend  closest hit for the queued rays of all jobs
 //   shade   path-tracer shading per job, material-sorted; finished paths leave their
 //           radiance in their slot and count their unit done
@@ -23,6 +25,7 @@
 #include <cstdint>
 #include <vector>
 
+#include "path_order.cuh"
 #include "runtime.hpp"
 
 namespace gr {
@@ -36,6 +39,7 @@ struct alignas(16) DevJob {
     uint32_t display;  // display-colour integrator
     uint32_t max_depth, rr_depth, rr_aggr;
     uint32_t live;  // 0: cancelled, its paths are dropped
+    PathOrder order;  // of one pass: the pixel of a unit's n-th path
 };
 
 struct DevUnit {
@@ -67,6 +71,9 @@ struct EngineCtl {
     uint32_t iter;
     uint32_t fetch;  // rays handed out by the refilling extension kernel this iteration
     uint32_t gather_next;  // film-tile items handed out by the gather this iteration
+    uint32_t loop_n;       // paths the path loop carries to their end this iteration
+    uint32_t loop_fetch;   // paths it has handed out
+    uint32_t loop_off;     // set by the host: a job's paths have no bounded length
     // Set by the host (0 = none): gather as soon as every unit below this one has
     // finished, without waiting for a larger batch, so the request those units complete
     // is done within one iteration.
@@ -123,6 +130,8 @@ class Engine {
   private:
     gr_status record_pair();
     gr_status enqueue_iteration(int cur);
+    template <int W>
+    gr_status launch_loop(EngineCtl* c, int cur);
     EngineConfig cfg_;
     cudaStream_t st_ = nullptr;
     uint32_t ring_ = 0;

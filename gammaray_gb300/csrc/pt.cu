@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
         if (!alive) L_buf[slot] = make_float4(L.x, L.y, L.z, 0.0f);
         return alive;
     };
-    count_rays(run_paths<W>(s, stk, n, fetch, err, take, shade), rays);
+    count_rays(run_paths<W>(stk, n, fetch, err, err + 1, [&]() -> const DeviceScene& { return s; }, take, shade), rays);
 }
 
 template <int W, bool CAMERA>
@@ -435,9 +435,8 @@ gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
     p.rr_aggr = rp.rr_aggressive_depth;
     uint64_t launches = 0;
     // Whether the path loop may take this render's short queues (it counts no traversal).
-    const bool bounded = rp.max_depth ? rp.max_depth <= PATH_LOOP_DEPTH
-                                      : std::max(rp.rr_depth, rp.rr_aggressive_depth) <= PATH_LOOP_RR_DEPTH;
-    const bool loop_ok = bounded && !display && !(rp.flags & GR_RENDER_COUNT_TRAVERSAL);
+    const bool loop_ok = path_loop_bounded(rp.max_depth, rp.rr_depth, rp.rr_aggressive_depth) && !display &&
+                         !(rp.flags & GR_RENDER_COUNT_TRAVERSAL);
 
     for (uint32_t done = 0; done < total; done += group) {
         uint32_t g = std::min(group, total - done);

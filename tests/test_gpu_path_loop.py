@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 import gammaray_gb300 as g
-from gammaray_gb300 import _abi, scenes
+from gammaray_gb300 import _abi, batch, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +47,23 @@ def test_path_loop_equals_launches_per_bounce(gpu, width, height, spp, depth, bv
     assert s.extension_rays == s_q.extension_rays and s.samples == s_q.samples
     if depth != 257:
         assert s.kernel_launches < s_q.kernel_launches or depth == 1
+
+
+@pytest.mark.parametrize("capacity", [1024, 1 << 14, 1 << 20])
+@pytest.mark.parametrize("depth", [3, 0, 257])  # 257: deeper than the loop takes
+def test_batch_equals_plain_renders(gpu, capacity, depth):
+    # A pool smaller than one image (its units start in pieces), a few images, and one that
+    # holds everything (the loop takes the queue's end).
+    jobs, refs = [], []
+    for k, (width, height, spp) in enumerate([(61, 47, 3), (33, 8, 5), (128, 96, 2)]):
+        w = scenes.cornell_spheres(width, height) if k else scenes.displaced_sphere(width, height, tris=3000)
+        st = g.Stage(w.prims, lib=gpu, environment=w.environment, seed=k)
+        integ = g.PathTracerIntegrator(max_depth=depth)
+        jobs.append(batch.Job(st, w.camera, integ, g.Film(width, height, lib=gpu), spp))
+        film = g.Film(width, height, lib=gpu)
+        g.Stage(w.prims, lib=gpu, environment=w.environment, seed=k).render(w.camera, integ, film, spp)
+        refs.append(film)
+    batch.render_batch(jobs, gpu, capacity)
+    for j, ref in zip(jobs, refs):
+        for a, b in zip(j.film.read(), ref.read()):
+            np.testing.assert_array_equal(a, b)
