@@ -380,15 +380,7 @@ gr_status gr_film_read(const gr_film* f, float* accum, float* weight) {
     if (!accum && !weight) return GR_OK;
     // The planes are split on the device and copied straight into the caller's arrays
     // (a DMA transfer when the caller's memory is pinned).
-    const size_t n = static_cast<size_t>(f->width) * f->height;
-    GR_CUDA_TRY(f->readback.ensure(n * 4 * sizeof(float)));
-    float* acc_d = f->readback.as<float>();
-    float* w_d = acc_d + 3 * n;
-    GR_TRY(film_split(f->pixels.as<float4>(), static_cast<uint32_t>(n), acc_d, w_d, 0));
-    if (accum) GR_CUDA_TRY(cudaMemcpyAsync(accum, acc_d, 3 * n * sizeof(float), cudaMemcpyDeviceToHost, 0));
-    if (weight) GR_CUDA_TRY(cudaMemcpyAsync(weight, w_d, n * sizeof(float), cudaMemcpyDeviceToHost, 0));
-    GR_CUDA_TRY(cudaStreamSynchronize(0));
-    return GR_OK;
+    return film_planes_to_host(f->pixels.as<float4>(), nullptr, f->width * f->height, f->readback, accum, weight, 0);
 }
 
 gr_status gr_film_resolve(const gr_film* f, float* rgb) {

@@ -338,6 +338,7 @@ struct gr_server {
     Engine engine;
     gr_server_options opts{};
     uint64_t budget = 0, used = 0;
+    DevBuf readback;  // planes of the film being read, the largest read so far
     uint64_t next_id = 1;
     std::vector<std::unique_ptr<ServerRequest>> reqs;
     // Scenes of taken requests that were cancelled while running: their paths may still
@@ -696,26 +697,14 @@ gr_status gr_server_cancel(gr_server* s, uint64_t id) {
 static gr_status copy_film(gr_server* s, const ServerRequest& r, float* accum, float* weight) {
     if (!accum && !weight) return GR_OK;
     const size_t n = static_cast<size_t>(r.req.width) * r.req.height;
-    std::vector<float4> px(n, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-    if (r.film.ptr) {
-        GR_CUDA_TRY(cudaStreamSynchronize(s->engine.stream()));
-        GR_CUDA_TRY(cudaMemcpy(px.data(), r.film.ptr, n * sizeof(float4), cudaMemcpyDeviceToHost));
-        if (r.progressive && r.film2.ptr) {  // even + odd passes
-            std::vector<float4> p2(n);
-            GR_CUDA_TRY(cudaMemcpy(p2.data(), r.film2.ptr, n * sizeof(float4), cudaMemcpyDeviceToHost));
-            for (size_t i = 0; i < n; ++i)
-                px[i] = make_float4(px[i].x + p2[i].x, px[i].y + p2[i].y, px[i].z + p2[i].z, px[i].w + p2[i].w);
-        }
+    if (!r.film.ptr) {
+        if (accum) std::fill(accum, accum + 3 * n, 0.0f);
+        if (weight) std::fill(weight, weight + n, 0.0f);
+        return GR_OK;
     }
-    for (size_t i = 0; i < n; ++i) {
-        if (accum) {
-            accum[3 * i] = px[i].x;
-            accum[3 * i + 1] = px[i].y;
-            accum[3 * i + 2] = px[i].z;
-        }
-        if (weight) weight[i] = px[i].w;
-    }
-    return GR_OK;
+    // On the engine's stream, after whatever it has queued for the film.
+    return film_planes_to_host(r.film.as<float4>(), r.progressive ? r.film2.as<float4>() : nullptr,
+                               static_cast<uint32_t>(n), s->readback, accum, weight, s->engine.stream());
 }
 
 gr_status gr_server_snapshot(gr_server* s, uint64_t id, float* accum, float* weight, uint32_t* passes) {

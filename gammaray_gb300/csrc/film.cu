@@ -124,11 +124,16 @@ __global__ void k_resolve(const float4* __restrict__ film, const float4* __restr
 }
 
 // Film::pixels as two planes: accum (3 floats per pixel) and weight (1 float per pixel).
-__global__ void k_film_split(const float4* __restrict__ film, uint32_t n, float* __restrict__ accum,
-                             float* __restrict__ weight) {
+// With a second film (a progressive request's other half), of their sum.
+__global__ void k_film_split(const float4* __restrict__ film, const float4* __restrict__ film2, uint32_t n,
+                             float* __restrict__ accum, float* __restrict__ weight) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float4 p = film[i];
+    if (film2) {
+        const float4 q = film2[i];
+        p = make_float4(p.x + q.x, p.y + q.y, p.z + q.z, p.w + q.w);
+    }
     accum[3 * i] = p.x;
     accum[3 * i + 1] = p.y;
     accum[3 * i + 2] = p.z;
@@ -198,9 +203,25 @@ gr_status film_resolve(const float4* film, const float4* splat, float splat_scal
     return GR_OK;
 }
 
-gr_status film_split(const float4* film, uint32_t n, float* accum, float* weight, cudaStream_t s) {
-    k_film_split<<<(n + 255) / 256, 256, 0, s>>>(film, n, accum, weight);
+gr_status film_split(const float4* film, const float4* film2, uint32_t n, float* accum, float* weight,
+                     cudaStream_t s) {
+    k_film_split<<<(n + 255) / 256, 256, 0, s>>>(film, film2, n, accum, weight);
     GR_CUDA_TRY(cudaGetLastError());
+    return GR_OK;
+}
+
+gr_status film_planes_to_host(const float4* film, const float4* film2, uint32_t n, DevBuf& planes, float* accum,
+                              float* weight, cudaStream_t s) {
+    GR_CUDA_TRY(planes.ensure(static_cast<size_t>(n) * 4 * sizeof(float)));
+    float* acc_d = planes.as<float>();
+    float* w_d = acc_d + 3 * static_cast<size_t>(n);
+    gr_status r = film_split(film, film2, n, acc_d, w_d, s);
+    if (r != GR_OK) return r;
+    if (accum)
+        GR_CUDA_TRY(cudaMemcpyAsync(accum, acc_d, 3 * static_cast<size_t>(n) * sizeof(float), cudaMemcpyDeviceToHost, s));
+    if (weight)
+        GR_CUDA_TRY(cudaMemcpyAsync(weight, w_d, static_cast<size_t>(n) * sizeof(float), cudaMemcpyDeviceToHost, s));
+    GR_CUDA_TRY(cudaStreamSynchronize(s));
     return GR_OK;
 }
 

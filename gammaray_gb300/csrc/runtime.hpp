@@ -226,8 +226,14 @@ size_t film_sched_words(uint32_t width, uint32_t height);
 // Resolve and EXR packing add splat * splat_scale when splat is not null.
 gr_status film_resolve(const float4* film, const float4* splat, float splat_scale, uint32_t n, float* rgb,
                        cudaStream_t s);
-// Splits the float4 film into an accum plane (3 floats per pixel) and a weight plane.
-gr_status film_split(const float4* film, uint32_t n, float* accum, float* weight, cudaStream_t s);
+// Splits the float4 film (film2: plus a second one, or null) into an accum plane (3 floats
+// per pixel) and a weight plane.
+gr_status film_split(const float4* film, const float4* film2, uint32_t n, float* accum, float* weight,
+                     cudaStream_t s);
+// The planes of film_split in host arrays (either may be null), through `planes`.  Returns
+// once they are there.
+gr_status film_planes_to_host(const float4* film, const float4* film2, uint32_t n, DevBuf& planes, float* accum,
+                              float* weight, cudaStream_t s);
 gr_status film_exr_pack(const float4* film, const float4* splat, float splat_scale, uint32_t width, uint32_t height,
                         unsigned char* out, size_t data_offset, cudaStream_t s);
 
