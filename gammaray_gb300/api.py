@@ -542,7 +542,7 @@ class Stage:
     # ---- ray queries (Bvh::intersect / intersect_naive / visibility / sample_light)
     def intersect(self, rays: np.ndarray) -> np.ndarray:
         rays = np.ascontiguousarray(rays, dtype=np.float32).reshape(-1, 6)
-        hits = np.zeros(len(rays), _abi.HIT_DTYPE)
+        hits = np.empty(len(rays), _abi.HIT_DTYPE)  # every element is written, or the call raises
         self.lib.call("gr_trace_rays", self.handle, fptr(rays), len(rays),
                       hits.ctypes.data_as(C.POINTER(_abi.Hit)))
         return hits
@@ -556,10 +556,10 @@ class Stage:
 
     def visibility(self, pairs: np.ndarray) -> np.ndarray:
         pairs = np.ascontiguousarray(pairs, dtype=np.float32).reshape(-1, 6)
-        vis = np.zeros(len(pairs), np.uint8)
+        vis = np.empty(len(pairs), np.uint8)  # every element is written as 0 or 1
         self.lib.call("gr_visibility", self.handle, fptr(pairs), len(pairs),
                       vis.ctypes.data_as(C.POINTER(C.c_uint8)))
-        return vis.astype(bool)
+        return vis.view(np.bool_)
 
     def sample_light(self, u: np.ndarray) -> np.ndarray:
         u = np.ascontiguousarray(u, dtype=np.float32).reshape(-1, 6)

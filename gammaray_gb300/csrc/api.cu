@@ -9,6 +9,7 @@
 #include <cstring>
 #include <thread>
 #include <fstream>
+#include <initializer_list>
 #include <memory>
 
 #include "runtime.hpp"
@@ -114,17 +115,31 @@ gr_status check_render_params(const gr_render_params* p) {
     return GR_OK;
 }
 
-// Scratch copy-in / copy-out helper for the host-buffer query calls.
+// Device buffers of one host-array query, carved from one allocation.  A scene keeps its
+// own between calls (a query of 1 M rays spent more time in cudaMalloc and cudaFree than in
+// its kernel), at most QUERY_KEEP bytes.
+constexpr size_t QUERY_KEEP = size_t(64) << 20;
 struct Scratch {
-    std::vector<DevBuf*> bufs;
+    DevBuf own;
+    DevBuf& buf;
+    size_t used = 0;
+    Scratch() : buf(own) {}
+    explicit Scratch(gr_scene* s) : buf(s->query) {}
     ~Scratch() {
-        for (DevBuf* b : bufs) delete b;
+        if (buf.bytes > QUERY_KEEP) buf.release();
     }
-    void* get(size_t bytes, cudaError_t& e) {
-        DevBuf* b = new DevBuf();
-        bufs.push_back(b);
-        e = b->ensure(bytes ? bytes : 16);
-        return b->ptr;
+    static size_t padded(size_t bytes) { return (std::max<size_t>(bytes, 16) + 255) & ~size_t(255); }
+    // Room for buffers of these sizes; get() then hands them out in order.
+    cudaError_t reserve(std::initializer_list<size_t> sizes) {
+        size_t total = 0;
+        for (size_t b : sizes) total += padded(b);
+        return buf.ensure(total);
+    }
+    template <class T>
+    T* get(size_t bytes) {
+        T* p = reinterpret_cast<T*>(buf.as<unsigned char>() + used);
+        used += padded(bytes);
+        return p;
     }
 };
 
@@ -557,17 +572,14 @@ gr_status gr_trace_rays(gr_scene* s, const float* rays, uint64_t n, gr_hit* hits
     if (!s || (n && (!rays || !hits))) return fail(GR_ERR_INVALID_ARGUMENT, "null argument");
     if (n == 0) return GR_OK;
     std::lock_guard<std::mutex> g(s->mu);
-    Scratch sc;
-    cudaError_t e;
-    float* dr = static_cast<float*>(sc.get(n * 6 * sizeof(float), e));
-    GR_CUDA_TRY(e);
-    gr_hit* dh = static_cast<gr_hit*>(sc.get(n * sizeof(gr_hit), e));
-    GR_CUDA_TRY(e);
-    int* derr = static_cast<int*>(sc.get(sizeof(int), e));
-    GR_CUDA_TRY(e);
+    Scratch sc(s);
+    GR_CUDA_TRY(sc.reserve({n * 6 * sizeof(float), n * sizeof(gr_hit), sizeof(int)}));
+    float* dr = sc.get<float>(n * 6 * sizeof(float));
+    gr_hit* dh = sc.get<gr_hit>(n * sizeof(gr_hit));
+    int* derr = sc.get<int>(sizeof(int));
     GR_CUDA_TRY(cudaMemsetAsync(derr, 0, sizeof(int), s->stream));
     GR_CUDA_TRY(cudaMemcpyAsync(dr, rays, n * 6 * sizeof(float), cudaMemcpyHostToDevice, s->stream));
-    GR_TRY(launch_trace(s->dev, dr, n, dh, false, nullptr, derr, s->stream));
+    GR_TRY(launch_trace(s->dev, dr, n, dh, derr, s->stream));
     GR_CUDA_TRY(cudaMemcpyAsync(hits, dh, n * sizeof(gr_hit), cudaMemcpyDeviceToHost, s->stream));
     int herr = 0;
     GR_CUDA_TRY(cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
@@ -581,19 +593,17 @@ gr_status gr_trace_rays_dev(gr_scene* s, const float* rays, uint64_t n, gr_hit* 
     if (!s || (n && (!rays || !hits))) return fail(GR_ERR_INVALID_ARGUMENT, "null argument");
     GR_CUDA_TRY(s->counters.ensure(NUM_COUNTERS * sizeof(uint32_t)));
     int* err = reinterpret_cast<int*>(s->counters.as<uint32_t>() + CNT_ERROR);
-    return launch_trace(s->dev, rays, n, hits, false, nullptr, err, static_cast<cudaStream_t>(stream));
+    return launch_trace(s->dev, rays, n, hits, err, static_cast<cudaStream_t>(stream));
 }
 
 gr_status gr_intersect_naive(gr_scene* s, const float* rays, uint64_t n, gr_hit* hits) {
     if (!s || (n && (!rays || !hits))) return fail(GR_ERR_INVALID_ARGUMENT, "null argument");
     if (n == 0) return GR_OK;
     std::lock_guard<std::mutex> g(s->mu);
-    Scratch sc;
-    cudaError_t e;
-    float* dr = static_cast<float*>(sc.get(n * 6 * sizeof(float), e));
-    GR_CUDA_TRY(e);
-    gr_hit* dh = static_cast<gr_hit*>(sc.get(n * sizeof(gr_hit), e));
-    GR_CUDA_TRY(e);
+    Scratch sc(s);
+    GR_CUDA_TRY(sc.reserve({n * 6 * sizeof(float), n * sizeof(gr_hit)}));
+    float* dr = sc.get<float>(n * 6 * sizeof(float));
+    gr_hit* dh = sc.get<gr_hit>(n * sizeof(gr_hit));
     GR_CUDA_TRY(cudaMemcpyAsync(dr, rays, n * 6 * sizeof(float), cudaMemcpyHostToDevice, s->stream));
     GR_TRY(launch_naive(s->dev, dr, n, dh, s->stream));
     GR_CUDA_TRY(cudaMemcpyAsync(hits, dh, n * sizeof(gr_hit), cudaMemcpyDeviceToHost, s->stream));
@@ -605,14 +615,11 @@ gr_status gr_visibility(gr_scene* s, const float* pairs, uint64_t n, uint8_t* vi
     if (!s || (n && (!pairs || !visible))) return fail(GR_ERR_INVALID_ARGUMENT, "null argument");
     if (n == 0) return GR_OK;
     std::lock_guard<std::mutex> g(s->mu);
-    Scratch sc;
-    cudaError_t e;
-    float* dp = static_cast<float*>(sc.get(n * 6 * sizeof(float), e));
-    GR_CUDA_TRY(e);
-    uint8_t* dv = static_cast<uint8_t*>(sc.get(n, e));
-    GR_CUDA_TRY(e);
-    int* derr = static_cast<int*>(sc.get(sizeof(int), e));
-    GR_CUDA_TRY(e);
+    Scratch sc(s);
+    GR_CUDA_TRY(sc.reserve({n * 6 * sizeof(float), n, sizeof(int)}));
+    float* dp = sc.get<float>(n * 6 * sizeof(float));
+    uint8_t* dv = sc.get<uint8_t>(n);
+    int* derr = sc.get<int>(sizeof(int));
     GR_CUDA_TRY(cudaMemsetAsync(derr, 0, sizeof(int), s->stream));
     GR_CUDA_TRY(cudaMemcpyAsync(dp, pairs, n * 6 * sizeof(float), cudaMemcpyHostToDevice, s->stream));
     GR_TRY(launch_visibility(s->dev, dp, n, dv, derr, s->stream));
@@ -630,12 +637,10 @@ gr_status gr_sample_light(gr_scene* s, const float* u, uint64_t n, gr_light_samp
     if (s->dev.num_lights == 0) return fail(GR_ERR_INVALID_ARGUMENT, "scene has no lights");
     if (n == 0) return GR_OK;
     std::lock_guard<std::mutex> g(s->mu);
-    Scratch sc;
-    cudaError_t e;
-    float* du = static_cast<float*>(sc.get(n * 6 * sizeof(float), e));
-    GR_CUDA_TRY(e);
-    gr_light_sample* dout = static_cast<gr_light_sample*>(sc.get(n * sizeof(gr_light_sample), e));
-    GR_CUDA_TRY(e);
+    Scratch sc(s);
+    GR_CUDA_TRY(sc.reserve({n * 6 * sizeof(float), n * sizeof(gr_light_sample)}));
+    float* du = sc.get<float>(n * 6 * sizeof(float));
+    gr_light_sample* dout = sc.get<gr_light_sample>(n * sizeof(gr_light_sample));
     GR_CUDA_TRY(cudaMemcpyAsync(du, u, n * 6 * sizeof(float), cudaMemcpyHostToDevice, s->stream));
     GR_TRY(launch_sample_light(s->dev, du, n, dout, s->stream));
     GR_CUDA_TRY(cudaMemcpyAsync(out, dout, n * sizeof(gr_light_sample), cudaMemcpyDeviceToHost, s->stream));
@@ -651,27 +656,22 @@ static gr_status bsdf_call(int op, const gr_material_desc* md, uint64_t n, const
     if (!build_material(*md, m, err)) return fail(GR_ERR_INVALID_ARGUMENT, err);
     if (n == 0) return GR_OK;
     Scratch sc;
-    cudaError_t e;
-    DevMaterial* dm = static_cast<DevMaterial*>(sc.get(sizeof(DevMaterial), e));
-    GR_CUDA_TRY(e);
-    gr_frame* df = static_cast<gr_frame*>(sc.get(n * sizeof(gr_frame), e));
-    GR_CUDA_TRY(e);
-    float* dwi = static_cast<float*>(sc.get(n * 3 * sizeof(float), e));
-    GR_CUDA_TRY(e);
+    const size_t v3_bytes = n * 3 * sizeof(float);
+    GR_CUDA_TRY(sc.reserve({sizeof(DevMaterial), n * sizeof(gr_frame), v3_bytes, v3_bytes, v3_bytes, out_bytes}));
+    DevMaterial* dm = sc.get<DevMaterial>(sizeof(DevMaterial));
+    gr_frame* df = sc.get<gr_frame>(n * sizeof(gr_frame));
+    float* dwi = sc.get<float>(v3_bytes);
     float* dwo = nullptr;
     float* du = nullptr;
     if (wo) {
-        dwo = static_cast<float*>(sc.get(n * 3 * sizeof(float), e));
-        GR_CUDA_TRY(e);
-        GR_CUDA_TRY(cudaMemcpy(dwo, wo, n * 3 * sizeof(float), cudaMemcpyHostToDevice));
+        dwo = sc.get<float>(v3_bytes);
+        GR_CUDA_TRY(cudaMemcpy(dwo, wo, v3_bytes, cudaMemcpyHostToDevice));
     }
     if (u) {
-        du = static_cast<float*>(sc.get(n * 3 * sizeof(float), e));
-        GR_CUDA_TRY(e);
-        GR_CUDA_TRY(cudaMemcpy(du, u, n * 3 * sizeof(float), cudaMemcpyHostToDevice));
+        du = sc.get<float>(v3_bytes);
+        GR_CUDA_TRY(cudaMemcpy(du, u, v3_bytes, cudaMemcpyHostToDevice));
     }
-    void* dout = sc.get(out_bytes, e);
-    GR_CUDA_TRY(e);
+    void* dout = sc.get<unsigned char>(out_bytes);
     GR_CUDA_TRY(cudaMemcpy(dm, &m, sizeof(m), cudaMemcpyHostToDevice));
     GR_CUDA_TRY(cudaMemcpy(df, fr, n * sizeof(gr_frame), cudaMemcpyHostToDevice));
     GR_CUDA_TRY(cudaMemcpy(dwi, wi, n * 3 * sizeof(float), cudaMemcpyHostToDevice));

@@ -1,6 +1,8 @@
 // Batched queries behind gr_trace_rays / gr_intersect_naive / gr_visibility /
-// gr_sample_light / gr_bsdf_*: one thread per query, used by the parity tests and by
-// callers that bring their own rays.
+// gr_sample_light / gr_bsdf_*, used by the parity tests and by callers that bring their own
+// rays.  Rays go through the warps' queue traversal, the other queries take a thread each.
+#include <algorithm>
+
 #include "runtime.hpp"
 #include "traverse.cuh"
 
@@ -28,21 +30,54 @@ GR_D void write_hit(const DeviceScene& s, gr_hit* out, const TraceResult& r) {
     *out = h;
 }
 
-template <int W, bool ANY>
+// A warp's share of n rays: every warps-th chunk of `chunk` rays, so that a costly part of
+// the rays is spread over all warps.  Few rays: smaller chunks, down to a ray per warp, since
+// lanes of a warp wait for each other's steps.  A share needs no counter in memory, so
+// queries on several streams at once share nothing.
+struct WarpShare {
+    uint32_t warps, warp;
+    uint32_t chunk, rays;       // rays of this warp
+    mutable uint32_t next = 0;  // the first one not taken yet
+    GR_D WarpShare(uint64_t n)
+        : warps(gridDim.x * (blockDim.x >> 5)), warp((threadIdx.x >> 5) * gridDim.x + blockIdx.x) {
+        const uint64_t each = (n + warps - 1) / warps;
+        chunk = each < 32u ? static_cast<uint32_t>(each) : 32u;
+        const uint64_t chunks = (n + chunk - 1) / chunk;
+        const uint64_t mine = warp < chunks ? (chunks - 1 - warp) / warps + 1 : 0;
+        rays = static_cast<uint32_t>(mine * chunk);
+        if (mine && (chunks - 1) % warps == warp) rays -= static_cast<uint32_t>(chunks * chunk - n);
+    }
+    GR_D uint32_t operator()(uint32_t k, unsigned) const {
+        const uint32_t base = next;
+        next += k;
+        return base;
+    }
+    // The warp's q-th ray (a chunk smaller than 32 is its only one).
+    GR_D uint64_t ray(uint32_t q) const {
+        return chunk == 32u ? (static_cast<uint64_t>(q >> 5) * warps + warp) * 32u + (q & 31u) : warp * chunk + q;
+    }
+};
+
+// Closest hits.  One ray per thread, a warp waiting for its longest ray, took 453 us for 1 M
+// rays (half toward a mesh of 102,422 triangles, half leaving its surface) and 53 us for 257
+// on 10,000; the shares 391 and 29.
+template <int W>
 __global__ void __launch_bounds__(QUERY_BLOCK) k_trace(DeviceScene s, const float* __restrict__ rays, uint64_t n,
-                                                       gr_hit* __restrict__ hits, const float* __restrict__ tmax,
-                                                       int* err) {
+                                                       gr_hit* __restrict__ hits, int* err) {
     extern __shared__ unsigned char smem[];
     int2 spill[MAX_STACK - SMEM_STACK];
     const auto stk = thread_stack<QUERY_BLOCK>(smem, spill);
-    uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float* r = rays + 6 * i;
-    V3 o = V3{r[0], r[1], r[2]};
-    V3 d = V3{r[3], r[4], r[5]};
-    float tm = tmax ? tmax[i] : FLT_MAX;
-    TraceResult res = trace_ray<W, ANY>(s, o, d, tm, stk, err);
-    write_hit(s, hits + i, res);
+    const WarpShare share(n);
+    trace_queue<W, false, false>(
+        share.rays, stk, err, nullptr, nullptr, share, [&]() -> const DeviceScene& { return s; },
+        [&](uint32_t q, TravState& t) {
+            const float* r = rays + 6 * share.ray(q);
+            trav_init(t, V3{r[0], r[1], r[2]}, V3{r[3], r[4], r[5]}, FLT_MAX);
+            return true;
+        },
+        [&](uint32_t q, const TravState& t) {
+            write_hit(s, hits + share.ray(q), TraceResult{t.closest, t.hit, t.hu, t.hv});
+        });
 }
 
 __global__ void k_naive(DeviceScene s, const float* __restrict__ rays, uint64_t n, gr_hit* __restrict__ hits) {
@@ -76,22 +111,25 @@ __global__ void __launch_bounds__(QUERY_BLOCK) k_visibility(DeviceScene s, const
     extern __shared__ unsigned char smem[];
     int2 spill[MAX_STACK - SMEM_STACK];
     const auto stk = thread_stack<QUERY_BLOCK>(smem, spill);
-    uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float* p = pairs + 6 * i;
-    V3 a = V3{p[0], p[1], p[2]};
-    V3 b = V3{p[3], p[4], p[5]};
-    // Bvh::visibility (geom/bvh.rs:460-477): a shadow ray from `a`, nudged, against
-    // target distance - 1e-3; any hit closer than that occludes.
-    if (fabsf(a.x - b.x) < 1e-3f && fabsf(a.y - b.y) < 1e-3f && fabsf(a.z - b.z) < 1e-3f) {
-        vis[i] = 0;
-        return;
-    }
-    V3 d = normalized(b - a);
-    V3 o = nudge(a, d);
-    float target = magnitude(b - o);
-    TraceResult r = trace_ray<W, true>(s, o, d, target - 1e-3f, stk, err);
-    vis[i] = r.k < 0 ? 1 : 0;
+    const WarpShare share(n);
+    trace_queue<W, true, false>(
+        share.rays, stk, err, nullptr, nullptr, share, [&]() -> const DeviceScene& { return s; },
+        [&](uint32_t q, TravState& t) {
+            const float* p = pairs + 6 * share.ray(q);
+            V3 a = V3{p[0], p[1], p[2]};
+            V3 b = V3{p[3], p[4], p[5]};
+            // Bvh::visibility (geom/bvh.rs:460-477): a shadow ray from `a`, nudged, against
+            // target distance - 1e-3; any hit closer than that occludes.
+            if (fabsf(a.x - b.x) < 1e-3f && fabsf(a.y - b.y) < 1e-3f && fabsf(a.z - b.z) < 1e-3f) {
+                vis[share.ray(q)] = 0;
+                return false;
+            }
+            V3 d = normalized(b - a);
+            V3 o = nudge(a, d);
+            trav_init(t, o, d, magnitude(b - o) - 1e-3f);
+            return true;
+        },
+        [&](uint32_t q, const TravState& t) { vis[share.ray(q)] = t.hit < 0 ? 1 : 0; });
 }
 
 __global__ void k_sample_light(DeviceScene s, const float* __restrict__ u, uint64_t n, gr_light_sample* out) {
@@ -168,42 +206,40 @@ __global__ void k_bsdf(int op, const DevMaterial* __restrict__ mp, uint64_t n, c
 
 unsigned blocks_for(uint64_t n, int b) { return static_cast<unsigned>((n + b - 1) / b); }
 
+// Blocks for n rays: every resident one, or one warp per ray when there are fewer.
+template <class K>
+unsigned share_blocks(K kernel, size_t smem, uint64_t n) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, QUERY_BLOCK, smem) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+    const uint64_t need = (n + QUERY_BLOCK / 32 - 1) / (QUERY_BLOCK / 32);
+    return static_cast<unsigned>(std::min<uint64_t>(need, static_cast<uint64_t>(per_sm) * device_sm_count()));
+}
+
 template <int W>
-gr_status trace_w(const DeviceScene& s, const float* rays, uint64_t n, gr_hit* hits, bool any, const float* tmax,
-                  int* err, cudaStream_t st) {
-    size_t smem = step_stack_smem_bytes(QUERY_BLOCK);
-    if (any) {
-        GR_CUDA_TRY(cudaFuncSetAttribute(k_trace<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem)));
-        k_trace<W, true><<<blocks_for(n, QUERY_BLOCK), QUERY_BLOCK, smem, st>>>(s, rays, n, hits, tmax, err);
-    } else {
-        GR_CUDA_TRY(cudaFuncSetAttribute(k_trace<W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem)));
-        k_trace<W, false><<<blocks_for(n, QUERY_BLOCK), QUERY_BLOCK, smem, st>>>(s, rays, n, hits, tmax, err);
-    }
+gr_status trace_w(const DeviceScene& s, const float* rays, uint64_t n, gr_hit* hits, int* err, cudaStream_t st) {
+    const size_t smem = step_stack_smem_bytes(QUERY_BLOCK);
+    k_trace<W><<<share_blocks(k_trace<W>, smem, n), QUERY_BLOCK, smem, st>>>(s, rays, n, hits, err);
     GR_CUDA_TRY(cudaGetLastError());
     return GR_OK;
 }
 
 template <int W>
 gr_status vis_w(const DeviceScene& s, const float* pairs, uint64_t n, uint8_t* vis, int* err, cudaStream_t st) {
-    size_t smem = step_stack_smem_bytes(QUERY_BLOCK);
-    GR_CUDA_TRY(
-        cudaFuncSetAttribute(k_visibility<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    k_visibility<W><<<blocks_for(n, QUERY_BLOCK), QUERY_BLOCK, smem, st>>>(s, pairs, n, vis, err);
+    const size_t smem = step_stack_smem_bytes(QUERY_BLOCK);
+    k_visibility<W><<<share_blocks(k_visibility<W>, smem, n), QUERY_BLOCK, smem, st>>>(s, pairs, n, vis, err);
     GR_CUDA_TRY(cudaGetLastError());
     return GR_OK;
 }
 
 }  // namespace
 
-gr_status launch_trace(const DeviceScene& s, const float* rays, uint64_t n, gr_hit* hits, bool any_hit,
-                       const float* tmax, int* err, cudaStream_t st) {
+gr_status launch_trace(const DeviceScene& s, const float* rays, uint64_t n, gr_hit* hits, int* err, cudaStream_t st) {
     if (n == 0) return GR_OK;
     switch (s.width) {
-        case 2: return trace_w<2>(s, rays, n, hits, any_hit, tmax, err, st);
-        case 4: return trace_w<4>(s, rays, n, hits, any_hit, tmax, err, st);
-        case 8: return trace_w<8>(s, rays, n, hits, any_hit, tmax, err, st);
+        case 2: return trace_w<2>(s, rays, n, hits, err, st);
+        case 4: return trace_w<4>(s, rays, n, hits, err, st);
+        case 8: return trace_w<8>(s, rays, n, hits, err, st);
     }
     set_error("unsupported BVH width");
     return GR_ERR_INTERNAL;

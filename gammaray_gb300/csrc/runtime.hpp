@@ -148,6 +148,7 @@ struct gr_scene {
     gr::SceneBuffers buf;
     gr::DeviceScene dev{};
     gr::DevBuf counters;  // [0..1] queue counts, [2] error flag, [3..] stats (gr::CNT_*)
+    gr::DevBuf query;     // buffers of the host-array queries, kept between calls (guarded by mu)
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     gr_render_stats stats{};
@@ -184,8 +185,7 @@ gr_status build_bvh_device(const HostBuild& h, SceneBuffers& b, cudaStream_t st,
                            uint32_t& stack_depth, uint64_t& bytes);
 
 // Kernel-side entry points (implemented in the .cu files).
-gr_status launch_trace(const DeviceScene& s, const float* rays, uint64_t n, gr_hit* hits, bool any_hit,
-                       const float* tmax, int* err, cudaStream_t st);
+gr_status launch_trace(const DeviceScene& s, const float* rays, uint64_t n, gr_hit* hits, int* err, cudaStream_t st);
 gr_status launch_naive(const DeviceScene& s, const float* rays, uint64_t n, gr_hit* hits, cudaStream_t st);
 gr_status launch_visibility(const DeviceScene& s, const float* pairs, uint64_t n, uint8_t* vis, int* err,
                             cudaStream_t st);
