@@ -24,8 +24,9 @@ GR_D void write_hit(const DeviceScene& s, gr_hit* out, const TraceResult& r) {
         h.t = r.t;
         h.prim = __float_as_int(__ldg(pr).w);
         h.component = __float_as_int(__ldg(pr + 1).w);
-        h.u = r.u;
-        h.v = r.v;
+        const bool triangle = __float_as_int(__ldg(pr + 2).w) == PRIM_TRIANGLE;  // a sphere's test leaves u and v unset
+        h.u = triangle ? r.u : 0.0f;
+        h.v = triangle ? r.v : 0.0f;
     }
     *out = h;
 }

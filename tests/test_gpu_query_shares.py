@@ -30,3 +30,18 @@ def test_shares_answer_every_query(gpu, bvh):
     for n in (1, 2, 31, 33, 257, 5471, 20_000, 175_105):
         np.testing.assert_array_equal(st.intersect(rays[:n]), hits[:n])
         np.testing.assert_array_equal(st.visibility(pairs[:n]), vis[:n])
+
+
+def test_sphere_hits_have_no_barycentrics(gpu):
+    """u and v of a sphere hit are 0, whatever triangle the same warp met before."""
+    w = scenes.displaced_sphere(8, 8, tris=3000)
+    ball = g.Sphere(w.prims[0].material, g.Mat.translation((1.3, 0.2, 0.1)), 0.5)
+    st = g.Stage([w.prims[0], ball], lib=gpu)
+    rng = np.random.default_rng(4)
+    o = rng.standard_normal((20_000, 3)) * 2.0
+    d = rng.standard_normal((20_000, 3)) - o
+    rays = np.concatenate([o, d / np.linalg.norm(d, axis=1, keepdims=True)], 1).astype(np.float32)
+    for hits in (st.intersect(rays), st.intersect_naive(rays)):
+        sphere = hits["prim"] == 1
+        assert sphere.sum() > 500 and (hits["prim"] == 0).sum() > 500
+        assert not hits["u"][sphere].any() and not hits["v"][sphere].any()
