@@ -218,7 +218,10 @@ gr_status gr_scene_create(const gr_scene_desc* desc, gr_scene** out) {
     auto t0 = std::chrono::steady_clock::now();
     std::unique_ptr<gr_scene> s(new gr_scene());
     std::string err;
-    if (!build_scene(*desc, s->host, err)) return fail(GR_ERR_INVALID_ARGUMENT, err);
+    // With the records left to the device, what fails is named by the host's own checks,
+    // which meet the first failing triangle or prim first.
+    if (!build_scene(*desc, s->host, err, false, true) && !build_scene(*desc, s->host, err))
+        return fail(GR_ERR_INVALID_ARGUMENT, err);
     GR_CUDA_TRY(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     GR_CUDA_TRY(cudaEventCreate(&s->ev0));
     GR_CUDA_TRY(cudaEventCreate(&s->ev1));
@@ -228,7 +231,12 @@ gr_status gr_scene_create(const gr_scene_desc* desc, gr_scene** out) {
     uint64_t total = 0;
     if (h.device_build) {
         uint32_t num_wide = 0, stack_depth = 0;
-        GR_TRY(build_bvh_device(h, b, st, num_wide, stack_depth, total));
+        const gr_status built = build_bvh_device(*desc, h, b, st, num_wide, stack_depth, total);
+        if (built == GR_ERR_INVALID_ARGUMENT) {
+            HostBuild checked;
+            return build_scene(*desc, checked, err) ? built : fail(built, err);
+        }
+        GR_TRY(built);
         h.num_wide_nodes = num_wide;
         h.stack_depth = stack_depth;
     } else {

@@ -179,10 +179,11 @@ struct gr_film {
 
 namespace gr {
 
-// Device BVH build (bvh_build.cu) for a HostBuild made with GR_BUILD_DEVICE_LBVH:
-// fills b.nodes, b.prims, b.tri_nidx, b.tri_uvidx (leaf order).
-gr_status build_bvh_device(const HostBuild& h, SceneBuffers& b, cudaStream_t st, uint32_t& num_wide,
-                           uint32_t& stack_depth, uint64_t& bytes);
+// Device BVH build (bvh_build.cu) for a HostBuild made from `desc` with
+// GR_BUILD_DEVICE_LBVH: fills b.nodes, b.prims, b.tri_nidx, b.tri_uvidx (leaf order).
+// GR_ERR_INVALID_ARGUMENT: h.device_records, and an index of desc is out of range.
+gr_status build_bvh_device(const gr_scene_desc& desc, const HostBuild& h, SceneBuffers& b, cudaStream_t st,
+                           uint32_t& num_wide, uint32_t& stack_depth, uint64_t& bytes);
 
 // Kernel-side entry points (implemented in the .cu files).
 gr_status launch_trace(const DeviceScene& s, const float* rays, uint64_t n, gr_hit* hits, int* err, cudaStream_t st);

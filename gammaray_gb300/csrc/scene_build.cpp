@@ -798,6 +798,10 @@ static bool build_lobes(const gr_material_desc& d, DevMaterial& m, std::string& 
     return true;
 }
 
+// See build_scene: fewest components and most prims of a scene whose records the device makes.
+static constexpr size_t DEVICE_RECORDS_MIN = 2048;
+static constexpr uint32_t DEVICE_RECORDS_PRIMS = 64;
+
 bool build_material(const gr_material_desc& d, DevMaterial& m, std::string& err) {
     if (!build_lobes(d, m, err)) return false;
     // The shading sort's key for the material's mixture: its lobe count and types.
@@ -845,7 +849,8 @@ static uint64_t tree_hash(const BinNodes& nodes, int32_t root, const std::vector
     return h;
 }
 
-bool build_scene(const gr_scene_desc& desc, HostBuild& out, std::string& err, bool want_tree_hash) {
+bool build_scene(const gr_scene_desc& desc, HostBuild& out, std::string& err, bool want_tree_hash,
+                 bool device_records) {
     out = HostBuild();
     uint32_t W = desc.bvh_width ? desc.bvh_width : 4;
     if (W != 2 && W != 4 && W != 8) {
@@ -869,14 +874,36 @@ bool build_scene(const gr_scene_desc& desc, HostBuild& out, std::string& err, bo
     }
     // Component list in prim order (Bvh::build, bvh.rs:340-350), with mesh data offsets.
     std::vector<Item> items;
-    {
-        size_t total = 0;
-        for (uint32_t p = 0; p < desc.num_prims && desc.prims; ++p)
-            total += desc.prims[p].kind == GR_PRIM_MESH ? desc.prims[p].num_tris : 1;
-        items.reserve(total);
+    size_t total = 0, vertices = 0;
+    for (uint32_t p = 0; p < desc.num_prims && desc.prims; ++p) {
+        const bool mesh = desc.prims[p].kind == GR_PRIM_MESH;
+        total += mesh ? desc.prims[p].num_tris : 1;
+        vertices += mesh ? desc.prims[p].num_vertices : 0;
     }
+    // The device makes the records of large scenes of few prims (a few copies per prim)
+    // whose meshes have no more vertices than their triangles can name (so that a small
+    // mesh cut from a large vertex array uploads only its records): 400,000 triangles took 1.5 to 2.5 ms on 16 host threads and 0.4 ms to upload, against
+    // 0.1 ms of index and vertex uploads and 20 us there.
+    out.device_records = device_records && desc.build == GR_BUILD_DEVICE_LBVH &&
+                         total >= DEVICE_RECORDS_MIN && desc.num_prims <= DEVICE_RECORDS_PRIMS &&
+                         vertices <= 3 * total;
+    if (!out.device_records) items.reserve(total);
     std::vector<uint32_t> vbase(desc.num_prims, 0), nbase(desc.num_prims, 0), ubase(desc.num_prims, 0);
     uint32_t nrm_total = 0, uv_total = 0;
+    auto add_attributes = [&](uint32_t p, const gr_prim_desc& d) {
+        if (d.tri_normals && d.num_normals) {
+            out.any_normals = true;
+            nbase[p] = nrm_total;
+            nrm_total += d.num_normals;
+            out.normals.insert(out.normals.end(), d.normals, d.normals + 3 * d.num_normals);
+        }
+        if (d.tri_uvs && d.num_uvs) {
+            out.any_uvs = true;
+            ubase[p] = uv_total;
+            uv_total += d.num_uvs;
+            out.uvs.insert(out.uvs.end(), d.uvs, d.uvs + 2 * d.num_uvs);
+        }
+    };
     for (uint32_t p = 0; p < desc.num_prims; ++p) {
         const gr_prim_desc& d = desc.prims[p];
         if (d.material >= desc.num_materials) {
@@ -889,6 +916,7 @@ bool build_scene(const gr_scene_desc& desc, HostBuild& out, std::string& err, bo
                 err = "sphere radius must be > 0";
                 return false;
             }
+            if (out.device_records) continue;
             Item it;
             it.prim = p;
             it.comp = 0;
@@ -903,11 +931,16 @@ bool build_scene(const gr_scene_desc& desc, HostBuild& out, std::string& err, bo
                 err = "mesh " + std::to_string(p) + " has no triangles";
                 return false;
             }
+            if (out.device_records && !out.materials[d.material].has_light) {
+                add_attributes(p, d);
+                continue;
+            }
             // Triangle t: its index checks (0: fine, else the first that fails) and its
-            // item.  Large meshes run on threads; the error reported is the first
+            // item (a light mesh with device records: the checks only, for the light
+            // tables).  Large meshes run on threads; the error reported is the first
             // failing triangle's, as in a serial pass.
             const size_t ibase = items.size();
-            items.resize(ibase + d.num_tris);
+            if (!out.device_records) items.resize(ibase + d.num_tris);
             auto triangle = [&](uint32_t t) -> int {
                 for (int k = 0; k < 3; ++k)
                     if (d.tri_vertices[3 * t + k] >= d.num_vertices) return 1;
@@ -917,6 +950,7 @@ bool build_scene(const gr_scene_desc& desc, HostBuild& out, std::string& err, bo
                 if (d.tri_uvs)
                     for (int k = 0; k < 3; ++k)
                         if (d.tri_uvs[3 * t + k] >= d.num_uvs) return 3;
+                if (out.device_records) return 0;
                 Item& it = items[ibase + t];
                 it.prim = p;
                 it.comp = t;
@@ -946,29 +980,18 @@ bool build_scene(const gr_scene_desc& desc, HostBuild& out, std::string& err, bo
                 err = c == 1 ? "vertex index out of range" : (c == 2 ? "normal index out of range" : "uv index out of range");
                 return false;
             }
-            if (d.tri_normals && d.num_normals) {
-                out.any_normals = true;
-                nbase[p] = nrm_total;
-                nrm_total += d.num_normals;
-                out.normals.insert(out.normals.end(), d.normals, d.normals + 3 * d.num_normals);
-            }
-            if (d.tri_uvs && d.num_uvs) {
-                out.any_uvs = true;
-                ubase[p] = uv_total;
-                uv_total += d.num_uvs;
-                out.uvs.insert(out.uvs.end(), d.uvs, d.uvs + 2 * d.num_uvs);
-            }
+            add_attributes(p, d);
         } else {
             err = "unknown prim kind";
             return false;
         }
     }
-    out.num_components = items.size();
-    if (items.empty()) {
+    out.num_components = total;
+    if (total == 0) {
         err = "scene has no components";
         return false;
     }
-    if (items.size() >= (1u << (31 - LEAF_COUNT_BITS))) {
+    if (total >= (1u << (31 - LEAF_COUNT_BITS))) {
         err = "too many components";
         return false;
     }
@@ -981,6 +1004,10 @@ bool build_scene(const gr_scene_desc& desc, HostBuild& out, std::string& err, bo
 
     // Primitive records: in leaf order for the host build, in component order for the
     // device build (which sorts them itself, bvh_build.cu).
+    if (out.device_records) {
+        out.nbase = nbase;
+        out.ubase = ubase;
+    }
     out.prims.resize(items.size() * 12);  // not filled: put_record writes all 12 floats
     if (out.any_normals) out.tri_normal_idx.assign(items.size() * 3, NO_INDEX);
     if (out.any_uvs) out.tri_uv_idx.assign(items.size() * 3, NO_INDEX);
