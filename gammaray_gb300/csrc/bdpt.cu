@@ -473,32 +473,48 @@ __global__ void __launch_bounds__(BSBLOCK, 768 / BSBLOCK)
     }
 }
 
-// Carries a queue's walks to their end (run_paths, wavefront.cuh).
+// A walk in the path loop; without the MIS extension its second half stays behind.
+struct LoopWalk {
+    uint32_t slot, unused;
+    Walk w;
+};
+static_assert(sizeof(Walk) == 64, "its first half is the walk without the MIS extension");
+template <bool MIS>
+constexpr int loop_words() {
+    return MIS ? 18 : 10;
+}
+
+// Carries a queue's walks to their end (run_paths).
 template <int W, bool MIS>
-__global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
+__global__ void __launch_bounds__(PATH_LOOP_THREADS, PATH_LOOP_BLOCKS)
     k_bdpt_walks(DeviceScene s, BdptParams p, Verts vs, PathOut out, const uint32_t* __restrict__ count,
                  const uint32_t* __restrict__ q_slot, const float4* __restrict__ q_o, const float4* __restrict__ q_d,
                  const float4* __restrict__ q_state, uint32_t* fetch, int* err, unsigned long long* rays) {
     extern __shared__ unsigned char smem[];
     int2 spill[MAX_STACK - SMEM_STACK];
-    const auto stk = thread_stack<BLOCK>(smem, spill);
+    const auto stk = thread_stack<PATH_LOOP_THREADS>(smem, spill);
     const uint32_t n = *count;
     if (n == 0) return;
-    uint32_t slot = 0;
-    Walk w{};
-    auto take = [&](uint32_t q, V3& o, V3& d) {
-        slot = q_slot[q];
+    auto take = [&](uint32_t q, LoopWalk& path, V3& o, V3& d) {
+        path.slot = q_slot[q];
+        path.unused = 0;
         const float4 o4 = q_o[q], d4 = q_d[q];
         o = V3{o4.x, o4.y, o4.z};
         d = V3{d4.x, d4.y, d4.z};
-        w = load_walk<MIS>(q_state, q);
-        return true;
+        path.w = load_walk<MIS>(q_state, q);
     };
-    auto shade = [&](uint32_t, const TravState& t, V3& no, V3& nd) {
-        const float4 h = make_float4(t.closest, __int_as_float(t.hit), t.hu, t.hv);
-        return walk_vertex<MIS>(s, p, vs, out, slot, w, ANY_LOBE, t.o, t.d, h, no, nd);
+    auto bucket = [&](const LoopWalk& path, int32_t k) {
+        const uint32_t walk = path.slot & 1u;
+        const uint32_t dim = (walk ? DIM_LIGHT_WALK : DIM_CAMERA_WALK) + 4 * path.w.k;
+        return shade_bucket(s, k, uniform01(path.w.key, dim), walk);
     };
-    count_rays(run_paths<W>(stk, n, fetch, err, err + 1, [&]() -> const DeviceScene& { return s; }, take, shade), rays);
+    auto shade = [&](LoopWalk& path, uint32_t lobe, V3 o, V3 d, float4 h, V3& no, V3& nd) {
+        return walk_vertex<MIS>(s, p, vs, out, path.slot, path.w, lobe, o, d, h, no, nd);
+    };
+    count_rays(run_paths<W, loop_words<MIS>(), LoopWalk>(
+                   stk, smem, n, fetch, err, err + 1, s.num_components >= GROUPED_COMPONENTS,
+                   [&]() -> const DeviceScene& { return s; }, take, bucket, shade),
+               rays);
 }
 
 // Capacities of the strategy entries and of the shadow queue, as BdptState::ensure sizes
@@ -1008,11 +1024,12 @@ gr_status shadow_launch(const DeviceScene& s, uint32_t cap, uint32_t* counters, 
 template <int W, bool MIS>
 gr_status walks_launch(const DeviceScene& s, const BdptParams& p, const Verts& vs, const PathOut& out, uint32_t most,
                        BdptState& bs, int cur, uint32_t* cnt, int* err, unsigned long long* rays, cudaStream_t st) {
-    const size_t smem = step_stack_smem_bytes(BLOCK);
-    const int grid = path_loop_grid(k_bdpt_walks<W, MIS>, smem, most);
-    k_bdpt_walks<W, MIS><<<grid, BLOCK, smem, st>>>(s, p, vs, out, cnt + CNT_LOOP, bs.q_slot[cur].as<uint32_t>(),
-                                                    bs.q_o[cur].as<float4>(), bs.q_d[cur].as<float4>(),
-                                                    bs.q_state[cur].as<float4>(), cnt + CNT_LOOP_FETCH, err, rays);
+    const size_t smem = path_loop_smem_bytes(loop_words<MIS>());
+    int grid;
+    GR_TRY_S(path_loop_grid(k_bdpt_walks<W, MIS>, smem, most, grid));
+    k_bdpt_walks<W, MIS><<<grid, PATH_LOOP_THREADS, smem, st>>>(
+        s, p, vs, out, cnt + CNT_LOOP, bs.q_slot[cur].as<uint32_t>(), bs.q_o[cur].as<float4>(),
+        bs.q_d[cur].as<float4>(), bs.q_state[cur].as<float4>(), cnt + CNT_LOOP_FETCH, err, rays);
     GR_CUDA_TRY(cudaGetLastError());
     return GR_OK;
 }

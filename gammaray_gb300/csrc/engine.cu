@@ -335,48 +335,61 @@ GR_D bool shade_job(const DevJob& J, uint32_t depth, uint64_t key, uint32_t lobe
     return !is_zero(tp) && (J.max_depth == 0 || depth + 1 < J.max_depth);
 }
 
+// Shading bucket of a hit: misses, cancelled and display-colour jobs share bucket 0.
+GR_D uint32_t job_bucket(const DevJob& J, int32_t k, uint64_t key, uint32_t depth) {
+    if (!J.live || J.display || k < 0) return 0u;
+    return shade_bucket(J.scene, k, uniform01(key, DIM_CAMERA_WALK + 4 * depth), 0);
+}
+
+// A path in the path loop.
+struct LoopPath {
+    V3 tp, L;
+    uint64_t key;
+    uint32_t slot, depth, job, unused;
+};
+constexpr int LOOP_WORDS = 11;  // all but `unused`
+
 // Carries the queue's last paths to their end (run_paths), as the plan decides.
 template <int W>
-__global__ void __launch_bounds__(EBLOCK, PATH_LOOP_BLOCKS)
+__global__ void __launch_bounds__(PATH_LOOP_THREADS, PATH_LOOP_BLOCKS)
     k_eng_loop(EngineCtl* c, const DevJob* __restrict__ jobs, uint32_t* unit_done, const uint32_t* __restrict__ q_slot,
                const float4* __restrict__ q_o, const float4* __restrict__ q_d, const float4* __restrict__ q_state,
                float4* __restrict__ s_hot, const uint4* __restrict__ s_cold) {
     extern __shared__ unsigned char smem[];
     int2 spill[MAX_STACK - SMEM_STACK];
-    const auto stk = thread_stack<EBLOCK>(smem, spill);
+    const auto stk = thread_stack<PATH_LOOP_THREADS>(smem, spill);
     const uint32_t n = c->loop_n;
     if (n == 0) return;
     TraceScene s{nullptr, nullptr, 0u};
-    V3 tp, L;
-    uint64_t key = 0;
-    uint32_t slot = 0, job = 0, depth = 0;
-    auto take = [&](uint32_t q, V3& o, V3& d) {
+    auto take = [&](uint32_t q, LoopPath& path, V3& o, V3& d) {
         const float4 o4 = q_o[q], d4 = q_d[q];
         const float4 ha = q_state[2 * static_cast<size_t>(q)], hb = q_state[2 * static_cast<size_t>(q) + 1];
-        slot = q_slot[q];
-        job = __float_as_uint(o4.w);
-        depth = __float_as_uint(d4.w);
-        const DeviceScene& js = jobs[job].scene;
+        path.slot = q_slot[q];
+        path.job = __float_as_uint(o4.w);
+        path.depth = __float_as_uint(d4.w);
+        const DeviceScene& js = jobs[path.job].scene;
         s = TraceScene{js.nodes, js.prims, js.step_budget};
         o = V3{o4.x, o4.y, o4.z};
         d = V3{d4.x, d4.y, d4.z};
-        tp = V3{ha.x, ha.y, ha.z};
-        L = V3{ha.w, hb.x, hb.y};
-        key = state_key(hb);
-        return true;
+        path.tp = V3{ha.x, ha.y, ha.z};
+        path.L = V3{ha.w, hb.x, hb.y};
+        path.key = state_key(hb);
     };
-    auto shade = [&](uint32_t, const TravState& t, V3& no, V3& nd) {
-        const float4 h = make_float4(t.closest, __int_as_float(t.hit), t.hu, t.hv);
-        const bool alive = shade_job(jobs[job], depth, key, ANY_LOBE, t.o, t.d, h, tp, L, no, nd);
-        ++depth;
+    auto bucket = [&](const LoopPath& path, int32_t k) {
+        return job_bucket(jobs[path.job], k, path.key, path.depth);
+    };
+    auto shade = [&](LoopPath& path, uint32_t lobe, V3 o, V3 d, float4 h, V3& no, V3& nd) {
+        const bool alive = shade_job(jobs[path.job], path.depth, path.key, lobe, o, d, h, path.tp, path.L, no, nd);
+        ++path.depth;
         if (!alive) {
-            s_hot[slot] = make_float4(L.x, L.y, L.z, 0.0f);
-            atomicAdd(unit_done + s_cold[slot].x, 1u);
+            s_hot[path.slot] = make_float4(path.L.x, path.L.y, path.L.z, 0.0f);
+            atomicAdd(unit_done + s_cold[path.slot].x, 1u);
         }
         return alive;
     };
-    count_rays(run_paths<W>(stk, n, &c->loop_fetch, &c->err, nullptr, [&]() -> const TraceScene& { return s; }, take,
-                            shade),
+    count_rays(run_paths<W, LOOP_WORDS, LoopPath>(
+                   stk, smem, n, &c->loop_fetch, &c->err, nullptr, true, [&]() -> const TraceScene& { return s; }, take,
+                   bucket, shade),
                &c->rays);
 }
 
@@ -401,12 +414,9 @@ __global__ void __launch_bounds__(ESBLOCK, 768 / ESBLOCK)
         const uint32_t cn = min(chunk, n - c0);
         sort_chunk<ESBLOCK, ESHADE_PER_THREAD>(sm, cn, per, [&](uint32_t i) {
             uint32_t q = c0 + i;
-            uint32_t jb = __float_as_uint(q_o[q].w);
-            const DevJob& J = jobs[jb];
-            int32_t k = __float_as_int(q_hit[q].y);
-            if (!J.live || J.display || k < 0) return 0u;
-            uint64_t key = state_key(q_state[2 * static_cast<size_t>(q) + 1]);
-            return shade_bucket(J.scene, k, uniform01(key, DIM_CAMERA_WALK + 4 * __float_as_uint(q_d[q].w)), 0);
+            const uint64_t key = state_key(q_state[2 * static_cast<size_t>(q) + 1]);
+            return job_bucket(jobs[__float_as_uint(q_o[q].w)], __float_as_int(q_hit[q].y), key,
+                              __float_as_uint(q_d[q].w));
         });
         for (uint32_t e = 0; e < per; ++e) {
             uint32_t i = e * ESBLOCK + threadIdx.x;
@@ -542,12 +552,12 @@ gr_status Engine::init(const EngineConfig& cfg, cudaStream_t) {
 
 template <int W>
 gr_status Engine::launch_loop(EngineCtl* c, int cur) {
-    const size_t smem = step_stack_smem_bytes(EBLOCK);
-    const int grid = grid_for(reinterpret_cast<const void*>(k_eng_loop<W>), EBLOCK, smem, cfg_.capacity);
-    k_eng_loop<W><<<grid, EBLOCK, smem, st_>>>(c, jobs_.as<DevJob>(), unit_done_.as<uint32_t>(),
-                                               q_slot_[cur].as<uint32_t>(), q_o_[cur].as<float4>(),
-                                               q_d_[cur].as<float4>(), q_state_[cur].as<float4>(),
-                                               s_hot_.as<float4>(), s_cold_.as<uint4>());
+    const size_t smem = path_loop_smem_bytes(LOOP_WORDS);
+    static_assert(path_loop_smem_bytes(LOOP_WORDS) <= 48 * 1024, "no attribute needed");
+    const int grid = grid_for(reinterpret_cast<const void*>(k_eng_loop<W>), PATH_LOOP_THREADS, smem, cfg_.capacity);
+    k_eng_loop<W><<<grid, PATH_LOOP_THREADS, smem, st_>>>(
+        c, jobs_.as<DevJob>(), unit_done_.as<uint32_t>(), q_slot_[cur].as<uint32_t>(), q_o_[cur].as<float4>(),
+        q_d_[cur].as<float4>(), q_state_[cur].as<float4>(), s_hot_.as<float4>(), s_cold_.as<uint4>());
     GR_CUDA_TRY(cudaGetLastError());
     return GR_OK;
 }

@@ -284,57 +284,68 @@ struct PathQueue {
     const float4* state;
 };
 
+// A path in the path loop.
+struct LoopPath {
+    V3 tp, L;
+    uint64_t key;
+    uint32_t slot, depth;
+};
+
 // Carries paths to their end (run_paths): CAMERA, the n_paths paths of a group from their
 // camera rays (no queue; their film positions are written here); else the queue of bounce
-// `depth0`.  Bound by latency: dependent node and record loads of one traversal step
-// after another, and the instruction fetch of the shading code.
+// `depth0`.  Bound by latency: the chain of dependent instructions of one traversal step
+// after another (7 cycles each) of a block's slowest ray, for which its warps wait half of
+// the time.
 template <int W, bool CAMERA>
-__global__ void __launch_bounds__(BLOCK, PATH_LOOP_BLOCKS)
+__global__ void __launch_bounds__(PATH_LOOP_THREADS, PATH_LOOP_BLOCKS)
     k_pt_finish(DeviceScene s, PTParams p, uint32_t depth0, uint32_t n_paths, PathQueue queue, float2* __restrict__ st,
                 float4* __restrict__ L_buf, uint32_t* fetch, int* err, unsigned long long* rays) {
     extern __shared__ unsigned char smem[];
     int2 spill[MAX_STACK - SMEM_STACK];
-    const auto stk = thread_stack<BLOCK>(smem, spill);
+    const auto stk = thread_stack<PATH_LOOP_THREADS>(smem, spill);
     const uint32_t n = CAMERA ? n_paths : *queue.count;
     if (n == 0) return;
-    V3 tp, L;
-    uint64_t key = 0;
-    uint32_t slot = 0, depth = 0;
-    auto take = [&](uint32_t q, V3& o, V3& d) {
-        depth = depth0;
+    auto take = [&](uint32_t q, LoopPath& path, V3& o, V3& d) {
+        path.depth = depth0;
         if (CAMERA) {
-            slot = camera_path(p, q, st, key, o, d);
-            tp = v3one();
-            L = v3zero();
+            path.slot = camera_path(p, q, st, path.key, o, d);
+            path.tp = v3one();
+            path.L = v3zero();
         } else {
-            slot = queue.slot[q];
+            path.slot = queue.slot[q];
             const float4 o4 = queue.o[q], d4 = queue.d[q];
             const float4 sa = queue.state[2 * static_cast<size_t>(q)], sb = queue.state[2 * static_cast<size_t>(q) + 1];
             o = V3{o4.x, o4.y, o4.z};
             d = V3{d4.x, d4.y, d4.z};
-            tp = V3{sa.x, sa.y, sa.z};
-            L = V3{sa.w, sb.x, sb.y};
-            key = state_key(sb);
+            path.tp = V3{sa.x, sa.y, sa.z};
+            path.L = V3{sa.w, sb.x, sb.y};
+            path.key = state_key(sb);
         }
-        return true;
     };
-    auto shade = [&](uint32_t, const TravState& t, V3& no, V3& nd) {
-        const float4 h = make_float4(t.closest, __int_as_float(t.hit), t.hu, t.hv);
-        const bool alive = shade_hit(s, p, depth, key, ANY_LOBE, t.o, t.d, h, tp, L, no, nd);
-        ++depth;
-        if (!alive) L_buf[slot] = make_float4(L.x, L.y, L.z, 0.0f);
+    auto bucket = [&](const LoopPath& path, int32_t k) {
+        return shade_bucket(s, k, uniform01(path.key, DIM_CAMERA_WALK + 4 * path.depth), 0);
+    };
+    auto shade = [&](LoopPath& path, uint32_t lobe, V3 o, V3 d, float4 h, V3& no, V3& nd) {
+        const bool alive = shade_hit(s, p, path.depth, path.key, lobe, o, d, h, path.tp, path.L, no, nd);
+        ++path.depth;
+        if (!alive) L_buf[path.slot] = make_float4(path.L.x, path.L.y, path.L.z, 0.0f);
         return alive;
     };
-    count_rays(run_paths<W>(stk, n, fetch, err, err + 1, [&]() -> const DeviceScene& { return s; }, take, shade), rays);
+    count_rays(run_paths<W, sizeof(LoopPath) / 4, LoopPath>(
+                   stk, smem, n, fetch, err, err + 1, s.num_components >= GROUPED_COMPONENTS,
+                   [&]() -> const DeviceScene& { return s; }, take, bucket, shade),
+               rays);
 }
 
 template <int W, bool CAMERA>
 gr_status launch_finish_w(const DeviceScene& s, const PTParams& p, uint32_t depth, uint32_t most, const PathQueue& q,
                           float2* film_pos, float4* L_buf, uint32_t* fetch, int* err, unsigned long long* rays,
                           cudaStream_t st) {
-    const size_t smem = step_stack_smem_bytes(BLOCK);
-    const int grid = path_loop_grid(k_pt_finish<W, CAMERA>, smem, most);
-    k_pt_finish<W, CAMERA><<<grid, BLOCK, smem, st>>>(s, p, depth, most, q, film_pos, L_buf, fetch, err, rays);
+    const size_t smem = path_loop_smem_bytes(sizeof(LoopPath) / 4);
+    int grid;
+    GR_TRY_S(path_loop_grid(k_pt_finish<W, CAMERA>, smem, most, grid));
+    k_pt_finish<W, CAMERA>
+        <<<grid, PATH_LOOP_THREADS, smem, st>>>(s, p, depth, most, q, film_pos, L_buf, fetch, err, rays);
     GR_CUDA_TRY(cudaGetLastError());
     return GR_OK;
 }

@@ -364,26 +364,26 @@ GR_D bool pop_next(TravState& t, const K& stk) {
     return false;
 }
 
-// One traversal step.  Returns true when the ray is finished (t.hit / t.closest hold
-// the closest hit).  With ANY_HIT it finishes at the first hit closer than t_max.
+// One traversal step towards the closest hit.  Returns true when the ray is finished (t.hit
+// / t.closest hold the hit).
 // S is DeviceScene or TraceScene: the step functions read only `nodes` and `prims`.
-template <int W, bool ANY_HIT, bool COUNT, class S, class K>
-GR_D bool trav_step(const S& s, TravState& t, const K& stk, int* err, uint32_t* counts) {
+template <int W, class S, class K>
+GR_D bool trav_step(const S& s, TravState& t, const K& stk, int* err) {
     if (t.ref >= 0) {
         bool overflow = false;
-        bool descended = visit_node<W, COUNT>(s, t, stk, err, counts, overflow);
+        const bool descended = visit_node<W, false>(s, t, stk, err, nullptr, overflow);
         if (overflow) {
             t.hit = -1;
             return true;
         }
         if (descended) return false;
-    } else if (visit_leaf<ANY_HIT, COUNT>(s, t, t.ref, counts)) {
-        return true;
+    } else {
+        visit_leaf<false, false>(s, t, t.ref, nullptr);
     }
     return !pop_next(t, stk);
 }
 
-inline size_t step_stack_smem_bytes(int threads) {
+GR_HD constexpr size_t step_stack_smem_bytes(int threads) {
     return static_cast<size_t>(SMEM_STACK) * threads * (sizeof(int32_t) + sizeof(float));
 }
 
@@ -395,26 +395,146 @@ GR_D StackView<STRIDE> thread_stack(unsigned char* smem, int2* spill) {
     return StackView<STRIDE>{reinterpret_cast<int2*>(smem) + threadIdx.x, spill};
 }
 
-// Traces one ray to the end.  ANY_HIT: stops at the first hit closer than t_max (shadow
-// rays).  A miss returns t = t_max and k = -1.  A ray that needs more than the scene's
-// step budget is abandoned as a miss and flagged: *err = 2 and, if err_ray is given, the
-// ray's index there.  A stack overflow (impossible for trees the builds accept) sets
-// *err = 1.  With COUNT, counts[0] / counts[1] accumulate nodes visited / primitives
-// tested.
-template <int W, bool ANY_HIT, bool COUNT = false, class K>
-GR_D TraceResult trace_ray(const DeviceScene& s, V3 o, V3 d, float t_max, const K& stk, int* err,
-                           int* err_ray = nullptr, uint32_t ray = 0, uint32_t* counts = nullptr) {
-    TravState t;
-    trav_init(t, o, d, t_max);
-    uint32_t steps = 0;
-    while (!trav_step<W, ANY_HIT, COUNT>(s, t, stk, err, counts)) {
-        if (++steps > s.step_budget) {
-            atomicExch(err, 2);
-            if (err_ray) atomicExch(err_ray, static_cast<int>(ray));
-            return TraceResult{t_max, -1, 0.0f, 0.0f};
+// ---------------------------------------------------------------------------
+// A lane's scene, held by lane `src`.
+GR_D TraceScene scene_of(const TraceScene& s, int src) {
+    return TraceScene{reinterpret_cast<const float4*>(
+                          __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(s.nodes), src)),
+                      reinterpret_cast<const float4*>(
+                          __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(s.prims), src)),
+                      __shfl_sync(0xffffffffu, s.step_budget, src)};
+}
+GR_D TraceScene scene_of(const DeviceScene& s, int) { return TraceScene{s.nodes, s.prims, s.step_budget}; }
+
+// Closest hits of the rays of the lanes in `mask` (at most 32 / W), W lanes each: a lane
+// tests one child of a node or one primitive of a leaf.  The same tests, order and hits as
+// trav_step, whose some 250 dependent instructions per node are what a ray alone in its warp
+// waits for.  `steps` counts on; a ray whose stack would outgrow its shared part is given
+// back unfinished (deep), one that runs out of steps with `over` set; the others end.  Every
+// lane of the warp calls it with the same mask.
+template <int W, class S, class K>
+GR_D void trace_grouped(unsigned mask, const S& scene, TravState& t, uint32_t& steps, const K& stk, bool& deep,
+                        bool& over) {
+    constexpr unsigned all = 0xffffffffu, ones = (1u << W) - 1u;
+    const unsigned lane = threadIdx.x & 31u, j = lane % W, g0 = lane - j;
+    const float inflate = 1.0f + 2.0f * gamma_n(3.0f);
+    unsigned rest = mask;
+    for (unsigned k = 0; k < lane / W; ++k) rest &= rest - 1u;
+    bool on = rest != 0u, out = false, late = false;
+    const int src = on ? __ffs(rest) - 1 : static_cast<int>(lane);
+    const TraceScene s = scene_of(scene, src);
+    auto of = [&](float x) { return __shfl_sync(all, x, src); };
+    const V3 o = V3{of(t.o.x), of(t.o.y), of(t.o.z)}, d = V3{of(t.d.x), of(t.d.y), of(t.d.z)};
+    const V3 inv = V3{of(t.inv.x), of(t.inv.y), of(t.inv.z)};
+    float closest = of(t.closest), hu = of(t.hu), hv = of(t.hv);
+    int32_t ref = __shfl_sync(all, t.ref, src), hit = __shfl_sync(all, t.hit, src);
+    int sp = __shfl_sync(all, t.sp, src);
+    uint32_t n = __shfl_sync(all, steps, src);
+    // Rows of this lane's child: near and far planes by the ray's direction signs.
+    const uint32_t xn = (d.x < 0.0f ? 3 : 0) * W + j, xf = (d.x < 0.0f ? 0 : 3) * W + j;
+    const uint32_t yn = (d.y < 0.0f ? 4 : 1) * W + j, yf = (d.y < 0.0f ? 1 : 4) * W + j;
+    const uint32_t zn = (d.z < 0.0f ? 5 : 2) * W + j, zf = (d.z < 0.0f ? 2 : 5) * W + j;
+    int2* col = stk.at(0) + (src - static_cast<int>(lane));
+    // The next stacked child that can hold a closer hit, as pop_next.
+    auto next = [&](bool want) {
+        bool found = false;
+        while (want && !found && sp > 0) {
+            --sp;
+            const int2 e = col[sp * K::stride];
+            found = __int_as_float(e.y) < closest;
+            ref = e.x;
+        }
+        if (want && !found) on = false;
+    };
+    __syncwarp();
+    for (;;) {
+        if (on && n > s.step_budget) {
+            on = false;
+            late = true;
+        }
+        if (on && sp + W - 1 > SMEM_STACK) {
+            on = false;
+            out = true;
+        }
+        if (!__any_sync(all, on)) break;
+        const bool node = on && ref >= 0;
+        if (__any_sync(all, node)) {
+            uint32_t key = KEY_MISS;
+            int32_t child = 0;
+            if (node) {
+                const float* f = reinterpret_cast<const float*>(s.nodes + static_cast<size_t>(ref) * (2 * W));
+                const float ax = __ldg(f + xn), ay = __ldg(f + yn), az = __ldg(f + zn);
+                const float bx = __ldg(f + xf), by = __ldg(f + yf), bz = __ldg(f + zf);
+                child = __float_as_int(__ldg(f + 6 * W + j));
+                const float tmin = fmaxf(fmaxf((ax - o.x) * inv.x, (ay - o.y) * inv.y), (az - o.z) * inv.z);
+                const float tmax = fminf(fminf((bx - o.x) * inv.x, (by - o.y) * inv.y), (bz - o.z) * inv.z) * inflate;
+                const float te = fmaxf(tmin, 0.0f);
+                if (te <= tmax && te < closest) key = (__float_as_uint(te) & ~7u) | j;
+                ++n;
+            }
+            uint32_t rank = 0;
+#pragma unroll
+            for (int x = 1; x < W; ++x) rank += __shfl_xor_sync(all, key, x) < key ? 1u : 0u;
+            const unsigned hits = (__ballot_sync(all, key != KEY_MISS) >> g0) & ones;
+            const unsigned first = (__ballot_sync(all, key != KEY_MISS && rank == 0u) >> g0) & ones;
+            const int32_t near = __shfl_sync(all, child, static_cast<int>(g0) + (first ? __ffs(first) - 1 : 0));
+            const int far = __popc(hits) - 1;
+            if (key != KEY_MISS && rank > 0u)
+                col[(sp + far - static_cast<int>(rank)) * K::stride] = make_int2(child, static_cast<int>(key & ~7u));
+            if (node && hits) {
+                sp += far;
+                ref = near;
+            }
+            __syncwarp();
+            next(node && !hits);
+        }
+        const bool leaf = on && ref < 0;
+        if (__any_sync(all, leaf)) {
+            const uint32_t enc = ~static_cast<uint32_t>(ref), at = enc >> LEAF_COUNT_BITS;
+            const uint32_t count = leaf ? (enc & (MAX_LEAF_PRIMS - 1)) + 1 : 0u;
+            for (uint32_t b = 0; __any_sync(all, b < count); b += W) {
+                float dist = 0.0f, u = 0.0f, v = 0.0f;
+                if (b + j < count) {
+                    const float4* pr = s.prims + 3 * static_cast<size_t>(at + b + j);
+                    dist = intersect_prim(__ldg(pr), __ldg(pr + 1), __ldg(pr + 2), o, d, u, v);
+                }
+                float best = dist != 0.0f && dist < closest ? dist : FLT_MAX;
+                const float mine = best;
+#pragma unroll
+                for (int x = 1; x < W; x <<= 1) best = fminf(best, __shfl_xor_sync(all, best, x));
+                const unsigned won = (__ballot_sync(all, mine == best && best < FLT_MAX) >> g0) & ones;
+                const int w = static_cast<int>(g0) + (won ? __ffs(won) - 1 : 0);
+                u = __shfl_sync(all, u, w);
+                v = __shfl_sync(all, v, w);
+                if (won) {
+                    closest = best;
+                    hit = static_cast<int32_t>(at + b) + (w - static_cast<int>(g0));
+                    hu = u;
+                    hv = v;
+                }
+            }
+            if (leaf) ++n;
+            next(leaf);
         }
     }
-    return TraceResult{t.closest, t.hit, t.hu, t.hv};
+    __syncwarp();
+    const int from = static_cast<int>(W * __popc(mask & ((1u << lane) - 1u))) & 31;
+    const float fc = __shfl_sync(all, closest, from), fu = __shfl_sync(all, hu, from), fv = __shfl_sync(all, hv, from);
+    const int32_t fr = __shfl_sync(all, ref, from), fh = __shfl_sync(all, hit, from);
+    const int fs = __shfl_sync(all, sp, from);
+    const uint32_t fn = __shfl_sync(all, n, from);
+    const int state = __shfl_sync(all, (out ? 1 : 0) | (late ? 2 : 0), from);
+    if ((mask >> lane) & 1u) {
+        t.closest = fc;
+        t.hu = fu;
+        t.hv = fv;
+        t.ref = fr;
+        t.hit = fh;
+        t.sp = fs;
+        steps = fn;
+        deep = state & 1;
+        over = state & 2;
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -71,10 +71,12 @@ int resident_grid(K kernel, size_t smem, uint32_t n, int block = BLOCK) {
     return static_cast<int>(std::max(1u, std::min(need, cap)));
 }
 
-// Grid of a path-loop kernel (blocks of BLOCK threads) for at most `most` paths.
+// Grid of a path-loop kernel for at most `most` paths; `smem` is the block's.
 template <class K>
-int path_loop_grid(K kernel, size_t smem, uint32_t most) {
-    return resident_grid(kernel, smem, (most + PATH_LOOP_MIN_LANES - 1) / PATH_LOOP_MIN_LANES * 32u);
+gr_status path_loop_grid(K kernel, size_t smem, uint32_t most, int& grid) {
+    if (smem > 48 * 1024) GR_CUDA_TRY(allow_sort_smem(kernel, smem));
+    grid = resident_grid(kernel, smem, (most + PATH_LOOP_MIN_LANES - 1) / PATH_LOOP_MIN_LANES * 32u, PATH_LOOP_THREADS);
+    return GR_OK;
 }
 
 // The start of a bounce whose queue is `cur`: a queue of at most `take` paths goes to the
