@@ -229,17 +229,26 @@ gr_status gr_scene_create(const gr_scene_desc* desc, gr_scene** out) {
     SceneBuffers& b = s->buf;
     cudaStream_t st = s->stream;
     uint64_t total = 0;
-    if (h.device_build) {
+    bool built = false;
+    if (h.device_build || h.device_sah) {
         uint32_t num_wide = 0, stack_depth = 0;
-        const gr_status built = build_bvh_device(*desc, h, b, st, num_wide, stack_depth, total);
-        if (built == GR_ERR_INVALID_ARGUMENT) {
+        const gr_status bs =
+            build_bvh_device(*desc, h, b, st, num_wide, stack_depth, h.num_binary_nodes, total);
+        if (bs == GR_ERR_INVALID_ARGUMENT && !h.device_sah) {
             HostBuild checked;
-            return build_scene(*desc, checked, err) ? built : fail(built, err);
+            return build_scene(*desc, checked, err) ? bs : fail(bs, err);
         }
-        GR_TRY(built);
-        h.num_wide_nodes = num_wide;
-        h.stack_depth = stack_depth;
-    } else {
+        if (bs != GR_OK && !h.device_sah) return bs;
+        built = bs == GR_OK;
+        if (built) {
+            h.num_wide_nodes = num_wide;
+            h.stack_depth = stack_depth;
+        } else {
+            cudaGetLastError();  // (an allocation that was refused)
+            if (!build_scene(*desc, h, err)) return fail(GR_ERR_INVALID_ARGUMENT, err);
+        }
+    }
+    if (!built) {
         GR_TRY(upload(b.nodes, h.nodes, st, total));
         GR_TRY(upload(b.prims, h.prims, st, total));
         GR_TRY(upload(b.tri_nidx, h.tri_normal_idx, st, total));

@@ -1,5 +1,6 @@
-// Device BVH build (GR_BUILD_DEVICE_LBVH): a linear BVH made on the GPU, then collapsed
-// into the same wide node layout as the host build, so traversal is unchanged.
+// Device BVH builds: a binary tree made on the GPU, then collapsed into the same wide node
+// layout as the host build, so traversal is unchanged.  GR_BUILD_DEVICE_LBVH makes a linear
+// BVH, as follows; the reference's SAH tree of large scenes is sah_build.cuh's.
 //
 //   records    boxes and primitive records from the caller's vertex and index arrays, with
 //              the index checks (large scenes of few prims; else the host makes them)
@@ -21,10 +22,14 @@
 //              stack use (the host collapse's: the largest sum of children - 1 along a path)
 //   permute    primitive records and attribute indices into leaf order
 //
-// The tree differs from the reference's SAH tree; closest hits do not (a ray keeps the
+// The linear tree differs from the reference's SAH tree; closest hits do not (a ray keeps the
 // nearest hit over all primitives), except that a tie at exactly equal distance may go
 // to the other primitive.
+#include <algorithm>
 #include <cfloat>
+#include <memory>
+#include <string>
+#include <utility>
 #include <vector>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -432,6 +437,16 @@ __global__ void k_permute(const float4* __restrict__ rec, const uint32_t* __rest
         for (int q = 0; q < 3; ++q) tu_out[3 * static_cast<size_t>(k) + q] = tu[3 * static_cast<size_t>(s) + q];
 }
 
+}  // namespace
+
+}  // namespace gr
+
+#include "sah_build.cuh"
+
+namespace gr {
+
+namespace {
+
 // One allocation carved into the build's scratch buffers: sizes are added first, then
 // reserve() makes the pointers valid.
 struct Slab {
@@ -455,18 +470,105 @@ cudaError_t put(void* dst, const T* src, size_t count, cudaStream_t st) {
     return cudaMemcpyAsync(dst, src, count * sizeof(T), cudaMemcpyHostToDevice, st);
 }
 
+// The order and the binary tree of the SAH build (sah_build.cuh): the host launches levels
+// of large nodes, SAH_LEVELS_AT_ONCE at a time (10 for 400,000 triangles), then the rest.
+constexpr uint32_t SAH_LEVELS_AT_ONCE = 12;
+
+struct SahScratch {
+    size_t ctl, order[2], bucket, moved, tile_left, best, left, small;
+    size_t nodes[2], tables[2], first_out[2], tile0[2], tiles[2];
+    uint32_t max_big, max_tiles, max_small;
+    SahScratch(Slab& m, uint32_t n) {
+        max_big = n / (SAH_SMALL + 1) + 1;
+        max_tiles = n / SAH_TILE + max_big + 1;
+        max_small = 2 * SAH_LEVELS * max_big;  // every large node leaves two at most
+        ctl = m.add(sizeof(SahCtl));
+        for (int k = 0; k < 2; ++k) {
+            order[k] = m.add(n * sizeof(uint32_t));
+            nodes[k] = m.add(max_big * sizeof(SahNode));
+            tables[k] = m.add(size_t(max_big) * SAH_BUCKETS * SAH_VALUES * sizeof(int));
+            first_out[k] = m.add(max_big * sizeof(uint32_t));
+            tile0[k] = m.add(max_big * sizeof(uint32_t));
+            tiles[k] = m.add(max_tiles * sizeof(uint2));
+        }
+        bucket = m.add(n);
+        moved = m.add(n * sizeof(uint32_t));
+        tile_left = m.add(max_tiles * sizeof(uint32_t));
+        best = m.add(max_big * sizeof(uint32_t));
+        left = m.add(max_big * sizeof(uint32_t));
+        small = m.add(max_small * sizeof(SahSmall));
+    }
+    SahView view(const Slab& m, const float* box, Opened* opened, uint32_t n) const {
+        SahView v;
+        v.ctl = m.at<SahCtl>(ctl);
+        v.box = box;
+        for (int k = 0; k < 2; ++k) {
+            v.order[k] = m.at<uint32_t>(order[k]);
+            v.level[k] = SahLevel{m.at<SahNode>(nodes[k]), m.at<int>(tables[k]), m.at<uint32_t>(first_out[k]),
+                                  m.at<uint32_t>(tile0[k]), m.at<uint2>(tiles[k])};
+        }
+        v.bucket = m.at<uint8_t>(bucket);
+        v.moved = m.at<uint32_t>(moved);
+        v.tile_left = m.at<uint32_t>(tile_left);
+        v.best = m.at<uint32_t>(best);
+        v.left = m.at<uint32_t>(left);
+        v.small = m.at<SahSmall>(small);
+        v.opened = reinterpret_cast<float*>(opened);
+        v.n = n;
+        v.max_big = max_big;
+        v.max_tiles = max_tiles;
+        v.max_small = max_small;
+        return v;
+    }
+};
+
+// GR_ERR_INTERNAL: the host build has to make this tree.
+gr_status sah_tree(const SahView& v, uint32_t* perm, cudaStream_t st, int& root) {
+    SahCtl h{};
+    for (int a = 0; a < 12; ++a) h.bounds[a] = a / 3 % 2 ? static_cast<int>(0x80000000u) : 0x7FFFFFFF;
+    GR_CUDA_TRY(cudaMemcpyAsync(v.ctl, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+    const uint32_t sms = static_cast<uint32_t>(device_sm_count());
+    k_sah_bounds<<<std::min((v.n + BB - 1) / BB, sms * 4u), BB, 0, st>>>(v);
+    GR_CUDA_TRY(cudaGetLastError());
+    k_sah_root<<<1, 32, 0, st>>>(v);
+    GR_CUDA_TRY(cudaGetLastError());
+    const uint32_t grid = std::min(v.max_tiles, sms * 8u);
+    for (uint32_t level = 0;;) {
+        const uint32_t stop = std::min(level + SAH_LEVELS_AT_ONCE, SAH_LEVELS);
+        for (; level < stop; ++level) {
+            k_sah_buckets<<<grid, BB, 0, st>>>(v, level);
+            k_sah_count<<<grid, BB, 0, st>>>(v, level);
+            k_sah_front<<<grid, BB, 0, st>>>(v, level);
+            k_sah_back<<<grid, BB, 0, st>>>(v, level);
+            GR_CUDA_TRY(cudaGetLastError());
+        }
+        GR_CUDA_TRY(cudaMemcpyAsync(&h, v.ctl, sizeof(h), cudaMemcpyDeviceToHost, st));
+        GR_CUDA_TRY(cudaStreamSynchronize(st));
+        if (h.failed || (h.big[level] && level == SAH_LEVELS)) {
+            set_error("device BVH build: left to the host");
+            return GR_ERR_INTERNAL;
+        }
+        if (h.big[level] == 0) break;
+    }
+    k_sah_small<<<std::min(h.small, sms * 4u), BB, sizeof(SahTree), st>>>(v, perm);
+    GR_CUDA_TRY(cudaGetLastError());
+    root = h.root;
+    return GR_OK;
+}
+
 // Levels launched before the host looks how many there were (18 for 400,000 triangles; an
 // empty level costs its launch).  A read-back per level and one launch per level for the
 // stack use took 930 us there, this way 330.
 constexpr uint32_t LEVELS_AT_ONCE = 22;
 
+// `root_ref`: the binary tree's root node (of a single component: its leaf, ~0).
 template <int W>
-gr_status collapse_levels(uint32_t n, CollapseCtl* ctl, const int* err, int4* todo, const Opened* opened,
+gr_status collapse_levels(int root_ref, uint32_t n, CollapseCtl* ctl, const int* err, int4* todo, const Opened* opened,
                           const float* box, const uint32_t* perm, uint32_t leaf_size, SceneBuffers& b,
                           cudaStream_t st, uint32_t& num_wide, uint32_t& stack_depth) {
     // Every wide node stands for a distinct binary node (or the root leaf): at most n.
     GR_CUDA_TRY(b.nodes.ensure(static_cast<size_t>(n) * 8 * W * sizeof(float)));
-    const int4 root = make_int4(n > 1 ? 0 : ~0, 0, static_cast<int>(n), 0);
+    const int4 root = make_int4(root_ref, 0, static_cast<int>(n), 0);
     const uint32_t one = 1;
     GR_CUDA_TRY(cudaMemsetAsync(ctl, 0, sizeof(CollapseCtl), st));
     GR_CUDA_TRY(cudaMemcpyAsync(ctl->count, &one, sizeof(one), cudaMemcpyHostToDevice, st));
@@ -500,26 +602,32 @@ gr_status collapse_levels(uint32_t n, CollapseCtl* ctl, const int* err, int4* to
 }  // namespace
 
 gr_status build_bvh_device(const gr_scene_desc& desc, const HostBuild& h, SceneBuffers& b, cudaStream_t st,
-                           uint32_t& num_wide, uint32_t& stack_depth, uint64_t& bytes) {
+                           uint32_t& num_wide, uint32_t& stack_depth, uint64_t& num_binary, uint64_t& bytes) {
     const uint32_t n = static_cast<uint32_t>(h.num_components);
     const uint32_t W = h.width, L = h.leaf_size;
     const uint32_t ni = n > 1 ? n - 1 : 1;  // internal nodes
     const uint32_t blocks = (n + BB - 1) / BB;
     size_t tmp_bytes = 0;
-    GR_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, static_cast<uint32_t*>(nullptr),
+    if (!h.device_sah)
+        GR_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, static_cast<uint32_t*>(nullptr),
                                                 static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
                                                 static_cast<uint32_t*>(nullptr), static_cast<int>(n), 0, 30, st));
     Slab m;
     const size_t o_box = m.add(size_t(n) * 6 * sizeof(float)), o_rec = m.add(size_t(n) * 3 * sizeof(float4));
     const size_t attr = size_t(n) * 3 * sizeof(uint32_t);
     const size_t o_tn = m.add(h.any_normals ? attr : 0), o_tu = m.add(h.any_uvs ? attr : 0);
-    const size_t o_bounds = m.add(6 * sizeof(int)), o_err = m.add(sizeof(int));
-    const size_t o_code = m.add(n * sizeof(uint32_t)), o_index = m.add(n * sizeof(uint32_t));
-    const size_t o_code_s = m.add(n * sizeof(uint32_t)), o_perm = m.add(n * sizeof(uint32_t));
-    const size_t o_tmp = m.add(std::max<size_t>(tmp_bytes, 16)), o_split = m.add(size_t(ni) * sizeof(int4));
-    const size_t o_par_i = m.add(ni * sizeof(int)), o_par_l = m.add(n * sizeof(int));
-    const size_t o_opened = m.add(size_t(ni) * sizeof(Opened)), o_visits = m.add(ni * sizeof(int));
+    const size_t o_err = m.add(sizeof(int)), o_perm = m.add(n * sizeof(uint32_t));
+    const size_t o_opened = m.add(size_t(ni) * sizeof(Opened));
     const size_t o_ctl = m.add(sizeof(CollapseCtl)), o_todo = m.add(size_t(n) * sizeof(int4));
+    // Of the linear build, or of the SAH build.
+    const size_t lin = h.device_sah ? 0 : n, lin_i = h.device_sah ? 0 : ni;
+    const size_t o_bounds = m.add(6 * sizeof(int));
+    const size_t o_code = m.add(lin * sizeof(uint32_t)), o_index = m.add(lin * sizeof(uint32_t));
+    const size_t o_code_s = m.add(lin * sizeof(uint32_t)), o_tmp = m.add(std::max<size_t>(tmp_bytes, 16));
+    const size_t o_split = m.add(lin_i * sizeof(int4)), o_par_i = m.add(lin_i * sizeof(int));
+    const size_t o_par_l = m.add(lin * sizeof(int)), o_visits = m.add(lin_i * sizeof(int));
+    std::unique_ptr<SahScratch> sah;
+    if (h.device_sah) sah.reset(new SahScratch(m, n));
     // The caller's arrays (records made on the device).
     std::vector<PrimSrc> src;
     std::vector<size_t> o_arrays;
@@ -587,42 +695,45 @@ gr_status build_bvh_device(const gr_scene_desc& desc, const HostBuild& h, SceneB
         GR_CUDA_TRY(put(tn, h.tri_normal_idx.data(), h.tri_normal_idx.size(), st));
         GR_CUDA_TRY(put(tu, h.tri_uv_idx.data(), h.tri_uv_idx.size(), st));
     }
-    int init[6];
-    for (int a = 0; a < 3; ++a) {
-        init[a] = 0x7FFFFFFF;  // ordered(+max)
-        init[3 + a] = static_cast<int>(0x80000000u);
-    }
-    int* bounds = m.at<int>(o_bounds);
-    GR_CUDA_TRY(cudaMemcpyAsync(bounds, init, sizeof(init), cudaMemcpyHostToDevice, st));
-    k_centroid_bounds<<<std::min(blocks, static_cast<uint32_t>(device_sm_count()) * 4u), BB, 0, st>>>(box, n, bounds);
-    GR_CUDA_TRY(cudaGetLastError());
-    uint32_t *code = m.at<uint32_t>(o_code), *index = m.at<uint32_t>(o_index), *code_s = m.at<uint32_t>(o_code_s);
-    k_morton<<<blocks, BB, 0, st>>>(box, n, bounds, code, index);
-    GR_CUDA_TRY(cudaGetLastError());
-    GR_CUDA_TRY(cub::DeviceRadixSort::SortPairs(m.at<void>(o_tmp), tmp_bytes, code, code_s, index, perm,
-                                                static_cast<int>(n), 0, 30, st));
-    int *par_i = m.at<int>(o_par_i), *par_l = m.at<int>(o_par_l), *visits = m.at<int>(o_visits);
-    int4* split = m.at<int4>(o_split);
     Opened* opened = m.at<Opened>(o_opened);
-    GR_CUDA_TRY(cudaMemsetAsync(par_i, 0xFF, ni * sizeof(int), st));  // root: -1
-    GR_CUDA_TRY(cudaMemsetAsync(par_l, 0xFF, n * sizeof(int), st));
-    GR_CUDA_TRY(cudaMemsetAsync(visits, 0, ni * sizeof(int), st));
-    if (n > 1) {
-        k_radix_tree<<<(n - 1 + BB - 1) / BB, BB, 0, st>>>(code_s, static_cast<int>(n), split, par_i, par_l);
+    int root = n > 1 ? 0 : ~0;
+    if (sah) {
+        const gr_status built = sah_tree(sah->view(m, box, opened, n), perm, st, root);
+        if (built != GR_OK) return built;
+    } else {
+        int init[6];
+        for (int a = 0; a < 3; ++a) {
+            init[a] = 0x7FFFFFFF;  // ordered(+max)
+            init[3 + a] = static_cast<int>(0x80000000u);
+        }
+        int* bounds = m.at<int>(o_bounds);
+        GR_CUDA_TRY(cudaMemcpyAsync(bounds, init, sizeof(init), cudaMemcpyHostToDevice, st));
+        const uint32_t grid = std::min(blocks, static_cast<uint32_t>(device_sm_count()) * 4u);
+        k_centroid_bounds<<<grid, BB, 0, st>>>(box, n, bounds);
         GR_CUDA_TRY(cudaGetLastError());
-        k_boxes<<<blocks, BB, 0, st>>>(box, perm, static_cast<int>(n), split, par_i, par_l, opened, visits, err);
+        uint32_t *code = m.at<uint32_t>(o_code), *index = m.at<uint32_t>(o_index), *code_s = m.at<uint32_t>(o_code_s);
+        k_morton<<<blocks, BB, 0, st>>>(box, n, bounds, code, index);
         GR_CUDA_TRY(cudaGetLastError());
+        GR_CUDA_TRY(cub::DeviceRadixSort::SortPairs(m.at<void>(o_tmp), tmp_bytes, code, code_s, index, perm,
+                                                    static_cast<int>(n), 0, 30, st));
+        int *par_i = m.at<int>(o_par_i), *par_l = m.at<int>(o_par_l), *visits = m.at<int>(o_visits);
+        int4* split = m.at<int4>(o_split);
+        GR_CUDA_TRY(cudaMemsetAsync(par_i, 0xFF, ni * sizeof(int), st));  // root: -1
+        GR_CUDA_TRY(cudaMemsetAsync(par_l, 0xFF, n * sizeof(int), st));
+        GR_CUDA_TRY(cudaMemsetAsync(visits, 0, ni * sizeof(int), st));
+        if (n > 1) {
+            k_radix_tree<<<(n - 1 + BB - 1) / BB, BB, 0, st>>>(code_s, static_cast<int>(n), split, par_i, par_l);
+            GR_CUDA_TRY(cudaGetLastError());
+            k_boxes<<<blocks, BB, 0, st>>>(box, perm, static_cast<int>(n), split, par_i, par_l, opened, visits, err);
+            GR_CUDA_TRY(cudaGetLastError());
+        }
     }
     int e = 0;
     GR_CUDA_TRY(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     CollapseCtl* ctl = m.at<CollapseCtl>(o_ctl);
     int4* todo = m.at<int4>(o_todo);
-    gr_status s;
-    switch (W) {
-        case 2: s = collapse_levels<2>(n, ctl, err, todo, opened, box, perm, L, b, st, num_wide, stack_depth); break;
-        case 8: s = collapse_levels<8>(n, ctl, err, todo, opened, box, perm, L, b, st, num_wide, stack_depth); break;
-        default: s = collapse_levels<4>(n, ctl, err, todo, opened, box, perm, L, b, st, num_wide, stack_depth); break;
-    }
+    auto collapse = W == 2 ? collapse_levels<2> : (W == 8 ? collapse_levels<8> : collapse_levels<4>);
+    const gr_status s = collapse(root, n, ctl, err, todo, opened, box, perm, L, b, st, num_wide, stack_depth);
     if (s != GR_OK) return s;  // (it has synchronised the stream, so `e` is there)
     if (e == ERR_BAD_INDEX) {
         set_error("device BVH build: an index is out of range");
@@ -636,6 +747,22 @@ gr_status build_bvh_device(const gr_scene_desc& desc, const HostBuild& h, SceneB
         set_error("device BVH build: the tree needs a traversal stack of " + std::to_string(stack_depth) +
                   " entries (limit " + std::to_string(MAX_STACK) + ")");
         return GR_ERR_STACK_OVERFLOW;
+    }
+    if (sah) {
+        SahCtl ctl_end;
+        const size_t used = size_t(num_wide) * 8 * W * sizeof(float);
+        DevBuf nodes;  // as many as there are: the collapse's were sized for the worst case
+        GR_CUDA_TRY(nodes.ensure(used));
+        GR_CUDA_TRY(cudaMemcpyAsync(nodes.ptr, b.nodes.ptr, used, cudaMemcpyDeviceToDevice, st));
+        GR_CUDA_TRY(cudaMemcpyAsync(&ctl_end, m.at<SahCtl>(sah->ctl), sizeof(ctl_end), cudaMemcpyDeviceToHost, st));
+        GR_CUDA_TRY(cudaStreamSynchronize(st));
+        if (ctl_end.failed) {
+            set_error("device BVH build: left to the host");
+            return GR_ERR_INTERNAL;
+        }
+        std::swap(nodes.ptr, b.nodes.ptr);
+        std::swap(nodes.bytes, b.nodes.bytes);
+        num_binary = 2 * (uint64_t(n) - ctl_end.excess) - 1;
     }
     const size_t rec_bytes = size_t(n) * 3 * sizeof(float4);
     GR_CUDA_TRY(b.prims.ensure(rec_bytes));

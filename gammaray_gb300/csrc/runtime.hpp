@@ -179,11 +179,12 @@ struct gr_film {
 
 namespace gr {
 
-// Device BVH build (bvh_build.cu) for a HostBuild made from `desc` with
-// GR_BUILD_DEVICE_LBVH: fills b.nodes, b.prims, b.tri_nidx, b.tri_uvidx (leaf order).
-// GR_ERR_INVALID_ARGUMENT: h.device_records, and an index of desc is out of range.
+// Device BVH build (bvh_build.cu) for a HostBuild made from `desc` whose tree is left to the
+// device: fills b.nodes, b.prims, b.tri_nidx, b.tri_uvidx (leaf order) and, of the SAH
+// build, num_binary.  GR_ERR_INVALID_ARGUMENT: h.device_records, and an index of desc is out
+// of range.  With h.device_sah whatever it cannot do the host build can still.
 gr_status build_bvh_device(const gr_scene_desc& desc, const HostBuild& h, SceneBuffers& b, cudaStream_t st,
-                           uint32_t& num_wide, uint32_t& stack_depth, uint64_t& bytes);
+                           uint32_t& num_wide, uint32_t& stack_depth, uint64_t& num_binary, uint64_t& bytes);
 
 // Kernel-side entry points (implemented in the .cu files).
 gr_status launch_trace(const DeviceScene& s, const float* rays, uint64_t n, gr_hit* hits, int* err, cudaStream_t st);

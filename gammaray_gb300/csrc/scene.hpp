@@ -107,6 +107,7 @@ struct HostBuild {
     // The device also makes the records and boxes, from the caller's arrays, and checks
     // their indices (no item_boxes, prims or attribute indices here).
     bool device_records = false;
+    bool device_sah = false;  // with device_records: the SAH build (bvh_build.cu makes its tree)
     std::vector<uint32_t> nbase, ubase;  // with device_records: each prim's attributes in normals / uvs
     uint32_t leaf_size = 0;
     std::vector<float, NoInitAlloc<float>> item_boxes;  // every element written
@@ -118,9 +119,9 @@ bool build_material(const gr_material_desc& d, DevMaterial& out, std::string& er
 
 // Validates the descriptor, runs the reference SAH build (geom/bvh.rs:182-382) and
 // collapses the binary tree into a width-W BVH.
-// device_records: a device build may leave the records to the device where that pays; the
-// triangles' indices are then not checked here, and a failure's text need not be the one
-// that a call without it gives.
+// device_records: the records, and of the SAH build the tree, may be left to the device
+// where that pays; the triangles' indices are then not checked here, and a failure's text
+// need not be the one that a call without it gives.
 bool build_scene(const gr_scene_desc& desc, HostBuild& out, std::string& err, bool tree_hash = false,
                  bool device_records = false);
 

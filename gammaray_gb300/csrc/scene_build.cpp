@@ -801,6 +801,10 @@ static bool build_lobes(const gr_material_desc& d, DevMaterial& m, std::string& 
 // See build_scene: fewest components and most prims of a scene whose records the device makes.
 static constexpr size_t DEVICE_RECORDS_MIN = 2048;
 static constexpr uint32_t DEVICE_RECORDS_PRIMS = 64;
+// Fewest components of a scene whose SAH tree the device builds (sah_build.cuh).  Scene
+// creation with the host's tree and with the device's (us): 3,000 triangles 1,048 / 970,
+// 5,000 1,222 / 1,117, 8,000 1,709 / 1,402, 20,000 2,955 / 1,546, 102,400 6,859 / 1,842.
+static constexpr size_t DEVICE_SAH_MIN = 4096;
 
 bool build_material(const gr_material_desc& d, DevMaterial& m, std::string& err) {
     if (!build_lobes(d, m, err)) return false;
@@ -884,9 +888,10 @@ bool build_scene(const gr_scene_desc& desc, HostBuild& out, std::string& err, bo
     // whose meshes have no more vertices than their triangles can name (so that a small
     // mesh cut from a large vertex array uploads only its records): 400,000 triangles took 1.5 to 2.5 ms on 16 host threads and 0.4 ms to upload, against
     // 0.1 ms of index and vertex uploads and 20 us there.
-    out.device_records = device_records && desc.build == GR_BUILD_DEVICE_LBVH &&
-                         total >= DEVICE_RECORDS_MIN && desc.num_prims <= DEVICE_RECORDS_PRIMS &&
-                         vertices <= 3 * total;
+    out.device_sah = desc.build == GR_BUILD_HOST_SAH;
+    out.device_records = device_records && total >= (out.device_sah ? DEVICE_SAH_MIN : DEVICE_RECORDS_MIN) &&
+                         desc.num_prims <= DEVICE_RECORDS_PRIMS && vertices <= 3 * total;
+    out.device_sah = out.device_sah && out.device_records;
     if (!out.device_records) items.reserve(total);
     std::vector<uint32_t> vbase(desc.num_prims, 0), nbase(desc.num_prims, 0), ubase(desc.num_prims, 0);
     uint32_t nrm_total = 0, uv_total = 0;
@@ -1043,7 +1048,7 @@ bool build_scene(const gr_scene_desc& desc, HostBuild& out, std::string& err, bo
         }
     };
 
-    if (out.device_build) {
+    if (out.device_build || out.device_sah) {
         out.leaf_size = L;
         out.item_boxes.resize(items.size() * 6);
         auto records = [&](unsigned, size_t b, size_t e) {
