@@ -39,12 +39,6 @@ constexpr int PATH_LOOP_BLOCKS = 2;
 // warp wait for each other.  4 / 8 measured 157 / 157 us for 96 x 54 paths of the Cornell
 // box, 487 / 486 for 300 x 200 x 4 spp of a mesh.
 constexpr uint32_t PATH_LOOP_MIN_LANES = 8;
-// Scenes of at least this many components have a warp's last rays traced by groups of
-// lanes (trace_grouped): 1,437 -> 1,386 us on 641 x 359 x 9 spp of 12,000 triangles, 293 ->
-// 278 on 64 x 64 x 2 spp of 50,000.  The few steps of a ray in a small scene do not repay
-// the hand-over (Cornell box 128 x 128 x 4 spp: 220 -> 230, BDPT 795 -> 813).
-constexpr uint32_t GROUPED_COMPONENTS = 1024;
-
 // A block's shared memory: its threads' traversal stacks, their paths (word by word, a
 // column each), and the shading order.
 constexpr size_t path_loop_smem_bytes(int words) {
@@ -148,7 +142,7 @@ GR_D uint32_t run_paths(const K& stk, unsigned char* smem, uint32_t n, uint32_t*
             const unsigned last = grouped ? __ballot_sync(0xffffffffu, trav && !deep) : 0u;
             bool over = false;
             if (last && __popc(last) <= 32 / W) {
-                trace_grouped<W>(last, scene(), t, steps, stk, deep, over);
+                trace_grouped<W, false>(last, scene(), t, steps, stk, deep, over);
                 trav = trav && deep;
             } else if (trav) {
                 const bool done = trav_step<W>(scene(), t, stk, err);

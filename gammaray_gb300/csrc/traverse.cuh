@@ -406,13 +406,19 @@ GR_D TraceScene scene_of(const TraceScene& s, int src) {
 }
 GR_D TraceScene scene_of(const DeviceScene& s, int) { return TraceScene{s.nodes, s.prims, s.step_budget}; }
 
-// Closest hits of the rays of the lanes in `mask` (at most 32 / W), W lanes each: a lane
+// Scenes of at least this many components have a warp's last rays traced by groups of
+// lanes (trace_grouped): 1,437 -> 1,386 us on 641 x 359 x 9 spp of 12,000 triangles, 293 ->
+// 278 on 64 x 64 x 2 spp of 50,000.  The few steps of a ray in a small scene do not repay
+// the hand-over (Cornell box 128 x 128 x 4 spp: 220 -> 230, BDPT 795 -> 813).
+constexpr uint32_t GROUPED_COMPONENTS = 1024;
+
+// Closest hits (ANY_HIT: any) of the rays of the lanes in `mask` (at most 32 / W), W lanes each: a lane
 // tests one child of a node or one primitive of a leaf.  The same tests, order and hits as
 // trav_step, whose some 250 dependent instructions per node are what a ray alone in its warp
 // waits for.  `steps` counts on; a ray whose stack would outgrow its shared part is given
 // back unfinished (deep), one that runs out of steps with `over` set; the others end.  Every
 // lane of the warp calls it with the same mask.
-template <int W, class S, class K>
+template <int W, bool ANY_HIT, class S, class K>
 GR_D void trace_grouped(unsigned mask, const S& scene, TravState& t, uint32_t& steps, const K& stk, bool& deep,
                         bool& over) {
     constexpr unsigned all = 0xffffffffu, ones = (1u << W) - 1u;
@@ -513,8 +519,11 @@ GR_D void trace_grouped(unsigned mask, const S& scene, TravState& t, uint32_t& s
                     hv = v;
                 }
             }
-            if (leaf) ++n;
-            next(leaf);
+            if (leaf) {
+                ++n;
+                if (ANY_HIT && hit >= 0) on = false;
+            }
+            next(leaf && on);
         }
     }
     __syncwarp();
@@ -549,7 +558,9 @@ GR_D void trace_grouped(unsigned mask, const S& scene, TravState& t, uint32_t& s
 // grabs that many rays and hands them to its idle lanes.  So a lane whose ray ended early
 // starts another one, instead of idling until the warp's longest ray ends.  A ray that
 // takes more than its scene's step budget is abandoned as a miss: *err = 2 and, if err_ray
-// is given, its index there.  With ANY_HIT a ray ends at its first hit.
+// is given, its index there.  With ANY_HIT a ray ends at its first hit.  `grouped` (with
+// GROUPED, and no COUNT): once no rays are left to grab, a warp's last ones are traced by groups of
+// lanes.
 //
 // Every warp intrinsic runs where control flow is warp-uniform: the loop's iterations are
 // the same for all lanes, the refill condition depends on ballot results and on the
@@ -559,14 +570,15 @@ GR_D void trace_grouped(unsigned mask, const S& scene, TravState& t, uint32_t& s
 //
 // Bound by instruction issue (71-77% active) and the L1 data pipe (54-67%: 112 bytes per
 // lane and node) on camera rays and first bounces, by node-load latency further on.
-template <int W, bool ANY_HIT, bool COUNT, class K, class Grab, class SceneOf, class Load, class Store>
+template <int W, bool ANY_HIT, bool COUNT, bool GROUPED = false, class K, class Grab, class SceneOf, class Load,
+          class Store>
 GR_D void trace_queue(uint32_t n, const K& stk, int* err, int* err_ray, uint32_t* counts, const Grab& grab,
-                      const SceneOf& scene, const Load& load, const Store& store) {
+                      const SceneOf& scene, const Load& load, const Store& store, bool grouped = false) {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
     TravState t;
     uint32_t q = 0, steps = 0;
-    bool busy = false, exhausted = false;
+    bool busy = false, exhausted = false, deep = false;  // deep: grouped lanes gave this ray back
     for (;;) {
         const unsigned idle = __ballot_sync(0xffffffffu, !busy);
         if (!exhausted && __popc(idle) >= EXTEND_REFILL) {
@@ -577,7 +589,25 @@ GR_D void trace_queue(uint32_t n, const K& stk, int* err, int* err_ray, uint32_t
                 if (q < n) {
                     busy = load(q, t);
                     steps = 0;
+                    deep = false;
                 }
+            }
+        }
+        if (GROUPED && grouped && exhausted) {
+            const unsigned last = __ballot_sync(0xffffffffu, busy && !deep);
+            if (last && __popc(last) <= 32 / W) {
+                bool over = false;
+                trace_grouped<W, ANY_HIT>(last, scene(), t, steps, stk, deep, over);
+                if (over) {
+                    atomicExch(err, 2);
+                    if (err_ray) atomicExch(err_ray, static_cast<int>(q));
+                    t.hit = -1;
+                }
+                if (((last >> lane) & 1u) && !deep) {
+                    store(q, t);
+                    busy = false;
+                }
+                continue;
             }
         }
         const bool leaf = busy && t.ref < 0, node = busy && t.ref >= 0;
