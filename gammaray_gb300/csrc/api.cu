@@ -102,6 +102,9 @@ DevCamera make_camera(const gr_camera& c) {
         }
     d.wx = c.horizontal_aperture / (c.focal_length * 2.0f);  // camera.rs:76-79
     d.wy = c.vertical_aperture / (c.focal_length * 2.0f);
+    float o[4];
+    for (int k = 0; k < 4; ++k) o[k] = 0.0f * d.m[0][k] + 0.0f * d.m[1][k] + 0.0f * d.m[2][k] + d.m[3][k];
+    for (int k = 0; k < 3; ++k) d.origin[k] = o[k] / o[3];
     return d;
 }
 

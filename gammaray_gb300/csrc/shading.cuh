@@ -82,16 +82,13 @@ GR_D V3 nudge(V3 o, V3 d) { return o + (d * RAY_PUSH_DIST); }  // Ray::nudge (co
 struct DevCamera {
     float m[4][4];
     float wx, wy;
+    float origin[3];  // every ray's: Xform::transform of the origin (xform.rs:41-47)
 };
 
 GR_D void camera_ray(const DevCamera& c, float s, float t, V3& o, V3& d) {
     V3 dir = normalized(V3{c.wx * s, c.wy * t, -1.0f});
-    // Xform::transform of the origin (xform.rs:41-47) and transform_dir (xform.rs:49-54)
-    float x = 0.0f * c.m[0][0] + 0.0f * c.m[1][0] + 0.0f * c.m[2][0] + c.m[3][0];
-    float y = 0.0f * c.m[0][1] + 0.0f * c.m[1][1] + 0.0f * c.m[2][1] + c.m[3][1];
-    float z = 0.0f * c.m[0][2] + 0.0f * c.m[1][2] + 0.0f * c.m[2][2] + c.m[3][2];
-    float w = 0.0f * c.m[0][3] + 0.0f * c.m[1][3] + 0.0f * c.m[2][3] + c.m[3][3];
-    o = V3{x / w, y / w, z / w};
+    // Xform::transform_dir (xform.rs:49-54)
+    o = V3{c.origin[0], c.origin[1], c.origin[2]};
     d = V3{dir.x * c.m[0][0] + dir.y * c.m[1][0] + dir.z * c.m[2][0],
            dir.x * c.m[0][1] + dir.y * c.m[1][1] + dir.z * c.m[2][1],
            dir.x * c.m[0][2] + dir.y * c.m[1][2] + dir.z * c.m[2][2]};
