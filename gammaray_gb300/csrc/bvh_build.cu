@@ -471,15 +471,15 @@ cudaError_t put(void* dst, const T* src, size_t count, cudaStream_t st) {
 }
 
 // The order and the binary tree of the SAH build (sah_build.cuh): the host launches levels
-// of large nodes, SAH_LEVELS_AT_ONCE at a time (10 for 400,000 triangles), then the rest.
-constexpr uint32_t SAH_LEVELS_AT_ONCE = 12;
+// of large nodes, SAH_LEVELS_FIRST of them (15 for 102,400 triangles), then SAH_LEVELS_MORE at a time.
+constexpr uint32_t SAH_LEVELS_FIRST = 16, SAH_LEVELS_MORE = 4;
 
 struct SahScratch {
     size_t ctl, order[2], bucket, moved, tile_left, best, left, small;
     size_t nodes[2], tables[2], first_out[2], tile0[2], tiles[2];
     uint32_t max_big, max_tiles, max_small;
     SahScratch(Slab& m, uint32_t n) {
-        max_big = n / (SAH_SMALL + 1) + 1;
+        max_big = n / (sah_small(n) + 1) + 1;
         max_tiles = n / SAH_TILE + max_big + 1;
         max_small = 2 * SAH_LEVELS * max_big;  // every large node leaves two at most
         ctl = m.add(sizeof(SahCtl));
@@ -515,6 +515,7 @@ struct SahScratch {
         v.small = m.at<SahSmall>(small);
         v.opened = reinterpret_cast<float*>(opened);
         v.n = n;
+        v.most_small = sah_small(n);
         v.max_big = max_big;
         v.max_tiles = max_tiles;
         v.max_small = max_small;
@@ -534,7 +535,7 @@ gr_status sah_tree(const SahView& v, uint32_t* perm, cudaStream_t st, int& root)
     GR_CUDA_TRY(cudaGetLastError());
     const uint32_t grid = std::min(v.max_tiles, sms * 8u);
     for (uint32_t level = 0;;) {
-        const uint32_t stop = std::min(level + SAH_LEVELS_AT_ONCE, SAH_LEVELS);
+        const uint32_t stop = std::min(level + (level ? SAH_LEVELS_MORE : SAH_LEVELS_FIRST), SAH_LEVELS);
         for (; level < stop; ++level) {
             k_sah_buckets<<<grid, BB, 0, st>>>(v, level);
             k_sah_count<<<grid, BB, 0, st>>>(v, level);
@@ -550,7 +551,12 @@ gr_status sah_tree(const SahView& v, uint32_t* perm, cudaStream_t st, int& root)
         }
         if (h.big[level] == 0) break;
     }
-    k_sah_small<<<std::min(h.small, sms * 4u), BB, sizeof(SahTree), st>>>(v, perm);
+    if (v.most_small == SAH_SMALL_FEW)
+        k_sah_small<SAH_SMALL_FEW>
+            <<<std::min(h.small, sms * 8u), BB, sizeof(SahTree<SAH_SMALL_FEW>), st>>>(v, perm);
+    else
+        k_sah_small<SAH_SMALL_MANY>
+            <<<std::min(h.small, sms * 4u), BB, sizeof(SahTree<SAH_SMALL_MANY>), st>>>(v, perm);
     GR_CUDA_TRY(cudaGetLastError());
     root = h.root;
     return GR_OK;

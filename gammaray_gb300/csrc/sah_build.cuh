@@ -11,7 +11,7 @@
 //   * a node whose centroids coincide is a leaf there.  Its components are halved here, as
 //     the collapse halves a range, down to single ones.
 //
-// Nodes of more than SAH_SMALL components are split level by level by the whole grid, four
+// Nodes of more than sah_small() components are split level by level by the whole grid, four
 // launches a level (k_sah_buckets, k_sah_count, k_sah_front, k_sah_back), in tiles.  A block
 // then builds each smaller subtree in shared memory (k_sah_small).  The binary tree has one
 // internal node per gap between neighbouring components of the final order, which is its
@@ -29,7 +29,15 @@ namespace {
 
 constexpr int SAH_BUCKETS = 12;
 constexpr int SAH_VALUES = 13;  // per bucket: count, box lo and hi, centroid lo and hi
-constexpr uint32_t SAH_SMALL = 1024;
+// Most components of a subtree that one block builds, by the scene's: a block takes its
+// subtree's first levels a warp at a time, so smaller subtrees, whose splits the whole grid
+// shares, end sooner, until there are so many nodes that the levels cost more.  256 / 512 /
+// 1024 measured 984 / 1069 / 1137 us of scene creation for 4,100 triangles, 1356 / 1408 /
+// 1541 for 20,000, 1658 / 1698 / 1830 for 102,400, 2190 / 2113 / 2159 for 200,000 and 2577 /
+// 2536 / 2399 for 400,000.
+constexpr uint32_t SAH_SMALL_FEW = 256, SAH_SMALL_MANY = 1024;
+constexpr uint32_t SAH_MANY = 150000;
+inline uint32_t sah_small(uint32_t n) { return n < SAH_MANY ? SAH_SMALL_FEW : SAH_SMALL_MANY; }
 constexpr uint32_t SAH_TILE = 1024;
 constexpr uint32_t SAH_ROOT = 0xFFFFFFFFu;
 constexpr uint32_t SAH_LEVELS = 64;  // of large nodes
@@ -44,7 +52,7 @@ struct SahCtl {
     int bounds[12];   // of all components: box lo, hi, centroid lo, hi (ordered)
 };
 
-// A node of more than SAH_SMALL components.
+// A large node.
 struct SahNode {
     uint32_t first, count;
     uint32_t slot;   // its place in its parent's record: 2 * parent + side, or SAH_ROOT
@@ -78,7 +86,7 @@ struct SahView {
     uint32_t* left;       // per node: components of the left side
     SahSmall* small;
     float* opened;  // the internal nodes' records (Opened), 16 floats each
-    uint32_t n, max_big, max_tiles, max_small;
+    uint32_t n, most_small, max_big, max_tiles, max_small;
     SahLevel level[2];
 };
 
@@ -211,7 +219,7 @@ GR_D void sah_enter(const SahView& s, uint32_t level, SahNode nd) {
     }
     uint32_t at = 0, tile = 0;
     const uint32_t tiles = (nd.count + SAH_TILE - 1) / SAH_TILE;
-    if (nd.count > SAH_SMALL) {
+    if (nd.count > s.most_small) {
         if (lane == 0) {
             at = atomicAdd(&s.ctl->big[level], 1u);
             tile = atomicAdd(&s.ctl->tiles[level], tiles);
@@ -490,18 +498,19 @@ __global__ void __launch_bounds__(BB) k_sah_back(SahView s, uint32_t level) {
     }
 }
 
-// A subtree in shared memory, of at most SAH_SMALL components.
+// A subtree in shared memory, of at most N components.
+template <uint32_t N>
 struct SahTree {
-    float box[6][SAH_SMALL];
-    uint32_t id[SAH_SMALL];
-    uint16_t order[2][SAH_SMALL], moved[SAH_SMALL];
-    uint8_t bucket[SAH_SMALL];
+    float box[6][N];
+    uint32_t id[N];
+    uint16_t order[2][N], moved[N];
+    uint8_t bucket[N];
     int tab[SAH_WARPS][SAH_BUCKETS * SAH_VALUES];
-    uint2 list[2][SAH_SMALL / 4];  // nodes of more than four: (first | count << 16, slot | range << 31)
-    uint2 tiny[SAH_SMALL / 2];     // nodes of two to four
+    uint2 list[2][N / 4];  // nodes of more than four: (first | count << 16, slot | range << 31)
+    uint2 tiny[N / 2];     // nodes of two to four
     uint32_t listed[2], tinies;
     GR_D float cen(uint32_t k, int dim) const {
-        k %= SAH_SMALL;
+        k %= N;
         return 0.5f * box[dim][k] + 0.5f * box[3 + dim][k];
     }
 };
@@ -509,7 +518,8 @@ constexpr uint32_t SAH_RANGE = 1u << 31;
 
 // The reference's nth_element (geom/util.rs), its swap partition and its shortened left side
 // included, on `s`.
-GR_D void sah_nth(const SahTree& T, uint16_t* s, uint32_t len, uint32_t nth, int dim) {
+template <uint32_t N>
+GR_D void sah_nth(const SahTree<N>& T, uint16_t* s, uint32_t len, uint32_t nth, int dim) {
     while (len >= 2) {
         const uint32_t pivot = len / 2;
         const uint16_t pe = s[pivot];
@@ -545,17 +555,19 @@ GR_D void sah_slot(const SahView& s, uint32_t slot, const float* b, int ref, uin
 }
 
 // A single component at position `at` of the subtree: its slot and its place in the order.
-GR_D void sah_single(const SahView& s, const SahTree& T, uint32_t first, uint32_t at, uint32_t e, uint32_t slot,
+template <uint32_t N>
+GR_D void sah_single(const SahView& s, const SahTree<N>& T, uint32_t first, uint32_t at, uint32_t e, uint32_t slot,
                      uint32_t* __restrict__ perm) {
     float b[6];
-    e %= SAH_SMALL;
+    e %= N;
     for (int a = 0; a < 6; ++a) b[a] = T.box[a][e];
     sah_slot(s, slot, b, ~static_cast<int>(first + at), 1);
     perm[first + at] = T.id[e];
 }
 
 // Subtrees of two to four components, by one thread.
-GR_D void sah_tiny(const SahView& s, SahTree& T, uint32_t first, uint16_t* order, uint2 node, uint32_t* perm) {
+template <uint32_t N>
+GR_D void sah_tiny(const SahView& s, SahTree<N>& T, uint32_t first, uint16_t* order, uint2 node, uint32_t* perm) {
     uint2 todo[4];
     int left = 0;
     todo[left++] = node;
@@ -572,7 +584,7 @@ GR_D void sah_tiny(const SahView& s, SahTree& T, uint32_t first, uint16_t* order
             b[3 + a] = cb[3 + a] = -FLT_MAX;
         }
         for (uint32_t i = f; i < f + n; ++i) {
-            const uint32_t e = order[i] % SAH_SMALL;
+            const uint32_t e = order[i] % N;
             for (int a = 0; a < 3; ++a) {
                 const float c = T.cen(e, a);
                 b[a] = fminf(b[a], T.box[a][e]);
@@ -598,9 +610,10 @@ GR_D void sah_tiny(const SahView& s, SahTree& T, uint32_t first, uint16_t* order
 // Builds the small subtrees, a block each, level by level: a warp a node, then a thread per
 // node of at most four components.  Bound by the chain of a warp's reductions in the first
 // levels and by the serial nth_element of the last ones.
+template <uint32_t N>
 __global__ void __launch_bounds__(BB) k_sah_small(SahView s, uint32_t* __restrict__ perm) {
     extern __shared__ unsigned char smem[];
-    SahTree& T = *reinterpret_cast<SahTree*>(smem);
+    SahTree<N>& T = *reinterpret_cast<SahTree<N>*>(smem);
     const unsigned all = 0xffffffffu, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
     const uint32_t trees = s.ctl->failed ? 0u : s.ctl->small;
     int* tab = T.tab[warp];
@@ -623,7 +636,7 @@ __global__ void __launch_bounds__(BB) k_sah_small(SahView s, uint32_t* __restric
         }
         __syncthreads();
         // A level leaves every node smaller: it ends.
-        for (uint32_t depth = 0; depth <= SAH_SMALL; ++depth) {
+        for (uint32_t depth = 0; depth <= N; ++depth) {
             const int cur = depth & 1;
             uint16_t *A = T.order[cur], *B = T.order[cur ^ 1];
             const uint32_t nodes = T.listed[cur];
@@ -634,7 +647,7 @@ __global__ void __launch_bounds__(BB) k_sah_small(SahView s, uint32_t* __restric
                 int v[12];  // ordered bounds: box lo, hi, centroid lo, hi
                 for (int a = 0; a < 12; ++a) v[a] = a / 3 % 2 ? static_cast<int>(0x80000000u) : 0x7FFFFFFF;
                 for (uint32_t j = lane; j < n; j += 32) {
-                    const uint32_t e = A[f + j] % SAH_SMALL;
+                    const uint32_t e = A[f + j] % N;
                     for (int a = 0; a < 3; ++a) {
                         const int c = ordered(T.cen(e, a));
                         v[a] = min(v[a], ordered(T.box[a][e]));
@@ -667,7 +680,7 @@ __global__ void __launch_bounds__(BB) k_sah_small(SahView s, uint32_t* __restric
                         float x[6] = {}, c[3] = {};
                         uint32_t k = 0;
                         if (in) {
-                            const uint32_t e = A[f + j] % SAH_SMALL;
+                            const uint32_t e = A[f + j] % N;
                             for (int a = 0; a < 6; ++a) x[a] = T.box[a][e];
                             for (int a = 0; a < 3; ++a) c[a] = 0.5f * x[a] + 0.5f * x[3 + a];
                             k = sah_bucket(dim == 0 ? c[0] : (dim == 1 ? c[1] : c[2]), lo, hi);
@@ -703,7 +716,7 @@ __global__ void __launch_bounds__(BB) k_sah_small(SahView s, uint32_t* __restric
                         for (uint32_t j = lane; j < n; j += 32) {
                             if (T.bucket[f + j] <= best) continue;
                             const uint32_t to = f + k + sah_back(T.moved + f, j - p1, R, p1) - R;
-                            if (to < SAH_SMALL) B[to] = A[f + j];
+                            if (to < N) B[to] = A[f + j];
                         }
                         mid = k;
                         if (k == 0 || k >= n) {  // cannot be: the first and last buckets hold components

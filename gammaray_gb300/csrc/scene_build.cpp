@@ -803,7 +803,7 @@ static constexpr size_t DEVICE_RECORDS_MIN = 2048;
 static constexpr uint32_t DEVICE_RECORDS_PRIMS = 64;
 // Fewest components of a scene whose SAH tree the device builds (sah_build.cuh).  Scene
 // creation with the host's tree and with the device's (us): 3,000 triangles 1,048 / 970,
-// 5,000 1,222 / 1,117, 8,000 1,709 / 1,402, 20,000 2,955 / 1,546, 102,400 6,859 / 1,842.
+// 8,000 1,709 / 1,229, 20,000 2,955 / 1,354, 102,400 6,859 / 1,649.
 static constexpr size_t DEVICE_SAH_MIN = 4096;
 
 bool build_material(const gr_material_desc& d, DevMaterial& m, std::string& err) {
