@@ -617,7 +617,10 @@ GR_D void trace_queue(uint32_t n, const K& stk, int* err, int* err_ray, uint32_t
             continue;
         }
         bool pop = false, done = false;
-        if (nodes == 0u || __popc(leaves) >= EXTEND_LEAVES) {
+        // The last rays of a warp wait for no more than a quarter of it: 512 x 512 x 4 spp of
+        // 102,400 triangles 1,171 -> 1,144 us, 1024 x 1024 x 64 spp 24.24 -> 24.16 ms.
+        const int enough = exhausted ? min(EXTEND_LEAVES, max(1, __popc(leaves | nodes) / 4)) : EXTEND_LEAVES;
+        if (nodes == 0u || __popc(leaves) >= enough) {
             if (leaf) {
                 done = visit_leaf<ANY_HIT, COUNT>(scene(), t, t.ref, counts);
                 pop = !done;
