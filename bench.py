@@ -29,13 +29,13 @@ import time
 import numpy as np
 
 ROOT = os.path.dirname(os.path.abspath(__file__))
-# DRAM bytes (read + written) per extension ray of k_extend_refill: ncu's
-# dram__bytes_read.sum + dram__bytes_write.sum summed over every k_extend_refill launch of
-# a 4-spp render of this workload (bench.py --profile-case --spp 4; its 4 M-ray queues
-# exceed L2 as the timed renders' do), divided by that render's extension rays.  Re-measured whenever the
+# DRAM bytes (read + written) per extension ray: ncu's dram__bytes_read.sum +
+# dram__bytes_write.sum summed over every k_extend_refill and k_pt_finish launch of a 4-spp
+# render of this workload (bench.py --profile-case --spp 4; its 4 M-ray queues exceed L2 as
+# the timed renders' do), divided by that render's extension rays.  Re-measured whenever the
 # extension kernel changes; EXTEND_DRAM_CAPTURE says which capture the figure comes from.
-EXTEND_DRAM_BYTES_PER_RAY = 46.5
-EXTEND_DRAM_CAPTURE = "ncu, 4-spp render of the bench workload, all 12 k_extend_refill launches"
+EXTEND_DRAM_BYTES_PER_RAY = 30.7
+EXTEND_DRAM_CAPTURE = "ncu, 4-spp render of the bench workload, every k_extend_refill and k_pt_finish launch"
 sys.path.insert(0, ROOT)
 
 MEASURED_PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
@@ -556,7 +556,7 @@ def run_ours(args, rank, world, local):
     per = float(args.steps)
     breakdown = {"extend": ext_ms / per, "shade": shade_ms / per, "raygen": raygen_ms / per, "film": film_ms / per}
     breakdown["between_launches"] = sum(dev_ms) / per - sum(breakdown.values())
-    # DRAM traffic of k_extend per launch: the captured bytes per ray (see
+    # DRAM traffic of the extension per launch: the captured bytes per ray (see
     # EXTEND_DRAM_BYTES_PER_RAY) times the rays of an average timed launch.
     roofline["traffic"] = EXTEND_DRAM_BYTES_PER_RAY * rays / max(1, ext_launch)
     roofline["traffic_source"] = (f"{EXTEND_DRAM_CAPTURE}: {EXTEND_DRAM_BYTES_PER_RAY} B/ray, "
