@@ -18,10 +18,13 @@ constexpr int EBLOCK = 128;
 // registers), so all of an SM's warps shade the same code path at a time, as in the
 // path tracer's k_shade.
 #ifndef GR_ENG_SHADE_BLOCK
-#define GR_ENG_SHADE_BLOCK 768
+#define GR_ENG_SHADE_BLOCK 896
 #endif
 constexpr int ESBLOCK = GR_ENG_SHADE_BLOCK;
-static_assert(ESBLOCK == 128 || ESBLOCK == 768, "engine shading block of 128 or 768 threads");
+static_assert(ESBLOCK == 128 || ESBLOCK == 768 || ESBLOCK == 896, "engine shading block of 128, 768 or 896 threads");
+// (72 registers, some spilled.  768 / 896 threads: 9.26 / 9.03 ms for 12 images in a batch,
+// 14.9 / 14.4 for 6 served requests: its entries wait longer for their loads than the path
+// tracer's.)
 // Entries per thread per chunk: fewer than the path tracer's, since the sort also reads an
 // entry's job and depth (two more lines that have to stay in L1).  12 images in a batch /
 // 6 served requests: 32 / 12 / 8 / 6 / 4 measured 10.81 / 9.91 / 9.97 / 9.78 / 9.73 and 19.40
@@ -393,7 +396,7 @@ __global__ void __launch_bounds__(PATH_LOOP_THREADS, PATH_LOOP_BLOCKS)
                &c->rays);
 }
 
-__global__ void __launch_bounds__(ESBLOCK, 768 / ESBLOCK)
+__global__ void __launch_bounds__(ESBLOCK, ESBLOCK < 768 ? 768 / ESBLOCK : 1)
     k_eng_shade(EngineCtl* c, int cur, const DevJob* __restrict__ jobs, uint32_t* unit_done,
                 const uint32_t* __restrict__ q_slot, const float4* __restrict__ q_o,
                 const float4* __restrict__ q_d, const float4* __restrict__ q_hit,

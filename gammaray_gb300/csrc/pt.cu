@@ -51,6 +51,16 @@ __global__ void k_set_count(uint32_t* c, uint32_t n) { *c = n; }
 #endif
 constexpr int SHADE_BIG = GR_SHADE_BLOCK;
 static_assert(SHADE_BIG == 128 || SHADE_BIG == 384 || SHADE_BIG == 768, "shading block of 128, 384 or 768 threads");
+// Long queues: 28 warps instead of 24 hide more of their latency than the spills at 71
+// registers cost (1024 x 1024 x 64 spp of 102,400 triangles 6.74 -> 6.50 ms of shading), but
+// a turn of the block through its queue takes about 1/8 longer, so only where it needs that
+// many fewer turns (641 x 359 x 9 spp, 18 and 16 turns: 1,373 and 1,391 us) and the queue is
+// more than one chunk (Cornell box, 1 M paths, up to 9 turns: 1,092 and 1,097).
+constexpr int SHADE_WIDE = 896;
+inline bool shade_wide(uint64_t n, uint32_t sms) {
+    auto turns = [&](uint64_t nt) { return (n + nt * sms - 1) / (nt * sms); };
+    return turns(SHADE_BIG) > SHADE_ONE_CHUNK && 9 * turns(SHADE_WIDE) < 8 * turns(SHADE_BIG);
+}
 // Most entries per thread of one chunk (shade_sort.cuh).
 template <int NT>
 constexpr uint32_t shade_per() {
@@ -171,7 +181,7 @@ GR_D bool shade_hit(const DeviceScene& s, const PTParams& p, uint32_t depth, uin
 
 // FIRST: the queue of camera rays (no slots or states stored; see first_key).
 template <int NT, bool FIRST>
-__global__ void __launch_bounds__(NT, 768 / NT) k_shade(DeviceScene s, PTParams p, uint32_t depth,
+__global__ void __launch_bounds__(NT, NT < 768 ? 768 / NT : 1) k_shade(DeviceScene s, PTParams p, uint32_t depth,
                                                  const uint32_t* __restrict__ count_in,
                                                  const uint32_t* __restrict__ q_slot, const float4* __restrict__ q_o,
                                                  const float4* __restrict__ q_d, const float4* __restrict__ q_hit,
@@ -264,12 +274,16 @@ gr_status launch_shade_nt(uint32_t n_bound, cudaStream_t st, A... a) {
     return GR_OK;
 }
 
-// Shades a queue of at most n_bound entries (the device holds the exact length): in
-// SHADE_BIG-thread blocks while that fills two blocks per SM, else in 128-thread blocks.
-// `first`: the queue of camera rays (depth 0).
+// Shades a queue of at most n_bound and probably `expected` entries (the device holds the
+// exact length): in SHADE_BIG- or SHADE_WIDE-thread blocks while that fills two blocks per
+// SM, else in 128-thread blocks.  `first`: the queue of camera rays (depth 0).
 template <class... A>
-gr_status launch_shade(uint32_t n_bound, bool first, cudaStream_t st, A... a) {
-    const bool big = SHADE_BIG != 128 && n_bound >= 2u * static_cast<uint32_t>(device_sm_count()) * SHADE_BIG;
+gr_status launch_shade(uint32_t n_bound, uint64_t expected, bool first, cudaStream_t st, A... a) {
+    const uint32_t sms = static_cast<uint32_t>(device_sm_count());
+    const bool big = SHADE_BIG != 128 && n_bound >= 2u * sms * SHADE_BIG;
+    if (SHADE_BIG == 768 && big && shade_wide(expected, sms))
+        return first ? launch_shade_nt<SHADE_WIDE, true>(n_bound, st, a...)
+                     : launch_shade_nt<SHADE_WIDE, false>(n_bound, st, a...);
     if (first) return big ? launch_shade_nt<SHADE_BIG, true>(n_bound, st, a...)
                           : launch_shade_nt<128, true>(n_bound, st, a...);
     return big ? launch_shade_nt<SHADE_BIG, false>(n_bound, st, a...) : launch_shade_nt<128, false>(n_bound, st, a...);
@@ -526,7 +540,8 @@ gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st) {
                 break;
             }
             if (timed) GR_TRY_S(mark(e0));
-            GR_TRY_S(launch_shade(look.bound, depth == 0, st, job.scene, p, depth, cnt + cur, ps.q_slot[cur].as<uint32_t>(),
+            GR_TRY_S(launch_shade(look.bound, look.expected, depth == 0, st, job.scene, p, depth, cnt + cur,
+                                  ps.q_slot[cur].as<uint32_t>(),
                                   ps.q_o[cur].as<float4>(), ps.q_d[cur].as<float4>(), ps.q_hit.as<float4>(),
                                   ps.q_state[cur].as<float4>(), ps.light.as<float4>(), cnt + nxt,
                                   ps.q_slot[nxt].as<uint32_t>(), ps.q_o[nxt].as<float4>(), ps.q_d[nxt].as<float4>(),
@@ -754,8 +769,8 @@ extern "C" gr_status gr_render_static(gr_scene* sc, const gr_camera* camera, con
                 break;
             }
             GR_CUDA_TRY(cudaMemsetAsync(cnt + nxt, 0, sizeof(uint32_t), st));
-            GR_TRY_S(launch_shade(n, depth == 0, st, sc->dev, p, depth, cnt + cur, q_slot[cur], q_o[cur], q_d[cur], q_hit,
-                                  q_state[cur], light, cnt + nxt, q_slot[nxt], q_o[nxt], q_d[nxt], q_state[nxt]));
+            GR_TRY_S(launch_shade(n, n, depth == 0, st, sc->dev, p, depth, cnt + cur, q_slot[cur], q_o[cur], q_d[cur],
+                                  q_hit, q_state[cur], light, cnt + nxt, q_slot[nxt], q_o[nxt], q_d[nxt], q_state[nxt]));
             GR_CUDA_TRY(cudaGetLastError());
             if (p.max_depth == 0 && (depth & 3) == 3) {
                 // Unbounded (reference) depth: stop once no path is left.  The copy goes
