@@ -501,10 +501,10 @@ def run_ours(args, rank, world, local):
         f2.close()
     e2e = {"value": world * samples_per_step / (statistics.median(e2e_ms) * 1e-3) / 1e6, "unit": "Msamples/s",
            "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
-           "includes": "host SAH build + wide collapse + upload, 64-spp render, film read-back into pinned host memory"}
+           "includes": "SAH build + wide collapse + upload, 64-spp render, film read-back into pinned host memory"}
 
     # The same render on a tree built on the GPU (GR_BUILD_DEVICE_LBVH), and end to end with
-    # that build: the reference's host SAH build is the default and the headline.
+    # that build: the reference's SAH tree is the default and the headline.
     dev_build = None
     if rank == 0:
         g.Stage(w.prims[-1:], lib=lib, device_build=True).close()  # build kernels loaded
