@@ -16,14 +16,6 @@ namespace {
 
 constexpr int BLOCK = 128;
 
-// Shading kernels are register-heavy (the Disney mixture); asking for 6 resident blocks
-// of 128 threads caps them at 85 registers, which measured 3% faster on the bench
-// workload than the uncapped 96 (occupancy 31% -> 37%).  GR_SHADE_MIN_BLOCKS overrides.
-#ifndef GR_SHADE_MIN_BLOCKS
-#define GR_SHADE_MIN_BLOCKS 6
-#endif
-#define GR_SHADE_BOUNDS __launch_bounds__(BLOCK, GR_SHADE_MIN_BLOCKS)
-
 // Closest hit for every queued ray (trace_queue); the queue's length is read on the
 // device, so launches never depend on a host read of it.
 // one_origin: every ray of the queue starts at q_o[0] (the path tracer's camera rays:
