@@ -44,8 +44,8 @@ __global__ void k_set_count(uint32_t* c, uint32_t n) { *c = n; }
 // / 36% / 31% of device time): one block per SM, whose warps all shade the same code
 // path, relieves the instruction fetch that bounded the kernel.  A queue too short to
 // give every SM two such blocks is shaded in 128-thread blocks instead, which spread
-// it over all SMs.  One block of 1024 threads per SM (64 registers, some spilled) was
-// slower than 768 (shading 9.38 vs 9.02 ms per render).
+// it over all SMs.  With chunks that stay in L1, 512 / 640 / 768 / 896 / 1024 threads take
+// 8.08 / 6.99 / 6.74 / 6.50 / 6.49 ms of shading per render (see SHADE_WIDE).
 #ifndef GR_SHADE_BLOCK
 #define GR_SHADE_BLOCK 768
 #endif
