@@ -81,6 +81,8 @@ gr_status run_engine_batch(const std::vector<const gr_job*>& jobs, const EngineC
         DevJob dj = make_job(j.scene, j.camera, j.params, j.film->width, j.film->height, film);
         s = e->add_job(dj, 0, 0, idx[k]);
         if (s != GR_OK) return s;
+        // The film was cleared on the default stream, which the engine's does not wait for.
+        if (!films_override) GR_CUDA_TRY(cudaStreamWaitEvent(e->stream(), j.film->cleared, 0));
         max_spp = std::max(max_spp, j.params.spp);
     }
     // Job-major order: a few scenes are live at a time, so their BVHs stay in L2; the
@@ -221,6 +223,7 @@ gr_status gr_batch_autotune(const gr_job* jobs, uint32_t n, gr_batch_options* ou
         GR_CUDA_TRY(cudaMemset(films[k].ptr, 0, bytes));
         fp[k] = films[k].as<float4>();
     }
+    GR_CUDA_TRY(cudaStreamSynchronize(0));  // cleared before an engine's own stream adds to them
     std::vector<const gr_job*> tj;
     for (auto& j : trial) tj.push_back(&j);
     double best = 0.0;
@@ -372,7 +375,7 @@ gr_status schedule(gr_server* s) {
         gr_status st;
         const size_t film_bytes = r->progressive ? r->bytes / 2 : r->bytes;
         GR_CUDA_TRY(r->film.ensure(film_bytes));
-        GR_CUDA_TRY(cudaMemset(r->film.ptr, 0, film_bytes));
+        GR_CUDA_TRY(cudaMemsetAsync(r->film.ptr, 0, film_bytes, s->engine.stream()));
         DevJob dj = make_job(r->req.scene, r->req.camera, r->req.params, r->req.width, r->req.height,
                              r->film.as<float4>());
         st = s->engine.add_job(dj, 0, 0, r->job);
@@ -380,7 +383,7 @@ gr_status schedule(gr_server* s) {
         if (r->progressive) {
             const size_t half = r->bytes / 2;
             GR_CUDA_TRY(r->film2.ensure(half));
-            GR_CUDA_TRY(cudaMemset(r->film2.ptr, 0, half));
+            GR_CUDA_TRY(cudaMemsetAsync(r->film2.ptr, 0, half, s->engine.stream()));
             DevJob d2 = make_job(r->req.scene, r->req.camera, r->req.params, r->req.width, r->req.height,
                                  r->film2.as<float4>());
             st = s->engine.add_job(d2, 0, 0, r->job2);
