@@ -8,8 +8,8 @@
 // (child, entry distance) pairs: the first SMEM_STACK entries in shared memory, column
 // `threadIdx.x`, deeper ones in a local array.  Popped entries whose entry distance is
 // no longer below the closest hit are skipped.  Every traversal (closest hit, shadow
-// rays, query kernels) runs the step functions below; visit_node and visit_leaf are the
-// only node and leaf tests.
+// rays, query kernels) runs the step functions below: visit_node and visit_leaf, one ray per
+// lane, or trace_grouped, which makes the same tests with W lanes per ray.
 // Leaves hold up to 16 consecutive primitive records.  The primitive tests are the
 // reference's Moller-Trumbore (geom/mesh.rs:270-308) and sphere quadratic
 // (geom/sphere.rs:70-101) with the same operation order, so a hit distance is
@@ -485,6 +485,7 @@ GR_D void trace_grouped(unsigned mask, const S& scene, TravState& t, uint32_t& s
             const unsigned first = (__ballot_sync(all, key != KEY_MISS && rank == 0u) >> g0) & ones;
             const int32_t near = __shfl_sync(all, child, static_cast<int>(g0) + (first ? __ffs(first) - 1 : 0));
             const int far = __popc(hits) - 1;
+            __syncwarp();  // every lane of the group has read the entries that are written over (next)
             if (key != KEY_MISS && rank > 0u)
                 col[(sp + far - static_cast<int>(rank)) * K::stride] = make_int2(child, static_cast<int>(key & ~7u));
             if (node && hits) {
