@@ -7,7 +7,8 @@
 //   * its partition swaps matches to the front.  With k matches, p1 the first non-match, T
 //     the positions of the matches after it and R = |T|, the matches keep their order at
 //     the front, and the non-match at position p ends at k + pos - R, where pos starts at
-//     p - p1 and steps pos = T[pos] - p1 while pos < R: every element finds its place alone;
+//     p - p1 and steps pos = T[pos] - p1 while pos < R: every element finds its place alone
+//     (sah_walk.cuh);
 //   * a node whose centroids coincide is a leaf there.  Its components are halved here, as
 //     the collapse halves a range, down to single ones.
 //
@@ -22,6 +23,8 @@
 // trees too deep for the level limits, are left to the host.  Positions read from the order
 // are kept inside their arrays whatever they hold.
 #pragma once
+
+#include "sah_walk.cuh"
 
 namespace gr {
 
@@ -183,18 +186,6 @@ GR_D void sah_add(int* tab, bool in, uint32_t b, const float* x, const float* c)
         }
         __syncwarp();
     }
-}
-
-// Where the swap partition leaves a non-match, R less: follows T (`moved`), whose entries
-// lie ahead of their positions, from `pos` until it is past it.
-template <class I>
-GR_D uint32_t sah_back(const I* moved, uint32_t pos, uint32_t R, uint32_t p1) {
-    while (pos < R) {
-        const uint32_t to = moved[pos] - p1;
-        if (to <= pos) break;  // cannot be: the walk would not end
-        pos = to;
-    }
-    return pos;
 }
 
 GR_D void sah_load(const SahView& s, uint32_t id, float* x, float* c) {
