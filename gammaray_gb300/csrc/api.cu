@@ -12,6 +12,7 @@
 #include <initializer_list>
 #include <memory>
 
+#include "film_clear.hpp"
 #include "runtime.hpp"
 
 namespace gr {
@@ -373,10 +374,9 @@ gr_status gr_film_create(uint32_t w, uint32_t h, gr_film** out) {
     f->height = h;
     size_t bytes = static_cast<size_t>(w) * h * sizeof(float4);
     GR_CUDA_TRY(f->pixels.ensure(bytes));
-    GR_CUDA_TRY(cudaMemset(f->pixels.ptr, 0, bytes));
+    GR_CUDA_TRY(cudaGetDevice(&f->device));
     GR_CUDA_TRY(cudaEventCreateWithFlags(&f->cleared, cudaEventDisableTiming));
-    GR_CUDA_TRY(cudaEventRecord(f->cleared, 0));
-    cudaGetDevice(&f->device);
+    GR_CUDA_TRY(clear_film(f->device, f->pixels.ptr, nullptr, bytes, f->cleared));
     *out = f.release();
     return GR_OK;
 }
@@ -388,9 +388,8 @@ gr_status gr_film_destroy(gr_film* f) {
 
 gr_status gr_film_clear(gr_film* f) {
     if (!f) return fail(GR_ERR_INVALID_ARGUMENT, "null film");
-    GR_CUDA_TRY(cudaMemset(f->pixels.ptr, 0, static_cast<size_t>(f->width) * f->height * sizeof(float4)));
-    if (f->splat.ptr) GR_CUDA_TRY(cudaMemset(f->splat.ptr, 0, static_cast<size_t>(f->width) * f->height * sizeof(float4)));
-    GR_CUDA_TRY(cudaEventRecord(f->cleared, 0));
+    const size_t bytes = static_cast<size_t>(f->width) * f->height * sizeof(float4);
+    GR_CUDA_TRY(clear_film(f->device, f->pixels.ptr, f->splat.ptr, bytes, f->cleared));
     f->passes = 0;
     return GR_OK;
 }
