@@ -178,6 +178,7 @@ gr_status gr_batch_release(void) {
     std::lock_guard<std::mutex> g(g_cache_mu);
     g_cache.clear();  // each engine waits for its stream, then frees its buffers
     g_cache_used.clear();
+    GR_CUDA_TRY(device_work().scratch.trim());
     return GR_OK;
 }
 

@@ -29,7 +29,6 @@
 #include <cfloat>
 #include <memory>
 #include <string>
-#include <utility>
 #include <vector>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -447,17 +446,47 @@ namespace gr {
 
 namespace {
 
+// Device memory for the build alone, allocated and freed in the order of its stream, from a
+// pool: cudaFree waits for all work on the device, so a creation would wait for every render
+// that other threads have running.
+struct StreamBuf {
+    cudaStream_t st;
+    void* ptr = nullptr;
+    explicit StreamBuf(cudaStream_t s) : st(s) {}
+    StreamBuf(const StreamBuf&) = delete;
+    StreamBuf& operator=(const StreamBuf&) = delete;
+    ~StreamBuf() { release(); }
+    void release() {
+        if (ptr) cudaFreeAsync(ptr, st);
+        ptr = nullptr;
+    }
+    cudaError_t allocate(size_t bytes) {
+        release();
+        if (alloc_should_fail()) return cudaErrorMemoryAllocation;
+        cudaMemPool_t pool;
+        cudaError_t e = device_work().scratch.get(pool);
+        if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&ptr, bytes, pool, st);
+        if (e != cudaSuccess) ptr = nullptr;
+        return e;
+    }
+    template <class T>
+    T* as() const {
+        return static_cast<T*>(ptr);
+    }
+};
+
 // One allocation carved into the build's scratch buffers: sizes are added first, then
 // reserve() makes the pointers valid.
 struct Slab {
-    DevBuf buf;
+    StreamBuf buf;
     size_t total = 0;
+    explicit Slab(cudaStream_t st) : buf(st) {}
     size_t add(size_t bytes) {
         const size_t at = total;
         total += (bytes + 255) & ~size_t(255);
         return at;
     }
-    cudaError_t reserve() { return buf.ensure(std::max<size_t>(total, 256)); }
+    cudaError_t reserve() { return buf.allocate(std::max<size_t>(total, 256)); }
     template <class T>
     T* at(size_t offset) const {
         return reinterpret_cast<T*>(buf.as<unsigned char>() + offset);
@@ -567,13 +596,12 @@ gr_status sah_tree(const SahView& v, uint32_t* perm, cudaStream_t st, int& root)
 // stack use took 930 us there, this way 330.
 constexpr uint32_t LEVELS_AT_ONCE = 22;
 
-// `root_ref`: the binary tree's root node (of a single component: its leaf, ~0).
+// `root_ref`: the binary tree's root node (of a single component: its leaf, ~0).  `nodes` has
+// room for n: every wide node stands for a distinct binary node (or the root leaf).
 template <int W>
 gr_status collapse_levels(int root_ref, uint32_t n, CollapseCtl* ctl, const int* err, int4* todo, const Opened* opened,
-                          const float* box, const uint32_t* perm, uint32_t leaf_size, SceneBuffers& b,
+                          const float* box, const uint32_t* perm, uint32_t leaf_size, float* nodes,
                           cudaStream_t st, uint32_t& num_wide, uint32_t& stack_depth) {
-    // Every wide node stands for a distinct binary node (or the root leaf): at most n.
-    GR_CUDA_TRY(b.nodes.ensure(static_cast<size_t>(n) * 8 * W * sizeof(float)));
     const int4 root = make_int4(root_ref, 0, static_cast<int>(n), 0);
     const uint32_t one = 1;
     GR_CUDA_TRY(cudaMemsetAsync(ctl, 0, sizeof(CollapseCtl), st));
@@ -586,8 +614,7 @@ gr_status collapse_levels(int root_ref, uint32_t n, CollapseCtl* ctl, const int*
         const uint32_t stop = std::min(level + LEVELS_AT_ONCE, MAX_LEVELS);
         for (; level < stop; ++level) {
             const uint32_t grid = std::min<uint64_t>(most, (width + BB - 1) / BB);
-            k_collapse<W><<<grid, BB, 0, st>>>(ctl, err, level, todo, opened, box, perm, leaf_size,
-                                                b.nodes.as<float>());
+            k_collapse<W><<<grid, BB, 0, st>>>(ctl, err, level, todo, opened, box, perm, leaf_size, nodes);
             GR_CUDA_TRY(cudaGetLastError());
             width = std::min<uint64_t>(width * W, n);
         }
@@ -618,7 +645,7 @@ gr_status build_bvh_device(const gr_scene_desc& desc, const HostBuild& h, SceneB
         GR_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, static_cast<uint32_t*>(nullptr),
                                                 static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
                                                 static_cast<uint32_t*>(nullptr), static_cast<int>(n), 0, 30, st));
-    Slab m;
+    Slab m(st);
     const size_t o_box = m.add(size_t(n) * 6 * sizeof(float)), o_rec = m.add(size_t(n) * 3 * sizeof(float4));
     const size_t attr = size_t(n) * 3 * sizeof(uint32_t);
     const size_t o_tn = m.add(h.any_normals ? attr : 0), o_tu = m.add(h.any_uvs ? attr : 0);
@@ -632,6 +659,9 @@ gr_status build_bvh_device(const gr_scene_desc& desc, const HostBuild& h, SceneB
     const size_t o_code_s = m.add(lin * sizeof(uint32_t)), o_tmp = m.add(std::max<size_t>(tmp_bytes, 16));
     const size_t o_split = m.add(lin_i * sizeof(int4)), o_par_i = m.add(lin_i * sizeof(int));
     const size_t o_par_l = m.add(lin * sizeof(int)), o_visits = m.add(lin_i * sizeof(int));
+    // The SAH scene keeps as many nodes as there are; the linear one the worst case's room.
+    const size_t node_bytes = size_t(8) * W * sizeof(float);
+    const size_t o_nodes = m.add(h.device_sah ? n * node_bytes : 0);
     std::unique_ptr<SahScratch> sah;
     if (h.device_sah) sah.reset(new SahScratch(m, n));
     // The caller's arrays (records made on the device).
@@ -738,8 +768,10 @@ gr_status build_bvh_device(const gr_scene_desc& desc, const HostBuild& h, SceneB
     GR_CUDA_TRY(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     CollapseCtl* ctl = m.at<CollapseCtl>(o_ctl);
     int4* todo = m.at<int4>(o_todo);
+    if (!sah) GR_CUDA_TRY(b.nodes.ensure(n * node_bytes));
+    float* nodes = sah ? m.at<float>(o_nodes) : b.nodes.as<float>();
     auto collapse = W == 2 ? collapse_levels<2> : (W == 8 ? collapse_levels<8> : collapse_levels<4>);
-    const gr_status s = collapse(root, n, ctl, err, todo, opened, box, perm, L, b, st, num_wide, stack_depth);
+    const gr_status s = collapse(root, n, ctl, err, todo, opened, box, perm, L, nodes, st, num_wide, stack_depth);
     if (s != GR_OK) return s;  // (it has synchronised the stream, so `e` is there)
     if (e == ERR_BAD_INDEX) {
         set_error("device BVH build: an index is out of range");
@@ -756,18 +788,14 @@ gr_status build_bvh_device(const gr_scene_desc& desc, const HostBuild& h, SceneB
     }
     if (sah) {
         SahCtl ctl_end;
-        const size_t used = size_t(num_wide) * 8 * W * sizeof(float);
-        DevBuf nodes;  // as many as there are: the collapse's were sized for the worst case
-        GR_CUDA_TRY(nodes.ensure(used));
-        GR_CUDA_TRY(cudaMemcpyAsync(nodes.ptr, b.nodes.ptr, used, cudaMemcpyDeviceToDevice, st));
+        GR_CUDA_TRY(b.nodes.ensure(num_wide * node_bytes));
+        GR_CUDA_TRY(cudaMemcpyAsync(b.nodes.ptr, nodes, num_wide * node_bytes, cudaMemcpyDeviceToDevice, st));
         GR_CUDA_TRY(cudaMemcpyAsync(&ctl_end, m.at<SahCtl>(sah->ctl), sizeof(ctl_end), cudaMemcpyDeviceToHost, st));
         GR_CUDA_TRY(cudaStreamSynchronize(st));
         if (ctl_end.failed) {
             set_error("device BVH build: left to the host");
             return GR_ERR_INTERNAL;
         }
-        std::swap(nodes.ptr, b.nodes.ptr);
-        std::swap(nodes.bytes, b.nodes.bytes);
         num_binary = 2 * (uint64_t(n) - ctl_end.excess) - 1;
     }
     const size_t rec_bytes = size_t(n) * 3 * sizeof(float4);
@@ -777,8 +805,9 @@ gr_status build_bvh_device(const gr_scene_desc& desc, const HostBuild& h, SceneB
     k_permute<<<blocks, BB, 0, st>>>(rec, tn, tu, perm, n, b.prims.as<float4>(), b.tri_nidx.as<uint32_t>(),
                                      b.tri_uvidx.as<uint32_t>());
     GR_CUDA_TRY(cudaGetLastError());
+    m.buf.release();  // (goes back to the device with the wait)
     GR_CUDA_TRY(cudaStreamSynchronize(st));
-    bytes += static_cast<uint64_t>(num_wide) * 8 * W * sizeof(float) + rec_bytes + (tn ? attr : 0) + (tu ? attr : 0);
+    bytes += num_wide * node_bytes + rec_bytes + (tn ? attr : 0) + (tu ? attr : 0);
     return GR_OK;
 }
 

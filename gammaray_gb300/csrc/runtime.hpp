@@ -115,8 +115,44 @@ struct BounceReadback {
     }
 };
 
+// A device's pool for scratch that is allocated and freed in the order of a stream (scene
+// creation).  It keeps up to KEEP bytes of what was freed for the next scene, and gives them
+// back in gr_batch_release.  Creation with nothing kept / 64 MB / 1 GB (ms): 5,000 triangles
+// 1.16 / 1.01 / 1.01, 102,400 1.67 / 1.45 / 1.45, 400,000 2.41 / 2.22 / 2.06, 1,000,000 4.03 /
+// 3.85 / 3.25 (350 bytes each); with cudaMalloc and cudaFree 1.00, 1.64, 2.26, 3.60.
+struct ScratchPool {
+    static constexpr uint64_t KEEP = uint64_t(512) << 20;
+    std::mutex mu;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t get(cudaMemPool_t& out) {  // of the current device
+        std::lock_guard<std::mutex> g(mu);
+        if (!pool) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            cudaError_t e = cudaGetDevice(&props.location.id);
+            cudaMemPool_t p = nullptr;
+            if (e == cudaSuccess) e = cudaMemPoolCreate(&p, &props);
+            uint64_t keep = KEEP;
+            if (e == cudaSuccess) e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+            if (e != cudaSuccess) {
+                if (p) cudaMemPoolDestroy(p);
+                return e;
+            }
+            pool = p;
+        }
+        out = pool;
+        return cudaSuccess;
+    }
+    cudaError_t trim() {
+        std::lock_guard<std::mutex> g(mu);
+        return pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
+    }
+};
+
 struct DeviceWork {
     std::mutex mu;
+    ScratchPool scratch;
     PathState paths;
     BdptState bdpt;
     BounceReadback readback;
