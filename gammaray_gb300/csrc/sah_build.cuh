@@ -433,7 +433,8 @@ static_assert(SAH_TILE / 32 == 32 && SAH_TILE % BB == 0, "a tile's chunks are on
 // The right sides, and the children.
 __global__ void __launch_bounds__(BB) k_sah_back(SahView s, uint32_t level) {
     const SahLevel& L = s.level[level & 1];
-    const uint32_t tiles = s.ctl->failed ? 0u : s.ctl->tiles[level];
+    // (one lane's reading: `failed` may be set by another block meanwhile)
+    const uint32_t tiles = __shfl_sync(0xffffffffu, s.ctl->failed ? 0u : s.ctl->tiles[level], 0);
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         const uint2 tile = L.tiles[t];
         const SahNode& nd = L.nodes[tile.x];
@@ -606,7 +607,9 @@ __global__ void __launch_bounds__(BB) k_sah_small(SahView s, uint32_t* __restric
     extern __shared__ unsigned char smem[];
     SahTree<N>& T = *reinterpret_cast<SahTree<N>*>(smem);
     const unsigned all = 0xffffffffu, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
-    const uint32_t trees = s.ctl->failed ? 0u : s.ctl->small;
+    // (not launched once `failed` is set; a block that sets it below has a tree all the same, and
+    // the barriers need every thread of a block to make the same turns)
+    const uint32_t trees = s.ctl->small;
     int* tab = T.tab[warp];
     for (uint32_t t = blockIdx.x; t < trees; t += gridDim.x) {
         const SahSmall root = s.small[t];
