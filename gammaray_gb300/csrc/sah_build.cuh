@@ -506,6 +506,7 @@ struct SahTree {
         return 0.5f * box[dim][k] + 0.5f * box[3 + dim][k];
     }
 };
+static_assert(sizeof(SahTree<SAH_SMALL_MANY>) <= 48 * 1024, "k_sah_small is launched without a shared memory attribute");
 constexpr uint32_t SAH_RANGE = 1u << 31;
 
 // The reference's nth_element (geom/util.rs), its swap partition and its shortened left side
