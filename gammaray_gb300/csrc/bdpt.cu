@@ -339,8 +339,7 @@ __global__ void __launch_bounds__(BLOCK) k_bdpt_raygen(DeviceScene s, BdptParams
 // One vertex of random_walk (integrators.rs:138-229) at the hit h = (t, leaf-order primitive
 // or -1, u, v) of walk `slot`'s ray (o, d): stores the vertex and advances w.  Returns
 // whether the walk goes on, with its next ray; a walk that ends leaves its vertex count.
-// `lobe`: the lobe already picked (sorted_lobe), or ANY_LOBE.
-constexpr uint32_t ANY_LOBE = 0xFFFFFFFFu;
+// `lobe`: the lobe that shade_bucket picked.
 template <bool MIS>
 GR_D bool walk_vertex(const DeviceScene& s, const BdptParams& p, const Verts& vs, const PathOut& out, uint32_t slot,
                       Walk& w, uint32_t lobe, V3 o, V3 d, float4 h, V3& new_o, V3& new_d) {
@@ -365,7 +364,6 @@ GR_D bool walk_vertex(const DeviceScene& s, const BdptParams& p, const Verts& vs
     uint32_t base = (walk ? DIM_LIGHT_WALK : DIM_CAMERA_WALK) + 4 * k;
     V3 incoming = -d;
     V3 hit_point = o + (d * h.x);
-    if (lobe == ANY_LOBE) lobe = pick_lobe(m, uniform01(w.key, base));
     MaterialSample ms = sample_lobe(m, incoming, f, c2l, static_cast<int>(lobe), uniform01(w.key, base + 1),
                                     uniform01(w.key, base + 2));
     bool connectible = count_lobes(m, LOBE_DIFFUSE | LOBE_GLOSSY) != 0;

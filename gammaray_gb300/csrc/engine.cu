@@ -299,8 +299,7 @@ __global__ void __launch_bounds__(BS) k_eng_extend_refill(EngineCtl* c, int cur,
 
 // One vertex of a job's path at the hit h = (t, leaf-order primitive or -1, u, v) of the ray
 // (o, d): radiance into L, the next throughput in tp and the next ray.  Returns whether the
-// path goes on.  `lobe`: the lobe already picked (sorted_lobe), or ANY_LOBE.
-constexpr uint32_t ANY_LOBE = 0xFFFFFFFFu;
+// path goes on.  `lobe`: the lobe that shade_bucket picked.
 GR_D bool shade_job(const DevJob& J, uint32_t depth, uint64_t key, uint32_t lobe, V3 o, V3 d, float4 h, V3& tp, V3& L,
                     V3& new_o, V3& new_d) {
     const DeviceScene& s = J.scene;
@@ -322,7 +321,6 @@ GR_D bool shade_job(const DevJob& J, uint32_t depth, uint64_t key, uint32_t lobe
     Frame f = hit_frame(s, k, o, d, h.x, h.z, h.w, prim);
     const DevMaterial& m = s.materials[__ldg(s.prim_material + prim)];
     const uint32_t base = DIM_CAMERA_WALK + 4 * depth;
-    if (lobe == ANY_LOBE) lobe = pick_lobe(m, uniform01(key, base));
     MaterialSample ms =
         sample_lobe(m, -d, f, true, static_cast<int>(lobe), uniform01(key, base + 1), uniform01(key, base + 2));
     L = L + mul(tp, ms.emission);

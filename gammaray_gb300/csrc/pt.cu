@@ -147,8 +147,7 @@ GR_D void push_path(bool alive, uint32_t* count_out, uint32_t slot, V3 o, V3 d, 
 // One vertex of PathTracerIntegrator::integrate (render/integrators.rs:42-100) at the hit
 // h = (t, leaf-order primitive or -1, u, v) of the ray (o, d): emission into L, the next
 // throughput in tp and the next ray.  Returns whether the path goes on.
-// `lobe`: the lobe already picked (sorted_lobe), or ANY_LOBE.
-constexpr uint32_t ANY_LOBE = 0xFFFFFFFFu;
+// `lobe`: the lobe that shade_bucket picked.
 GR_D bool shade_hit(const DeviceScene& s, const PTParams& p, uint32_t depth, uint64_t key, uint32_t lobe, V3 o, V3 d,
                     float4 h, V3& tp, V3& L, V3& new_o, V3& new_d) {
     const int32_t k = __float_as_int(h.y);
@@ -160,7 +159,6 @@ GR_D bool shade_hit(const DeviceScene& s, const PTParams& p, uint32_t depth, uin
     uint32_t prim;
     Frame f = hit_frame(s, k, o, d, h.x, h.z, h.w, prim);
     const DevMaterial& m = s.materials[__ldg(s.prim_material + prim)];
-    if (lobe == ANY_LOBE) lobe = pick_lobe(m, uniform01(key, base));
     MaterialSample ms =
         sample_lobe(m, -d, f, true, static_cast<int>(lobe), uniform01(key, base + 1), uniform01(key, base + 2));
     L = L + mul(tp, ms.emission);
