@@ -111,7 +111,7 @@ gr_status run_engine_batch(const std::vector<const gr_job*>& jobs, const EngineC
     if (s != GR_OK) return s;
     st.samples += c.paths_total;  // all finished: the batch ran to completion
     st.extension_rays += c.rays;
-    st.kernel_launches += static_cast<uint64_t>(c.iter) * 6;
+    st.kernel_launches += static_cast<uint64_t>(c.iter) * Engine::KERNELS_PER_ITERATION;
     st.device_ms += ms;
     if (!done) {
         set_error("batch did not complete");

@@ -94,6 +94,7 @@ struct EngineConfig {
 
 class Engine {
   public:
+    static constexpr uint32_t KERNELS_PER_ITERATION = 6;  // plan, gather, fill, loop, extend, shade
     Engine() {}
     ~Engine();
     gr_status init(const EngineConfig& cfg, cudaStream_t st);
