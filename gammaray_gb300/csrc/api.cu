@@ -238,6 +238,7 @@ gr_status gr_scene_create(const gr_scene_desc* desc, gr_scene** out) {
         uint32_t num_wide = 0, stack_depth = 0;
         const gr_status bs =
             build_bvh_device(*desc, h, b, st, num_wide, stack_depth, h.num_binary_nodes, total);
+        GR_TRY(build_index_check());
         if (bs == GR_ERR_INVALID_ARGUMENT && !h.device_sah) {
             HostBuild checked;
             return build_scene(*desc, checked, err) ? bs : fail(bs, err);
@@ -605,7 +606,7 @@ gr_status gr_trace_rays(gr_scene* s, const float* rays, uint64_t n, gr_hit* hits
     GR_CUDA_TRY(cudaStreamSynchronize(s->stream));
     if (herr == 2) return fail(GR_ERR_TIMEOUT, "traversal step budget exceeded");
     if (herr) return fail(GR_ERR_STACK_OVERFLOW, "traversal stack bound exceeded");
-    return GR_OK;
+    return query_index_check();
 }
 
 gr_status gr_trace_rays_dev(gr_scene* s, const float* rays, uint64_t n, gr_hit* hits, void* stream) {
@@ -648,7 +649,7 @@ gr_status gr_visibility(gr_scene* s, const float* pairs, uint64_t n, uint8_t* vi
     GR_CUDA_TRY(cudaStreamSynchronize(s->stream));
     if (herr == 2) return fail(GR_ERR_TIMEOUT, "traversal step budget exceeded");
     if (herr) return fail(GR_ERR_STACK_OVERFLOW, "traversal stack bound exceeded");
-    return GR_OK;
+    return query_index_check();
 }
 
 gr_status gr_sample_light(gr_scene* s, const float* u, uint64_t n, gr_light_sample* out) {

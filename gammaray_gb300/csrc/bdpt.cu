@@ -344,6 +344,7 @@ template <bool MIS>
 GR_D bool walk_vertex(const DeviceScene& s, const BdptParams& p, const Verts& vs, const PathOut& out, uint32_t slot,
                       Walk& w, uint32_t lobe, V3 o, V3 d, float4 h, V3& new_o, V3& new_d) {
     const uint32_t walk = slot & 1u, path = slot >> 1, k = w.k;
+    if (!GR_IN_RANGE(k, p.max_len) || !GR_IN_RANGE(slot, p.nslots)) return false;
     const bool c2l = walk == 0;
     const int32_t pk = __float_as_int(h.y);
     if (pk < 0) {
@@ -758,7 +759,8 @@ __global__ void __launch_bounds__(BLOCK) k_bdpt_len_scatter(uint32_t n, const ui
         if (in && static_cast<int>(lane) == leader)
             base = atomicAdd(&items->hist[key], static_cast<uint32_t>(__popc(same)));
         base = __shfl_sync(0xffffffffu, base, leader);
-        if (in) order[base + __popc(same & ((1u << lane) - 1u))] = i;
+        const uint32_t at = base + __popc(same & ((1u << lane) - 1u));
+        if (in && GR_IN_RANGE(at, n)) order[at] = i;
     }
 }
 

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(BB) k_collapse(CollapseCtl* ctl, const int* __
                                                  int4* __restrict__ todo,
                                                  const Opened* __restrict__ opened, const float* __restrict__ box,
                                                  const uint32_t* __restrict__ perm, uint32_t leaf_size,
-                                                 float* __restrict__ nodes) {
+                                                 float* __restrict__ nodes, [[maybe_unused]] uint32_t room) {
     const uint32_t n = ctl->count[level];
     if (n == 0 || *err) return;  // (a flagged tree is not walked)
     uint32_t begin = 0;
@@ -320,7 +320,8 @@ __global__ void __launch_bounds__(BB) k_collapse(CollapseCtl* ctl, const int* __
                                             static_cast<uint32_t>(c[j].count - 1));
                 } else {
                     ref = static_cast<int>(next);
-                    todo[next++] = make_int4(c[j].ref, c[j].first, c[j].count, static_cast<int>(held));
+                    if (GR_IN_RANGE(next, room)) todo[next] = make_int4(c[j].ref, c[j].first, c[j].count, static_cast<int>(held));
+                    ++next;
                 }
             }
             for (int a = 0; a < 3; ++a) {
@@ -614,7 +615,7 @@ gr_status collapse_levels(int root_ref, uint32_t n, CollapseCtl* ctl, const int*
         const uint32_t stop = std::min(level + LEVELS_AT_ONCE, MAX_LEVELS);
         for (; level < stop; ++level) {
             const uint32_t grid = std::min<uint64_t>(most, (width + BB - 1) / BB);
-            k_collapse<W><<<grid, BB, 0, st>>>(ctl, err, level, todo, opened, box, perm, leaf_size, nodes);
+            k_collapse<W><<<grid, BB, 0, st>>>(ctl, err, level, todo, opened, box, perm, leaf_size, nodes, n);
             GR_CUDA_TRY(cudaGetLastError());
             width = std::min<uint64_t>(width * W, n);
         }
@@ -808,6 +809,18 @@ gr_status build_bvh_device(const gr_scene_desc& desc, const HostBuild& h, SceneB
     m.buf.release();  // (goes back to the device with the wait)
     GR_CUDA_TRY(cudaStreamSynchronize(st));
     bytes += num_wide * node_bytes + rec_bytes + (tn ? attr : 0) + (tu ? attr : 0);
+    return GR_OK;
+}
+
+gr_status build_index_check() {
+#if GR_CHECKED
+    bool bad = false;
+    GR_CUDA_TRY(take_bad_index(bad));
+    if (bad) {
+        set_error("device BVH build: an index was out of range (checked build)");
+        return GR_ERR_INTERNAL;
+    }
+#endif
     return GR_OK;
 }
 

@@ -14,10 +14,12 @@
 #define GR_HD __host__ __device__ __forceinline__
 #define GR_D __device__ __forceinline__
 
-// Checked build (-DGR_CHECKED=1, the stand-in for a memory checker): every queue, entry
-// and shadow-queue write tests its index against its buffer's capacity, skips the write
-// when it is out of range and sets this file's flag, which the host reads after the
-// render (GR_ERR_INTERNAL).  Off by default; then GR_IN_RANGE is `true`.
+// Checked build (-DGR_CHECKED=1, the stand-in for a memory checker): every write to a place
+// that a kernel computes from data (queues, path and ring slots, vertices, entries, shadow
+// queue, query results, the SAH build's tree and lists, wide nodes to open) tests its index
+// against its buffer's capacity, skips the write when it is out of range and sets this file's
+// flag, which the host reads after the work (GR_ERR_INTERNAL).  Off by default; then
+// GR_IN_RANGE is `true`.
 #ifndef GR_CHECKED
 #define GR_CHECKED 0
 #endif

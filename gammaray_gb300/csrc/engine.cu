@@ -384,7 +384,8 @@ __global__ void __launch_bounds__(PATH_LOOP_THREADS, PATH_LOOP_BLOCKS)
         ++path.depth;
         if (!alive) {
             s_hot[path.slot] = make_float4(path.L.x, path.L.y, path.L.z, 0.0f);
-            atomicAdd(unit_done + s_cold[path.slot].x, 1u);
+            const uint32_t unit = s_cold[path.slot].x;
+            if (GR_IN_RANGE(unit, c->units_count)) atomicAdd(unit_done + unit, 1u);
         }
         return alive;
     };
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(ESBLOCK, ESBLOCK < 768 ? 768 / ESBLOCK : 1)
             // launches on the same stream.
             if (__any_sync(0xffffffffu, finished)) {
                 unsigned same = __match_any_sync(0xffffffffu, unit);
-                if (finished && lane == static_cast<unsigned>(__ffs(same) - 1))
+                if (finished && lane == static_cast<unsigned>(__ffs(same) - 1) && GR_IN_RANGE(unit, c->units_count))
                     atomicAdd(unit_done + unit, static_cast<uint32_t>(__popc(same)));
             }
             push_ray(alive, &c->q[nxt], slot, new_o, new_d, job, depth + 1, sa, sb, nslot, no, nd, nstate, cap);

@@ -180,7 +180,8 @@ GR_D uint32_t run_paths(const K& stk, unsigned char* smem, uint32_t n, uint32_t*
             if (tid == 31) *total = x;
         }
         __syncthreads();
-        if (busy) order[count[b % SORT_BUCKETS] + pos] = tid | (b / SORT_BUCKETS << 16);
+        if (busy && GR_IN_RANGE(count[b % SORT_BUCKETS] + pos, NT))
+            order[count[b % SORT_BUCKETS] + pos] = tid | (b / SORT_BUCKETS << 16);
         __syncthreads();
         const uint32_t m = *total, share = (m + NT / 32 - 1) / (NT / 32), at = (tid >> 5) * share + lane;
         if (tid < SORT_BUCKETS) count[tid] = 0;

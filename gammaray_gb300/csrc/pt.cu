@@ -106,7 +106,7 @@ GR_D uint32_t camera_path(const PTParams& p, uint32_t q, float2* __restrict__ st
     float s, t;
     film_sample_point(p.order.width, p.order.height, ps.row, ps.col, key, s, t);
     camera_ray(p.cam, s, t, o, d);
-    st[ps.slot] = make_float2(s, t);
+    if (GR_IN_RANGE(ps.slot, p.qcap)) st[ps.slot] = make_float2(s, t);
     return ps.slot;
 }
 
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(NT, NT < 768 ? 768 / NT : 1) k_shade(DeviceSce
                 if (alive) {
                     sa = make_float4(tp.x, tp.y, tp.z, L.x);
                     sb = make_float4(L.y, L.z, sb.z, sb.w);
-                } else {
+                } else if (GR_IN_RANGE(slot, p.qcap)) {
                     L_buf[slot] = make_float4(L.x, L.y, L.z, 0.0f);
                 }
             }
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(PATH_LOOP_THREADS, PATH_LOOP_BLOCKS)
     auto shade = [&](LoopPath& path, uint32_t lobe, V3 o, V3 d, float4 h, V3& no, V3& nd) {
         const bool alive = shade_hit(s, p, path.depth, path.key, lobe, o, d, h, path.tp, path.L, no, nd);
         ++path.depth;
-        if (!alive) L_buf[path.slot] = make_float4(path.L.x, path.L.y, path.L.z, 0.0f);
+        if (!alive && GR_IN_RANGE(path.slot, p.qcap)) L_buf[path.slot] = make_float4(path.L.x, path.L.y, path.L.z, 0.0f);
         return alive;
     };
     count_rays(run_paths<W, sizeof(LoopPath) / 4, LoopPath>(

@@ -79,7 +79,8 @@ __global__ void __launch_bounds__(QUERY_BLOCK) k_trace(DeviceScene s, const floa
             return true;
         },
         [&](uint32_t q, const TravState& t) {
-            write_hit(s, hits + share.ray(q), TraceResult{t.closest, t.hit, t.hu, t.hv});
+            if (GR_IN_RANGE(share.ray(q), n))
+                write_hit(s, hits + share.ray(q), TraceResult{t.closest, t.hit, t.hu, t.hv});
         },
         s.num_components >= GROUPED_COMPONENTS);
 }
@@ -133,7 +134,9 @@ __global__ void __launch_bounds__(QUERY_BLOCK) k_visibility(DeviceScene s, const
             trav_init(t, o, d, magnitude(b - o) - 1e-3f);
             return true;
         },
-        [&](uint32_t q, const TravState& t) { vis[share.ray(q)] = t.hit < 0 ? 1 : 0; },
+        [&](uint32_t q, const TravState& t) {
+            if (GR_IN_RANGE(share.ray(q), n)) vis[share.ray(q)] = t.hit < 0 ? 1 : 0;
+        },
         s.num_components >= GROUPED_COMPONENTS);
 }
 
@@ -248,6 +251,18 @@ gr_status launch_trace(const DeviceScene& s, const float* rays, uint64_t n, gr_h
     }
     set_error("unsupported BVH width");
     return GR_ERR_INTERNAL;
+}
+
+gr_status query_index_check() {
+#if GR_CHECKED
+    bool bad = false;
+    GR_CUDA_TRY(take_bad_index(bad));
+    if (bad) {
+        set_error("ray query: a ray's index was out of range (checked build)");
+        return GR_ERR_INTERNAL;
+    }
+#endif
+    return GR_OK;
 }
 
 gr_status launch_naive(const DeviceScene& s, const float* rays, uint64_t n, gr_hit* hits, cudaStream_t st) {

@@ -244,15 +244,17 @@ struct RenderJob {
 
 gr_status render_pt(gr_scene* sc, const RenderJob& job, cudaStream_t st);
 gr_status render_bdpt(gr_scene* sc, const RenderJob& job, cudaStream_t st);
-// Checked builds (GR_CHECKED): whether a render's kernels wrote out of range (read after
-// the render's work has finished); GR_OK otherwise.
 // Scene lifetime across server requests: a request retains its scene from submission
 // until no queued path can reach it any more; gr_scene_destroy waits for the last release.
 void scene_retain(gr_scene* s);
 void scene_release(gr_scene* s);
 
+// Checked builds (GR_CHECKED): whether kernels of a render, a ray query or a device build
+// wrote out of range (read after their work has finished); GR_OK otherwise.
 gr_status pt_index_check();
 gr_status bdpt_index_check();
+gr_status query_index_check();
+gr_status build_index_check();
 // Adds `passes` passes of samples (pass k at k * width * height in st_buf and color) to
 // `film`, each pixel's sum in the reference's serial order.  With `sched` (device
 // scratch of film_sched_words(width, height) words) and `err` (the error word; 3 = a

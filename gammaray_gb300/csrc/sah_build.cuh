@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(BB) k_sah_back(SahView s, uint32_t level) {
             if (threadIdx.x == 0) atomicExch(&s.ctl->failed, 1u);
             continue;
         }
-        if ((threadIdx.x & 31u) == 0) {
+        if ((threadIdx.x & 31u) == 0 && GR_IN_RANGE(c.slot, 2 * (s.n - 1))) {
             float* o = s.opened + 8 * static_cast<size_t>(c.slot);
             for (int a = 0; a < 3; ++a) {
                 o[a] = c.box[a];
@@ -542,6 +542,7 @@ GR_D void sah_nth(const SahTree<N>& T, uint16_t* s, uint32_t len, uint32_t nth, 
 }
 
 GR_D void sah_slot(const SahView& s, uint32_t slot, const float* b, int ref, uint32_t count) {
+    if (!GR_IN_RANGE(slot, 2 * (s.n - 1))) return;
     float4* o = reinterpret_cast<float4*>(s.opened + 8 * static_cast<size_t>(slot));
     o[0] = make_float4(b[0], b[1], b[2], __int_as_float(ref));
     o[1] = make_float4(b[3], b[4], b[5], __int_as_float(static_cast<int>(count)));
@@ -555,7 +556,7 @@ GR_D void sah_single(const SahView& s, const SahTree<N>& T, uint32_t first, uint
     e %= N;
     for (int a = 0; a < 6; ++a) b[a] = T.box[a][e];
     sah_slot(s, slot, b, ~static_cast<int>(first + at), 1);
-    perm[first + at] = T.id[e];
+    if (GR_IN_RANGE(first + at, s.n)) perm[first + at] = T.id[e];
 }
 
 // Subtrees of two to four components, by one thread.
@@ -734,9 +735,13 @@ __global__ void __launch_bounds__(BB) k_sah_small(SahView s, uint32_t* __restric
                 if (lane < 2) {
                     const uint32_t cf = lane ? f + mid : f, cn = lane ? n - mid : mid, slot = 2 * id + lane;
                     const uint2 c = make_uint2(cf | (cn << 16), slot | range);
-                    if (cn > 4) T.list[cur ^ 1][atomicAdd(&T.listed[cur ^ 1], 1u)] = c;
-                    else if (cn > 1) T.tiny[atomicAdd(&T.tinies, 1u)] = c;
-                    else sah_single(s, T, first, cf, B[cf], slot, perm);
+                    if (cn > 4) {
+                        const uint32_t at = atomicAdd(&T.listed[cur ^ 1], 1u);
+                        if (GR_IN_RANGE(at, N / 4)) T.list[cur ^ 1][at] = c;
+                    } else if (cn > 1) {
+                        const uint32_t at = atomicAdd(&T.tinies, 1u);
+                        if (GR_IN_RANGE(at, N / 2)) T.tiny[at] = c;
+                    } else sah_single(s, T, first, cf, B[cf], slot, perm);
                 }
             }
             __syncthreads();
