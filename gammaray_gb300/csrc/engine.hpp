@@ -59,6 +59,7 @@ struct EngineCtl {
     unsigned long long fill_base;
     unsigned long long rays;
     uint32_t units_count;
+    uint32_t loop_grouped;  // set by the host (with units_count): the path loop's last rays take groups of lanes
     uint32_t g_lo;  // oldest unit not yet gathered
     uint32_t q[2];
     uint32_t fill_n;
@@ -136,6 +137,7 @@ class Engine {
     EngineConfig cfg_;
     cudaStream_t st_ = nullptr;
     uint32_t ring_ = 0;
+    bool grouped_ = false;  // a job's scene is large enough for groups of lanes
     DevBuf ctl_, jobs_, units_, unit_done_;
     DevBuf s_hot_, s_cold_;  // path state ring (see engine.cu)
     DevBuf q_slot_[2], q_o_[2], q_d_[2], q_state_[2], q_hit_;
