@@ -220,8 +220,9 @@ GR_D Cand cand_of(const float4 c0, const float4 c1, int first) {
     return c;
 }
 
-// Levels of the wide tree.  The binary tree is at most 30 (code bits) + 32 (index bits of
-// equal codes) deep, so no collapse has more.
+// Levels of the wide tree.  The linear tree is at most 30 (code bits) + 32 (index bits of
+// equal codes) deep, so its collapse has no more.  A SAH tree can be deeper: one whose
+// collapse is goes to the host build.
 constexpr uint32_t MAX_LEVELS = 64;
 
 struct CollapseCtl {

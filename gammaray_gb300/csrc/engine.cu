@@ -13,16 +13,16 @@ namespace gr {
 namespace {
 
 constexpr int EBLOCK = 128;
-// The engine's shading kernel: blocks of GR_ENG_SHADE_BLOCK threads (128 or 768), each
-// sorting its chunk of the queue by code path.  At 768 one block fills an SM (85
-// registers), so all of an SM's warps shade the same code path at a time, as in the
-// path tracer's k_shade.
+// The engine's shading kernel: blocks of GR_ENG_SHADE_BLOCK threads (128, 768 or 896), each
+// sorting its chunk of the queue by code path.  At 768 (85 registers) and 896 (72) one block
+// fills an SM, so all of an SM's warps shade the same code path at a time, as in the path
+// tracer's k_shade.
 #ifndef GR_ENG_SHADE_BLOCK
 #define GR_ENG_SHADE_BLOCK 896
 #endif
 constexpr int ESBLOCK = GR_ENG_SHADE_BLOCK;
 static_assert(ESBLOCK == 128 || ESBLOCK == 768 || ESBLOCK == 896, "engine shading block of 128, 768 or 896 threads");
-// (72 registers, some spilled.  768 / 896 threads: 9.26 / 9.03 ms for 12 images in a batch,
+// (At 72 registers some are spilled.  768 / 896 threads: 9.26 / 9.03 ms for 12 images in a batch,
 // 14.9 / 14.4 for 6 served requests: its entries wait longer for their loads than the path
 // tracer's.)
 // Entries per thread per chunk: fewer than the path tracer's, since the sort also reads an

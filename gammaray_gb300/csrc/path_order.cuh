@@ -5,9 +5,9 @@
 // row * width + col is where the film gather finds it.  Entry q of the camera-ray queue
 // is not sample q: the queue runs through the image in patches, every pass of a few
 // neighbouring pixels together.  A warp's camera rays then cover a patch of 4 pixels x 8
-// passes instead of 32 pixels of a row, and the rays of a shading chunk (24,576 entries,
-// 48 x 8 pixels x 64 passes) leave from one small part of the scene, so both they and
-// the rays they continue as share nodes and primitives in L1.
+// passes instead of 32 pixels of a row, and the rays of a shading chunk (6,144 entries of
+// 768 threads: 12 x 8 pixels x 64 passes) leave from one small part of the scene, so both
+// they and the rays they continue as share nodes and primitives in L1.
 // Which entry a path has changes no result.
 //
 //   quads   runs of ORDER_QUAD pixels of the pixel order, all passes of a quad together,

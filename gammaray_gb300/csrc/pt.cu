@@ -54,8 +54,11 @@ static_assert(SHADE_BIG == 128 || SHADE_BIG == 384 || SHADE_BIG == 768, "shading
 // Long queues: 28 warps instead of 24 hide more of their latency than the spills at 71
 // registers cost (1024 x 1024 x 64 spp of 102,400 triangles 6.74 -> 6.50 ms of shading), but
 // a turn of the block through its queue takes about 1/8 longer, so only where it needs that
-// many fewer turns (641 x 359 x 9 spp, 18 and 16 turns: 1,373 and 1,391 us) and the queue is
-// more than one chunk (Cornell box, 1 M paths, up to 9 turns: 1,092 and 1,097).
+// many fewer turns and the queue is more than one chunk.  This rule against 896 threads for
+// every long queue, three runs each of 10 sizes (0.3 to 12.6 M paths), 3 scenes and 2 depths:
+// 0.966 to 1.028 of the time, 1.002 on average (runs of one side differ by up to 2%, twice by
+// 3.6%).  It gains most on 640 x 480 x 1 and 641 x 359 x 9 spp of 3,000 triangles (519 and
+// 537 us, 1,098 and 1,119) and loses on 256 x 256 x 8 of the Cornell box (623 and 610).
 constexpr int SHADE_WIDE = 896;
 inline bool shade_wide(uint64_t n, uint32_t sms) {
     auto turns = [&](uint64_t nt) { return (n + nt * sms - 1) / (nt * sms); };

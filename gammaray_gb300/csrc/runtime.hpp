@@ -75,7 +75,7 @@ struct DevBuf {
     }
 };
 
-// Path-tracer wavefront state, reused across renders of a scene (grown on demand).
+// Path-tracer wavefront state, reused across the renders of a device (grown on demand).
 struct PathState {
     DevBuf light, st;  // per slot: final radiance, film (s, t)
     // Ping-pong queues of live paths: slot, ray, and state (throughput, radiance so far,
@@ -96,11 +96,10 @@ struct BdptState {
     static size_t bytes_per_path(uint32_t max_len);  // device bytes ensure() needs per path
 };
 
-// The large wavefront buffers are shared by every scene on a device (renders on one
-// GPU run one after another anyway); a scene keeps only its small counter block.
 // The host's view of the queue lengths: what the last four bounces' starts saw, written to
-// pinned memory by k_bounce_begin, and an event after each.  Made once per device and kept (freeing pinned
-// memory synchronises the device), so a render starts without host allocations.
+// pinned memory by k_bounce_begin, and an event after each.  Made once per device and kept
+// (freeing pinned memory synchronises the device), so a render starts without host
+// allocations.
 struct BounceReadback {
     uint32_t* host = nullptr;
     cudaEvent_t ev[4] = {};
@@ -150,6 +149,9 @@ struct ScratchPool {
     }
 };
 
+// The large wavefront buffers are shared by every scene on a device (renders on one
+// GPU run one after another anyway); a scene keeps its small counter block and the buffers
+// of its ray queries.
 struct DeviceWork {
     std::mutex mu;
     ScratchPool scratch;

@@ -799,11 +799,15 @@ static bool build_lobes(const gr_material_desc& d, DevMaterial& m, std::string& 
 }
 
 // See build_scene: fewest components and most prims of a scene whose records the device makes.
+// Creation with the linear build, records made on the host and on the device (us): 700
+// triangles 403 / 397, 1,400 469 / 429, 2,100 507 / 441, 4,100 569 / 467, 20,000 1,041 / 639,
+// 200,000 2,322 / 798.  The prims bound the copies, four a prim, and are no crossing: 4,100
+// triangles in 64 meshes 988 / 907, 200,000 in 64 3,934 / 1,431 and in 256 5,254 / 2,787.
 static constexpr size_t DEVICE_RECORDS_MIN = 2048;
 static constexpr uint32_t DEVICE_RECORDS_PRIMS = 64;
 // Fewest components of a scene whose SAH tree the device builds (sah_build.cuh).  Scene
-// creation with the host's tree and with the device's (us): 3,000 triangles 1,048 / 970,
-// 8,000 1,709 / 1,229, 20,000 2,955 / 1,354, 102,400 6,859 / 1,649.
+// creation with the host's tree and with the device's (us): 1,400 triangles 646 / 784, 2,100
+// 797 / 854, 3,000 995 / 900, 4,100 1,270 / 934, 20,000 2,763 / 1,073, 200,000 11,596 / 1,797.
 static constexpr size_t DEVICE_SAH_MIN = 4096;
 
 bool build_material(const gr_material_desc& d, DevMaterial& m, std::string& err) {
@@ -886,8 +890,9 @@ bool build_scene(const gr_scene_desc& desc, HostBuild& out, std::string& err, bo
     }
     // The device makes the records of large scenes of few prims (a few copies per prim)
     // whose meshes have no more vertices than their triangles can name (so that a small
-    // mesh cut from a large vertex array uploads only its records): 400,000 triangles took 1.5 to 2.5 ms on 16 host threads and 0.4 ms to upload, against
-    // 0.1 ms of index and vertex uploads and 20 us there.
+    // mesh cut from a large vertex array uploads only its records): 400,000 triangles took
+    // 1.5 to 2.5 ms on 16 host threads and 0.4 ms to upload, against 0.1 ms of index and
+    // vertex uploads and 20 us there.
     out.device_sah = desc.build == GR_BUILD_HOST_SAH;
     out.device_records = device_records && total >= (out.device_sah ? DEVICE_SAH_MIN : DEVICE_RECORDS_MIN) &&
                          desc.num_prims <= DEVICE_RECORDS_PRIMS && vertices <= 3 * total;
