@@ -118,7 +118,8 @@ struct BounceReadback {
 // creation).  It keeps up to KEEP bytes of what was freed for the next scene, and gives them
 // back in gr_batch_release.  Creation with nothing kept / 64 MB / 1 GB (ms): 5,000 triangles
 // 1.16 / 1.01 / 1.01, 102,400 1.67 / 1.45 / 1.45, 400,000 2.41 / 2.22 / 2.06, 1,000,000 4.03 /
-// 3.85 / 3.25 (350 bytes each); with cudaMalloc and cudaFree 1.00, 1.64, 2.26, 3.60.
+// 3.85 / 3.25 (350 bytes each); with cudaMalloc and cudaFree 1.00, 1.64, 2.26, 3.60.  (A
+// process's first allocation from any pool takes 2.1 ms more, once.)
 struct ScratchPool {
     static constexpr uint64_t KEEP = uint64_t(512) << 20;
     std::mutex mu;

@@ -166,8 +166,9 @@ typedef struct gr_scene_info {
 } gr_scene_info;
 
 /* Replaces Stage::new / Bvh::build (render/stage.rs:15-20, geom/bvh.rs:339-382):
- * copies the prims, runs the reference SAH build on the host and (GPU library)
- * uploads a wide BVH.  The descriptors may be freed when this returns. */
+ * copies the prims, builds the reference's SAH tree and (GPU library) keeps it as a wide
+ * BVH on the device (gr_scene_desc.build: large scenes' trees are built there).  It waits
+ * for its own device work only.  The descriptors may be freed when this returns. */
 gr_status gr_scene_create(const gr_scene_desc* desc, gr_scene** out);
 /* The handle is dead when this returns.  A scene that server requests still use
  * (gr_server_submit) is freed when the last of them lets go: at gr_server_take, or for a
@@ -200,6 +201,8 @@ typedef struct gr_film gr_film;
 /* Film::new(width, height) (render/film.rs:45-53): accum and weight start at zero. */
 gr_status gr_film_create(uint32_t width, uint32_t height, gr_film** out);
 gr_status gr_film_destroy(gr_film* film);
+/* Zeroes the film, its splats and its pass count, on the film's device whichever is
+ * current; renders and batches that start later add to the cleared film. */
 gr_status gr_film_clear(gr_film* film);
 /* Copies Film::pixels out: accum as 3 floats and weight as 1 float per pixel,
  * row-major, row 0 first (render/film.rs:26-36). */
@@ -319,6 +322,9 @@ typedef struct gr_render_stats {
 gr_status gr_scene_last_stats(const gr_scene* scene, gr_render_stats* out);
 
 /* ---------------------------------------------------------------- ray queries */
+
+/* The queries on host arrays keep their device buffers with the scene, up to 64 MB (about
+ * 1.5 million rays), until it is destroyed; a larger call allocates and frees its own. */
 
 /* Closest hit.  prim = -1 for a miss (Intersection::NoHit).  component is the
  * triangle index within the mesh (0 for spheres); u, v are the Moller-Trumbore
